@@ -209,6 +209,38 @@ def test_block_residual_loss_matches_oracle():
     assert np.all(grad.cpu().numpy()[3] == 0.0)
 
 
+@pytest.mark.parametrize("batch", [1, 7, 8, 9, 128, 129, 1024])
+def test_block_residual_loss_item_counts(batch):
+    """Item counts around the CTAs (8) and items in flight (128) of the loss kernel. FP32 stencils of
+    at most 13 terms: 1e-5; the loss and V summed in FP64; twice gives the same bits."""
+    import torch
+
+    rng = np.random.default_rng(batch)
+    x = rng.normal(size=(batch, 2, 10, 10, 10)).astype(np.float32)
+    x[:, 1] = rng.choice([1.0, 0.0, -1.0], p=[0.7, 0.2, 0.1], size=(batch, 10, 10, 10))
+    x[batch // 2 + 1:batch // 2 + 2, 0] = 0.0  # an item without residual
+    y = rng.normal(size=(batch, 512)).astype(np.float32)
+    some = np.unique(np.r_[0, batch // 2, batch - 1])  # the oracle's dense operators cost 2 MB an item
+    loss, grad = torch.zeros(1, device="cuda"), torch.full((batch, 512), 7.0, device="cuda")
+    fb.UNet.block_residual_loss(_t(y), _t(x), loss, grad)
+    again = torch.zeros_like(grad)
+    fb.UNet.block_residual_loss(_t(y), _t(x), torch.zeros(1, device="cuda"), again)
+    assert torch.equal(grad, again)
+    want = np.zeros((batch, 512))
+    total, valid = 0.0, 0
+    for b in range(batch):
+        if b in some or batch <= 129:
+            item_loss, item_grad = U.block_residual_loss(y[b:b + 1], x[b:b + 1])
+            want[b] = item_grad[0]
+            total += item_loss
+        valid += bool(np.any((x[b, 1] == 1.0)[1:9, 1:9, 1:9] & (x[b, 0, 1:9, 1:9, 1:9] != 0)))
+    got = grad.cpu().numpy() * max(valid, 1)
+    rows = some if batch > 129 else np.arange(batch)
+    assert _rel(got[rows], want[rows]) <= 1e-5
+    if batch <= 129:
+        assert float(loss) == pytest.approx(total / max(valid, 1), rel=1e-5)
+
+
 def _held_out(scene, n, steps=7):
     soa, mass = scenes.SCENES[scene](n)
     ctx = fb.LiquidContext(n, capacity=soa.shape[1])
