@@ -256,3 +256,38 @@ def test_empty_and_invalid_particles():
     with pytest.raises(fb.FluidityError) as e:
         ctx.upload(np.zeros((15, 65), np.float32))
     assert e.value.code == fb.RESOURCE_EXHAUSTED
+
+
+@pytest.mark.parametrize("count", [1, 31, 33, 1023, 1024, 1025, 5000])
+def test_topology_from_unordered_particles(count):
+    """Blocks marked by particles in no order, at counts around a warp and around the 1024
+    particles of a CTA, against the blocks (and their ring) found on the host; a particle that
+    has no block is reported with its index."""
+    import torch
+
+    n, rng = 64, np.random.default_rng(count)
+    soa = np.zeros((15, count), np.float32)
+    soa[0:3] = rng.uniform(1.0 / n, 1.0 - 1.0 / n, size=(3, count))
+    soa[0, ::2] *= 0.25  # uneven: some blocks with many particles
+    ctx = fb.LiquidContext(n, capacity=count)
+    dev = torch.from_numpy(soa).cuda()
+    p = fb.Particles()
+    p.x[:] = [dev[d].data_ptr() for d in range(3)]
+    p.v[:] = [dev[3 + d].data_ptr() for d in range(3)]
+    p.c[:] = [dev[6 + d].data_ptr() for d in range(9)]
+    p.mass, p.count = None, count
+    lib, rep = fb.library(), fb.Report()
+    assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(p), None, ctypes.byref(rep)) == fb.OK
+    blk = np.floor(soa[0:3] * np.float32(n)).astype(int) // 8
+    occ = np.zeros((10, 10, 10), bool)
+    for dz in range(3):
+        for dy in range(3):
+            for dx in range(3):
+                occ[blk[2] + dz, blk[1] + dy, blk[0] + dx] = True
+    z, y, x = np.nonzero(occ[1:9, 1:9, 1:9])
+    np.testing.assert_array_equal(ctx.active_blocks(), np.stack([x, y, z], 1))
+    for bad, code in ((np.nan, fb.OUT_OF_RANGE), (1.5, fb.FAILED_PRECONDITION)):
+        dev[1, count - 1] = bad
+        assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(p), None, ctypes.byref(rep)) == code
+        assert rep.first_bad_index == count - 1
+    ctx.close()
