@@ -224,3 +224,53 @@ def test_normalized_p2g_reports_face_validity():
         seen |= set(np.unique(got[have]).tolist())
     assert seen == {0, 1, 3}
     ctx.close()
+
+
+@pytest.mark.parametrize("counts", [(1,), (31, 1), (32, 33), (255, 256), (257, 700, 5)])
+@pytest.mark.parametrize("with_old", [True, False])
+def test_full_gather_block_counts(counts, with_old):
+    """The full gather with block populations around a warp and around the CTA's 256 particles, in
+    blocks of their own, against the FP64 restatement: 81-term FP32 sums, 1e-5 of each group's
+    largest value. What lies after the last record stays as it was."""
+    import ctypes
+
+    import torch
+
+    from helpers import box_for
+
+    n, rng = 40, np.random.default_rng(sum(counts))
+    x = np.concatenate([rng.uniform([[8.0 * (k + 1)], [8.0], [16.0]], [[8.0 * (k + 2)], [16.0], [24.0]], (3, c))
+                        for k, c in enumerate(counts)], 1) / n
+    count = x.shape[1]
+    soa = np.zeros((15, count), np.float32)
+    soa[0:3] = x
+    src, dst = torch.from_numpy(soa).cuda(), torch.zeros((15, count), device="cuda")
+
+    def parts(t):
+        p = fb.Particles()
+        p.x[:] = [t[d].data_ptr() for d in range(3)]
+        p.v[:] = [t[3 + d].data_ptr() for d in range(3)]
+        p.c[:] = [t[6 + d].data_ptr() for d in range(9)]
+        p.mass, p.count = None, count
+        return p
+
+    ctx = fb.LiquidContext(n, capacity=count)
+    lib, rep, a, b = fb.library(), fb.Report(), parts(src), parts(dst)
+    assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(a), None, ctypes.byref(rep)) == fb.OK
+    assert lib.fl_sort_particles_by_block(ctx.handle, ctypes.byref(a), ctypes.byref(b), None, ctypes.byref(rep)) == fb.OK
+    blocks = ctx.active_blocks()
+    new, old = ([rng.normal(size=len(blocks) * 512).astype(np.float32) for _ in range(3)] for _ in range(2))
+    dn, do = ([torch.from_numpy(u).cuda() for u in f] for f in (new, old))
+    out = torch.full((count + 2, 24), 7.0, device="cuda")
+    arr = lambda ts: (ctypes.c_void_p * 3)(*[t.data_ptr() for t in ts])  # noqa: E731
+    assert lib.fl_g2p(ctx.handle, ctypes.byref(b), arr(dn), arr(do) if with_old else (ctypes.c_void_p * 3)(), 0.0,
+                      out.data_ptr(), None, ctypes.byref(rep)) == fb.OK and rep.error == 0
+    dense = lambda f: [fb.sparse_faces_to_dense(blocks, f[k].astype(np.float64), (n, n, n), k) for k in range(3)]  # noqa: E731
+    want = oracle.g2p(box_for(n), dst[0:3].cpu().numpy().T.astype(np.float64), dense(new), dense(old) if with_old else None)
+    if not with_old:
+        want[:, 3:6] = want[:, 0:3]
+    got = out.cpu().numpy()
+    for lo, hi in ((0, 3), (3, 6), (6, 15), (15, 24)):
+        assert _rel(got[:count, lo:hi], want[:, lo:hi]) <= TOL, (lo, hi)
+    assert np.all(got[count:] == 7.0)
+    ctx.close()
