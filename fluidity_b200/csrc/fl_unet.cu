@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
@@ -39,48 +40,199 @@ constexpr int kT = 256;
 
 // ---------------------------------------------------------------- forward
 
-// out[b][co][cell] = act(bias[co] + sum_ci sum_tap w[co][ci][tap] in[b][ci][cell + tap]).
-// VALID: the input is already (S+2)^3; otherwise it is S^3, zero padded here.
-// One CTA per (batch item, chunk of output channels); the input item sits in
-// shared memory as [ci][(S+2)^3].
-template <int S, bool VALID>
-__global__ void __launch_bounds__(kT) k_conv3_fwd(const float* __restrict__ in, int cin, const float* __restrict__ w,
-                                                  const float* __restrict__ bias, int cout, int co_chunk,
-                                                  float* __restrict__ out, int relu) {
-  constexpr int P = S + 2, P3 = P * P * P, S3 = S * S * S;
-  extern __shared__ float tile[];
-  const int b = blockIdx.x;
-  const int co0 = blockIdx.y * co_chunk;
-  if (VALID) {
-    const float* src = in + (size_t)b * cin * P3;
-    for (int i = threadIdx.x; i < cin * P3; i += kT) tile[i] = src[i];
+// The FP32 3x3x3 convolutions, forward and data gradient. Both are
+//   out[b][o][cell] = f(sum_i sum_tap W[o][i][tap] in[b][i][cell + tap - 1]),
+// the data gradient with i over the layer's output channels and
+// W[o][i][tap] = w[i][o][26 - tap]. Bound by the FP32 pipe once the loads are
+// amortised: a thread owns four x-adjacent cells and kCo output channels, so
+// one input row (a 16- and an 8-byte shared load) serves 3 taps x 4 cells x
+// kCo channels in packed FMAs (channel pairs). At 45 items a 4^3 layer
+// of 32 to 32 channels takes 23 us (26 us its data gradient) and an 8^3 layer of
+// 16 to 16 24 us (23 us); one thread per output, with an input and a weight load
+// per FMA, took 160 (127) and 152 (130) us. Staging is most of what is left.
+// One CTA of 128 threads per item, slab of kZ output planes and 16 output
+// channels; the slab's zero-padded input (rows padded to a multiple of four
+// words, planes so that the eight lanes of a 16-byte access touch all banks)
+// and the 16 channels' weights ([input channel][tap][channel]) are staged in
+// shared memory. Sums run over input channels, then taps in ascending order.
+template <int S>
+struct ConvTile {
+  static constexpr int kZ = S == 8 ? 2 : 4;   // output planes per CTA
+  static constexpr int kCo = S == 8 ? 4 : 2;  // output channels per thread
+  static constexpr int kRow = S == 8 ? 12 : 8;
+  static constexpr int kPlane = S == 8 ? 10 * 12 : 6 * 8 + 4;
+  static constexpr int kChannel = (kZ + 2) * kPlane;
+  static constexpr size_t smem(int cin) { return sizeof(float) * cin * (kChannel + 27 * kConvW); }
+  static constexpr int kConvW = 20;  // words per (channel, tap): 16 weights, padded against store conflicts
+};
+
+template <int S, bool VALID, bool DATA>
+__global__ void __launch_bounds__(128) k_conv3(const float* __restrict__ in, int cin, const float* __restrict__ w,
+                                               const float* __restrict__ bias, int cout, float* __restrict__ out,
+                                               int relu, const float* __restrict__ act) {
+  using T = ConvTile<S>;
+  constexpr int E = S + 2, S3 = S * S * S, EIN = VALID ? E : S, EIN3 = EIN * EIN * EIN, OFF = VALID ? 0 : 1;
+  constexpr int kSlabs = S / T::kZ, kCells = (T::kZ + 2) * E * E;
+  extern __shared__ __align__(16) float conv_smem[];
+  float* tile = conv_smem;
+  float* wt = tile + cin * T::kChannel;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int b = blockIdx.x / kSlabs, z0 = (blockIdx.x % kSlabs) * T::kZ, co0 = blockIdx.y * 16;
+  const float* src = in + (size_t)b * cin * EIN3;
+  for (int i = t; i < cin * kCells; i += 128) {
+    const int ci = i / kCells, r = i % kCells;
+    const int pz = r / (E * E), py = (r / E) % E, px = r % E;
+    const int z = z0 + pz - OFF, y = py - OFF, x = px - OFF;
+    float v = 0.0f;
+    if (VALID || (z >= 0 && z < S && y >= 0 && y < S && x >= 0 && x < S)) v = src[ci * EIN3 + (z * EIN + y) * EIN + x];
+    tile[ci * T::kChannel + pz * T::kPlane + py * T::kRow + px] = v;
+  }
+  if (DATA) {  // in channel i = a layer output, the 16 layer inputs co0 .. co0 + 15 contiguous in w[i]
+    for (int e = t; e < cin * 16 * 27; e += 128) {
+      const int i = e / (16 * 27), r = e % (16 * 27), o = r / 27, tap = r % 27;
+      wt[(i * 27 + 26 - tap) * T::kConvW + o] = w[((size_t)i * cout + co0 + o) * 27 + tap];
+    }
   } else {
-    const float* src = in + (size_t)b * cin * S3;
-    for (int i = threadIdx.x; i < cin * P3; i += kT) {
-      const int ci = i / P3, r = i - ci * P3;
-      const int pz = r / (P * P), py = (r / P) % P, px = r % P;
-      const bool inside = pz >= 1 && pz <= S && py >= 1 && py <= S && px >= 1 && px <= S;
-      tile[i] = inside ? src[ci * S3 + ((pz - 1) * S + (py - 1)) * S + (px - 1)] : 0.0f;
+    for (int e = t; e < 16 * cin * 27; e += 128) {
+      const int o = e / (cin * 27), r = e % (cin * 27);
+      wt[r * T::kConvW + o] = w[(size_t)(co0 + o) * cin * 27 + r];
     }
   }
   __syncthreads();
-  const int n_out = min(co_chunk, cout - co0) * S3;
-  for (int idx = threadIdx.x; idx < n_out; idx += kT) {
-    const int co = co0 + idx / S3, cell = idx % S3;
-    const int z = cell / (S * S), y = (cell / S) % S, x = cell % S;
-    float acc = bias[co];
-    const float* wc = w + (size_t)co * cin * 27;
-    for (int ci = 0; ci < cin; ++ci) {
-      const float* t = tile + ci * P3 + (z * P + y) * P + x;
-      const float* wk = wc + ci * 27;
+  // S = 8: lanes (y, x half, z), warp = channel quad; S = 4: lanes (y, z, channel pair of the warp's quad)
+  const int y = S == 8 ? lane & 7 : lane & 3, z = S == 8 ? lane >> 4 : (lane >> 2) & 3;
+  const int x0 = S == 8 ? 4 * ((lane >> 3) & 1) : 0;
+  const int co = 4 * warp + (S == 8 ? 0 : 2 * (lane >> 4));
+  float2 acc[4][T::kCo / 2];
 #pragma unroll
-      for (int dz = 0; dz < 3; ++dz)
+  for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int dy = 0; dy < 3; ++dy)
+    for (int h = 0; h < T::kCo / 2; ++h)
+      acc[c][h] = DATA ? make_float2(0.0f, 0.0f)
+                       : make_float2(__ldg(&bias[co0 + co + 2 * h]), __ldg(&bias[co0 + co + 2 * h + 1]));
+  for (int ci = 0; ci < cin; ++ci) {
+    const float* base = tile + ci * T::kChannel + z * T::kPlane + y * T::kRow + x0;
+    const float* wc = wt + ci * 27 * T::kConvW + co;
 #pragma unroll
-          for (int dx = 0; dx < 3; ++dx) acc = fmaf(__ldg(&wk[(dz * 3 + dy) * 3 + dx]), t[(dz * P + dy) * P + dx], acc);
+    for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+      for (int dy = 0; dy < 3; ++dy) {
+        const float4 a = *reinterpret_cast<const float4*>(base + dz * T::kPlane + dy * T::kRow);
+        const float2 e = *reinterpret_cast<const float2*>(base + dz * T::kPlane + dy * T::kRow + 4);
+        const float v[6] = {a.x, a.y, a.z, a.w, e.x, e.y};
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx) {
+          const float* wp = wc + ((dz * 3 + dy) * 3 + dx) * T::kConvW;
+          float2 wv[T::kCo / 2];
+          if constexpr (T::kCo == 4) {
+            const float4 q = *reinterpret_cast<const float4*>(wp);
+            wv[0] = make_float2(q.x, q.y);
+            wv[1] = make_float2(q.z, q.w);
+          } else {
+            wv[0] = *reinterpret_cast<const float2*>(wp);
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int h = 0; h < T::kCo / 2; ++h)
+              acc[c][h] = __ffma2_rn(make_float2(v[c + dx], v[c + dx]), wv[h], acc[c][h]);
+        }
+      }
+  }
+#pragma unroll
+  for (int k = 0; k < T::kCo; ++k) {
+    const size_t o = ((size_t)b * cout + co0 + co + k) * S3 + ((z0 + z) * S + y) * S + x0;
+    float r[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) r[c] = (k & 1) ? acc[c][k >> 1].y : acc[c][k >> 1].x;
+    if (DATA && act != nullptr) {
+      const float4 m = *reinterpret_cast<const float4*>(act + o);
+      r[0] = m.x > 0.0f ? r[0] : 0.0f;
+      r[1] = m.y > 0.0f ? r[1] : 0.0f;
+      r[2] = m.z > 0.0f ? r[2] : 0.0f;
+      r[3] = m.w > 0.0f ? r[3] : 0.0f;
+    } else if (!DATA && relu) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) r[c] = fmaxf(r[c], 0.0f);
     }
-    out[((size_t)b * cout + co) * S3 + cell] = relu ? fmaxf(acc, 0.0f) : acc;
+    *reinterpret_cast<float4*>(out + o) = make_float4(r[0], r[1], r[2], r[3]);
+  }
+}
+
+// The 2^3 layer: an output cell sees all eight input cells, each through one
+// tap, so only 8 of its 27 taps are formed. Lanes hold 32 items, a warp one
+// (z, y) row of two cells and four output channels: the weights of a tap are
+// then one broadcast 16-byte load for the warp. One CTA of 8 warps per 32 items
+// and 8 output channels.
+constexpr int kConv2Items = 33;  // words per (channel, cell): 32 items, padded
+constexpr int kConv2W = 12;      // words per (channel, tap): 8 weights, padded
+constexpr size_t conv2_smem(int cin) { return sizeof(float) * cin * (8 * kConv2Items + 27 * kConv2W); }
+
+template <bool DATA>
+__global__ void __launch_bounds__(256) k_conv3_2(const float* __restrict__ in, int cin, const float* __restrict__ w,
+                                                 const float* __restrict__ bias, int cout, int batch,
+                                                 float* __restrict__ out, int relu, const float* __restrict__ act) {
+  extern __shared__ __align__(16) float conv_smem[];
+  float* wt = conv_smem;
+  float* tile = wt + cin * 27 * kConv2W;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int b0 = blockIdx.x * 32, co0 = blockIdx.y * 8;
+  const int items = min(32, batch - b0);
+  for (int e = t; e < 32 * cin * 8; e += 256) {
+    const int b = e / (cin * 8), r = e % (cin * 8);
+    tile[r * kConv2Items + b] = b < items ? in[(size_t)(b0 + b) * cin * 8 + r] : 0.0f;
+  }
+  for (int e = t; e < cin * 8 * 27; e += 256) {
+    if (DATA) {
+      const int i = e / (8 * 27), r = e % (8 * 27), o = r / 27, tap = r % 27;
+      wt[(i * 27 + 26 - tap) * kConv2W + o] = w[((size_t)i * cout + co0 + o) * 27 + tap];
+    } else {
+      const int o = e / (cin * 27), r = e % (cin * 27);
+      wt[r * kConv2W + o] = w[(size_t)(co0 + o) * cin * 27 + r];
+    }
+  }
+  __syncthreads();
+  const int z = (warp >> 1) & 1, y = warp & 1, co = 4 * (warp >> 2);
+  float2 acc[2][2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      acc[c][h] = DATA ? make_float2(0.0f, 0.0f)
+                       : make_float2(__ldg(&bias[co0 + co + 2 * h]), __ldg(&bias[co0 + co + 2 * h + 1]));
+  for (int ci = 0; ci < cin; ++ci) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {  // input row (z', y'): taps z' - z + 1 and y' - y + 1
+      const int tap = ((r >> 1) - z + 1) * 9 + ((r & 1) - y + 1) * 3;
+      const float* v = tile + (ci * 8 + 2 * r) * kConv2Items + lane;
+      const float2 v0 = make_float2(v[0], v[0]), v1 = make_float2(v[kConv2Items], v[kConv2Items]);
+      const float* wp = wt + (ci * 27 + tap) * kConv2W + co;
+      float2 wv[3][2];
+#pragma unroll
+      for (int dx = 0; dx < 3; ++dx) {
+        const float4 q = *reinterpret_cast<const float4*>(wp + dx * kConv2W);
+        wv[dx][0] = make_float2(q.x, q.y);
+        wv[dx][1] = make_float2(q.z, q.w);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        acc[0][h] = __ffma2_rn(v1, wv[2][h], __ffma2_rn(v0, wv[1][h], acc[0][h]));
+        acc[1][h] = __ffma2_rn(v1, wv[1][h], __ffma2_rn(v0, wv[0][h], acc[1][h]));
+      }
+    }
+  }
+  if (lane >= items) return;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const size_t o = ((size_t)(b0 + lane) * cout + co0 + co + k) * 8 + z * 4 + y * 2;
+    float r[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      r[c] = (k & 1) ? acc[c][k >> 1].y : acc[c][k >> 1].x;
+      if (DATA && act != nullptr && !(act[o + c] > 0.0f)) r[c] = 0.0f;
+      if (!DATA && relu) r[c] = fmaxf(r[c], 0.0f);
+    }
+    *reinterpret_cast<float2*>(out + o) = make_float2(r[0], r[1]);
   }
 }
 
@@ -128,122 +280,130 @@ __global__ void k_up_add_relu(const float* __restrict__ coarse, const float* __r
 
 // ---------------------------------------------------------------- backward
 
-// din[b][ci][i] = (sum_co sum_tap w[co][ci][tap] g[b][co][i - tap + 1]) * (act[b][ci][i] > 0 if act).
-// The gradient item sits in shared memory zero padded as [co][(S+2)^3].
-template <int S>
-__global__ void __launch_bounds__(kT) k_conv3_bwd_data(const float* __restrict__ g, int cout,
-                                                       const float* __restrict__ w, int cin, int ci_chunk,
-                                                       const float* __restrict__ act, float* __restrict__ din) {
-  constexpr int P = S + 2, P3 = P * P * P, S3 = S * S * S;
-  extern __shared__ float tile[];
-  const int b = blockIdx.x;
-  const int ci0 = blockIdx.y * ci_chunk;
-  const float* src = g + (size_t)b * cout * S3;
-  for (int i = threadIdx.x; i < cout * P3; i += kT) {
-    const int co = i / P3, r = i - co * P3;
-    const int pz = r / (P * P), py = (r / P) % P, px = r % P;
-    const bool inside = pz >= 1 && pz <= S && py >= 1 && py <= S && px >= 1 && px <= S;
-    tile[i] = inside ? src[co * S3 + ((pz - 1) * S + (py - 1)) * S + (px - 1)] : 0.0f;
-  }
-  __syncthreads();
-  const int n_out = min(ci_chunk, cin - ci0) * S3;
-  for (int idx = threadIdx.x; idx < n_out; idx += kT) {
-    const int ci = ci0 + idx / S3, cell = idx % S3;
-    const size_t o = ((size_t)b * cin + ci) * S3 + cell;
-    if (act != nullptr && !(act[o] > 0.0f)) {
-      din[o] = 0.0f;
-      continue;
-    }
-    const int z = cell / (S * S), y = (cell / S) % S, x = cell % S;
-    float acc = 0.0f;
-    for (int co = 0; co < cout; ++co) {
-      const float* t = tile + co * P3 + ((z + 2) * P + (y + 2)) * P + (x + 2);
-      const float* wk = w + ((size_t)co * cin + ci) * 27;
-#pragma unroll
-      for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-        for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-          for (int dx = 0; dx < 3; ++dx)
-            acc = fmaf(__ldg(&wk[(dz * 3 + dy) * 3 + dx]), t[-((dz * P + dy) * P + dx)], acc);
-    }
-    din[o] = acc;
-  }
-}
+// Weight and bias gradient of a 3x3x3 layer:
+//   dw[co][ci][tap] = sum_b sum_o g[b][co][o] in[b][ci][o + tap - pad], db[co] = sum_b sum_o g[b][co][o].
+// A thread owns one input channel, one (dz, dy) and eight output channels: per
+// cell one input value (three kept for the dx taps) and two broadcast 16-byte
+// loads of g (staged [cell][channel]) feed 12 packed FMAs. An 8^3
+// layer of 16 to 16 channels takes 33 us at 45 items; a CTA per channel pair
+// reading both operands from global memory took 102 us.
+// Work units (an item's slab of two planes at 8^3, an item at 4^3, four items
+// at 2^3) are dealt to gridDim.x CTAs in order and each CTA writes one partial
+// row; k_wgrad_sum adds the rows in order, so the result is reproducible.
+// With two input channels (the first layer) kSplit threads share a role, each
+// taking every kSplit-th row of cells into a partial row of its own.
+template <int S, bool VALID, int CIN>
+struct WgradTile {
+  static constexpr int kSplit = CIN == 2 ? 8 : 1;
+  static constexpr int kThreads = CIN * 18 * kSplit;  // channels x 9 x 2 octets of output channels
+  static constexpr int kZ = S == 8 ? 2 : S;
+  static constexpr int kItems = S == 2 ? 4 : 1;
+  static constexpr int kSlabs = S / kZ;
+  static constexpr int kCh = CIN + 1;                                 // words per cell: odd or whole-warp reads
+  static constexpr int kRow = (S + 2) * kCh + (CIN == 16 && S == 8 ? 6 : 0);  // 16 mod 32: half-warps on two rows
+  static constexpr int kPlane = (S + 2) * kRow + (CIN == 16 && S == 8 ? 16 : 0);
+  static constexpr int kItem = (kZ + 2) * kPlane;
+  static constexpr int kG = 20;  // words per cell of g: 16 channels, padded
+  static constexpr size_t kSmem = sizeof(float) * (kItems * (kItem + kZ * S * S * kG) + 4);
+};
+constexpr long long kWgradPart = 1 << 21;  // floats of the partial rows
 
-// 27 partial sums -> shared result in fixed order (warp shuffles, then warps in order).
-__device__ __forceinline__ void block_sum27(float (&acc)[27], float* red /* 27 * (kT/32) */, float* out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+template <int S, bool VALID, int CIN>
+__global__ void __launch_bounds__(WgradTile<S, VALID, CIN>::kThreads)
+    k_conv3_wgrad(const float* __restrict__ in, const float* __restrict__ g, int cout, int batch, int units,
+                  float* __restrict__ part) {
+  using T = WgradTile<S, VALID, CIN>;
+  constexpr int E = S + 2, S3 = S * S * S, EIN = VALID ? E : S, EIN3 = EIN * EIN * EIN, OFF = VALID ? 0 : 1;
+  constexpr int kInCells = (T::kZ + 2) * E * E, kOutCells = T::kZ * S * S;
+  extern __shared__ __align__(16) float wg_smem[];
+  float* gt = wg_smem;                                // [item][cell][16, padded]
+  float* it = gt + T::kItems * kOutCells * T::kG;     // [item][z][y][x][channel]
+  const int t = threadIdx.x, co0 = blockIdx.y * 16;
+  const int ci = t % CIN, rest = t / CIN, dzy = rest % 9, oct = (rest / 9) & 1, split = rest / 18;
+  const int dz = dzy / 3, dy = dzy % 3;
+  float2 acc[3][4], bsum[4];
 #pragma unroll
-  for (int t = 0; t < 27; ++t) {
-    float v = acc[t];
+  for (int h = 0; h < 4; ++h) {
+    bsum[h] = make_float2(0.0f, 0.0f);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[t * (kT / 32) + warp] = v;
+    for (int dx = 0; dx < 3; ++dx) acc[dx][h] = make_float2(0.0f, 0.0f);
   }
-  __syncthreads();
-  if (threadIdx.x < 27) {
-    float s = 0.0f;
-    for (int k = 0; k < kT / 32; ++k) s += red[threadIdx.x * (kT / 32) + k];
-    out[threadIdx.x] = s;
-  }
-}
-
-// dw[co][ci][tap] = sum_b sum_o g[b][co][o] in[b][ci][o + tap - pad]; db[co] = sum_b sum_o g[b][co][o]
-// (written by the ci == 0 CTA). One CTA per (ci, co). VALID: input extent S+2, pad 0.
-template <int S, bool VALID>
-__global__ void __launch_bounds__(kT) k_conv3_bwd_weight(const float* __restrict__ in, int cin,
-                                                         const float* __restrict__ g, int cout, int batch,
-                                                         float* __restrict__ dw, float* __restrict__ db) {
-  constexpr int S3 = S * S * S;
-  constexpr int E = VALID ? S + 2 : S;  // input extent
-  constexpr int E3 = E * E * E;
-  __shared__ float red[27 * (kT / 32)];
-  __shared__ float res[27];
-  __shared__ float bred[kT / 32];
-  const int ci = blockIdx.x, co = blockIdx.y;
-  float acc[27];
-#pragma unroll
-  for (int t = 0; t < 27; ++t) acc[t] = 0.0f;
-  float bsum = 0.0f;
-  const int total = batch * S3;
-  for (int idx = threadIdx.x; idx < total; idx += kT) {
-    const int b = idx / S3, o = idx % S3;
-    const float gv = g[((size_t)b * cout + co) * S3 + o];
-    bsum += gv;
-    const int z = o / (S * S), y = (o / S) % S, x = o % S;
-    const float* src = in + ((size_t)b * cin + ci) * E3;
-#pragma unroll
-    for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-      for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-        for (int dx = 0; dx < 3; ++dx) {
-          int zz = z + dz, yy = y + dy, xx = x + dx;
-          if (!VALID) {
-            zz -= 1;
-            yy -= 1;
-            xx -= 1;
-          }
-          float v = 0.0f;
-          if (VALID || (zz >= 0 && zz < S && yy >= 0 && yy < S && xx >= 0 && xx < S)) v = src[(zz * E + yy) * E + xx];
-          acc[(dz * 3 + dy) * 3 + dx] = fmaf(gv, v, acc[(dz * 3 + dy) * 3 + dx]);
-        }
-  }
-  block_sum27(acc, red, res);
-  __syncthreads();
-  if (threadIdx.x < 27) dw[((size_t)co * cin + ci) * 27 + threadIdx.x] = res[threadIdx.x];
-  if (ci == 0) {
-    float v = bsum;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) bred[threadIdx.x >> 5] = v;
+  for (int u = blockIdx.x; u < units; u += gridDim.x) {
+    const int b0 = u / T::kSlabs * T::kItems, z0 = (u % T::kSlabs) * T::kZ;
+    __syncthreads();  // the previous unit's reads
+    for (int i = t; i < T::kItems * CIN * kInCells; i += T::kThreads) {
+      const int k = i / (CIN * kInCells), r = i % (CIN * kInCells), c = r / kInCells, cell = r % kInCells;
+      const int pz = cell / (E * E), py = (cell / E) % E, px = cell % E;
+      const int z = z0 + pz - OFF, y = py - OFF, x = px - OFF;
+      float v = 0.0f;
+      if (b0 + k < batch && (VALID || (z >= 0 && z < S && y >= 0 && y < S && x >= 0 && x < S)))
+        v = in[((size_t)(b0 + k) * CIN + c) * EIN3 + (z * EIN + y) * EIN + x];
+      it[k * T::kItem + pz * T::kPlane + py * T::kRow + px * T::kCh + c] = v;
+    }
+    for (int i = t; i < T::kItems * 16 * kOutCells; i += T::kThreads) {
+      const int k = i / (16 * kOutCells), r = i % (16 * kOutCells), o = r / kOutCells, cell = r % kOutCells;
+      gt[(k * kOutCells + cell) * T::kG + o] =
+          b0 + k < batch ? g[((size_t)(b0 + k) * cout + co0 + o) * S3 + z0 * S * S + cell] : 0.0f;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      float s = 0.0f;
-      for (int k = 0; k < kT / 32; ++k) s += bred[k];
-      db[co] = s;
+    for (int row = split; row < T::kItems * T::kZ * S; row += T::kSplit) {
+      const int k = row / (T::kZ * S), z = (row / S) % T::kZ, y = row % S;
+      const float* v = it + k * T::kItem + (z + dz) * T::kPlane + (y + dy) * T::kRow + ci;
+      const float* gp = gt + (size_t)row * S * T::kG + 8 * oct;
+      float v0 = v[0], v1 = v[T::kCh];
+#pragma unroll
+      for (int x = 0; x < S; ++x) {
+        const float v2 = v[(x + 2) * T::kCh];
+        const float4 ga = *reinterpret_cast<const float4*>(gp + x * T::kG);
+        const float4 gb = *reinterpret_cast<const float4*>(gp + x * T::kG + 4);
+        const float2 gv[4] = {make_float2(ga.x, ga.y), make_float2(ga.z, ga.w), make_float2(gb.x, gb.y),
+                              make_float2(gb.z, gb.w)};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          acc[0][h] = __ffma2_rn(make_float2(v0, v0), gv[h], acc[0][h]);
+          acc[1][h] = __ffma2_rn(make_float2(v1, v1), gv[h], acc[1][h]);
+          acc[2][h] = __ffma2_rn(make_float2(v2, v2), gv[h], acc[2][h]);
+          if (dzy == 0) bsum[h] = __fadd2_rn(bsum[h], gv[h]);
+        }
+        v0 = v1;
+        v1 = v2;
+      }
     }
+  }
+  const int nw = cout * CIN * 27;
+  float* row = part + ((size_t)blockIdx.x * T::kSplit + split) * (nw + cout);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int o = co0 + 8 * oct + k;
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx)
+      row[((size_t)o * CIN + ci) * 27 + dzy * 3 + dx] = (k & 1) ? acc[dx][k >> 1].y : acc[dx][k >> 1].x;
+    if (dzy == 0 && ci == 0) row[nw + o] = (k & 1) ? bsum[k >> 1].y : bsum[k >> 1].x;
+  }
+}
+
+// dw, db = the partial rows added in order: 32 values per CTA, eight warps taking
+// every eighth row, then the eight sums in order.
+__global__ void __launch_bounds__(kT) k_wgrad_sum(const float* __restrict__ part, int rows, int nw, int cout,
+                                                  float* __restrict__ dw, float* __restrict__ db) {
+  __shared__ float red[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e = blockIdx.x * 32 + lane, n = nw + cout;
+  float s = 0.0f;
+  if (e < n) {
+#pragma unroll 8
+    for (int r = warp; r < rows; r += 8) s += part[(size_t)r * n + e];
+  }
+  red[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && e < n) {
+    float v = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v += red[k][lane];
+    if (e < nw)
+      dw[e] = v;
+    else
+      db[e - nw] = v;
   }
 }
 
@@ -567,29 +727,52 @@ unsigned grid_for(long long n) {
 template <int S, bool VALID>
 void conv3_fwd(const float* in, int cin, const float* w, const float* bias, int cout, float* out, int batch, int relu,
                cudaStream_t s) {
-  constexpr int P3 = (S + 2) * (S + 2) * (S + 2);
-  const int chunk = S == 8 ? 8 : cout;
-  const size_t smem = sizeof(float) * cin * P3;
   ++g_kernel_launches;
-  k_conv3_fwd<S, VALID><<<dim3(batch, (cout + chunk - 1) / chunk), kT, smem, s>>>(in, cin, w, bias, cout, chunk, out,
-                                                                                  relu);
+  if constexpr (S == 2)
+    k_conv3_2<false><<<dim3((batch + 31) / 32, cout / 8), 256, conv2_smem(cin), s>>>(in, cin, w, bias, cout, batch, out,
+                                                                                     relu, nullptr);
+  else
+    k_conv3<S, VALID, false><<<dim3(batch * (S / ConvTile<S>::kZ), cout / 16), 128, ConvTile<S>::smem(cin), s>>>(
+        in, cin, w, bias, cout, out, relu, nullptr);
 }
 
+// g has the layer's cout channels, din its cin: the roles of k_conv3's cin and cout.
 template <int S>
 void conv3_bwd_data(const float* g, int cout, const float* w, int cin, const float* act, float* din, int batch,
                     cudaStream_t s) {
-  constexpr int P3 = (S + 2) * (S + 2) * (S + 2);
-  const int chunk = S == 8 ? 8 : cin;
-  const size_t smem = sizeof(float) * cout * P3;
   ++g_kernel_launches;
-  k_conv3_bwd_data<S><<<dim3(batch, (cin + chunk - 1) / chunk), kT, smem, s>>>(g, cout, w, cin, chunk, act, din);
+  if constexpr (S == 2)
+    k_conv3_2<true><<<dim3((batch + 31) / 32, cin / 8), 256, conv2_smem(cout), s>>>(g, cout, w, nullptr, cin, batch,
+                                                                                    din, 0, act);
+  else
+    k_conv3<S, false, true><<<dim3(batch * (S / ConvTile<S>::kZ), cin / 16), 128, ConvTile<S>::smem(cout), s>>>(
+        g, cout, w, nullptr, cin, din, 0, act);
 }
 
+template <int S, bool VALID, int CIN>
+void wgrad(const float* in, const float* g, int cout, int batch, float* part, float* dw, float* db, cudaStream_t s) {
+  using T = WgradTile<S, VALID, CIN>;
+  const int nw = cout * CIN * 27;
+  const int units = (batch + T::kItems - 1) / T::kItems * T::kSlabs;
+  // one CTA per SM where the units and the partial rows' space allow it
+  const int ctas = (int)std::min<long long>({(long long)units, 148, kWgradPart / ((long long)T::kSplit * (nw + cout))});
+  g_kernel_launches += 2;
+  k_conv3_wgrad<S, VALID, CIN><<<dim3(ctas, cout / 16), T::kThreads, T::kSmem, s>>>(in, g, cout, batch, units, part);
+  k_wgrad_sum<<<(nw + cout + 31) / 32, kT, 0, s>>>(part, ctas * T::kSplit, nw, cout, dw, db);
+}
+
+// The network's layers: 2 input channels (first layer) or 16 at 8^3, 16 or 32 at 4^3, 32 at 2^3.
 template <int S, bool VALID>
-void conv3_bwd_weight(const float* in, int cin, const float* g, int cout, int batch, float* dw, float* db,
+void conv3_bwd_weight(const float* in, int cin, const float* g, int cout, int batch, float* part, float* dw, float* db,
                       cudaStream_t s) {
-  ++g_kernel_launches;
-  k_conv3_bwd_weight<S, VALID><<<dim3(cin, cout), kT, 0, s>>>(in, cin, g, cout, batch, dw, db);
+  if constexpr (VALID)
+    wgrad<S, true, 2>(in, g, cout, batch, part, dw, db, s);
+  else if constexpr (S == 8)
+    wgrad<S, false, 16>(in, g, cout, batch, part, dw, db, s);
+  else if (S == 4 && cin == 16)
+    wgrad<S, false, 16>(in, g, cout, batch, part, dw, db, s);
+  else
+    wgrad<S, false, 32>(in, g, cout, batch, part, dw, db, s);
 }
 
 // A 3x3x3 layer on the SIMT kernels (tc == nullptr) or as a tensor-core GEMM;
@@ -608,8 +791,8 @@ void bwd3_data(UNetTcTrain* tc, cudaError_t& e, const float* g, int cout, const 
 }
 template <int S, bool VALID>
 void bwd3_weight(UNetTcTrain* tc, cudaError_t& e, const float* in, int cin, const float* g, int cout, int batch,
-                 float* dw, float* db, cudaStream_t s) {
-  if (tc == nullptr) return conv3_bwd_weight<S, VALID>(in, cin, g, cout, batch, dw, db, s);
+                 float* part, float* dw, float* db, cudaStream_t s) {
+  if (tc == nullptr) return conv3_bwd_weight<S, VALID>(in, cin, g, cout, batch, part, dw, db, s);
   if (e == cudaSuccess) e = conv3_bwd_weight_tc<S, VALID>(*tc, in, cin, g, cout, batch, dw, db, s);
 }
 
@@ -666,6 +849,9 @@ UNetCache unet_cache_layout(int batch) {
   C.g4c = take(32 * 64);
   C.g2a = take(64 * 8);
   C.g2b = take(64 * 8);
+  off = (off + 3) / 4 * 4;
+  C.part = off;  // partial rows of the weight gradients
+  off += kWgradPart;
   C.total = off;
   return C;
 }
@@ -673,10 +859,21 @@ UNetCache unet_cache_layout(int batch) {
 void configure_unet_kernels() {
   static bool done = false;
   if (done) return;
-  const int big = sizeof(float) * 32 * 1000;  // largest padded tile: 32 channels of 10^3
-  cudaFuncSetAttribute(k_conv3_fwd<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(k_conv3_fwd<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(k_conv3_bwd_data<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  auto allow = [](auto* kernel, size_t bytes) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  allow(k_conv3<8, true, false>, ConvTile<8>::smem(2));
+  allow(k_conv3<8, false, false>, ConvTile<8>::smem(16));
+  allow(k_conv3<8, false, true>, ConvTile<8>::smem(16));
+  allow(k_conv3<4, false, false>, ConvTile<4>::smem(32));
+  allow(k_conv3<4, false, true>, ConvTile<4>::smem(32));
+  allow(k_conv3_2<false>, conv2_smem(32));
+  allow(k_conv3_2<true>, conv2_smem(64));
+  allow(k_conv3_wgrad<8, true, 2>, WgradTile<8, true, 2>::kSmem);
+  allow(k_conv3_wgrad<8, false, 16>, WgradTile<8, false, 16>::kSmem);
+  allow(k_conv3_wgrad<4, false, 16>, WgradTile<4, false, 16>::kSmem);
+  allow(k_conv3_wgrad<4, false, 32>, WgradTile<4, false, 32>::kSmem);
+  allow(k_conv3_wgrad<2, false, 32>, WgradTile<2, false, 32>::kSmem);
   done = true;
 }
 
@@ -732,7 +929,7 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   k_conv1_bwd_weight<1024><<<dim3(16, 1), 1024, 0, s>>>(A + C.d1, 16, gy, 1, 512, batch, GW(9), GB(9));
   k_conv1_bwd_data<<<grid_for(B * 16 * 512), kT, 0, s>>>(gy, 1, W(9), 16, 512, B * 16 * 512, A + C.d1, A + C.g8a);
   // d1 (conv3 16->16 on u1); gu1 pre-activation -> g8b
-  bwd3_weight<8, false>(tc, tce, A + C.u1, 16, A + C.g8a, 16, batch, GW(8), GB(8), s);
+  bwd3_weight<8, false>(tc, tce, A + C.u1, 16, A + C.g8a, 16, batch, A + C.part, GW(8), GB(8), s);
   bwd3_data<8>(tc, tce, A + C.g8a, 16, W(8), 16, A + C.u1, A + C.g8b, batch, s);
   // u1 = relu(up(c1) + s1): c1 = conv1(d2, 32->16)
   g_kernel_launches += 3;
@@ -741,7 +938,7 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   k_conv1_bwd_data<<<grid_for(B * 32 * 64), kT, 0, s>>>(A + C.g4c, 16, W(7), 32, 64, B * 32 * 64, A + C.d2,
                                                         A + C.g4a);
   // d2 (conv3 32->32 on u2); gu2 pre-activation -> g4b
-  bwd3_weight<4, false>(tc, tce, A + C.u2, 32, A + C.g4a, 32, batch, GW(6), GB(6), s);
+  bwd3_weight<4, false>(tc, tce, A + C.u2, 32, A + C.g4a, 32, batch, A + C.part, GW(6), GB(6), s);
   bwd3_data<4>(tc, tce, A + C.g4a, 32, W(6), 32, A + C.u2, A + C.g4b, batch, s);
   // u2 = relu(up(c2) + s2): c2 = conv1(bt, 64->32)
   g_kernel_launches += 3;
@@ -749,27 +946,27 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   k_conv1_bwd_weight<kT><<<dim3(64, 32), kT, 0, s>>>(A + C.bt, 64, A + C.g2b, 32, 8, batch, GW(5), GB(5));
   k_conv1_bwd_data<<<grid_for(B * 64 * 8), kT, 0, s>>>(A + C.g2b, 32, W(5), 64, 8, B * 64 * 8, A + C.bt, A + C.g2a);
   // bt (conv3 32->64 on p2) -> gp2 (g2b, 32 channels)
-  bwd3_weight<2, false>(tc, tce, A + C.p2, 32, A + C.g2a, 64, batch, GW(4), GB(4), s);
+  bwd3_weight<2, false>(tc, tce, A + C.p2, 32, A + C.g2a, 64, batch, A + C.part, GW(4), GB(4), s);
   bwd3_data<2>(tc, tce, A + C.g2a, 64, W(4), 32, nullptr, A + C.g2b, batch, s);
   // s2 gradient: (gu2 + pool_back(gp2)) * (s2 > 0) -> g4a
   g_kernel_launches += 1;
   k_pool_back_add_mask<<<grid_for(B * 32 * 64), kT, 0, s>>>(A + C.g4b, A + C.g2b, A + C.s2, 4, B * 32 * 64,
                                                             A + C.g4a);
   // e2b (conv3 32->32 on e2a) -> ge2a (g4c)
-  bwd3_weight<4, false>(tc, tce, A + C.e2a, 32, A + C.g4a, 32, batch, GW(3), GB(3), s);
+  bwd3_weight<4, false>(tc, tce, A + C.e2a, 32, A + C.g4a, 32, batch, A + C.part, GW(3), GB(3), s);
   bwd3_data<4>(tc, tce, A + C.g4a, 32, W(3), 32, A + C.e2a, A + C.g4c, batch, s);
   // e2a (conv3 16->32 on p1) -> gp1 (g4b, 16 channels)
-  bwd3_weight<4, false>(tc, tce, A + C.p1, 16, A + C.g4c, 32, batch, GW(2), GB(2), s);
+  bwd3_weight<4, false>(tc, tce, A + C.p1, 16, A + C.g4c, 32, batch, A + C.part, GW(2), GB(2), s);
   bwd3_data<4>(tc, tce, A + C.g4c, 32, W(2), 16, nullptr, A + C.g4b, batch, s);
   // s1 gradient: (gu1 + pool_back(gp1)) * (s1 > 0) -> g8a
   g_kernel_launches += 1;
   k_pool_back_add_mask<<<grid_for(B * 16 * 512), kT, 0, s>>>(A + C.g8b, A + C.g4b, A + C.s1, 8, B * 16 * 512,
                                                              A + C.g8a);
   // e1b (conv3 16->16 on e1a) -> ge1a (g8c)
-  bwd3_weight<8, false>(tc, tce, A + C.e1a, 16, A + C.g8a, 16, batch, GW(1), GB(1), s);
+  bwd3_weight<8, false>(tc, tce, A + C.e1a, 16, A + C.g8a, 16, batch, A + C.part, GW(1), GB(1), s);
   bwd3_data<8>(tc, tce, A + C.g8a, 16, W(1), 16, A + C.e1a, A + C.g8c, batch, s);
   // e1a (valid conv3 2->16 on x)
-  bwd3_weight<8, true>(tc, tce, A + C.x, 2, A + C.g8c, 16, batch, GW(0), GB(0), s);
+  bwd3_weight<8, true>(tc, tce, A + C.x, 2, A + C.g8c, 16, batch, A + C.part, GW(0), GB(0), s);
   if (tce != cudaSuccess) return tce;
   return cudaGetLastError();
 }

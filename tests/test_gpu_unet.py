@@ -376,3 +376,46 @@ def test_zero_network_breaks_down_and_falls_back_at_once():
     assert d.fell_back == 1 and d.learned_iterations == 0
     assert d.relative_residual <= 1e-6
     ctx.close()
+
+
+def _open_network(seed):
+    """Parameters whose every ReLU is open on _inputs: weights a tenth of the initialisation's and
+    biases 1, so a layer's sum has a standard deviation of about 0.15 around at least 1. With masks
+    that rounding cannot flip, the errors are those of the sums alone (one flipped mask of the 10^6
+    that 40 items have moves a gradient of the first layer by 3e-3)."""
+    th, off = 0.1 * U.init_params(seed), 0
+    for name, nw, nb in U.layer_sizes():
+        th[off + nw:off + nw + nb] = 1.0
+        off += nw + nb
+    return th
+
+
+@pytest.mark.parametrize("batch", [1, 5, 33, 40])
+def test_fp32_convolutions_at_item_counts(batch):
+    """The FP32 forward and backward at item counts around the items a CTA takes (4, 32) and the
+    work units of one CTA per SM (40 items are 160 slabs), against the FP64 oracle: sums of at most
+    864 FP32 terms in the forward, 20k in a gradient, 1e-4 per layer; twice gives the same bits."""
+    import torch
+
+    rng = np.random.default_rng(batch)
+    th = _open_network(3)
+    x = _inputs(rng, batch)
+    y_ref, cache = U.forward(th, x)
+    dy = rng.normal(size=y_ref.shape)
+    g_ref = U.backward(th, cache, dy)
+    P, X, DY = _t(th), _t(x), _t(dy.reshape(batch, 512))
+    Y, G, again = torch.zeros((batch, 512), device="cuda"), torch.zeros_like(P), torch.zeros_like(P)
+    n = fb.UNet(batch)
+    n.forward(P, X, Y)
+    n.backward(P, DY, G)
+    n.forward(P, X, Y)
+    n.backward(P, DY, again)
+    torch.cuda.synchronize()
+    n.close()
+    assert torch.equal(G, again)
+    assert _rel(Y.cpu().numpy(), y_ref.reshape(batch, 512)) <= TOL
+    g, off = G.cpu().numpy(), 0
+    for name, nw, nb in U.layer_sizes():
+        assert _rel(g[off:off + nw], g_ref[off:off + nw]) <= TOL, name
+        assert _rel(g[off + nw:off + nw + nb], g_ref[off + nw:off + nw + nb]) <= TOL, name
+        off += nw + nb
