@@ -15,16 +15,23 @@
 // InitializeMacPressure3D (mac_pressure_3d_multigrid.cc:401-419) and the
 // evaluation and identity check of mac_pressure_workspace_3d.cc:399-461.
 //
-// B200 layout. Such a system is a few hundred KB, so one CTA of 1024 threads
-// on one SM does all of it in a single launch, in FP64: per-face
-// coefficients, then per cell the right-hand side and the diagonal summed over
-// its incident faces in increasing face order (the order of the reference's
-// face loop, so the compensated sums are the reference's sums), the gauge
-// balance of every unanchored component, Jacobi-preconditioned CG from the
-// warm start with its six vectors in shared memory (each face entry resolved
-// once to its other cell and conductance), and the evaluation (corrected face
-// velocities, residuals, physical defects, the residual/defect identity). The
-// host does only index
+// B200 layout. Such a system is a few hundred KB and its solve a chain of some
+// hundred dependent sums, so it is bound by the latency of a CG iteration. One
+// cluster of 8 CTAs x 512 threads does all of it in a single launch, in FP64,
+// with one cell per thread: a thread keeps its cell's row (six conductances and
+// the addresses of the six neighbours), residual, preconditioned residual and
+// pressure in registers; only the search direction is shared, through
+// distributed shared memory. A sum over all cells is warp shuffles, one remote
+// store per warp and CTA, and a cluster barrier, after which every warp adds the
+// 128 warp sums itself in a fixed order: three cluster barriers per iteration.
+// The 3375-cell dam break to the reference's gate takes 175 us; one CTA of 1024
+// threads with the vectors in its shared memory took 643 us.
+// Before the solve: per-face coefficients, then per cell the right-hand side and
+// the diagonal summed over its incident faces in increasing face order (the
+// order of the reference's face loop, so the compensated sums are the
+// reference's sums) and the gauge balance of every unanchored component; after
+// it the evaluation (corrected face velocities, residuals, physical defects, the
+// residual/defect identity). The host does only index
 // work: face endpoints by binary search, per-cell face lists, connected
 // components and gauges. This file is compiled with -fmad=false so that no
 // product is fused into a sum, as in the reference's FP64 arithmetic.
@@ -45,8 +52,11 @@
 namespace fl {
 namespace {
 
-constexpr int kMpThreads = 1024;
+constexpr int kMpCtas = 8, kMpThreads = 512;  // one cluster
+constexpr int kMpAll = kMpCtas * kMpThreads;
+constexpr int kMpWarps = kMpAll / 32;
 constexpr uint64_t kMpMaxCells = 4096;   // mac_pressure_3d_arithmetic.h:19
+static_assert(kMpMaxCells <= (uint64_t)kMpAll, "one cell per thread");
 constexpr uint64_t kMpMaxFaces = 24576;  // mac_pressure_3d_arithmetic.h:20
 constexpr int kMpMaxIterations = 65536;
 
@@ -72,8 +82,7 @@ struct MpSystem {
   const int* face_kind;
   const int* tail;
   const int* head;
-  const int* cell_off;  // nc + 1
-  const int* cell_ent;
+  const int* cell_ent;  // 6 nc
   const int* root;       // component root (smallest ordinal) per cell
   const unsigned char* pinned;
   const int* comp_cell_off;  // ncomp + 1 (unanchored components only)
@@ -81,11 +90,8 @@ struct MpSystem {
   const int* comp_face_off;
   const int* comp_faces;  // (face << 1) | (1 when the component holds the head)
   // work and results
-  int* ent_other;                                         // per face entry: (other cell << 1) | side
-  double* ent_cond;                                       // per face entry: the face's conductance
-  double *scale, *cond, *wall_face;                       // nf
-  double *compliance, *rhs, *rhs_abs;                    // nc
-  double *p, *residual, *defect;                          // nc (the solver's vectors are in shared memory)
+  double *scale, *cond, *wall_face;  // nf
+  double *rhs, *p, *residual, *defect;  // nc
   double* corrected_u;                                    // nf
   MpStatus* out;
 };
@@ -111,77 +117,83 @@ struct Row {
   }
 };
 
-// Sum of v over the CTA, returned to every thread (fixed order for a fixed launch).
-__device__ double cta_sum(double v, double* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();  // red may still be read from the previous call
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  double s = 0.0;
-  for (int k = 0; k < kMpThreads / 32; ++k) s += red[k];
-  return s;
+__device__ __forceinline__ unsigned mp_map(unsigned a, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
 }
-// Two sums over the CTA in one pair of barriers, each exactly as cta_sum forms it.
-__device__ double2 cta_sum2(double a, double b, double* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
-  }
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) {
-    red[w] = a;
-    red[kMpThreads / 32 + w] = b;
-  }
-  __syncthreads();
-  double sa = 0.0, sb = 0.0;
-  for (int k = 0; k < kMpThreads / 32; ++k) {
-    sa += red[k];
-    sb += red[kMpThreads / 32 + k];
-  }
-  return make_double2(sa, sb);
+__device__ __forceinline__ double mp_ld(unsigned a) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  return v;
 }
-__device__ double cta_max(double v, double* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  double s = 0.0;
-  for (int k = 0; k < kMpThreads / 32; ++k) s = fmax(s, red[k]);
-  return s;
+__device__ __forceinline__ void mp_st(unsigned a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+// Cluster barrier; orders the cluster's shared and global memory accesses.
+__device__ __forceinline__ void mp_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// out_i = (A x)_i: compliance, then each incident face's flux in face order.
-// Entries are resolved once (other endpoint, conductance), so a row needs no
-// face lookup; the flux is c (x_tail - x_head) as in the face loop, with a
-// missing endpoint at zero.
-// Every cell lists exactly its six incident faces (the host checks the face
-// set), so row i's entries are 6i .. 6i+5: all twelve loads are issued
-// before the sum, which keeps the face order.
-__device__ double apply_row(const MpSystem& S, const double* x, int i) {
-  const double xi = x[i];
-  double out = S.compliance[i] * xi;
-  double c[6];
-  int o[6];
+// Sums (and, for the last N - kSums values, maxima) of v[N] over the cluster,
+// returned to every thread: `slots` holds N doubles per warp of the cluster, is
+// written by every CTA and may be written again only after a further barrier.
+template <int N, int kSums>
+__device__ void mp_reduce(double (&v)[N], double* slots, unsigned rank) {
+  const int lane = threadIdx.x & 31, warp = (int)rank * (kMpThreads / 32) + (threadIdx.x >> 5);
 #pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    c[k] = S.ent_cond[6 * i + k];
-    o[k] = S.ent_other[6 * i + k];
+  for (int n = 0; n < N; ++n) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double w = __shfl_xor_sync(0xffffffffu, v[n], o);
+      v[n] = n < kSums ? v[n] + w : fmax(v[n], w);
+    }
   }
+  if (lane < kMpCtas) {
+    const unsigned to = mp_map((unsigned)__cvta_generic_to_shared(slots + warp * N), (unsigned)lane);
+#pragma unroll
+    for (int n = 0; n < N; ++n) mp_st(to + 8u * n, v[n]);
+  }
+  mp_sync();
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    double s = slots[lane * N + n];
+#pragma unroll
+    for (int k = 1; k < kMpWarps / 32; ++k) {
+      const double w = slots[(lane + 32 * k) * N + n];
+      s = n < kSums ? s + w : fmax(s, w);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double w = __shfl_xor_sync(0xffffffffu, s, o);
+      s = n < kSums ? s + w : fmax(s, w);
+    }
+    v[n] = s;
+  }
+}
+
+// One cell's row: its compliance, then per incident face (increasing face
+// order) the conductance (0: no flux), the address of the other cell's entry of
+// the shared vector, whether there is such a cell (its value is zero otherwise)
+// and the side this cell is on.
+struct MpRow {
+  double compliance, c[6];
+  unsigned other[6], has, head;  // bit k: face k has another cell; this cell is face k's head
+};
+// (A x)_i for x_i = xi: the flux is c (x_tail - x_head) as in the face loop.
+__device__ __forceinline__ double mp_apply(const MpRow& r, double xi) {
+  double out = r.compliance * xi, xo[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) xo[k] = (r.has >> k) & 1u ? mp_ld(r.other[k]) : 0.0;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
-    if (c[k] == 0.0) continue;
-    const int other = o[k] >> 1;  // -1: no cell at the other end
-    const double xo = other >= 0 ? x[other] : 0.0;
-    if (o[k] & 1)
-      out -= c[k] * (xo - xi);  // this cell is the head
+    if (r.c[k] == 0.0) continue;
+    if ((r.head >> k) & 1u)
+      out -= r.c[k] * (xo[k] - xi);
     else
-      out += c[k] * (xi - xo);
+      out += r.c[k] * (xi - xo[k]);
   }
   return out;
 }
@@ -200,27 +212,18 @@ __device__ double corrected_velocity(const MpSystem& S, const double* p, int f) 
   return u;
 }
 
-__global__ void __launch_bounds__(kMpThreads, 1) k_mac_pressure(MpSystem S) {
-  __shared__ double red[kMpThreads / 32];
-  __shared__ int status;
-  const int t = threadIdx.x;
+__global__ void __cluster_dims__(kMpCtas, 1, 1) __launch_bounds__(kMpThreads, 1) k_mac_pressure(MpSystem S) {
+  __shared__ double vec[kMpThreads];  // the shared vector: this CTA's cells
+  __shared__ double slots_a[kMpWarps], slots_b[2 * kMpWarps], slots_c[5 * kMpWarps];
+  unsigned rank;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int t = (int)rank * kMpThreads + threadIdx.x;  // this thread's cell
   const int nc = S.nc, nf = S.nf;
-  // The solver's vectors (at most 6 x 4096 doubles) live in shared memory;
-  // the pressure goes to global memory at the end for the host.
-  extern __shared__ double vec[];
-  double* P = vec;
-  double* D = P + nc;
-  double* R = D + nc;
-  double* Q = R + nc;
-  double* Z = Q + nc;
-  double* DG = Z + nc;
-  if (t == 0) {
-    status = FL_OK;
-    S.out->arch = compiled_arch();
-  }
+  const bool mine = t < nc;
+  if (t == 0) S.out->arch = compiled_arch();
   const double full_area = S.h * S.h;
   // Face coefficients (FreezeLinkFromIncidence).
-  for (int f = t; f < nf; f += kMpThreads) {
+  for (int f = t; f < nf; f += kMpAll) {
     const double* v = S.face_values + 6 * f;
     double sc = 0.0, c = 0.0;
     if (v[0] > 0.0) {
@@ -231,49 +234,59 @@ __global__ void __launch_bounds__(kMpThreads, 1) k_mac_pressure(MpSystem S) {
     S.cond[f] = c;
     S.wall_face[f] = (full_area - v[0]) * v[4];
   }
-  for (int i = t; i < nc; i += kMpThreads) {
-    const double* v = S.cell_values + 5 * i;
-    S.compliance[i] = v[2] == 0.0 ? 0.0 : v[0] / (v[2] * S.dt);
-  }
-  __syncthreads();
+  mp_sync();
   // Right-hand side and diagonal (AssembleIntegratedRhsInto): the cell's own
-  // terms, then its faces in increasing face order; each face entry resolved
-  // for the operator rows.
-  for (int i = t; i < nc; i += kMpThreads) {
-    for (int e = S.cell_off[i]; e < S.cell_off[i + 1]; ++e) {
-      const int f = S.cell_ent[e] >> 1, side = S.cell_ent[e] & 1;
-      const int other = side ? S.tail[f] : S.head[f];
-      S.ent_other[e] = other * 2 + side;  // other = -1 gives -2 + side: >> 1 is -1, & 1 the side
-      S.ent_cond[e] = S.cond[f];
-    }
-    const double* v = S.cell_values + 5 * i;
-    Row row;
-    row.add(v[0] * v[1]);
-    row.add(v[4]);
-    row.add(S.compliance[i] * v[3]);
-    double dg = S.compliance[i];
-    for (int e = S.cell_off[i]; e < S.cell_off[i + 1]; ++e) {
-      const int f = S.cell_ent[e] >> 1;
-      const bool is_head = S.cell_ent[e] & 1;
+  // terms, then its six faces in increasing face order; each face entry resolved
+  // for the operator row. Every cell lists exactly its six incident faces (the
+  // host checks the face set), so cell i's entries are 6i .. 6i + 5.
+  MpRow row{};
+  double dg = 0.0, rhs = 0.0, rhs_abs = 0.0, start = 0.0;
+  bool pinned = false;
+  const unsigned vec_a = (unsigned)__cvta_generic_to_shared(vec);
+  if (mine) {
+    const double* v = S.cell_values + 5 * t;
+    row.compliance = v[2] == 0.0 ? 0.0 : v[0] / (v[2] * S.dt);
+    Row sum;
+    sum.add(v[0] * v[1]);
+    sum.add(v[4]);
+    sum.add(row.compliance * v[3]);
+    dg = row.compliance;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int ent = S.cell_ent[6 * t + k], f = ent >> 1;
+      const bool is_head = ent & 1;
+      const int other = is_head ? S.tail[f] : S.head[f];
+      const double c = S.cond[f];
+      row.c[k] = c;
+      if (other >= 0) {
+        row.other[k] = mp_map(vec_a + 8u * (unsigned)(other % kMpThreads), (unsigned)(other / kMpThreads));
+        row.has |= 1u << k;
+      }
+      row.head |= is_head ? 1u << k : 0u;
       const double* fv = S.face_values + 6 * f;
       const double fluid_flux = fv[0] * fv[3];
       const double sgn = is_head ? 1.0 : -1.0;
-      row.add(sgn * fluid_flux);
-      row.add(sgn * S.wall_face[f]);
+      sum.add(sgn * fluid_flux);
+      sum.add(sgn * S.wall_face[f]);
       const int kind = S.face_kind[f];
       if (kind == kLinkInternal)
-        row.add(sgn * (S.cond[f] * fv[5]));
+        sum.add(sgn * (c * fv[5]));
       else if (kind == kLinkDirichlet)
-        row.add(S.cond[f] * fv[5]);
-      dg += S.cond[f];
+        sum.add(c * fv[5]);
+      dg += c;
     }
-    S.rhs[i] = row.flux.total();
-    S.rhs_abs[i] = row.absolute.total();
-    DG[i] = dg;
+    rhs = sum.flux.total();
+    rhs_abs = sum.absolute.total();
+    S.rhs[t] = rhs;
+    pinned = S.pinned[t] != 0;
+    // Warm start: the previous pressure, less the pin's on unanchored components.
+    const int rt = S.root[t];
+    start = v[3] - (S.pinned[rt] ? S.cell_values[5 * rt + 3] : 0.0);
   }
   // Gauge balance of each unanchored component (SelectGaugesInto): its cells'
   // source and wall terms, then the wall flux of its faces, in order.
-  for (int k = t; k < S.ncomp; k += kMpThreads) {
+  double unbalanced = 0.0;
+  for (int k = t; k < S.ncomp; k += kMpAll) {
     Row bal;
     for (int e = S.comp_cell_off[k]; e < S.comp_cell_off[k + 1]; ++e) {
       const double* v = S.cell_values + 5 * S.comp_cells[e];
@@ -284,110 +297,82 @@ __global__ void __launch_bounds__(kMpThreads, 1) k_mac_pressure(MpSystem S) {
       const int f = S.comp_faces[e] >> 1;
       bal.add((S.comp_faces[e] & 1) ? S.wall_face[f] : -1.0 * S.wall_face[f]);
     }
-    if (fabs(bal.flux.total()) > 32.0 * DBL_EPSILON * bal.absolute.total()) atomicExch(&status, FL_FAILED_PRECONDITION);
+    if (fabs(bal.flux.total()) > 32.0 * DBL_EPSILON * bal.absolute.total()) unbalanced = 1.0;
   }
-  __syncthreads();
-  if (status != FL_OK) {
+  double P = start, D = 0.0;
+  vec[threadIdx.x] = P;
+  double first[2] = {rhs * rhs, unbalanced};
+  mp_reduce<2, 1>(first, slots_b, rank);
+  if (first[1] != 0.0) {  // the same for every thread of the cluster
     if (t == 0) {
-      S.out->status = status;
+      S.out->status = FL_FAILED_PRECONDITION;
       S.out->iterations = 0;
       S.out->true_residual_l2 = S.out->max_volume_scaled_residual = S.out->max_defect = S.out->rhs_l2 = 0.0;
     }
-    return;  // (uniform: every thread read the same status after the barrier)
+    return;
   }
-  // Warm start: the previous pressure, less the pin's on unanchored components.
-  for (int i = t; i < nc; i += kMpThreads) {
-    const int rt = S.root[i];
-    const double shift = S.pinned[rt] ? S.cell_values[5 * rt + 3] : 0.0;
-    P[i] = S.cell_values[5 * i + 3] - shift;
-  }
-  __syncthreads();
-  double bb = 0.0;
-  for (int i = t; i < nc; i += kMpThreads) {
-    const double q = apply_row(S, P, i);
-    R[i] = S.pinned[i] ? 0.0 : S.rhs[i] - q;
-    bb += S.rhs[i] * S.rhs[i];
-  }
-  const double bnorm = sqrt(cta_sum(bb, red));
+  const double bnorm = sqrt(first[0]);
   // ||b - Ap||_2 <= rel_tol ||b||_2, or the reference's gate 2e-6 + 2e-6 ||b||_2
   const double limit = S.rel_tol > 0.0 ? S.rel_tol * bnorm : 2e-6 + 2e-6 * bnorm;
-  // Jacobi-preconditioned CG; the pinned rows stay at their warm start. The
-  // residual norm, the preconditioned residual z = r / diag and r.z of each
-  // iterate are formed in the pass that updates r (every thread visits its
-  // rows in the same order as a separate pass would, so the sums are the same
-  // bits), and both sums share one reduction.
-  __shared__ double red2[2 * (kMpThreads / 32)];
-  double rr = 0.0, rz = 0.0;
-  for (int i = t; i < nc; i += kMpThreads) rr += R[i] * R[i];
-  for (int i = t; i < nc; i += kMpThreads) {
-    const double zi = (S.pinned[i] || DG[i] == 0.0) ? 0.0 : R[i] / DG[i];
-    Z[i] = zi;
-    rz += R[i] * zi;
-  }
-  {
-    const double2 sums = cta_sum2(rr, rz, red2);
-    rr = sums.x;
-    rz = sums.y;
-  }
-  double rz_prev = 0.0;
+  // Jacobi-preconditioned CG; the pinned rows stay at their warm start.
+  const bool solved = mine && !pinned, scaled = solved && dg != 0.0;
+  double R = solved ? rhs - mp_apply(row, P) : 0.0;
+  double Z = scaled ? R / dg : 0.0;
+  double sums[2] = {R * R, R * Z};
+  mp_sync();  // every CTA has read slots_b and its neighbours' starts
+  mp_reduce<2, 2>(sums, slots_b, rank);
+  double rr = sums[0], rz = sums[1], rz_prev = 0.0;
   int it = 0;
+  double status = FL_OK;
   for (; it < S.max_iterations; ++it) {
     if (sqrt(rr) <= limit) break;
     const double beta = it == 0 ? 0.0 : rz / rz_prev;
-    for (int i = t; i < nc; i += kMpThreads) D[i] = it == 0 ? Z[i] : Z[i] + beta * D[i];
-    __syncthreads();
-    double dq = 0.0;
-    for (int i = t; i < nc; i += kMpThreads) {
-      const double qi = S.pinned[i] ? 0.0 : apply_row(S, D, i);
-      Q[i] = qi;
-      dq += D[i] * qi;
-    }
-    dq = cta_sum(dq, red);
-    if (!(dq > 0.0)) {
-      if (t == 0) status = FL_ABORTED;
+    D = it == 0 ? Z : Z + beta * D;
+    vec[threadIdx.x] = D;
+    mp_sync();
+    const double Q = solved ? mp_apply(row, D) : 0.0;
+    double dq[1] = {D * Q};
+    mp_reduce<1, 1>(dq, slots_a, rank);  // its barrier also ends the reads of vec
+    if (!(dq[0] > 0.0)) {
+      status = FL_ABORTED;
       break;
     }
-    const double alpha = rz / dq;
-    double rr_next = 0.0, rz_next = 0.0;
-    for (int i = t; i < nc; i += kMpThreads) {
-      P[i] += alpha * D[i];
-      const double ri = R[i] - alpha * Q[i];
-      R[i] = ri;
-      rr_next += ri * ri;
-      const double zi = (S.pinned[i] || DG[i] == 0.0) ? 0.0 : ri / DG[i];
-      Z[i] = zi;
-      rz_next += ri * zi;
-    }
-    const double2 sums = cta_sum2(rr_next, rz_next, red2);
+    const double alpha = rz / dq[0];
+    P += alpha * D;
+    R = R - alpha * Q;
+    Z = scaled ? R / dg : 0.0;
+    double next[2] = {R * R, R * Z};
+    mp_reduce<2, 2>(next, slots_b, rank);
     rz_prev = rz;
-    rr = sums.x;
-    rz = sums.y;
+    rr = next[0];
+    rz = next[1];
   }
-  __syncthreads();
   // Evaluation: corrected faces, residuals b - Ap, physical defects and the
   // identity V d + r = 0 within 64 ulp of the terms' magnitudes.
-  for (int f = t; f < nf; f += kMpThreads) {
-    const double u = corrected_velocity(S, P, f);
-    if (!isfinite(u)) atomicExch(&status, FL_OUT_OF_RANGE);
+  if (mine) S.p[t] = P;
+  mp_sync();
+  for (int f = t; f < nf; f += kMpAll) {
+    const double u = corrected_velocity(S, S.p, f);
+    if (!isfinite(u)) status = fmax(status, (double)FL_OUT_OF_RANGE);
     S.corrected_u[f] = u;
   }
-  __syncthreads();
-  double l2 = 0.0, bl2 = 0.0, maxr = 0.0, maxd = 0.0;
-  for (int i = t; i < nc; i += kMpThreads) {
-    const double* v = S.cell_values + 5 * i;
+  mp_sync();
+  double l2 = 0.0, maxr = 0.0, maxd = 0.0;
+  if (mine) {
+    const double* v = S.cell_values + 5 * t;
     Row op, ph;
-    op.add(S.compliance[i] * P[i]);
+    op.add(row.compliance * P);
     ph.add(-v[0] * v[1]);
     ph.add(-v[4]);
-    if (S.compliance[i] > 0.0) ph.add(S.compliance[i] * (P[i] - v[3]));
-    for (int e = S.cell_off[i]; e < S.cell_off[i + 1]; ++e) {
-      const int f = S.cell_ent[e] >> 1;
-      const bool is_head = S.cell_ent[e] & 1;
-      const double c = S.cond[f];
-      if (c != 0.0) {
+    if (row.compliance > 0.0) ph.add(row.compliance * (P - v[3]));
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int ent = S.cell_ent[6 * t + k], f = ent >> 1;
+      const bool is_head = ent & 1;
+      if (row.c[k] != 0.0) {
         const int tl = S.tail[f], hd = S.head[f];
-        const double pt = tl >= 0 ? P[tl] : 0.0, phd = hd >= 0 ? P[hd] : 0.0;
-        const double flux = c * (pt - phd);
+        const double pt = tl >= 0 ? S.p[tl] : 0.0, phd = hd >= 0 ? S.p[hd] : 0.0;
+        const double flux = row.c[k] * (pt - phd);
         op.add(is_head ? -flux : flux);
       }
       const double flux = S.face_values[6 * f] * S.corrected_u[f];
@@ -399,33 +384,29 @@ __global__ void __launch_bounds__(kMpThreads, 1) k_mac_pressure(MpSystem S) {
         ph.add(S.wall_face[f]);
       }
     }
-    const double r = S.rhs[i] - op.flux.total();
+    const double r = rhs - op.flux.total();
     const double dd = ph.flux.total() / v[0];
     const double ident = v[0] * dd + r;
-    const double absterms = S.rhs_abs[i] + op.absolute.total() + ph.absolute.total();
-    if (fabs(ident) > 64.0 * DBL_EPSILON * absterms) atomicExch(&status, FL_INTERNAL);
-    S.residual[i] = r;
-    S.defect[i] = dd;
-    S.p[i] = P[i];
-    l2 += r * r;
-    bl2 += S.rhs[i] * S.rhs[i];
-    maxr = fmax(maxr, fabs(r) / v[0]);
-    maxd = fmax(maxd, fabs(dd));
+    const double absterms = rhs_abs + op.absolute.total() + ph.absolute.total();
+    if (fabs(ident) > 64.0 * DBL_EPSILON * absterms) status = fmax(status, (double)FL_INTERNAL);
+    S.residual[t] = r;
+    S.defect[t] = dd;
+    l2 = r * r;
+    maxr = fabs(r) / v[0];
+    maxd = fabs(dd);
   }
-  l2 = sqrt(cta_sum(l2, red));
-  bl2 = sqrt(cta_sum(bl2, red));
-  maxr = cta_max(maxr, red);
-  maxd = cta_max(maxd, red);
-  __syncthreads();
+  double ends[5] = {l2, rhs * rhs, maxr, maxd, status};
+  mp_reduce<5, 2>(ends, slots_c, rank);
   if (t == 0) {
-    int st = status;
-    if (st == FL_OK && l2 > limit * 1.000001 + 1e-300) st = FL_ABORTED;
+    const double norm = sqrt(ends[0]);
+    int st = (int)ends[4];  // the gravest of the cells' and faces' codes
+    if (st == FL_OK && norm > limit * 1.000001 + 1e-300) st = FL_ABORTED;
     S.out->status = st;
     S.out->iterations = it;
-    S.out->true_residual_l2 = l2;
-    S.out->max_volume_scaled_residual = maxr;
-    S.out->max_defect = maxd;
-    S.out->rhs_l2 = bl2;
+    S.out->true_residual_l2 = norm;
+    S.out->max_volume_scaled_residual = ends[2];
+    S.out->max_defect = ends[3];
+    S.out->rhs_l2 = sqrt(ends[1]);
   }
 }
 
@@ -489,9 +470,9 @@ int find_root(std::vector<int>& parent, int c) {
 // unanchored components, comp_faces component face entries.
 size_t mp_arena_bytes(size_t nc, size_t nf, size_t ent, size_t ncomp, size_t comp_faces) {
   const size_t nd_in = 5 * nc + 6 * nf;
-  const size_t nd_work = 3 * nf + 6 * nc + nf + ent;
-  const size_t ni = 3 * nf + (nc + 1) + ent + nc + (ncomp + 1) + nc + (ncomp + 1) + comp_faces;
-  return sizeof(double) * (nd_in + nd_work) + sizeof(MpStatus) + sizeof(int) * (ni + ent) + nc + 64;
+  const size_t nd_work = 3 * nf + 4 * nc + nf;
+  const size_t ni = 3 * nf + ent + nc + (ncomp + 1) + nc + (ncomp + 1) + comp_faces;
+  return sizeof(double) * (nd_in + nd_work) + sizeof(MpStatus) + sizeof(int) * ni + nc + 64;
 }
 
 bool MpScratch::reserve_caps() {
@@ -786,14 +767,11 @@ int mp_project(MpScratch& X, cudaStream_t stream, double h, double dt, const int
   S.scale = take_d(nf);
   S.cond = take_d(nf);
   S.wall_face = take_d(nf);
-  S.compliance = take_d(nc);
   S.rhs = take_d(nc);
-  S.rhs_abs = take_d(nc);
   S.p = take_d(nc);
   S.residual = take_d(nc);
   S.defect = take_d(nc);
   S.corrected_u = take_d(nf);
-  S.ent_cond = take_d(cell_ent.size());
   S.out = reinterpret_cast<MpStatus*>(dp);
   int* ip = reinterpret_cast<int*>(S.out + 1);
   auto& host_ints = X.host_ints;
@@ -806,15 +784,13 @@ int mp_project(MpScratch& X, cudaStream_t stream, double h, double dt, const int
   S.face_kind = put(face_kind, nf);
   S.tail = put(tail.data(), nf);
   S.head = put(head.data(), nf);
-  S.cell_off = put(cell_off.data(), nc + 1);
   S.cell_ent = put(cell_ent.data(), cell_ent.size());
   S.root = put(root.data(), nc);
   S.comp_cell_off = put(comp_cell_off.data(), ncomp + 1);
   S.comp_cells = put(comp_cells.data(), comp_cells.size());
   S.comp_face_off = put(comp_face_off.data(), ncomp + 1);
   S.comp_faces = put(comp_faces.data(), comp_faces.size());
-  S.ent_other = ip + host_ints.size();  // written by the kernel
-  unsigned char* d_pinned = reinterpret_cast<unsigned char*>(S.ent_other + cell_ent.size());
+  unsigned char* d_pinned = reinterpret_cast<unsigned char*>(ip + host_ints.size());
   S.pinned = d_pinned;
   S.cell_values = d_cells;
   S.face_values = d_faces;
@@ -829,13 +805,8 @@ int mp_project(MpScratch& X, cudaStream_t stream, double h, double dt, const int
             cudaMemcpyAsync(d_pinned, pinned.data(), nc, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaEventRecord(X.e0, s) == cudaSuccess;
   if (ok) {
-    const size_t vec_bytes = sizeof(double) * 6 * (size_t)nc;
-    static unsigned long long configured = 0;
-    if (first_on_device(configured))
-      cudaFuncSetAttribute(k_mac_pressure, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(sizeof(double) * 6 * kMpMaxCells));
     ++g_kernel_launches;
-    k_mac_pressure<<<1, kMpThreads, vec_bytes, s>>>(S);
+    k_mac_pressure<<<kMpCtas, kMpThreads, 0, s>>>(S);
     ok = cudaGetLastError() == cudaSuccess && cudaEventRecord(X.e1, s) == cudaSuccess &&
          cudaMemcpyAsync(&res, S.out, sizeof(MpStatus), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
          cudaStreamSynchronize(s) == cudaSuccess && cudaEventElapsedTime(&ms, X.e0, X.e1) == cudaSuccess;

@@ -128,3 +128,28 @@ def test_solves_are_bitwise_reproducible():
     for k in ("pressure", "rhs", "residual", "defect", "corrected_u"):
         np.testing.assert_array_equal(a[k], b[k])
     assert a["diag"]["iterations"] == b["diag"]["iterations"] == 95  # as the FP64 oracle
+
+
+@pytest.mark.parametrize("size", [(1, 1, 1), (7, 8, 9), (8, 8, 8), (27, 19, 1), (16, 16, 16)])
+def test_brick_sizes(size):
+    """Bricks of 1, 504, 512, 513 and 4096 cells (a CTA of the cluster has 512) with air on their
+    high sides, against the FP64 oracle solved to the same 1e-12: the right-hand side bit for bit,
+    pressures to 1e-8 of the largest."""
+    rng = np.random.default_rng(size[0])
+    z, y, x = np.meshgrid(*[np.arange(s) for s in size[::-1]], indexing="ij")
+    ci = np.stack([x.ravel(), y.ravel(), z.ravel()], 1).astype(np.int32)
+    cv = np.zeros((len(ci), 5))
+    cv[:, 0] = 1.0
+    opens = {}
+    for c in ci.tolist():
+        for a in range(3):
+            hi = list(c)
+            hi[a] += 1
+            opens[(a, *hi)] = (2 if hi[a] == size[a] else 1, [1.0, 1e-3, 1.0, rng.normal(), 0.0, 0.0])
+    fi, fk, fv = closed_system(ci, opens)
+    args = (ci, cv, fi, fk, fv, 1.0, 0.01)
+    out = fb.project_mac_pressure_3d(*args, rel_tol=1e-12, max_iterations=4000)
+    ref = oracle.pressure_solve(*args, rel_tol=1e-12, max_iterations=4000)
+    np.testing.assert_array_equal(out["rhs"], ref["rhs"])
+    assert np.abs(out["pressure"] - ref["pressure"]).max() <= 1e-8 * np.abs(ref["pressure"]).max()
+    assert out["diag"]["true_residual_l2"] <= 1e-12 * out["diag"]["rhs_l2"] * 1.000001
