@@ -74,7 +74,7 @@ def build(verbose: bool = False, force: bool = False) -> Path:
         if verbose:
             sys.stdout.write(out.decode())
     if force or _stale(LIB, objs):
-        cmd = [nvcc(), "-shared", *ARCH, "-o", str(LIB), *map(str, objs), "-lcudart", "-lcublas"]
+        cmd = [nvcc(), "-shared", *ARCH, "-o", str(LIB), *map(str, objs), "-lcudart"]
         subprocess.check_call(cmd)
     build_backend(force)
     return LIB

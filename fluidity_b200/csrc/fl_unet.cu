@@ -306,7 +306,6 @@ struct WgradTile {
   static constexpr int kG = 20;  // words per cell of g: 16 channels, padded
   static constexpr size_t kSmem = sizeof(float) * (kItems * (kItem + kZ * S * S * kG) + 4);
 };
-constexpr long long kWgradPart = 1 << 21;  // floats of the partial rows
 
 template <int S, bool VALID, int CIN>
 __global__ void __launch_bounds__(WgradTile<S, VALID, CIN>::kThreads)
@@ -756,9 +755,9 @@ void wgrad(const float* in, const float* g, int cout, int batch, float* part, fl
   const int units = (batch + T::kItems - 1) / T::kItems * T::kSlabs;
   // one CTA per SM where the units and the partial rows' space allow it
   const int ctas = (int)std::min<long long>({(long long)units, 148, kWgradPart / ((long long)T::kSplit * (nw + cout))});
-  g_kernel_launches += 2;
+  ++g_kernel_launches;
   k_conv3_wgrad<S, VALID, CIN><<<dim3(ctas, cout / 16), T::kThreads, T::kSmem, s>>>(in, g, cout, batch, units, part);
-  k_wgrad_sum<<<(nw + cout + 31) / 32, kT, 0, s>>>(part, ctas * T::kSplit, nw, cout, dw, db);
+  wgrad_sum(part, ctas * T::kSplit, nw, cout, dw, db, s);
 }
 
 // The network's layers: 2 input channels (first layer) or 16 at 8^3, 16 or 32 at 4^3, 32 at 2^3.
@@ -775,28 +774,33 @@ void conv3_bwd_weight(const float* in, int cin, const float* g, int cout, int ba
     wgrad<S, false, 32>(in, g, cout, batch, part, dw, db, s);
 }
 
-// A 3x3x3 layer on the SIMT kernels (tc == nullptr) or as a tensor-core GEMM;
+// A 3x3x3 layer in the FP32 kernels (tc == nullptr) or on the tensor cores;
 // the first tensor-core failure is kept in `e` and the remaining layers skip.
 template <int S, bool VALID>
-void fwd3(UNetTcTrain* tc, cudaError_t& e, const float* in, int cin, const float* w, const float* bias, int cout,
-          float* out, int batch, int relu, cudaStream_t s) {
+void fwd3(UNetTcTrain* tc, cudaError_t& e, int layer, const float* in, int cin, const float* w, const float* bias,
+          int cout, float* out, int batch, int relu, cudaStream_t s) {
   if (tc == nullptr) return conv3_fwd<S, VALID>(in, cin, w, bias, cout, out, batch, relu, s);
-  if (e == cudaSuccess) e = conv3_fwd_tc<S, VALID>(*tc, in, cin, w, bias, cout, out, batch, relu, s);
+  if (e == cudaSuccess) e = conv3_fwd_tc(*tc, layer, in, bias, out, batch, s);
 }
 template <int S>
-void bwd3_data(UNetTcTrain* tc, cudaError_t& e, const float* g, int cout, const float* w, int cin, const float* act,
-               float* din, int batch, cudaStream_t s) {
+void bwd3_data(UNetTcTrain* tc, cudaError_t& e, int layer, const float* g, int cout, const float* w, int cin,
+               const float* act, float* din, int batch, cudaStream_t s) {
   if (tc == nullptr) return conv3_bwd_data<S>(g, cout, w, cin, act, din, batch, s);
-  if (e == cudaSuccess) e = conv3_bwd_data_tc<S>(*tc, g, cout, w, cin, act, din, batch, s);
+  if (e == cudaSuccess) e = conv3_bwd_data_tc(*tc, layer, g, act, din, batch, s);
 }
 template <int S, bool VALID>
-void bwd3_weight(UNetTcTrain* tc, cudaError_t& e, const float* in, int cin, const float* g, int cout, int batch,
-                 float* part, float* dw, float* db, cudaStream_t s) {
+void bwd3_weight(UNetTcTrain* tc, cudaError_t& e, int layer, const float* in, int cin, const float* g, int cout,
+                 int batch, float* part, float* dw, float* db, cudaStream_t s) {
   if (tc == nullptr) return conv3_bwd_weight<S, VALID>(in, cin, g, cout, batch, part, dw, db, s);
-  if (e == cudaSuccess) e = conv3_bwd_weight_tc<S, VALID>(*tc, in, cin, g, cout, batch, dw, db, s);
+  if (e == cudaSuccess) e = conv3_bwd_weight_tc(layer, in, g, batch, part, dw, db, s);
 }
 
 }  // namespace
+
+void wgrad_sum(const float* part, int rows, int nw, int cout, float* dw, float* db, cudaStream_t s) {
+  ++g_kernel_launches;
+  k_wgrad_sum<<<(nw + cout + 31) / 32, kT, 0, s>>>(part, rows, nw, cout, dw, db);
+}
 
 UNetLayout unet_layout() {
   static const int kCin[kUNetLayers] = {2, 16, 16, 32, 32, 64, 32, 32, 16, 16};
@@ -888,23 +892,23 @@ cudaError_t unet_forward(const float* P, const float* x, int batch, float* cache
   if (x != A + C.x) cudaMemcpyAsync(A + C.x, x, sizeof(float) * 2000 * B, cudaMemcpyDeviceToDevice, s);
   auto W = [&](int l) { return P + L.offset[l]; };
   auto Bi = [&](int l) { return P + L.bias[l]; };
-  cudaError_t tce = cudaSuccess;
-  fwd3<8, true>(tc, tce, A + C.x, 2, W(0), Bi(0), 16, A + C.e1a, batch, 1, s);
-  fwd3<8, false>(tc, tce, A + C.e1a, 16, W(1), Bi(1), 16, A + C.s1, batch, 1, s);
+  cudaError_t tce = tc != nullptr ? unet_tc_train_pack(*tc, P, false, s) : cudaSuccess;
+  fwd3<8, true>(tc, tce, 0, A + C.x, 2, W(0), Bi(0), 16, A + C.e1a, batch, 1, s);
+  fwd3<8, false>(tc, tce, 1, A + C.e1a, 16, W(1), Bi(1), 16, A + C.s1, batch, 1, s);
   g_kernel_launches += 1;
   k_pool<<<grid_for(B * 16 * 64), kT, 0, s>>>(A + C.s1, 8, B * 16 * 64, A + C.p1);
-  fwd3<4, false>(tc, tce, A + C.p1, 16, W(2), Bi(2), 32, A + C.e2a, batch, 1, s);
-  fwd3<4, false>(tc, tce, A + C.e2a, 32, W(3), Bi(3), 32, A + C.s2, batch, 1, s);
+  fwd3<4, false>(tc, tce, 2, A + C.p1, 16, W(2), Bi(2), 32, A + C.e2a, batch, 1, s);
+  fwd3<4, false>(tc, tce, 3, A + C.e2a, 32, W(3), Bi(3), 32, A + C.s2, batch, 1, s);
   g_kernel_launches += 1;
   k_pool<<<grid_for(B * 32 * 8), kT, 0, s>>>(A + C.s2, 4, B * 32 * 8, A + C.p2);
-  fwd3<2, false>(tc, tce, A + C.p2, 32, W(4), Bi(4), 64, A + C.bt, batch, 1, s);
+  fwd3<2, false>(tc, tce, 4, A + C.p2, 32, W(4), Bi(4), 64, A + C.bt, batch, 1, s);
   g_kernel_launches += 6;
   k_conv1_fwd<<<grid_for(B * 32 * 8), kT, 0, s>>>(A + C.bt, 64, W(5), Bi(5), 32, 8, B * 32 * 8, A + C.c2);
   k_up_add_relu<<<grid_for(B * 32 * 64), kT, 0, s>>>(A + C.c2, A + C.s2, 4, B * 32 * 64, A + C.u2);
-  fwd3<4, false>(tc, tce, A + C.u2, 32, W(6), Bi(6), 32, A + C.d2, batch, 1, s);
+  fwd3<4, false>(tc, tce, 6, A + C.u2, 32, W(6), Bi(6), 32, A + C.d2, batch, 1, s);
   k_conv1_fwd<<<grid_for(B * 16 * 64), kT, 0, s>>>(A + C.d2, 32, W(7), Bi(7), 16, 64, B * 16 * 64, A + C.c1);
   k_up_add_relu<<<grid_for(B * 16 * 512), kT, 0, s>>>(A + C.c1, A + C.s1, 8, B * 16 * 512, A + C.u1);
-  fwd3<8, false>(tc, tce, A + C.u1, 16, W(8), Bi(8), 16, A + C.d1, batch, 1, s);
+  fwd3<8, false>(tc, tce, 8, A + C.u1, 16, W(8), Bi(8), 16, A + C.d1, batch, 1, s);
   k_conv1_fwd<<<grid_for(B * 512), kT, 0, s>>>(A + C.d1, 16, W(9), Bi(9), 1, 512, B * 512, A + C.y);
   if (y != nullptr && y != A + C.y)
     cudaMemcpyAsync(y, A + C.y, sizeof(float) * 512 * B, cudaMemcpyDeviceToDevice, s);
@@ -916,7 +920,7 @@ cudaError_t unet_forward(const float* P, const float* x, int batch, float* cache
 cudaError_t unet_backward(const float* P, float* cache, const float* gy, int batch, float* G, cudaStream_t s,
                           UNetTcTrain* tc) {
   configure_unet_kernels();
-  cudaError_t tce = cudaSuccess;
+  cudaError_t tce = tc != nullptr ? unet_tc_train_pack(*tc, P, true, s) : cudaSuccess;
   const UNetLayout L = unet_layout();
   const UNetCache C = unet_cache_layout(batch);
   float* A = cache;
@@ -929,8 +933,8 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   k_conv1_bwd_weight<1024><<<dim3(16, 1), 1024, 0, s>>>(A + C.d1, 16, gy, 1, 512, batch, GW(9), GB(9));
   k_conv1_bwd_data<<<grid_for(B * 16 * 512), kT, 0, s>>>(gy, 1, W(9), 16, 512, B * 16 * 512, A + C.d1, A + C.g8a);
   // d1 (conv3 16->16 on u1); gu1 pre-activation -> g8b
-  bwd3_weight<8, false>(tc, tce, A + C.u1, 16, A + C.g8a, 16, batch, A + C.part, GW(8), GB(8), s);
-  bwd3_data<8>(tc, tce, A + C.g8a, 16, W(8), 16, A + C.u1, A + C.g8b, batch, s);
+  bwd3_weight<8, false>(tc, tce, 8, A + C.u1, 16, A + C.g8a, 16, batch, A + C.part, GW(8), GB(8), s);
+  bwd3_data<8>(tc, tce, 8, A + C.g8a, 16, W(8), 16, A + C.u1, A + C.g8b, batch, s);
   // u1 = relu(up(c1) + s1): c1 = conv1(d2, 32->16)
   g_kernel_launches += 3;
   k_up_back<<<grid_for(B * 16 * 64), kT, 0, s>>>(A + C.g8b, 8, B * 16 * 64, A + C.g4c);
@@ -938,35 +942,35 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   k_conv1_bwd_data<<<grid_for(B * 32 * 64), kT, 0, s>>>(A + C.g4c, 16, W(7), 32, 64, B * 32 * 64, A + C.d2,
                                                         A + C.g4a);
   // d2 (conv3 32->32 on u2); gu2 pre-activation -> g4b
-  bwd3_weight<4, false>(tc, tce, A + C.u2, 32, A + C.g4a, 32, batch, A + C.part, GW(6), GB(6), s);
-  bwd3_data<4>(tc, tce, A + C.g4a, 32, W(6), 32, A + C.u2, A + C.g4b, batch, s);
+  bwd3_weight<4, false>(tc, tce, 6, A + C.u2, 32, A + C.g4a, 32, batch, A + C.part, GW(6), GB(6), s);
+  bwd3_data<4>(tc, tce, 6, A + C.g4a, 32, W(6), 32, A + C.u2, A + C.g4b, batch, s);
   // u2 = relu(up(c2) + s2): c2 = conv1(bt, 64->32)
   g_kernel_launches += 3;
   k_up_back<<<grid_for(B * 32 * 8), kT, 0, s>>>(A + C.g4b, 4, B * 32 * 8, A + C.g2b);
   k_conv1_bwd_weight<kT><<<dim3(64, 32), kT, 0, s>>>(A + C.bt, 64, A + C.g2b, 32, 8, batch, GW(5), GB(5));
   k_conv1_bwd_data<<<grid_for(B * 64 * 8), kT, 0, s>>>(A + C.g2b, 32, W(5), 64, 8, B * 64 * 8, A + C.bt, A + C.g2a);
   // bt (conv3 32->64 on p2) -> gp2 (g2b, 32 channels)
-  bwd3_weight<2, false>(tc, tce, A + C.p2, 32, A + C.g2a, 64, batch, A + C.part, GW(4), GB(4), s);
-  bwd3_data<2>(tc, tce, A + C.g2a, 64, W(4), 32, nullptr, A + C.g2b, batch, s);
+  bwd3_weight<2, false>(tc, tce, 4, A + C.p2, 32, A + C.g2a, 64, batch, A + C.part, GW(4), GB(4), s);
+  bwd3_data<2>(tc, tce, 4, A + C.g2a, 64, W(4), 32, nullptr, A + C.g2b, batch, s);
   // s2 gradient: (gu2 + pool_back(gp2)) * (s2 > 0) -> g4a
   g_kernel_launches += 1;
   k_pool_back_add_mask<<<grid_for(B * 32 * 64), kT, 0, s>>>(A + C.g4b, A + C.g2b, A + C.s2, 4, B * 32 * 64,
                                                             A + C.g4a);
   // e2b (conv3 32->32 on e2a) -> ge2a (g4c)
-  bwd3_weight<4, false>(tc, tce, A + C.e2a, 32, A + C.g4a, 32, batch, A + C.part, GW(3), GB(3), s);
-  bwd3_data<4>(tc, tce, A + C.g4a, 32, W(3), 32, A + C.e2a, A + C.g4c, batch, s);
+  bwd3_weight<4, false>(tc, tce, 3, A + C.e2a, 32, A + C.g4a, 32, batch, A + C.part, GW(3), GB(3), s);
+  bwd3_data<4>(tc, tce, 3, A + C.g4a, 32, W(3), 32, A + C.e2a, A + C.g4c, batch, s);
   // e2a (conv3 16->32 on p1) -> gp1 (g4b, 16 channels)
-  bwd3_weight<4, false>(tc, tce, A + C.p1, 16, A + C.g4c, 32, batch, A + C.part, GW(2), GB(2), s);
-  bwd3_data<4>(tc, tce, A + C.g4c, 32, W(2), 16, nullptr, A + C.g4b, batch, s);
+  bwd3_weight<4, false>(tc, tce, 2, A + C.p1, 16, A + C.g4c, 32, batch, A + C.part, GW(2), GB(2), s);
+  bwd3_data<4>(tc, tce, 2, A + C.g4c, 32, W(2), 16, nullptr, A + C.g4b, batch, s);
   // s1 gradient: (gu1 + pool_back(gp1)) * (s1 > 0) -> g8a
   g_kernel_launches += 1;
   k_pool_back_add_mask<<<grid_for(B * 16 * 512), kT, 0, s>>>(A + C.g8b, A + C.g4b, A + C.s1, 8, B * 16 * 512,
                                                              A + C.g8a);
   // e1b (conv3 16->16 on e1a) -> ge1a (g8c)
-  bwd3_weight<8, false>(tc, tce, A + C.e1a, 16, A + C.g8a, 16, batch, A + C.part, GW(1), GB(1), s);
-  bwd3_data<8>(tc, tce, A + C.g8a, 16, W(1), 16, A + C.e1a, A + C.g8c, batch, s);
+  bwd3_weight<8, false>(tc, tce, 1, A + C.e1a, 16, A + C.g8a, 16, batch, A + C.part, GW(1), GB(1), s);
+  bwd3_data<8>(tc, tce, 1, A + C.g8a, 16, W(1), 16, A + C.e1a, A + C.g8c, batch, s);
   // e1a (valid conv3 2->16 on x)
-  bwd3_weight<8, true>(tc, tce, A + C.x, 2, A + C.g8c, 16, batch, A + C.part, GW(0), GB(0), s);
+  bwd3_weight<8, true>(tc, tce, 0, A + C.x, 2, A + C.g8c, 16, batch, A + C.part, GW(0), GB(0), s);
   if (tce != cudaSuccess) return tce;
   return cudaGetLastError();
 }
@@ -1211,7 +1215,7 @@ int fl_unet_set_tensor_cores(fl_unet* u, int enable) {
   int st = fl::check_device();
   if (st != FL_OK) return st;
   auto* t = new fl::UNetTcTrain();
-  if (fl::unet_tc_train_create(u->max_batch, t) != cudaSuccess) {
+  if (fl::unet_tc_train_create(t) != cudaSuccess) {
     cudaGetLastError();
     delete t;
     return FL_RESOURCE_EXHAUSTED;

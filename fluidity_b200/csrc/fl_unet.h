@@ -32,34 +32,30 @@ UNetLayout unet_layout();
 void configure_unet_kernels();
 UNetCache unet_cache_layout(int batch);
 
-// Scratch of the tensor-core training convolutions (fl_unet_train_tc.cu): the
-// cuBLAS handle, the BF16 im2col, packed-weight and gradient-row operands and
-// the FP32 GEMM result, sized for a batch of up to max_batch items.
-struct UNetTcTrain {
-  void* handle = nullptr;  // cublasHandle_t
-  __nv_bfloat16* col = nullptr;
-  __nv_bfloat16* w = nullptr;
-  __nv_bfloat16* g = nullptr;
-  float* out = nullptr;
-  float* part = nullptr;  // bias-gradient partial sums, 64 x 32
-};
-// Largest batch of the tensor-core path: its operands (at most 512 x 432 BF16
-// per item) stay below 2^31 elements, so every index is 32-bit.
-constexpr int kUNetTcMaxBatch = 8192;
-cudaError_t unet_tc_train_create(int max_batch, UNetTcTrain* t);
-void unet_tc_train_destroy(UNetTcTrain* t);
-template <int S, bool VALID>
-cudaError_t conv3_fwd_tc(UNetTcTrain& t, const float* in, int cin, const float* w, const float* bias, int cout,
-                         float* out, int batch, int relu, cudaStream_t s);
-template <int S>
-cudaError_t conv3_bwd_data_tc(UNetTcTrain& t, const float* g, int cout, const float* w, int cin, const float* act,
-                              float* din, int batch, cudaStream_t s);
-template <int S, bool VALID>
-cudaError_t conv3_bwd_weight_tc(UNetTcTrain& t, const float* in, int cin, const float* g, int cout, int batch,
-                                float* dw, float* db, cudaStream_t s);
+// Weight gradients: CTAs write partial rows (weights, then biases) into kWgradPart
+// floats of the training cache; wgrad_sum adds `rows` of them in order.
+constexpr long long kWgradPart = 1 << 21;
+void wgrad_sum(const float* part, int rows, int nw, int cout, float* dw, float* db, cudaStream_t s);
 
-// tc == nullptr: the FP32 SIMT convolutions; otherwise the 3x3x3 convolutions
-// run as BF16 tensor-core GEMMs with FP32 accumulation.
+// Tensor-core training convolutions (fl_unet_train_tc.cu): the BF16 weights,
+// packed from the parameters once per pass (forward, or data = backward). `layer`
+// is the parameter layout's layer index.
+struct UNetTcTrain {
+  __nv_bfloat16* w = nullptr;
+};
+constexpr int kUNetTcMaxBatch = 8192;  // largest batch of the tensor-core path
+cudaError_t unet_tc_train_create(UNetTcTrain* t);
+void unet_tc_train_destroy(UNetTcTrain* t);
+cudaError_t unet_tc_train_pack(const UNetTcTrain& t, const float* params, bool data, cudaStream_t s);
+cudaError_t conv3_fwd_tc(const UNetTcTrain& t, int layer, const float* in, const float* bias, float* out, int batch,
+                         cudaStream_t s);
+cudaError_t conv3_bwd_data_tc(const UNetTcTrain& t, int layer, const float* g, const float* act, float* din, int batch,
+                              cudaStream_t s);
+cudaError_t conv3_bwd_weight_tc(int layer, const float* in, const float* g, int batch, float* part, float* dw, float* db,
+                                cudaStream_t s);
+
+// tc == nullptr: the FP32 convolutions; otherwise the 3x3x3 convolutions run on
+// the tensor cores, BF16 operands with FP32 accumulation.
 cudaError_t unet_forward(const float* params, const float* x, int batch, float* cache, float* y, cudaStream_t s,
                          UNetTcTrain* tc = nullptr);
 cudaError_t unet_backward(const float* params, float* cache, const float* grad_y, int batch, float* grad_params,

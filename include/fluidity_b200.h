@@ -314,10 +314,9 @@ int fl_unet_create(int max_batch, fl_unet** out);
 int fl_unet_destroy(fl_unet* net);
 /* Training precision of fl_unet_forward / fl_unet_backward: 0 (default) the
  * FP32 convolution kernels; 1 each 3x3x3 convolution (forward, data and weight
- * gradients) as a GEMM of BF16 operands with FP32 accumulation on the tensor
- * cores (im2col operands formed by this library's kernels, the GEMM by
- * cuBLAS), parameters, activations, gradients and Adam in FP32. Enabling
- * reserves the operand buffers: FL_OUT_OF_RANGE for a workspace of more than
+ * gradients) as an implicit GEMM of BF16 operands with FP32 accumulation on the
+ * tensor cores, parameters, activations, gradients and Adam in FP32. Enabling
+ * reserves the packed weights: FL_OUT_OF_RANGE for a workspace of more than
  * 8192 items, FL_RESOURCE_EXHAUSTED if they cannot be allocated. */
 int fl_unet_set_tensor_cores(fl_unet* net, int enable);
 /* He-uniform weights from a counter-based stream (SplitMix64 of seed and index), zero biases. */

@@ -419,3 +419,35 @@ def test_fp32_convolutions_at_item_counts(batch):
         assert _rel(g[off:off + nw], g_ref[off:off + nw]) <= TOL, name
         assert _rel(g[off + nw:off + nw + nb], g_ref[off + nw:off + nw + nb]) <= TOL, name
         off += nw + nb
+
+
+@pytest.mark.parametrize("batch", [1, 3, 17, 40])
+def test_tensor_core_convolutions_at_item_counts(batch):
+    """The tensor-core forward, and the backward from the FP32 forward's cache, at item counts
+    around the items a CTA takes (2, 4, 16) and the work units of one CTA per SM, against the FP64
+    oracle at BF16 tolerances (as test_tensor_core_training_matches_oracle_at_bf16_tolerance)."""
+    import torch
+
+    rng = np.random.default_rng(batch)
+    th = _open_network(5)
+    x = _inputs(rng, batch)
+    y_ref, cache = U.forward(th, x)
+    dy = rng.normal(size=y_ref.shape)
+    g_ref = U.backward(th, cache, dy)
+    P, X, DY = _t(th), _t(x), _t(dy.reshape(batch, 512))
+    Y, G, again = torch.zeros((batch, 512), device="cuda"), torch.zeros_like(P), torch.zeros_like(P)
+    n = fb.UNet(batch)
+    n.forward(P, X, Y)
+    n.set_tensor_cores(True)
+    n.backward(P, DY, G)
+    n.backward(P, DY, again)
+    n.forward(P, X, Y)
+    torch.cuda.synchronize()
+    n.close()
+    assert torch.equal(G, again)
+    assert _rel(Y.cpu().numpy(), y_ref.reshape(batch, 512)) <= 1e-2
+    g, off = G.cpu().numpy(), 0
+    for name, nw, nb in U.layer_sizes():
+        assert _rel(g[off:off + nw], g_ref[off:off + nw]) <= 3e-2, name
+        assert _rel(g[off + nw:off + nw + nb], g_ref[off + nw:off + nw + nb]) <= 3e-2, name
+        off += nw + nb
