@@ -19,6 +19,7 @@
 #include <cstring>
 #include <map>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "../../include/fluidity_b200.h"
@@ -39,8 +40,21 @@ using namespace fl;
 
 constexpr int kStateBuffers = 4;
 
+// What the host reads back from the device.
+struct HostBlock {
+  SolverState st;
+  DeviceReport rep;
+  int nb;
+};
+
 struct fl_context {
   int device = 0;
+  // Every buffer below that is not said to be grown on demand lies in one device
+  // allocation (`slab`): an allocation and its release cost the driver up to a
+  // few hundred microseconds each, and a context has some seventy buffers.
+  void* slab = nullptr;
+  HostBlock* host = nullptr;  // pinned; plain memory in a context for the transfers alone
+  bool host_pinned = false;
   fl_grid_desc desc{};
   size_t pcap = 0;
   int lattice = 0;  // blocks in the lattice
@@ -216,6 +230,26 @@ fl_particles state_particles(fl_context* c, int which) {
   p.mass = nullptr;
   p.count = c->count;
   return p;
+}
+
+// The 15 arrays of a particle state between a buffer of `from` and one of `to`
+// floats per array. One contiguous copy where both are full; short arrays as
+// one strided copy, since 15 copies of a few microseconds each cost their
+// submissions; long ones array by array (each runs at the link's rate, from
+// pageable memory too). With the context's single allocation the 32^3 step with
+// host buffers went from 1082 to 973 us.
+cudaError_t copy_state(float* dst, size_t to, const float* src, size_t from, size_t count, cudaMemcpyKind kind,
+                       cudaStream_t s) {
+  const size_t row = sizeof(float) * count;
+  if (count == 0) return cudaSuccess;
+  if (to == count && from == count) return cudaMemcpyAsync(dst, src, 15 * row, kind, s);
+  if (row <= (4u << 20))
+    return cudaMemcpy2DAsync(dst, sizeof(float) * to, src, sizeof(float) * from, row, 15, kind, s);
+  for (size_t k = 0; k < 15; ++k) {
+    const cudaError_t e = cudaMemcpyAsync(dst + k * to, src + k * from, row, kind, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // Orders `s` after every snapshot copy of any particle buffer.
@@ -692,6 +726,8 @@ int validate_particles(const double* parts, uint64_t np, double h, bool need_mas
   return FL_OK;
 }
 
+int create_context(const fl_grid_desc* grid, uint64_t particle_capacity, bool solver, fl_context** out);
+
 struct TempContext {
   fl_context* ctx = nullptr;
   ~TempContext() {
@@ -709,7 +745,7 @@ int make_ref_context(const double origin[3], double h, const RefLayout& L, uint6
     d.solid_hi[k] = INT_MAX;
   }
   d.h = h;
-  int st = fl_context_create(&d, std::max<uint64_t>(np, 1), &tc.ctx);
+  int st = create_context(&d, std::max<uint64_t>(np, 1), false, &tc.ctx);
   if (st != FL_OK) return st;
   std::vector<int32_t> coords;
   for (auto& b : L.blocks8) {
@@ -814,6 +850,157 @@ int post_vcycle_residual(fl_context* c, const fl_pressure_options* opt, const fl
 }
 }  // namespace fl
 
+namespace {
+
+// solver = false: a context for one call of the topology, sort and transfer
+// operators (the reference-shaped operators), without the pressure solver's
+// buffers, streams and pinned memory and without snapshot fences.
+int create_context(const fl_grid_desc* grid, uint64_t particle_capacity, bool solver, fl_context** out) {
+  if (!grid || !out) return FL_INVALID_ARGUMENT;
+  *out = nullptr;
+  if (!(grid->h > 0.0) || !std::isfinite(grid->h)) return FL_INVALID_ARGUMENT;
+  for (int d = 0; d < 3; ++d)
+    if (grid->block_dim[d] <= 0 || !std::isfinite(grid->origin[d])) return FL_INVALID_ARGUMENT;
+  const long long lattice = (long long)grid->block_dim[0] * grid->block_dim[1] * grid->block_dim[2];
+  if (lattice > (1LL << 21)) return FL_RESOURCE_EXHAUSTED;
+  if (particle_capacity >= (1ULL << 31)) return FL_RESOURCE_EXHAUSTED;
+  int st = device_ready();
+  if (st != FL_OK) return st;
+  fl_context* c = new fl_context();
+  cudaGetDevice(&c->device);
+  c->desc = *grid;
+  c->pcap = std::max<uint64_t>(particle_capacity, 1);
+  c->lattice = (int)lattice;
+  const size_t cells = (size_t)lattice * kBlockCells;
+  // The slab's pieces: listed first, then placed (512-byte aligned) in one allocation.
+  std::vector<std::pair<void**, size_t>> pieces;
+  size_t total = 0;
+  auto piece = [&](auto** p, size_t bytes) {
+    pieces.emplace_back(reinterpret_cast<void**>(p), total);
+    total += (std::max<size_t>(bytes, 1) + 511) / 512 * 512;
+  };
+  auto array = [&](auto** p, size_t count) { piece(p, sizeof(**p) * count); };
+  array(&c->occ, lattice);
+  array(&c->flag, lattice);
+  array(&c->ordinal, lattice);
+  array(&c->table, lattice);
+  array(&c->coord, 3 * lattice);
+  array(&c->nbr27, 27 * lattice);
+  array(&c->nb_dev, 1);
+  array(&c->keys, c->pcap);
+  array(&c->index, c->pcap);
+  array(&c->index_alt, c->pcap);
+  array(&c->counts, cells + 1);
+  array(&c->cell_start, cells + 1);
+  c->temp_bytes = std::max(sort_temp_bytes(c->pcap, cells), (size_t)lattice * 8 + 4096);
+  piece(&c->temp, c->temp_bytes);
+  for (int b = 0; b < 2; ++b) array(&c->pbuf[b], 16 * c->pcap);
+  for (int a = 0; a < 3; ++a) {
+    array(&c->u_pred[a], cells);
+    array(&c->u_new[a], cells);
+    array(&c->fmass[a], cells);
+  }
+  array(&c->tiles, (size_t)lattice * 3 * kTileFaces);
+  array(&c->rep, 1);
+  if (solver) {
+    array(&c->type, cells);
+    array(&c->b64, cells);
+    array(&c->p64, cells);
+    array(&c->p_nat, cells);
+    array(&c->p_keep, cells);
+    array(&c->p_keep_prev, cells);
+    for (int k = 0; k < 2; ++k) {
+      array(&c->r[k], cells);
+      array(&c->d[k], cells);
+    }
+    array(&c->q, cells);
+    array(&c->e, cells);
+    array(&c->partial, 2 * (cells / 256 + 1024));
+    array(&c->st, 1);
+    // multigrid levels (x and k sized for FP32)
+    array(&c->lv_mask0, cells);
+    int maxbd = std::max(grid->block_dim[0], std::max(grid->block_dim[1], grid->block_dim[2]));
+    int L = 4;
+    while (L < 12 && dense_dim(maxbd, L - 1) > 1) ++L;
+    c->max_levels = L;
+    for (int l = 0; l < L; ++l) {
+      long long cnt;
+      if (l < 3) {
+        const int S = 8 >> l;
+        cnt = lattice * S * S * S;
+      } else {
+        cnt = 1;
+        for (int d = 0; d < 3; ++d) cnt *= dense_dim(grid->block_dim[d], l);
+      }
+      c->lv_cap[l] = cnt;
+      array(&c->lv_fluid[l], cnt);
+      for (int a = 0; a < 3; ++a) piece(&c->lv_k[l][a], sizeof(float) * cnt);
+      array(&c->lv_anchor[l], cnt);
+      array(&c->lv_diag[l], cnt);
+      piece(&c->lv_x[l], sizeof(float) * cnt);
+      array(&c->lv_b[l], cnt);
+    }
+  }
+  int e = FL_OK;
+  auto chk = [&](int v) {
+    if (v != FL_OK && e == FL_OK) e = v;
+  };
+  if (cudaMalloc(&c->slab, total) == cudaSuccess) {
+    for (auto& [p, at] : pieces) *p = static_cast<unsigned char*>(c->slab) + at;
+  } else {
+    cudaGetLastError();
+    c->slab = nullptr;
+    chk(FL_RESOURCE_EXHAUSTED);
+  }
+  if (solver) {
+    c->host_pinned = cudaMallocHost(&c->host, sizeof(HostBlock)) == cudaSuccess;
+    if (!c->host_pinned) {
+      cudaGetLastError();
+      c->host = nullptr;
+      chk(FL_RESOURCE_EXHAUSTED);
+    }
+  } else {
+    c->host = new HostBlock();
+  }
+  if (c->host != nullptr) {
+    c->nb_host = &c->host->nb;
+    c->st_host = &c->host->st;
+    c->rep_host = &c->host->rep;
+  }
+  if (cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) chk(FL_INTERNAL);
+  if (solver) {
+    if (cudaStreamCreateWithFlags(&c->work, cudaStreamNonBlocking) != cudaSuccess) chk(FL_INTERNAL);
+    if (cudaStreamCreateWithFlags(&c->cap, cudaStreamNonBlocking) != cudaSuccess) chk(FL_INTERNAL);
+    if (cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming) != cudaSuccess) chk(FL_INTERNAL);
+    if (cudaEventCreateWithFlags(&c->ev_out, cudaEventDisableTiming) != cudaSuccess) chk(FL_INTERNAL);
+    for (int b = 0; b < 2; ++b)
+      if (cudaEventCreateWithFlags(&c->fence[b], cudaEventDisableTiming) != cudaSuccess) chk(FL_INTERNAL);
+    for (int k = 0; k < 5; ++k)
+      if (cudaEventCreate(&c->phase[k]) != cudaSuccess) chk(FL_INTERNAL);
+    configure_pressure_kernels();
+  } else {
+    c->nbuf = 0;  // no buffer has a fence
+  }
+  if (e == FL_OK) {
+    cudaMemset(c->rep, 0, sizeof(DeviceReport));
+    if (solver) {
+      cudaMemset(c->st, 0, sizeof(SolverState));
+      cudaMemset(c->lv_x[0], 0, sizeof(float) * c->lv_cap[0]);
+      // dense levels: zero once so cells never written read as non-fluid
+      for (int l = 3; l < c->max_levels; ++l) cudaMemset(c->lv_fluid[l], 0, c->lv_cap[l]);
+    }
+    if (cudaDeviceSynchronize() != cudaSuccess) e = FL_INTERNAL;
+  }
+  if (e != FL_OK) {
+    fl_context_destroy(c);
+    return e;
+  }
+  *out = c;
+  return FL_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 int fl_runtime_info(int* compiled_architecture, int* device_count, int* device_major, int* device_minor) {
@@ -850,147 +1037,14 @@ int fl_copy_to_device(void* device, const void* host, uint64_t bytes) {
 }
 
 int fl_context_create(const fl_grid_desc* grid, uint64_t particle_capacity, fl_context** out) {
-  if (!grid || !out) return FL_INVALID_ARGUMENT;
-  *out = nullptr;
-  if (!(grid->h > 0.0) || !std::isfinite(grid->h)) return FL_INVALID_ARGUMENT;
-  for (int d = 0; d < 3; ++d)
-    if (grid->block_dim[d] <= 0 || !std::isfinite(grid->origin[d])) return FL_INVALID_ARGUMENT;
-  const long long lattice = (long long)grid->block_dim[0] * grid->block_dim[1] * grid->block_dim[2];
-  if (lattice > (1LL << 21)) return FL_RESOURCE_EXHAUSTED;
-  if (particle_capacity >= (1ULL << 31)) return FL_RESOURCE_EXHAUSTED;
-  int st = device_ready();
-  if (st != FL_OK) return st;
-  fl_context* c = new fl_context();
-  cudaGetDevice(&c->device);
-  c->desc = *grid;
-  c->pcap = std::max<uint64_t>(particle_capacity, 1);
-  c->lattice = (int)lattice;
-  const size_t cells = (size_t)lattice * kBlockCells;
-  int e = FL_OK;
-  auto chk = [&](int v) {
-    if (v != FL_OK && e == FL_OK) e = v;
-  };
-  chk(dalloc(&c->occ, lattice));
-  chk(dalloc(&c->flag, lattice));
-  chk(dalloc(&c->ordinal, lattice));
-  chk(dalloc(&c->table, lattice));
-  chk(dalloc(&c->coord, 3 * lattice));
-  chk(dalloc(&c->nbr27, 27 * lattice));
-  chk(dalloc(&c->nb_dev, 1));
-  chk(cudaMallocHost(&c->nb_host, sizeof(int)) == cudaSuccess ? FL_OK : FL_RESOURCE_EXHAUSTED);
-  chk(dalloc(&c->keys, c->pcap));
-  chk(dalloc(&c->index, c->pcap));
-  chk(dalloc(&c->index_alt, c->pcap));
-  chk(dalloc(&c->counts, cells + 1));
-  chk(dalloc(&c->cell_start, cells + 1));
-  c->temp_bytes = std::max(sort_temp_bytes(c->pcap, cells), (size_t)lattice * 8 + 4096);
-  chk(cudaMalloc(&c->temp, c->temp_bytes) == cudaSuccess ? FL_OK : FL_RESOURCE_EXHAUSTED);
-  for (int b = 0; b < 2; ++b) chk(dalloc(&c->pbuf[b], 16 * c->pcap));
-  for (int a = 0; a < 3; ++a) {
-    chk(dalloc(&c->u_pred[a], cells));
-    chk(dalloc(&c->u_new[a], cells));
-    chk(dalloc(&c->fmass[a], cells));
-  }
-  chk(dalloc(&c->tiles, (size_t)lattice * 3 * kTileFaces));
-  chk(dalloc(&c->type, cells));
-  chk(dalloc(&c->b64, cells));
-  chk(dalloc(&c->p64, cells));
-  chk(dalloc(&c->p_nat, cells));
-  chk(dalloc(&c->p_keep, cells));
-  chk(dalloc(&c->p_keep_prev, cells));
-  if (cudaStreamCreateWithFlags(&c->work, cudaStreamNonBlocking) != cudaSuccess) chk(FL_INTERNAL);
-  if (cudaStreamCreateWithFlags(&c->cap, cudaStreamNonBlocking) != cudaSuccess) chk(FL_INTERNAL);
-  if (cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming) != cudaSuccess) chk(FL_INTERNAL);
-  if (cudaEventCreateWithFlags(&c->ev_out, cudaEventDisableTiming) != cudaSuccess) chk(FL_INTERNAL);
-  for (int b = 0; b < 2; ++b)
-    if (cudaEventCreateWithFlags(&c->fence[b], cudaEventDisableTiming) != cudaSuccess) chk(FL_INTERNAL);
-  configure_pressure_kernels();
-  for (int k = 0; k < 2; ++k) {
-    chk(dalloc(&c->r[k], cells));
-    chk(dalloc(&c->d[k], cells));
-  }
-  chk(dalloc(&c->q, cells));
-  chk(dalloc(&c->e, cells));
-  chk(dalloc(&c->partial, 2 * (cells / 256 + 1024)));
-  chk(dalloc(&c->st, 1));
-  chk(cudaMallocHost(&c->st_host, sizeof(SolverState)) == cudaSuccess ? FL_OK : FL_RESOURCE_EXHAUSTED);
-  chk(dalloc(&c->rep, 1));
-  chk(cudaMallocHost(&c->rep_host, sizeof(DeviceReport)) == cudaSuccess ? FL_OK : FL_RESOURCE_EXHAUSTED);
-  // multigrid levels
-  chk(dalloc(&c->lv_mask0, cells));
-  int maxbd = std::max(grid->block_dim[0], std::max(grid->block_dim[1], grid->block_dim[2]));
-  int L = 4;
-  while (L < 12 && dense_dim(maxbd, L - 1) > 1) ++L;
-  c->max_levels = L;
-  for (int l = 0; l < L; ++l) {
-    long long cnt;
-    if (l < 3) {
-      const int S = 8 >> l;
-      cnt = lattice * S * S * S;
-    } else {
-      cnt = 1;
-      for (int d = 0; d < 3; ++d) cnt *= dense_dim(grid->block_dim[d], l);
-    }
-    c->lv_cap[l] = cnt;
-    chk(dalloc(&c->lv_fluid[l], cnt));
-    for (int a = 0; a < 3; ++a) chk(dalloc(reinterpret_cast<float**>(&c->lv_k[l][a]), cnt));
-    chk(dalloc(&c->lv_anchor[l], cnt));
-    chk(dalloc(&c->lv_diag[l], cnt));
-    chk(dalloc(reinterpret_cast<float**>(&c->lv_x[l]), cnt));
-    chk(dalloc(&c->lv_b[l], cnt));
-    if (l >= 3) {
-      // dense levels: zero once so cells never written read as non-fluid
-      cudaMemset(c->lv_fluid[l], 0, cnt);
-    }
-  }
-  if (cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) chk(FL_INTERNAL);
-  for (int k = 0; k < 5; ++k)
-    if (cudaEventCreate(&c->phase[k]) != cudaSuccess) chk(FL_INTERNAL);
-  if (e == FL_OK) {
-    cudaMemset(c->st, 0, sizeof(SolverState));
-    cudaMemset(c->rep, 0, sizeof(DeviceReport));
-    cudaMemset(c->lv_x[0], 0, sizeof(float) * c->lv_cap[0]);
-    if (cudaDeviceSynchronize() != cudaSuccess) e = FL_INTERNAL;
-  }
-  if (e != FL_OK) {
-    fl_context_destroy(c);
-    return e;
-  }
-  *out = c;
-  return FL_OK;
+  return create_context(grid, particle_capacity, true, out);
 }
 
 int fl_context_destroy(fl_context* c) {
   if (!c) return FL_OK;
   if (c->snapshot_queues > 0) return FL_FAILED_PRECONDITION;  // destroy its snapshot queues first
-  cudaFree(c->occ);
-  cudaFree(c->flag);
-  cudaFree(c->ordinal);
-  cudaFree(c->table);
-  cudaFree(c->coord);
-  cudaFree(c->nbr27);
-  cudaFree(c->nb_dev);
-  if (c->nb_host) cudaFreeHost(c->nb_host);
-  cudaFree(c->keys);
-  cudaFree(c->index);
-  cudaFree(c->index_alt);
-  cudaFree(c->counts);
-  cudaFree(c->cell_start);
-  cudaFree(c->temp);
   if (c->stage_stream) cudaStreamSynchronize(c->stage_stream);
-  for (int b = 0; b < kStateBuffers; ++b) cudaFree(c->pbuf[b]);
-  for (int a = 0; a < 3; ++a) {
-    cudaFree(c->u_pred[a]);
-    cudaFree(c->u_new[a]);
-    cudaFree(c->fmass[a]);
-  }
-  cudaFree(c->tiles);
-  cudaFree(c->type);
-  cudaFree(c->b64);
-  cudaFree(c->p64);
-  cudaFree(c->p_nat);
-  cudaFree(c->p_keep);
-  cudaFree(c->p_keep_prev);
+  for (int b = 2; b < kStateBuffers; ++b) cudaFree(c->pbuf[b]);  // staged inputs' (the first two are the slab's)
   if (c->fcg_exec) cudaGraphExecDestroy(c->fcg_exec);
   if (c->fcg_nn_exec) cudaGraphExecDestroy(c->fcg_nn_exec);
   cudaFree(c->nn_params);
@@ -1008,30 +1062,15 @@ int fl_context_destroy(fl_context* c) {
     if (c->staged[b]) cudaEventDestroy(c->staged[b]);
   }
   if (c->stage_stream) cudaStreamDestroy(c->stage_stream);
-  for (int k = 0; k < 2; ++k) {
-    cudaFree(c->r[k]);
-    cudaFree(c->d[k]);
-  }
-  cudaFree(c->q);
-  cudaFree(c->e);
-  cudaFree(c->partial);
-  cudaFree(c->st);
-  if (c->st_host) cudaFreeHost(c->st_host);
-  cudaFree(c->rep);
-  if (c->rep_host) cudaFreeHost(c->rep_host);
-  cudaFree(c->lv_mask0);
-  for (int l = 0; l < 12; ++l) {
-    cudaFree(c->lv_fluid[l]);
-    for (int a = 0; a < 3; ++a) cudaFree(c->lv_k[l][a]);
-    cudaFree(c->lv_anchor[l]);
-    cudaFree(c->lv_diag[l]);
-    cudaFree(c->lv_x[l]);
-    cudaFree(c->lv_b[l]);
-  }
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (int k = 0; k < 5; ++k)
     if (c->phase[k]) cudaEventDestroy(c->phase[k]);
+  cudaFree(c->slab);
+  if (c->host_pinned)
+    cudaFreeHost(c->host);
+  else
+    delete c->host;
   delete c;
   return FL_OK;
 }
@@ -1196,9 +1235,7 @@ int fl_upload_particles(fl_context* c, const float* host, uint64_t count, void* 
   c->occ_ready = false;
   FL_CUDA(cudaStreamWaitEvent(s, c->fence[b], 0));  // a snapshot copy of the buffer still in flight
   if (c->staged[b]) FL_CUDA(cudaStreamWaitEvent(s, c->staged[b], 0));  // a dropped staging copy into it
-  for (int k = 0; k < 15; ++k)
-    FL_CUDA(cudaMemcpyAsync(c->pbuf[b] + (size_t)k * c->pcap, host + (size_t)k * count, sizeof(float) * count,
-                            cudaMemcpyHostToDevice, s));
+  FL_CUDA(copy_state(c->pbuf[b], c->pcap, host, count, count, cudaMemcpyHostToDevice, s));
   return FL_OK;
 }
 
@@ -1218,9 +1255,7 @@ int fl_stage_particles(fl_context* c, const float* host, uint64_t count) {
   const int b = pick_buffer(c, (1u << c->cur) | staged_mask(c));
   cudaStream_t s = c->stage_stream;
   FL_CUDA(cudaStreamWaitEvent(s, c->fence[b], 0));
-  for (int k = 0; k < 15; ++k)
-    FL_CUDA(cudaMemcpyAsync(c->pbuf[b] + (size_t)k * c->pcap, host + (size_t)k * count, sizeof(float) * count,
-                            cudaMemcpyHostToDevice, s));
+  FL_CUDA(copy_state(c->pbuf[b], c->pcap, host, count, count, cudaMemcpyHostToDevice, s));
   FL_CUDA(cudaEventRecord(c->staged[b], s));
   c->stage_buf[c->nstage] = b;
   c->stage_count[c->nstage] = count;
@@ -1231,9 +1266,7 @@ int fl_stage_particles(fl_context* c, const float* host, uint64_t count) {
 int fl_download_particles(fl_context* c, float* host, void* stream) {
   if (!c || !host) return FL_INVALID_ARGUMENT;
   cudaStream_t s = (cudaStream_t)stream;
-  for (int k = 0; k < 15; ++k)
-    FL_CUDA(cudaMemcpyAsync(host + (size_t)k * c->count, c->pbuf[c->cur] + (size_t)k * c->pcap,
-                            sizeof(float) * c->count, cudaMemcpyDeviceToHost, s));
+  FL_CUDA(copy_state(host, c->count, c->pbuf[c->cur], c->pcap, c->count, cudaMemcpyDeviceToHost, s));
   FL_CUDA(cudaStreamSynchronize(s));
   return FL_OK;
 }

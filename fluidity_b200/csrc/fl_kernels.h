@@ -240,10 +240,10 @@ struct OwnedFaceKey {
 // call.
 struct MpScratch {
   std::vector<int> tail, head, cell_off, cell_ent, fill, parent, root, comp_of, gauges, comp_cell_off, comp_cells,
-      comp_face_off, comp_faces, host_ints;
+      comp_face_off, comp_faces;
   std::vector<int> lut;  // cell ordinal per lattice position of the cells' bounding box (-1: none), when it fits
-  std::vector<unsigned char> anchored, pinned;
-  std::vector<double> hp, hr, hd, hb, hu;
+  std::vector<unsigned char> anchored, pinned, host_in;
+  std::vector<double> host_out;
   char* arena = nullptr;
   size_t arena_bytes = 0;
   cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -466,13 +466,18 @@ int find_root(std::vector<int>& parent, int c) {
 
 }  // namespace
 
-// Device arena bytes for nc cells, nf faces, ent cell-face entries, ncomp
-// unanchored components, comp_faces component face entries.
-size_t mp_arena_bytes(size_t nc, size_t nf, size_t ent, size_t ncomp, size_t comp_faces) {
-  const size_t nd_in = 5 * nc + 6 * nf;
-  const size_t nd_work = 3 * nf + 4 * nc + nf;
+static_assert(sizeof(MpStatus) % sizeof(double) == 0, "the status follows the results in one copy");
+
+// Bytes of the arena's inputs for nc cells, nf faces, ent cell-face entries,
+// ncomp unanchored components, comp_faces component face entries.
+size_t mp_input_bytes(size_t nc, size_t nf, size_t ent, size_t ncomp, size_t comp_faces) {
   const size_t ni = 3 * nf + ent + nc + (ncomp + 1) + nc + (ncomp + 1) + comp_faces;
-  return sizeof(double) * (nd_in + nd_work) + sizeof(MpStatus) + sizeof(int) * ni + nc + 64;
+  return sizeof(double) * (5 * nc + 6 * nf) + sizeof(int) * ni + nc;
+}
+// The whole arena.
+size_t mp_arena_bytes(size_t nc, size_t nf, size_t ent, size_t ncomp, size_t comp_faces) {
+  return (mp_input_bytes(nc, nf, ent, ncomp, comp_faces) + 15) / 16 * 16 + sizeof(double) * (4 * nf + 4 * nc) +
+         sizeof(MpStatus);
 }
 
 bool MpScratch::reserve_caps() {
@@ -492,11 +497,10 @@ bool MpScratch::reserve_caps() {
     comp_cells.reserve(nc);
     comp_face_off.reserve(nc + 1);
     comp_faces.reserve(2 * nf);
-    host_ints.reserve(4 * nf + 5 * nc + 3);
+    host_in.reserve(mp_input_bytes(nc, nf, 2 * nf, nc, 2 * nf));
     anchored.reserve(nc);
     pinned.reserve(nc);
-    for (auto* v : {&hp, &hr, &hd, &hb}) v->reserve(nc);
-    hu.reserve(nf);
+    host_out.reserve(4 * nc + nf + sizeof(MpStatus) / sizeof(double));
   } catch (...) {
     return false;
   }
@@ -756,14 +760,36 @@ int mp_project(MpScratch& X, cudaStream_t stream, double h, double dt, const int
   S.dt = dt;
   S.rel_tol = rel_tol;
   S.max_iterations = max_iterations;
-  double* dp = reinterpret_cast<double*>(X.arena);
+  // The arena: the inputs (values, index lists, pins), sent as one copy, then the
+  // work arrays, then the results and the status, fetched as one copy.
+  auto& host_in = X.host_in;
+  host_in.clear();
+  auto put = [&](const void* src, size_t n) {
+    const size_t at = host_in.size();
+    const unsigned char* b = static_cast<const unsigned char*>(src);
+    host_in.insert(host_in.end(), b, b + n);
+    return X.arena + at;
+  };
+  auto put_d = [&](const double* src, size_t n) { return reinterpret_cast<const double*>(put(src, sizeof(double) * n)); };
+  auto put_i = [&](const int* src, size_t n) { return reinterpret_cast<const int*>(put(src, sizeof(int) * n)); };
+  S.cell_values = put_d(cell_values, (size_t)5 * nc);
+  S.face_values = put_d(face_values, (size_t)6 * nf);
+  S.face_kind = put_i(face_kind, nf);
+  S.tail = put_i(tail.data(), nf);
+  S.head = put_i(head.data(), nf);
+  S.cell_ent = put_i(cell_ent.data(), cell_ent.size());
+  S.root = put_i(root.data(), nc);
+  S.comp_cell_off = put_i(comp_cell_off.data(), ncomp + 1);
+  S.comp_cells = put_i(comp_cells.data(), comp_cells.size());
+  S.comp_face_off = put_i(comp_face_off.data(), ncomp + 1);
+  S.comp_faces = put_i(comp_faces.data(), comp_faces.size());
+  S.pinned = reinterpret_cast<const unsigned char*>(put(pinned.data(), nc));
+  double* dp = reinterpret_cast<double*>(X.arena + (host_in.size() + 15) / 16 * 16);
   auto take_d = [&](size_t n) {
     double* r = dp;
     dp += n;
     return r;
   };
-  double* d_cells = take_d((size_t)5 * nc);
-  double* d_faces = take_d((size_t)6 * nf);
   S.scale = take_d(nf);
   S.cond = take_d(nf);
   S.wall_face = take_d(nf);
@@ -773,63 +799,27 @@ int mp_project(MpScratch& X, cudaStream_t stream, double h, double dt, const int
   S.defect = take_d(nc);
   S.corrected_u = take_d(nf);
   S.out = reinterpret_cast<MpStatus*>(dp);
-  int* ip = reinterpret_cast<int*>(S.out + 1);
-  auto& host_ints = X.host_ints;
-  host_ints.clear();
-  auto put = [&](const int* src, size_t n) {
-    int* r = ip + host_ints.size();
-    host_ints.insert(host_ints.end(), src, src + n);
-    return r;
-  };
-  S.face_kind = put(face_kind, nf);
-  S.tail = put(tail.data(), nf);
-  S.head = put(head.data(), nf);
-  S.cell_ent = put(cell_ent.data(), cell_ent.size());
-  S.root = put(root.data(), nc);
-  S.comp_cell_off = put(comp_cell_off.data(), ncomp + 1);
-  S.comp_cells = put(comp_cells.data(), comp_cells.size());
-  S.comp_face_off = put(comp_face_off.data(), ncomp + 1);
-  S.comp_faces = put(comp_faces.data(), comp_faces.size());
-  unsigned char* d_pinned = reinterpret_cast<unsigned char*>(ip + host_ints.size());
-  S.pinned = d_pinned;
-  S.cell_values = d_cells;
-  S.face_values = d_faces;
+  auto& host_out = X.host_out;  // rhs, p, residual, defect, corrected_u, status
+  const size_t results = (size_t)4 * nc + nf;
+  host_out.resize(results + sizeof(MpStatus) / sizeof(double));
   cudaStream_t s = stream;
-  MpStatus res{};
   float ms = 0.0f;
-  bool ok = cudaMemcpyAsync(d_cells, cell_values, sizeof(double) * 5 * nc, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-            (nf == 0 || cudaMemcpyAsync(d_faces, face_values, sizeof(double) * 6 * nf, cudaMemcpyHostToDevice, s) ==
-                            cudaSuccess) &&
-            cudaMemcpyAsync(ip, host_ints.data(), sizeof(int) * host_ints.size(), cudaMemcpyHostToDevice, s) ==
-                cudaSuccess &&
-            cudaMemcpyAsync(d_pinned, pinned.data(), nc, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+  bool ok = cudaMemcpyAsync(X.arena, host_in.data(), host_in.size(), cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaEventRecord(X.e0, s) == cudaSuccess;
   if (ok) {
     ++g_kernel_launches;
     k_mac_pressure<<<kMpCtas, kMpThreads, 0, s>>>(S);
     ok = cudaGetLastError() == cudaSuccess && cudaEventRecord(X.e1, s) == cudaSuccess &&
-         cudaMemcpyAsync(&res, S.out, sizeof(MpStatus), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+         cudaMemcpyAsync(host_out.data(), S.rhs, sizeof(double) * results + sizeof(MpStatus), cudaMemcpyDeviceToHost,
+                         s) == cudaSuccess &&
          cudaStreamSynchronize(s) == cudaSuccess && cudaEventElapsedTime(&ms, X.e0, X.e1) == cudaSuccess;
-  }
-  auto &hp = X.hp, &hr = X.hr, &hd = X.hd, &hb = X.hb, &hu = X.hu;
-  if (ok && res.status == FL_OK) {
-    hp.resize(nc);
-    hr.resize(nc);
-    hd.resize(nc);
-    hb.resize(nc);
-    hu.resize(std::max(nf, 1));
-    ok = cudaMemcpyAsync(hp.data(), S.p, sizeof(double) * nc, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-         cudaMemcpyAsync(hr.data(), S.residual, sizeof(double) * nc, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-         cudaMemcpyAsync(hd.data(), S.defect, sizeof(double) * nc, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-         cudaMemcpyAsync(hb.data(), S.rhs, sizeof(double) * nc, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-         (nf == 0 || cudaMemcpyAsync(hu.data(), S.corrected_u, sizeof(double) * nf, cudaMemcpyDeviceToHost, s) ==
-                         cudaSuccess) &&
-         cudaStreamSynchronize(s) == cudaSuccess;
   }
   if (!ok) {
     cudaGetLastError();
     return FL_INTERNAL;
   }
+  MpStatus res;
+  std::memcpy(&res, host_out.data() + results, sizeof(MpStatus));
   if (diagnostics) {
     diagnostics->iterations = (uint64_t)res.iterations;
     diagnostics->true_residual_l2 = res.true_residual_l2;
@@ -843,11 +833,12 @@ int mp_project(MpScratch& X, cudaStream_t stream, double h, double dt, const int
     measurement->kernel_ms = ms;
   }
   if (res.status != FL_OK) return res.status;  // no projection is published
-  std::memcpy(pressure, hp.data(), sizeof(double) * nc);
-  std::memcpy(residual, hr.data(), sizeof(double) * nc);
-  std::memcpy(defect, hd.data(), sizeof(double) * nc);
-  std::memcpy(rhs, hb.data(), sizeof(double) * nc);
-  if (nf) std::memcpy(corrected_u, hu.data(), sizeof(double) * nf);
+  const double* r = host_out.data();
+  std::memcpy(rhs, r, sizeof(double) * nc);
+  std::memcpy(pressure, r + nc, sizeof(double) * nc);
+  std::memcpy(residual, r + 2 * nc, sizeof(double) * nc);
+  std::memcpy(defect, r + 3 * nc, sizeof(double) * nc);
+  if (nf) std::memcpy(corrected_u, r + 4 * nc, sizeof(double) * nf);
   if (gauge_ordinals)
     for (int k = 0; k < ncomp; ++k) gauge_ordinals[k] = (uint64_t)gauges[k];
   return FL_OK;
