@@ -12,7 +12,12 @@
 // memory descriptor (K-major, no swizzle) starts at that row, its 8-row groups
 // 128 bytes apart (SBO) and its two 8-channel K halves one channel group apart
 // (LBO). Rows that are pads produce garbage outputs, which the epilogue drops.
-// The block's input window (8^3 + one-cell halo) uses Px = Py = Pz = 10.
+// The block's input window (8^3 + one-cell halo) uses Px = Py = Pz = 10, and its
+// two channels would leave six of a row's eight empty, so a window row holds the
+// three x-neighbours' channels (x - 1, x, x + 1) and a (dz, dy) pair of taps is
+// one K half: the two halves of an MMA are two consecutive (dz, dy) rows, their
+// distance given as the descriptor's K-half stride, and the layer takes 5 MMAs
+// per tile instead of 27: 18 instead of 60 us at the 128^3 splash's 1.9k blocks.
 //
 // Per conv layer one persistent kernel: each CTA keeps the layer's packed
 // weights in shared memory ([tap][K chunk][K half][Cout][8]), and per block it
@@ -101,6 +106,10 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uin
                "l"(src), "r"(bytes), "r"(mbar)
                : "memory");
 }
+
+// Weight K chunks (of 16) of a layer with KG input channel groups: per tap and 16
+// channels, or for the window (KG = 1) per pair of (dz, dy) rows.
+__host__ __device__ constexpr int weight_chunks(int kg) { return kg == 1 ? 5 : 27 * (kg / 2); }
 
 // TMEM columns of one accumulator stage (a power of two, at least 32).
 __host__ __device__ constexpr int tc_cols(int used) { return used <= 32 ? 32 : (used <= 64 ? 64 : (used <= 128 ? 128 : 256)); }
@@ -194,8 +203,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
 
 // One conv layer over all blocks. IN/OUT: geometry of the input columns and of
 // the output layout (same D except for the valid first layer, whose input is
-// the 10^3 window). KG: input channel groups (1 = the 2-channel window, whose
-// second K half re-reads the first with zero weights). N: output channels.
+// the 10^3 window). KG: input channel groups (1 = the window, a (dz, dy) row of
+// taps per K half). N: output channels.
 //
 // A CTA handles blocks blockIdx.x, blockIdx.x + gridDim.x, ... through a
 // two-stage pipeline. Warp 4's first thread copies block k + 1's operand
@@ -215,7 +224,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
   constexpr int KC = KG >= 2 ? KG / 2 : 1;
   constexpr int TILES = IN.tiles;
   constexpr int NCOLS = tc_cols(TILES * N);
-  constexpr uint32_t W_BYTES = 27u * KC * 2u * N * 16u;
+  constexpr uint32_t W_BYTES = (uint32_t)weight_chunks(KG) * 2u * N * 16u;
   constexpr uint32_t A_BYTES = (uint32_t)KG * IN.rows * 16u;
   constexpr uint32_t GROUP_BYTES = (uint32_t)IN.rows * 16u;
   constexpr uint32_t IDESC = instr_desc(128, N);
@@ -289,21 +298,31 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
         // so each tap's operands are the tile's base descriptors plus constant
         // row offsets (every address stays below 256 KB: no carry out of the
         // field; the static_assert above keeps shifted rows inside the column).
-        const uint64_t a0 =
-            smem_desc(a_addr + (uint32_t)st * A_BYTES + (uint32_t)IN.r_lo * 16u, KG >= 2 ? GROUP_BYTES : 0u, 128u);
         const uint64_t b0 = smem_desc(w_addr, N * 16u, 128u);
+        const uint32_t a_row = a_addr + (uint32_t)st * A_BYTES + (uint32_t)IN.r_lo * 16u;
 #pragma unroll 1
         for (int t = 0; t < TILES; ++t) {
-          const uint64_t at = a0 + (uint64_t)(128 * t);
           const uint32_t dt = tmem + (uint32_t)(st * NCOLS + t * N);
+          if constexpr (KG == 1) {
 #pragma unroll
-          for (int tap = 0; tap < 27; ++tap) {
-            const int shift = ((tap / 9 - 1) * IN.Py + ((tap / 3) % 3 - 1)) * IN.Px + (tap % 3 - 1);
+            for (int p = 0; p < 5; ++p) {  // rows 2p and 2p + 1 of the nine (dz, dy); row 9 has zero weights
+              const int r = 2 * p, next = r < 8 ? r + 1 : r;
+              const int shift = ((r / 3 - 1) * IN.Py + (r % 3 - 1)) * IN.Px;
+              const int step = ((next / 3 - 1) * IN.Py + (next % 3 - 1)) * IN.Px - shift;
+              const uint64_t ad = smem_desc(a_row, (uint32_t)step * 16u, 128u) + (uint64_t)(int64_t)(128 * t + shift);
+              mma_bf16(dt, ad, b0 + (uint64_t)(p * 2 * N), IDESC, p != 0 ? 1u : 0u);
+            }
+          } else {
+            const uint64_t at = smem_desc(a_row, GROUP_BYTES, 128u) + (uint64_t)(128 * t);
 #pragma unroll
-            for (int kc = 0; kc < KC; ++kc) {
-              const uint64_t ad = at + (uint64_t)(int64_t)(shift + 2 * kc * IN.rows);
-              const uint64_t bd = b0 + (uint64_t)((tap * KC + kc) * 2 * N);
-              mma_bf16(dt, ad, bd, IDESC, (tap | kc) != 0 ? 1u : 0u);
+            for (int tap = 0; tap < 27; ++tap) {
+              const int shift = ((tap / 9 - 1) * IN.Py + ((tap / 3) % 3 - 1)) * IN.Px + (tap % 3 - 1);
+#pragma unroll
+              for (int kc = 0; kc < KC; ++kc) {
+                const uint64_t ad = at + (uint64_t)(int64_t)(shift + 2 * kc * IN.rows);
+                const uint64_t bd = b0 + (uint64_t)((tap * KC + kc) * 2 * N);
+                mma_bf16(dt, ad, bd, IDESC, (tap | kc) != 0 ? 1u : 0u);
+              }
             }
           }
         }
@@ -385,8 +404,10 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * NCOLS)));
 }
 
-// Input window of block b in the 10^3 layout (one channel group: residual / s,
-// cell mask, six zero channels) and the block scale s (max |residual| over the window).
+// Input window of block b in the 10^3 layout (one channel group: residual / s and
+// cell mask of the cells x - 1, x and x + 1, two zero channels; the rows at the
+// window's x ends, whose neighbours are another line's, are never a tap's centre)
+// and the block scale s (max |residual| over the window).
 // z_zero (not null when the network's output replaces z): a block whose window
 // holds no residual is skipped by every layer, so its correction, zero, is
 // written here.
@@ -396,6 +417,7 @@ __global__ void __launch_bounds__(512) k_tc_gather(GridView g, const float* __re
                                                    float* __restrict__ scale, T* __restrict__ z_zero) {
   constexpr PadGeom W = geom10();
   __shared__ float red[16];
+  __shared__ float2 win[1002];  // (residual, mask) of the window, one entry of margin at each end
   const int b = blockIdx.x;
   float rv[2], mv[2], mx = 0.0f;
 #pragma unroll
@@ -427,12 +449,20 @@ __global__ void __launch_bounds__(512) k_tc_gather(GridView g, const float* __re
 #pragma unroll
   for (int k = 0; k < 16; ++k) sc = fmaxf(sc, red[k]);
   if (sc == 0.0f && z_zero != nullptr) z_zero[(size_t)b * 512 + threadIdx.x] = static_cast<T>(0.0f);
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int i = threadIdx.x + 512 * k;
+    if (i < 1000) win[i + 1] = make_float2(sc > 0.0f ? rv[k] / sc : 0.0f, mv[k]);
+  }
+  if (threadIdx.x < 2) win[threadIdx.x * 1001] = make_float2(0.0f, 0.0f);
+  __syncthreads();
   uint4* dst = x + (size_t)b * W.rows;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const int i = threadIdx.x + 512 * k;
-    if (i < 1000) {  // window row (hz+1, hy+1, hx+1) == i in the 10^3 layout
-      float v[8] = {sc > 0.0f ? rv[k] / sc : 0.0f, mv[k], 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (i < 1000) {  // window row (hz+1, hy+1, hx+1) == i in the 10^3 layout: its cell and the two beside it in x
+      const float2 lo = win[i], at = win[i + 1], hi = win[i + 2];
+      const float v[8] = {lo.x, lo.y, at.x, at.y, hi.x, hi.y, 0.f, 0.f};
       dst[i] = pack8(v);
     }
   }
@@ -542,16 +572,23 @@ __global__ void __launch_bounds__(256) k_tc_upadd1(const uint4* __restrict__ d2,
 }
 
 // Packs one FP32 conv layer (w[co][ci][27]) into [27][kc][2][cout][8] BF16 with
-// input channels padded to 16 * kc (zeros).
+// input channels padded to 16 * kc (zeros); the first layer (two channels) into
+// [5][2][cout][8]: K half h of chunk p is (dz, dy) row 2p + h, channel 2 dx + ci.
 __global__ void k_pack_conv(const float* __restrict__ w, int cin, int cout, int kc, __nv_bfloat16* __restrict__ out) {
-  const int total = 27 * kc * 2 * cout * 8;
+  const int total = (cin == 2 ? 5 : 27 * kc) * 2 * cout * 8;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int j = i & 7;
     const int n = (i >> 3) % cout;
     const int kh = (i / (8 * cout)) & 1;
-    const int k = (i / (16 * cout)) % kc;
-    const int tap = i / (16 * cout * kc);
-    const int ci = k * 16 + kh * 8 + j;
+    int ci, tap;
+    if (cin == 2) {
+      const int row = 2 * (i / (16 * cout)) + kh;
+      ci = row < 9 && j < 6 ? j & 1 : cin;
+      tap = row * 3 + (j >> 1);
+    } else {
+      ci = (i / (16 * cout)) % kc * 16 + kh * 8 + j;
+      tap = i / (16 * cout * kc);
+    }
     out[i] = __float2bfloat16_rn(ci < cin ? w[((size_t)n * cin + ci) * 27 + tap] : 0.0f);
   }
 }
@@ -567,8 +604,7 @@ constexpr int conv_ctas_per_sm() {
 template <int KG, int N, int MODE, int IN_KIND, int OUT_KIND>
 constexpr size_t conv_smem() {
   constexpr PadGeom IN = IN_KIND == 10 ? geom10() : (IN_KIND == 8 ? geom8() : (IN_KIND == 4 ? geom4() : geom2()));
-  constexpr int KC = KG >= 2 ? KG / 2 : 1;
-  constexpr size_t bytes = 27u * KC * 2u * N * 16u + 2u * (size_t)KG * IN.rows * 16u + 9 * 8 + 8;
+  constexpr size_t bytes = (size_t)weight_chunks(KG) * 2u * N * 16u + 2u * (size_t)KG * IN.rows * 16u + 9 * 8 + 8;
   // Ask for enough shared memory that one more CTA than the TMEM allows does
   // not fit the SM (228 KB, 1 KB reserved per CTA), so no TMEM allocation
   // waits for another CTA's release.
@@ -621,7 +657,7 @@ UNetTcLayout unet_tc_layout() {
   for (int k = 0; k < 7; ++k) {
     const int kc = cin[k] >= 32 ? 2 : 1;
     L.w_off[k] = w;
-    w += 27ll * kc * 2 * cout[k] * 8;
+    w += (cin[k] == 2 ? 5ll : 27ll * kc) * 2 * cout[k] * 8;
   }
   L.w_total = w;
   return L;
