@@ -497,13 +497,16 @@ __global__ void k_tc_pool(const uint4* __restrict__ in, uint4* __restrict__ out,
 }
 
 // u2 = relu(up(W_u2 bt + b_u2) + s2) at 4^3 (32 channels): one CTA per block,
-// bt is [8 cells][64] FP32, s2 and u2 are 4-group padded 4^3 columns.
+// bt is [8 cells][64] FP32, s2 and u2 are 4-group padded 4^3 columns. Bound by
+// shared-memory accesses: with unpadded weight rows (32-way conflicts of the
+// transposing stores) it took 26 us at 1.9k blocks, now 15.
 __global__ void __launch_bounds__(256) k_tc_upadd2(const float* __restrict__ bt, const uint4* __restrict__ s2,
                                                    const float* __restrict__ w, const float* __restrict__ bias,
                                                    uint4* __restrict__ u2) {
   constexpr PadGeom L = geom4();
   __shared__ float c2[8][32];
-  __shared__ float wt[64][32];  // the 1x1 weights transposed: a warp's 32 output channels read one row
+  __shared__ float wt[64][33];  // the 1x1 weights transposed: a warp's 32 output channels read one row (padded:
+                                // the transposing stores of a warp go down a column)
   __shared__ float in[8][64];
   const int b = blockIdx.x;
   for (int i = threadIdx.x; i < 64 * 32; i += 256) wt[i & 63][i >> 6] = __ldg(&w[i]);  // w[co][ci], coalesced
@@ -537,37 +540,53 @@ __global__ void __launch_bounds__(256) k_tc_upadd1(const uint4* __restrict__ d2,
   constexpr PadGeom L4 = geom4();
   constexpr PadGeom L8 = geom8();
   __shared__ float din[64][33];
-  __shared__ float c1[64][16];
-  __shared__ float wt[32][16];  // the 1x1 weights transposed (w[co][ci] -> wt[ci][co])
+  __shared__ __align__(16) float c1[64][16];
+  __shared__ __align__(16) float wt[32][20];  // the 1x1 weights transposed (w[co][ci] -> wt[ci][co]), rows padded
   const int b = blockIdx.x;
+  // s1 does not depend on the 1x1 layer: in flight while it is formed
+  uint4 skip[4];
+  size_t idx[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = threadIdx.x + 256 * k, gi = i & 1, c = i >> 1;
+    idx[k] = (size_t)b * 2 * L8.rows + (size_t)gi * L8.rows + pad_row(L8, c & 7, (c >> 3) & 7, c >> 6);
+    skip[k] = s1[idx[k]];
+  }
   for (int i = threadIdx.x; i < 16 * 32; i += 256) wt[i & 31][i >> 5] = __ldg(&w[i]);
-  for (int i = threadIdx.x; i < 64 * 4; i += 256) {
-    const int gi = i & 3, c = i >> 2;
-    const int x = c & 3, y = (c >> 2) & 3, z = c >> 4;
+  {
+    const int gi = threadIdx.x & 3, c = threadIdx.x >> 2;
     float v[8];
-    unpack8(d2[(size_t)b * 4 * L4.rows + (size_t)gi * L4.rows + pad_row(L4, x, y, z)], v);
+    unpack8(d2[(size_t)b * 4 * L4.rows + (size_t)gi * L4.rows + pad_row(L4, c & 3, (c >> 2) & 3, c >> 4)], v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) din[c][8 * gi + j] = v[j];
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-    const int co = i & 15, c = i >> 4;
-    float acc = bias[co];
+  {  // four output channels of one cell per thread: one input and one 16-byte weight load serve four FMAs
+    const int q = threadIdx.x & 3, c = threadIdx.x >> 2;
+    float acc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = bias[4 * q + k];
 #pragma unroll 8
-    for (int ci = 0; ci < 32; ++ci) acc = fmaf(wt[ci][co], din[c][ci], acc);
-    c1[c][co] = acc;
+    for (int ci = 0; ci < 32; ++ci) {
+      const float v = din[c][ci];
+      const float4 wv = *reinterpret_cast<const float4*>(&wt[ci][4 * q]);
+      acc[0] = fmaf(wv.x, v, acc[0]);
+      acc[1] = fmaf(wv.y, v, acc[1]);
+      acc[2] = fmaf(wv.z, v, acc[2]);
+      acc[3] = fmaf(wv.w, v, acc[3]);
+    }
+    *reinterpret_cast<float4*>(&c1[c][4 * q]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 512 * 2; i += 256) {
-    const int gi = i & 1, c = i >> 1;
-    const int x = c & 7, y = (c >> 3) & 7, z = c >> 6;
-    const int parent = ((z >> 1) * 4 + (y >> 1)) * 4 + (x >> 1);
-    const size_t idx = (size_t)b * 2 * L8.rows + (size_t)gi * L8.rows + pad_row(L8, x, y, z);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = threadIdx.x + 256 * k, gi = i & 1, c = i >> 1;
+    const int parent = ((c >> 7) * 4 + ((c >> 4) & 3)) * 4 + ((c >> 1) & 3);
     float v[8];
-    unpack8(s1[idx], v);
+    unpack8(skip[k], v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j] + c1[parent][8 * gi + j], 0.0f);
-    u1[idx] = pack8(v);
+    u1[idx[k]] = pack8(v);
   }
 }
 
