@@ -46,12 +46,12 @@ constexpr int kT = 256;
 // W[o][i][tap] = w[i][o][26 - tap]. Bound by the FP32 pipe once the loads are
 // amortised: a thread owns four x-adjacent cells and kCo output channels, so
 // one input row (a 16- and an 8-byte shared load) serves 3 taps x 4 cells x
-// kCo channels in packed FMAs (channel pairs). At 45 items a 4^3 layer
-// of 32 to 32 channels takes 23 us (26 us its data gradient) and an 8^3 layer of
-// 16 to 16 24 us (23 us); one thread per output, with an input and a weight load
-// per FMA, took 160 (127) and 152 (130) us. Staging is most of what is left.
-// One CTA of 128 threads per item, slab of kZ output planes and 16 output
-// channels; the slab's zero-padded input (rows padded to a multiple of four
+// kCo channels in packed FMAs (channel pairs). A training step of 45
+// items takes 549 us; with one output per thread and an input and a weight load
+// per FMA it took 1821, with one group of 128 threads per CTA here and at most one
+// CTA per SM in the weight gradients 629. Staging is most of what is left.
+// One CTA per item, slab of kZ output planes and 16 output channels, two groups
+// of 128 threads each taking half of the input channels; the slab's zero-padded input (rows padded to a multiple of four
 // words, planes so that the eight lanes of a 16-byte access touch all banks)
 // and the 16 channels' weights ([input channel][tap][channel]) are staged in
 // shared memory. Sums run over input channels, then taps in ascending order.
@@ -62,12 +62,18 @@ struct ConvTile {
   static constexpr int kRow = S == 8 ? 12 : 8;
   static constexpr int kPlane = S == 8 ? 10 * 12 : 6 * 8 + 4;
   static constexpr int kChannel = (kZ + 2) * kPlane;
-  static constexpr size_t smem(int cin) { return sizeof(float) * cin * (kChannel + 27 * kConvW); }
+  // (at least what the exchange of the two groups' sums needs)
+  static constexpr size_t smem(int cin) {
+    const size_t staged = sizeof(float) * cin * (kChannel + 27 * kConvW), sums = sizeof(float) * 128 * 4 * kCo;
+    return staged > sums ? staged : sums;
+  }
   static constexpr int kConvW = 20;  // words per (channel, tap): 16 weights, padded against store conflicts
 };
 
+constexpr int kConvThreads = 256;
+
 template <int S, bool VALID, bool DATA>
-__global__ void __launch_bounds__(128) k_conv3(const float* __restrict__ in, int cin, const float* __restrict__ w,
+__global__ void __launch_bounds__(kConvThreads) k_conv3(const float* __restrict__ in, int cin, const float* __restrict__ w,
                                                const float* __restrict__ bias, int cout, float* __restrict__ out,
                                                int relu, const float* __restrict__ act) {
   using T = ConvTile<S>;
@@ -76,10 +82,11 @@ __global__ void __launch_bounds__(128) k_conv3(const float* __restrict__ in, int
   extern __shared__ __align__(16) float conv_smem[];
   float* tile = conv_smem;
   float* wt = tile + cin * T::kChannel;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int t = threadIdx.x, lane = t & 31, warp = (t >> 5) & 3, half = t >> 7;
   const int b = blockIdx.x / kSlabs, z0 = (blockIdx.x % kSlabs) * T::kZ, co0 = blockIdx.y * 16;
   const float* src = in + (size_t)b * cin * EIN3;
-  for (int i = t; i < cin * kCells; i += 128) {
+#pragma unroll 4
+  for (int i = t; i < cin * kCells; i += kConvThreads) {
     const int ci = i / kCells, r = i % kCells;
     const int pz = r / (E * E), py = (r / E) % E, px = r % E;
     const int z = z0 + pz - OFF, y = py - OFF, x = px - OFF;
@@ -88,12 +95,14 @@ __global__ void __launch_bounds__(128) k_conv3(const float* __restrict__ in, int
     tile[ci * T::kChannel + pz * T::kPlane + py * T::kRow + px] = v;
   }
   if (DATA) {  // in channel i = a layer output, the 16 layer inputs co0 .. co0 + 15 contiguous in w[i]
-    for (int e = t; e < cin * 16 * 27; e += 128) {
+#pragma unroll 4
+    for (int e = t; e < cin * 16 * 27; e += kConvThreads) {
       const int i = e / (16 * 27), r = e % (16 * 27), o = r / 27, tap = r % 27;
       wt[(i * 27 + 26 - tap) * T::kConvW + o] = w[((size_t)i * cout + co0 + o) * 27 + tap];
     }
   } else {
-    for (int e = t; e < 16 * cin * 27; e += 128) {
+#pragma unroll 4
+    for (int e = t; e < 16 * cin * 27; e += kConvThreads) {
       const int o = e / (cin * 27), r = e % (cin * 27);
       wt[r * T::kConvW + o] = w[(size_t)(co0 + o) * cin * 27 + r];
     }
@@ -108,9 +117,10 @@ __global__ void __launch_bounds__(128) k_conv3(const float* __restrict__ in, int
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int h = 0; h < T::kCo / 2; ++h)
-      acc[c][h] = DATA ? make_float2(0.0f, 0.0f)
-                       : make_float2(__ldg(&bias[co0 + co + 2 * h]), __ldg(&bias[co0 + co + 2 * h + 1]));
-  for (int ci = 0; ci < cin; ++ci) {
+      acc[c][h] = DATA || half != 0
+                      ? make_float2(0.0f, 0.0f)
+                      : make_float2(__ldg(&bias[co0 + co + 2 * h]), __ldg(&bias[co0 + co + 2 * h + 1]));
+  for (int ci = half * (cin / 2); ci < (half + 1) * (cin / 2); ++ci) {
     const float* base = tile + ci * T::kChannel + z * T::kPlane + y * T::kRow + x0;
     const float* wc = wt + ci * 27 * T::kConvW + co;
 #pragma unroll
@@ -139,6 +149,20 @@ __global__ void __launch_bounds__(128) k_conv3(const float* __restrict__ in, int
         }
       }
   }
+  // the second group's sums, added by the first (through the tile's shared memory)
+  __syncthreads();
+  float2* other = reinterpret_cast<float2*>(tile) + (t & 127);
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int h = 0; h < T::kCo / 2; ++h)
+      if (half != 0) other[(c * (T::kCo / 2) + h) * 128] = acc[c][h];
+  __syncthreads();
+  if (half != 0) return;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int h = 0; h < T::kCo / 2; ++h) acc[c][h] = __fadd2_rn(acc[c][h], other[(c * (T::kCo / 2) + h) * 128]);
 #pragma unroll
   for (int k = 0; k < T::kCo; ++k) {
     const size_t o = ((size_t)b * cout + co0 + co + k) * S3 + ((z0 + z) * S + y) * S + x0;
@@ -284,9 +308,7 @@ __global__ void k_up_add_relu(const float* __restrict__ coarse, const float* __r
 //   dw[co][ci][tap] = sum_b sum_o g[b][co][o] in[b][ci][o + tap - pad], db[co] = sum_b sum_o g[b][co][o].
 // A thread owns one input channel, one (dz, dy) and eight output channels: per
 // cell one input value (three kept for the dx taps) and two broadcast 16-byte
-// loads of g (staged [cell][channel]) feed 12 packed FMAs. An 8^3
-// layer of 16 to 16 channels takes 33 us at 45 items; a CTA per channel pair
-// reading both operands from global memory took 102 us.
+// loads of g (staged [cell][channel]) feed 12 packed FMAs.
 // Work units (an item's slab of two planes at 8^3, an item at 4^3, four items
 // at 2^3) are dealt to gridDim.x CTAs in order and each CTA writes one partial
 // row; k_wgrad_sum adds the rows in order, so the result is reproducible.
@@ -731,7 +753,7 @@ void conv3_fwd(const float* in, int cin, const float* w, const float* bias, int 
     k_conv3_2<false><<<dim3((batch + 31) / 32, cout / 8), 256, conv2_smem(cin), s>>>(in, cin, w, bias, cout, batch, out,
                                                                                      relu, nullptr);
   else
-    k_conv3<S, VALID, false><<<dim3(batch * (S / ConvTile<S>::kZ), cout / 16), 128, ConvTile<S>::smem(cin), s>>>(
+    k_conv3<S, VALID, false><<<dim3(batch * (S / ConvTile<S>::kZ), cout / 16), kConvThreads, ConvTile<S>::smem(cin), s>>>(
         in, cin, w, bias, cout, out, relu, nullptr);
 }
 
@@ -744,7 +766,7 @@ void conv3_bwd_data(const float* g, int cout, const float* w, int cin, const flo
     k_conv3_2<true><<<dim3((batch + 31) / 32, cin / 8), 256, conv2_smem(cout), s>>>(g, cout, w, nullptr, cin, batch,
                                                                                     din, 0, act);
   else
-    k_conv3<S, false, true><<<dim3(batch * (S / ConvTile<S>::kZ), cin / 16), 128, ConvTile<S>::smem(cout), s>>>(
+    k_conv3<S, false, true><<<dim3(batch * (S / ConvTile<S>::kZ), cin / 16), kConvThreads, ConvTile<S>::smem(cout), s>>>(
         g, cout, w, nullptr, cin, din, 0, act);
 }
 
@@ -753,8 +775,8 @@ void wgrad(const float* in, const float* g, int cout, int batch, float* part, fl
   using T = WgradTile<S, VALID, CIN>;
   const int nw = cout * CIN * 27;
   const int units = (batch + T::kItems - 1) / T::kItems * T::kSlabs;
-  // one CTA per SM where the units and the partial rows' space allow it
-  const int ctas = (int)std::min<long long>({(long long)units, 148, kWgradPart / ((long long)T::kSplit * (nw + cout))});
+  // two CTAs per SM where the units and the partial rows' space allow it
+  const int ctas = (int)std::min<long long>({(long long)units, 2 * 148, kWgradPart / ((long long)T::kSplit * (nw + cout))});
   ++g_kernel_launches;
   k_conv3_wgrad<S, VALID, CIN><<<dim3(ctas, cout / 16), T::kThreads, T::kSmem, s>>>(in, g, cout, batch, units, part);
   wgrad_sum(part, ctas * T::kSplit, nw, cout, dw, db, s);

@@ -15,8 +15,10 @@
 // operands and by launch latency, so warp-level MMAs (m16n8k16), which read
 // their operands from where they were staged and need no tensor-memory
 // allocation or epilogue copy, are enough to take the matrix work off the
-// critical path. A training step of 64 items takes 494 us; with im2col operands
-// written to memory and library GEMMs between them (92 + 20 launches) it took 664.
+// critical path. A training step of 64 items takes 429 us; with im2col operands
+// written to memory and library GEMMs between them (92 + 20 launches) it took 664,
+// with up to 32 channels per CTA and several items per weight-gradient unit (so 8
+// to 64 CTAs a layer) 494.
 // Bias, ReLU and the ReLU mask are applied in the epilogue. Sums and every
 // result are FP32, as are the parameters and Adam's state; every reduction has a
 // fixed order. The FP32 kernels of fl_unet.cu remain the exact path.
@@ -140,6 +142,7 @@ template <int S, bool VALID, int CIN, int ITEMS, int Z, int THREADS>
 __device__ __forceinline__ void stage(const float* __restrict__ in, int b0, int z0, int batch, __nv_bfloat16* tile) {
   using T = Tile<S, CIN, ITEMS, Z>;
   constexpr int EIN = VALID ? S + 2 : S, EIN3 = EIN * EIN * EIN, OFF = VALID ? 0 : 1, HC = CIN / 2;
+#pragma unroll 4
   for (int i = threadIdx.x; i < ITEMS * T::kPos * HC; i += THREADS) {
     const int p = i % (ITEMS * T::kPos), c = i / (ITEMS * T::kPos), item = p / T::kPos, r = p % T::kPos;
     const int z = z0 + r / (T::E * T::E) - OFF, y = (r / T::E) % T::E - OFF, x = r % T::E - OFF;
@@ -158,16 +161,18 @@ __device__ __forceinline__ void stage(const float* __restrict__ in, int b0, int 
 template <int S>
 struct ConvShape {
   static constexpr int kItems = S == 2 ? 4 : 1, kZ = S == 8 ? 4 : S;
+  static constexpr int kCo = S == 2 ? 32 : 16;  // output channels of one CTA
   static constexpr int kWm = S == 8 ? 8 : (S == 4 ? 4 : 2), kWn = 8 / kWm;  // warps over rows and channels
   static constexpr int kMw = S == 8 ? 2 : 1;                               // 16-row tiles per warp
 };
-template <int S, int CIN, int COUT>
+template <int S, int CIN>
 constexpr size_t conv_smem() {
   using T = Tile<S, CIN, ConvShape<S>::kItems, ConvShape<S>::kZ>;
-  return T::kBytes + sizeof(__nv_bfloat16) * (CIN == 2 ? 32 * COUT * 2 : 27 * COUT * (CIN + 8));
+  constexpr int kCo = ConvShape<S>::kCo;
+  return T::kBytes + sizeof(__nv_bfloat16) * (CIN == 2 ? 32 * kCo * 2 : 27 * kCo * (CIN + 8));
 }
 
-// One CTA: kItems items' slab of kZ planes, all COUT channels. The epilogue adds
+// One CTA: kItems items' slab of kZ planes, kCo of the COUT channels. The epilogue adds
 // the bias and applies the ReLU (forward), or the ReLU mask of `act` (data gradient).
 template <int S, bool VALID, int CIN, int COUT, bool DATA>
 __global__ void __launch_bounds__(kConvThreads)
@@ -175,7 +180,8 @@ __global__ void __launch_bounds__(kConvThreads)
                float* __restrict__ out, int batch, int relu, const float* __restrict__ act) {
   using C = ConvShape<S>;
   using T = Tile<S, CIN, C::kItems, C::kZ>;
-  constexpr int kSlabs = S / C::kZ, S3 = S * S * S, kNw = COUT / 8 / C::kWn;
+  constexpr int kSlabs = S / C::kZ, S3 = S * S * S, kNw = C::kCo / 8 / C::kWn;
+  const int co0 = blockIdx.y * C::kCo;
   constexpr int kW = CIN + 8;  // BF16 per (tap, output channel) row
   extern __shared__ __align__(16) unsigned char conv_bytes[];
   __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(conv_bytes);
@@ -183,12 +189,17 @@ __global__ void __launch_bounds__(kConvThreads)
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, wm = warp % C::kWm, wn = warp / C::kWm;
   const int b0 = blockIdx.x / kSlabs * C::kItems, z0 = (blockIdx.x % kSlabs) * C::kZ;
   if constexpr (CIN == 2) {
+    static_assert(CIN != 2 || COUT == C::kCo, "the first layer's channels are one CTA's");
     for (int i = t; i < 32 * COUT * 2 / 8; i += kConvThreads)
       reinterpret_cast<uint4*>(wt)[i] = reinterpret_cast<const uint4*>(w)[i];
   } else {
     constexpr int kChunks = CIN / 8;
-    for (int i = t; i < 27 * COUT * kChunks; i += kConvThreads)
-      *reinterpret_cast<uint4*>(wt + (i / kChunks) * kW + (i % kChunks) * 8) = reinterpret_cast<const uint4*>(w)[i];
+#pragma unroll 4
+    for (int i = t; i < 27 * C::kCo * kChunks; i += kConvThreads) {
+      const int row = i / kChunks, tap = row / C::kCo, o = row % C::kCo;
+      *reinterpret_cast<uint4*>(wt + row * kW + (i % kChunks) * 8) =
+          reinterpret_cast<const uint4*>(w)[(tap * COUT + co0 + o) * kChunks + i % kChunks];
+    }
   }
   stage<S, VALID, CIN, C::kItems, C::kZ, kConvThreads>(in, b0, z0, batch, tile);
   __syncthreads();
@@ -241,7 +252,7 @@ __global__ void __launch_bounds__(kConvThreads)
       for (int c = 0; c < CIN / 16; ++c) {
         unsigned b[(kNw + 1) / 2][4];
 #pragma unroll
-        for (int n = 0; n < (kNw + 1) / 2; ++n) ldsm4(b[n], brow + 2 * ((tap * COUT + 16 * n) * kW + 16 * c));
+        for (int n = 0; n < (kNw + 1) / 2; ++n) ldsm4(b[n], brow + 2 * ((tap * C::kCo + 16 * n) * kW + 16 * c));
 #pragma unroll
         for (int m = 0; m < C::kMw; ++m) {
           unsigned a[4];
@@ -264,7 +275,7 @@ __global__ void __launch_bounds__(kConvThreads)
       for (int n = 0; n < kNw; ++n)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          const int co = (wn * kNw + n) * 8 + 2 * q + k;
+          const int co = co0 + (wn * kNw + n) * 8 + 2 * q + k;
           const size_t o = ((size_t)(b0 + item) * COUT + co) * S3 + r;
           float v = acc[m][n][2 * h + k];
           if (DATA) {
@@ -282,8 +293,8 @@ __global__ void __launch_bounds__(kConvThreads)
 
 template <int S, int CIN, int COUT>
 struct WgradShape {
-  static constexpr int kItems = S == 8 ? 1 : (S == 4 ? 2 : 16), kZ = S == 8 ? 4 : S;
-  static constexpr int kCo = COUT < 32 ? COUT : 32;  // output channels of one CTA
+  static constexpr int kItems = S == 2 ? 4 : 1, kZ = S == 8 ? 4 : S;
+  static constexpr int kCo = 16;  // output channels of one CTA
   using T = Tile<S, CIN, kItems, kZ>;
   static constexpr int kG = T::kCells + 8;  // BF16 per row of g
   static constexpr size_t kSmem = T::kBytes + sizeof(__nv_bfloat16) * kCo * kG;
@@ -399,9 +410,9 @@ template <int S, bool VALID, int CIN, int COUT>
 cudaError_t conv(const UNetTcTrain& t, int layer, bool data, const float* in, const float* bias, float* out, int batch,
                  int relu, const float* act, cudaStream_t s) {
   using C = ConvShape<S>;
-  constexpr size_t smem = conv_smem<S, CIN, COUT>();
+  constexpr size_t smem = conv_smem<S, CIN>();
   const PackLayer p = pack_table().l[pack_index(layer)];
-  const unsigned grid = (unsigned)((batch + C::kItems - 1) / C::kItems * (S / C::kZ));
+  const dim3 grid((unsigned)((batch + C::kItems - 1) / C::kItems * (S / C::kZ)), COUT / C::kCo);
   ++g_kernel_launches;
   static unsigned long long configured[2] = {0, 0};
   if constexpr (VALID) {
