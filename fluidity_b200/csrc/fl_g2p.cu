@@ -25,20 +25,24 @@ constexpr int kG2PThreads = 256;
 __device__ __forceinline__ int tile_ext0(int a) { return a == 0 ? 11 : 10; }
 __device__ __forceinline__ int tile_ext1(int a) { return a == 1 ? 11 : 10; }
 
+// Entry n of the block's three halo tiles in the owned-face arrays (its component
+// in *a), or -1 where no active block owns the face.
+__device__ __forceinline__ long long tile_source(const GridView& g, int b, int n, int* a) {
+  *a = n / kTileFaces;
+  const int idx = n % kTileFaces;
+  const int e0 = tile_ext0(*a), e1 = tile_ext1(*a);
+  const int nx = idx % e0 - 1, ny = (idx / e0) % e1 - 1, nz = idx / (e0 * e1) - 1;
+  const int dx = nx < 0 ? -1 : (nx > 7 ? 1 : 0), dy = ny < 0 ? -1 : (ny > 7 ? 1 : 0),
+            dz = nz < 0 ? -1 : (nz > 7 ? 1 : 0);
+  const int nb = g.nbr27[b * 27 + nbr_index(dx, dy, dz)];
+  return nb < 0 ? -1 : (long long)nb * kBlockCells + ((nz - 8 * dz) * 8 + (ny - 8 * dy)) * 8 + (nx - 8 * dx);
+}
+
 __device__ void load_tile(const GridView& g, int b, const float* const u[3], float* tile, int t) {
   for (int n = t; n < 3 * kTileFaces; n += kG2PThreads) {
-    const int a = n / kTileFaces, idx = n % kTileFaces;
-    const int e0 = tile_ext0(a), e1 = tile_ext1(a);
-    const int nx = idx % e0 - 1, ny = (idx / e0) % e1 - 1, nz = idx / (e0 * e1) - 1;
-    const int dx = nx < 0 ? -1 : (nx > 7 ? 1 : 0), dy = ny < 0 ? -1 : (ny > 7 ? 1 : 0),
-              dz = nz < 0 ? -1 : (nz > 7 ? 1 : 0);
-    const int nb = g.nbr27[b * 27 + nbr_index(dx, dy, dz)];
-    float v = 0.0f;
-    if (nb >= 0) {
-      const int l = ((nz - 8 * dz) * 8 + (ny - 8 * dy)) * 8 + (nx - 8 * dx);
-      v = u[a][(size_t)nb * kBlockCells + l];
-    }
-    tile[n] = v;
+    int a;
+    const long long src = tile_source(g, b, n, &a);
+    tile[n] = src >= 0 ? u[a][src] : 0.0f;
   }
 }
 
@@ -221,11 +225,14 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
 // The full gather (24 values per particle: velocity, increment over the old
 // faces, fitted slopes, gradients). Bound by instruction issue: 81 x 2 node
 // values and about 330 FMAs a particle, contracted axis by axis in packed pairs
-// ((u, old) share their weights, so dw0 u and w0 old are one FMA). A particle's
+// (u and old share their weights and lie side by side in the tile: one 8-byte load
+// is the pair that dw0 u + w0 old's FMA takes, without moves; two tiles of their
+// own cost 6% of the whole call below). A particle's
 // record is 96 contiguous bytes, so a warp's 32 records are staged in shared
 // memory (rows of 25 words: no conflicts) and stored as 24 contiguous 128-byte
 // lines; a lane storing its own record touches 32 lines per instruction. The
-// 120 x 104 x 88 transfers, whose gather this is, went from 616 to 534 us.
+// 120 x 104 x 88 transfers, whose gather this is, went from 616 to 534 us with the
+// staged records and to 500 with the pairs.
 constexpr int kFullRow = 25;
 constexpr size_t kFullSmem = sizeof(float) * (6 * kTileFaces + kG2PThreads * kFullRow);
 
@@ -233,20 +240,19 @@ __global__ void __launch_bounds__(kG2PThreads, 3)
     k_g2p_full(GridView g, ParticlesView p, const int* cell_start, const float* u0, const float* u1, const float* u2,
                const float* o0, const float* o1, const float* o2, float* full_out, DeviceReport* rep) {
   extern __shared__ float full_smem[];
-  float* tile = full_smem;
-  float* tile_old = tile + 3 * kTileFaces;
+  float2* tile = reinterpret_cast<float2*>(full_smem);  // (new, old) face velocities
   const int b = blockIdx.x, t = threadIdx.x, lane = t & 31;
-  float* rows = tile_old + 3 * kTileFaces + (t - lane) * kFullRow;  // the warp's staged records
+  float* rows = full_smem + 6 * kTileFaces + (t - lane) * kFullRow;  // the warp's staged records
   if (b == 0 && t == 0 && rep != nullptr) rep->compiled_architecture = compiled_arch();
   const int pbeg = cell_start[b * kBlockCells], pend = cell_start[(b + 1) * kBlockCells];
   if (pbeg == pend) return;
   const float* un[3] = {u0, u1, u2};
   const float* uo[3] = {o0, o1, o2};
-  load_tile(g, b, un, tile, t);
-  if (o0 != nullptr)
-    load_tile(g, b, uo, tile_old, t);
-  else
-    for (int n = t; n < 3 * kTileFaces; n += kG2PThreads) tile_old[n] = 0.0f;
+  for (int n = t; n < 3 * kTileFaces; n += kG2PThreads) {
+    int a;
+    const long long src = tile_source(g, b, n, &a);
+    tile[n] = make_float2(src >= 0 ? un[a][src] : 0.0f, src >= 0 && o0 != nullptr ? uo[a][src] : 0.0f);
+  }
   __syncthreads();
   const int bc[3] = {g.coord[3 * b] * 8, g.coord[3 * b + 1] * 8, g.coord[3 * b + 2] * 8};
   const float four_inv_h = 4.0f * g.inv_h;
@@ -296,8 +302,7 @@ __global__ void __launch_bounds__(kG2PThreads, 3)
         }
         const int e0 = tile_ext0(a), e1 = tile_ext1(a);
         const int n0 = ((first[2] - bc[2] + 1) * e1 + (first[1] - bc[1] + 1)) * e0 + (first[0] - bc[0] + 1);
-        const float* ta = tile + a * kTileFaces + n0;
-        const float* to = tile_old + a * kTileFaces + n0;
+        const float2* ta = tile + a * kTileFaces + n0;
         float2 pm0 = make_float2(0.0f, 0.0f), m1g1 = pm0, m2g2 = pm0, g0old = pm0;
 #pragma unroll
         for (int kz = 0; kz < 3; ++kz) {
@@ -308,10 +313,11 @@ __global__ void __launch_bounds__(kG2PThreads, 3)
             float2 U01, Uo;
 #pragma unroll
             for (int kx = 0; kx < 3; ++kx) {
-              const float u = ta[at + kx], old = to[at + kx];
+              const float2 node = ta[at + kx];  // one 8-byte load, and the pair that Uo's FMA takes
+              const float u = node.x;
               const float2 wx = make_float2(w[0][kx], wr[0][kx]), dx = make_float2(dw[0][kx], w[0][kx]);
               U01 = kx == 0 ? __fmul2_rn(wx, make_float2(u, u)) : __ffma2_rn(wx, make_float2(u, u), U01);
-              Uo = kx == 0 ? __fmul2_rn(dx, make_float2(u, old)) : __ffma2_rn(dx, make_float2(u, old), Uo);
+              Uo = kx == 0 ? __fmul2_rn(dx, node) : __ffma2_rn(dx, node, Uo);
             }
             const float2 wy = make_float2(w[1][ky], w[1][ky]);
             V01 = __ffma2_rn(wy, U01, V01);
