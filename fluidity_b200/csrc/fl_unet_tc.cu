@@ -4,27 +4,38 @@
 //
 // Activation layout (BF16, one copy per active block, zero pads kept zero):
 // a D^3 tensor with C channels is C/8 channel groups, each a column of rows of
-// 8 channels (16 bytes). Rows follow a padded box whose x and y pads are shared
-// between neighbouring lines and planes: Px = Py = D+1, Pz = D+2, and cell
-// (x,y,z) sits at row ((z+1) Py + (y+1)) Px + (x+1). A tap (dz,dy,dx) is then a
-// constant row shift dz Py Px + dy Px + dx, so the A operand of one tap for 128
-// consecutive output rows is the activation column itself, shifted: the shared
-// memory descriptor (K-major, no swizzle) starts at that row, its 8-row groups
-// 128 bytes apart (SBO) and its two 8-channel K halves one channel group apart
-// (LBO). Rows that are pads produce garbage outputs, which the epilogue drops.
-// The block's input window (8^3 + one-cell halo) uses Px = Py = Pz = 10, and its
-// two channels would leave six of a row's eight empty, so a window row holds the
-// three x-neighbours' channels (x - 1, x, x + 1) and a (dz, dy) pair of taps is
-// one K half: the two halves of an MMA are two consecutive (dz, dy) rows, their
+// 8 channels (16 bytes). Rows follow a box whose lines are the D cells alone and
+// whose planes share their y pads: Py = D+1, Pz = D+2, and cell (x,y,z) sits at
+// row ((z+1) Py + (y+1)) D + x. A (dz, dy) pair of taps is then a constant row
+// shift (dz Py + dy) D, so the A operand of one pair for 128 consecutive output
+// rows is the activation column itself, shifted: the shared memory descriptor
+// (K-major, no swizzle) starts at that row, its 8-row groups 128 bytes apart
+// (SBO) and its two 8-channel K halves one channel group apart (LBO). Rows that
+// are pads produce garbage outputs, which the epilogue drops. The three taps of a
+// line (dx = -1, 0, 1) are three N-wide column sets of the same MMA, and the
+// epilogue adds them, D-1[x-1] + D0[x] + D+1[x+1], from the neighbouring lanes: a
+// tile row's 32 lanes are whole lines, so a line's ends need no other warp. An
+// MMA at N = 16 is bound by reading its A operand (128 x 32 bytes of shared
+// memory, ~46 cycles an MMA measured); with 3N columns a tile takes 9 of them per
+// 16 channels instead of 27 (the 16-channel 8^3 layers 45-48 -> 30 us, the 32-channel
+// 4^3 layers 25.5 -> 18.4 at the 128^3 splash's 1.9k blocks; one application, with
+// k_bt_tc, 352 -> 259).
+// The block's input window (8^3 + one-cell halo, Py = Pz = 10) has two channels,
+// which would leave six of a row's eight empty, so a window row holds the three
+// x-neighbours' channels (x - 1, x, x + 1) and a (dz, dy) pair of taps is one K
+// half: the two halves of an MMA are two consecutive (dz, dy) rows, their
 // distance given as the descriptor's K-half stride, and the layer takes 5 MMAs
-// per tile instead of 27: 18 instead of 60 us at the 128^3 splash's 1.9k blocks.
+// per tile instead of 27: 18 instead of 60 us at 1.9k blocks, 15 with lines of 8
+// cells alone (5 tiles instead of 7).
+// The 2^3 layer sees all eight cells of its block from every output cell, so it
+// is a plain GEMM over the blocks (k_bt_tc).
 //
 // Per conv layer one persistent kernel: each CTA keeps the layer's packed
-// weights in shared memory ([tap][K chunk][K half][Cout][8]), and per block it
-// copies the input rows in, one thread issues tiles x 27 x K-chunks MMAs
-// (M = 128, N = Cout, K = 16), a commit arrives on an mbarrier, and four warps
-// read the accumulators back (tcgen05.ld 32x32b) for bias, ReLU and the store
-// to the next layout. The 1x1 layers, pooling and upsampling run as small
+// weights in shared memory ([(dz, dy)][K chunk][K half][dx][Cout][8]), and per block it
+// copies the input rows in, one thread issues tiles x 9 x K-chunks MMAs
+// (M = 128, N = 3 Cout, K = 16), a commit arrives on an mbarrier, and four or
+// eight warps read the accumulators back (tcgen05.ld 32x32b) for the sum over dx,
+// bias, ReLU and the store to the next layout. The 1x1 layers, pooling and upsampling run as small
 // SIMT kernels on the same layouts; the last layer's epilogue also applies the
 // 16->1 output layer and writes the correction into the solver's vector.
 #include <cuda_bf16.h>
@@ -41,20 +52,22 @@ namespace fl {
 
 namespace {
 
-constexpr int kTcThreads = 160;  // warps 0-3 read TMEM lanes 32w..32w+31; warp 4 copies and issues MMAs
 constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at 1.9 GHz: mbarrier wait bound
 
 struct PadGeom {
   int D, Px, Py, rows, r_lo, tiles;
 };
 // rows >= 128 * tiles + 2 * r_lo, so every shifted tile stays inside the column
-__host__ __device__ constexpr PadGeom geom8() { return {8, 9, 9, 824, 91, 5}; }
-__host__ __device__ constexpr PadGeom geom4() { return {4, 5, 5, 192, 31, 1}; }
-__host__ __device__ constexpr PadGeom geom2() { return {2, 3, 3, 160, 13, 1}; }
-__host__ __device__ constexpr PadGeom geom10() { return {8, 10, 10, 1120, 111, 7}; }
+__host__ __device__ constexpr PadGeom geom8() { return {8, 8, 9, 800, 80, 5}; }
+__host__ __device__ constexpr PadGeom geom4() { return {4, 4, 5, 176, 24, 1}; }
+__host__ __device__ constexpr PadGeom geom10() { return {8, 8, 10, 816, 88, 5}; }
+
+// Warps 0..kTcEpilogue-1 read TMEM lanes 32 (w % 4)..; the next one copies and issues MMAs.
+__host__ __device__ constexpr int tc_epilogue_warps(int tiles) { return tiles > 1 ? 8 : 4; }
+constexpr int kBtThreads = 160;
 
 __device__ __forceinline__ int pad_row(const PadGeom& g, int x, int y, int z) {
-  return ((z + 1) * g.Py + (y + 1)) * g.Px + (x + 1);
+  return ((z + 1) * g.Py + (y + 1)) * g.Px + x;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -98,18 +111,27 @@ __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // One contiguous global -> shared copy through the bulk-copy engine (no
-// multicast; this GPU's own memory), completing on `mbar` as transaction bytes.
+// multicast; this GPU's own memory), completing on `mbar` as transaction bytes
+// (bulk_copy_part: the bytes are announced by the caller).
 // Both addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+__device__ __forceinline__ void bulk_copy_part(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(mbar)
                : "memory");
 }
 
-// Weight K chunks (of 16) of a layer with KG input channel groups: per tap and 16
-// channels, or for the window (KG = 1) per pair of (dz, dy) rows.
-__host__ __device__ constexpr int weight_chunks(int kg) { return kg == 1 ? 5 : 27 * (kg / 2); }
+__device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+  bulk_copy_part(dst, src, bytes, mbar);
+}
+
+// Weight K chunks (of 16) of a layer with KG input channel groups: per (dz, dy) and
+// 16 channels, or for the window (KG = 1) per pair of (dz, dy) rows.
+__host__ __device__ constexpr int weight_chunks(int kg) { return kg == 1 ? 5 : 9 * (kg / 2); }
+
+// Columns of an MMA: the layer's N outputs for each of the line's three taps (the
+// window's rows hold the taps themselves).
+__host__ __device__ constexpr int mma_columns(int kg, int n) { return kg == 1 ? n : 3 * n; }
 
 // TMEM columns of one accumulator stage (a power of two, at least 32).
 __host__ __device__ constexpr int tc_cols(int used) { return used <= 32 ? 32 : (used <= 64 ? 64 : (used <= 128 ? 128 : 256)); }
@@ -141,16 +163,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
   }
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// The registers of an asynchronous load, usable only after the wait.
+__device__ __forceinline__ void tmem_ld_done(uint32_t (&r)[16]) {
 #pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
+  for (int k = 0; k < 16; ++k) asm volatile("" : "+r"(r[k]));
 }
 
 __device__ __forceinline__ uint4 pack8(const float* v) {
@@ -177,14 +202,13 @@ __device__ __forceinline__ void unpack8(uint4 u, float* v) {
   }
 }
 
-enum ConvMode : int { kToPadded = 0, kToPlain = 1, kToCorrection = 2 };
+enum ConvMode : int { kToPadded = 0, kToCorrection = 1 };
 
 struct ConvArgs {
   const uint4* in;        // [nb][in_groups][rows_in] rows of 8 BF16 channels
-  const uint4* weights;   // packed [27][kc][2][N] rows of 8 BF16
+  const uint4* weights;   // packed [9][kc][2][3][N] rows of 8 BF16
   const float* bias;      // N
   uint4* out;             // kToPadded: [nb][N/8][rows_out]
-  float* out_plain;       // kToPlain: [nb][D^3][N]
   int nb;
   // final layer (kToCorrection)
   const float* w_out;     // 16
@@ -197,6 +221,10 @@ struct ConvArgs {
   int* error;             // set to 1 when an mbarrier wait gives up
 };
 
+// Geometry of a layout: 10 = the window, 8 and 4 = the padded columns of that level.
+__host__ __device__ constexpr PadGeom in_geom(int kind) { return kind == 10 ? geom10() : (kind == 8 ? geom8() : geom4()); }
+__host__ __device__ constexpr int conv_threads(int kind) { return 32 * (tc_epilogue_warps(in_geom(kind).tiles) + 1); }
+
 __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
@@ -207,29 +235,33 @@ __device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
 // taps per K half). N: output channels.
 //
 // A CTA handles blocks blockIdx.x, blockIdx.x + gridDim.x, ... through a
-// two-stage pipeline. Warp 4's first thread copies block k + 1's operand
+// two-stage pipeline. The last warp's first thread copies block k + 1's operand
 // columns into one shared-memory stage (a bulk copy) while it issues block
 // k's MMAs from the other stage into one of two TMEM accumulator stages;
-// warps 0-3 (TMEM lanes 32w..32w+31) drain the other accumulator stage,
-// block k - 1's, for bias, ReLU and the store. Barriers per stage: operands
+// the epilogue warps (warp w: TMEM lanes 32 (w % 4)..; eight warps take the tiles
+// in turn, even and odd) drain the other accumulator stage, block k - 1's, for the
+// sum over dx, bias, ReLU and the store. Barriers per stage: operands
 // arrived (full), operands consumed by the MMAs (empty), accumulators written
 // (accf), accumulators read (acce, one arrival per epilogue warp). Every wait
 // is bounded (~1 s); a wait that gives up sets the error flag and its role
 // stops, and the TMEM is released only after a final commit shows every
 // issued MMA complete.
 template <int KG, int N, int MODE, int IN_KIND, int OUT_KIND>
-__global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
-  constexpr PadGeom IN = IN_KIND == 10 ? geom10() : (IN_KIND == 8 ? geom8() : (IN_KIND == 4 ? geom4() : geom2()));
-  constexpr PadGeom OUT = OUT_KIND == 8 ? geom8() : (OUT_KIND == 4 ? geom4() : geom2());
+__global__ void __launch_bounds__(conv_threads(IN_KIND)) k_conv_tc(ConvArgs a) {
+  constexpr PadGeom IN = in_geom(IN_KIND);
+  constexpr PadGeom OUT = in_geom(OUT_KIND);
   constexpr int KC = KG >= 2 ? KG / 2 : 1;
   constexpr int TILES = IN.tiles;
-  constexpr int NCOLS = tc_cols(TILES * N);
-  constexpr uint32_t W_BYTES = (uint32_t)weight_chunks(KG) * 2u * N * 16u;
+  constexpr int EPI = tc_epilogue_warps(TILES);
+  constexpr int NM = mma_columns(KG, N);
+  constexpr int NCOLS = tc_cols(TILES * NM);
+  constexpr uint32_t W_BYTES = (uint32_t)weight_chunks(KG) * 2u * NM * 16u;
   constexpr uint32_t A_BYTES = (uint32_t)KG * IN.rows * 16u;
   constexpr uint32_t GROUP_BYTES = (uint32_t)IN.rows * 16u;
-  constexpr uint32_t IDESC = instr_desc(128, N);
+  constexpr uint32_t IDESC = instr_desc(128, NM);
   static_assert(IN.rows >= 128 * TILES + 2 * IN.r_lo, "shifted tiles must stay inside the column");
-  static_assert(N % 16 == 0 && N >= 16 && N <= 256, "M = 128 needs N in 16..256, multiple of 16");
+  static_assert(NM % 16 == 0 && NM >= 16 && NM <= 256, "M = 128 needs N in 16..256, multiple of 16");
+  static_assert(32 % IN.Px == 0 && IN.r_lo % IN.Px == 0, "a warp's 32 rows must be whole lines");
   static_assert(W_BYTES % 16 == 0 && A_BYTES % 16 == 0, "bulk copies need 16-byte alignment and sizes");
   static_assert(2 * NCOLS <= 512, "two accumulator stages within the SM's TMEM");
 
@@ -240,10 +272,10 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
   enum { kFull = 0, kEmpty = 2, kAccF = 4, kAccE = 6, kDrain = 8 };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (uint32_t i = tid; i < W_BYTES / 16; i += kTcThreads) w_s[i] = a.weights[i];
+  for (uint32_t i = tid; i < W_BYTES / 16; i += conv_threads(IN_KIND)) w_s[i] = a.weights[i];
   if (tid == 0) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) mbar_init_count(smem_u32(bars + k), (k == kAccE || k == kAccE + 1) ? 4u : 1u);
+    for (int k = 0; k < 9; ++k) mbar_init_count(smem_u32(bars + k), (k == kAccE || k == kAccE + 1) ? (uint32_t)EPI : 1u);
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -269,7 +301,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
     }
   };
 
-  if (warp == 4) {
+  if (warp == EPI) {
     if (lane == 0) {
       bool ok = true;
       int issued = -1, arrived = -1;  // last block (in this CTA's sequence) copied / waited for
@@ -298,11 +330,11 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
         // so each tap's operands are the tile's base descriptors plus constant
         // row offsets (every address stays below 256 KB: no carry out of the
         // field; the static_assert above keeps shifted rows inside the column).
-        const uint64_t b0 = smem_desc(w_addr, N * 16u, 128u);
+        const uint64_t b0 = smem_desc(w_addr, NM * 16u, 128u);
         const uint32_t a_row = a_addr + (uint32_t)st * A_BYTES + (uint32_t)IN.r_lo * 16u;
 #pragma unroll 1
         for (int t = 0; t < TILES; ++t) {
-          const uint32_t dt = tmem + (uint32_t)(st * NCOLS + t * N);
+          const uint32_t dt = tmem + (uint32_t)(st * NCOLS + t * NM);
           if constexpr (KG == 1) {
 #pragma unroll
             for (int p = 0; p < 5; ++p) {  // rows 2p and 2p + 1 of the nine (dz, dy); row 9 has zero weights
@@ -310,18 +342,18 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
               const int shift = ((r / 3 - 1) * IN.Py + (r % 3 - 1)) * IN.Px;
               const int step = ((next / 3 - 1) * IN.Py + (next % 3 - 1)) * IN.Px - shift;
               const uint64_t ad = smem_desc(a_row, (uint32_t)step * 16u, 128u) + (uint64_t)(int64_t)(128 * t + shift);
-              mma_bf16(dt, ad, b0 + (uint64_t)(p * 2 * N), IDESC, p != 0 ? 1u : 0u);
+              mma_bf16(dt, ad, b0 + (uint64_t)(p * 2 * NM), IDESC, p != 0 ? 1u : 0u);
             }
           } else {
             const uint64_t at = smem_desc(a_row, GROUP_BYTES, 128u) + (uint64_t)(128 * t);
 #pragma unroll
-            for (int tap = 0; tap < 27; ++tap) {
-              const int shift = ((tap / 9 - 1) * IN.Py + ((tap / 3) % 3 - 1)) * IN.Px + (tap % 3 - 1);
+            for (int line = 0; line < 9; ++line) {
+              const int shift = ((line / 3 - 1) * IN.Py + (line % 3 - 1)) * IN.Px;
 #pragma unroll
               for (int kc = 0; kc < KC; ++kc) {
                 const uint64_t ad = at + (uint64_t)(int64_t)(shift + 2 * kc * IN.rows);
-                const uint64_t bd = b0 + (uint64_t)((tap * KC + kc) * 2 * N);
-                mma_bf16(dt, ad, bd, IDESC, (tap | kc) != 0 ? 1u : 0u);
+                const uint64_t bd = b0 + (uint64_t)((line * KC + kc) * 2 * NM);
+                mma_bf16(dt, ad, bd, IDESC, (line | kc) != 0 ? 1u : 0u);
               }
             }
           }
@@ -349,20 +381,43 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
         break;
       }
       fence_after_sync();
-      // warp w owns tile rows 32w..32w+31
+      // warp w owns tile rows 32 (w % 4)..+31
+      const int row_warp = warp & 3;
 #pragma unroll 1
-      for (int t = 0; t < TILES; ++t) {
-        const int r = IN.r_lo + 128 * t + 32 * warp + lane;
-        const int px = r % IN.Px, py = (r / IN.Px) % IN.Py, pz = r / (IN.Px * IN.Py);
-        const bool interior = px >= 1 && px <= IN.D && py >= 1 && py <= IN.D && pz >= 1 && pz <= IN.D;
-        const int x = px - 1, y = py - 1, z = pz - 1;
+      for (int t = warp >> 2; t < TILES; t += EPI / 4) {
+        const int r = IN.r_lo + 128 * t + 32 * row_warp + lane;
+        const int x = r % IN.Px, y = (r / IN.Px) % IN.Py - 1, z = r / (IN.Px * IN.Py) - 1;
+        const bool interior = y >= 0 && y < IN.D && z >= 0 && z < IN.D;
         float acc[N];
+        const uint32_t tt = tmem + ((uint32_t)(32 * row_warp) << 16) + (uint32_t)(st * NCOLS + t * NM);
 #pragma unroll
         for (int c = 0; c < N; c += 16) {
-          float v[16];
-          tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(st * NCOLS + t * N + c), v);
+          if constexpr (KG == 1) {
+            uint32_t v[16];
+            tmem_ld16_async(tt + c, v);
+            tmem_ld_wait();
+            tmem_ld_done(v);
 #pragma unroll
-          for (int q = 0; q < 16; ++q) acc[c + q] = fmaxf(v[q] + __ldg(&a.bias[c + q]), 0.0f);
+            for (int q = 0; q < 16; ++q) acc[c + q] = fmaxf(__uint_as_float(v[q]) + __ldg(&a.bias[c + q]), 0.0f);
+          } else {
+            uint32_t lo[16], mid[16], hi[16];
+            tmem_ld16_async(tt + c, lo);
+            tmem_ld16_async(tt + N + c, mid);
+            tmem_ld16_async(tt + 2 * N + c, hi);
+            tmem_ld_wait();
+            tmem_ld_done(lo);
+            tmem_ld_done(mid);
+            tmem_ld_done(hi);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              const float left = __uint_as_float(__shfl_up_sync(0xffffffffu, lo[q], 1));
+              const float right = __uint_as_float(__shfl_down_sync(0xffffffffu, hi[q], 1));
+              float v = __uint_as_float(mid[q]);
+              if (x > 0) v += left;
+              if (x < IN.D - 1) v += right;
+              acc[c + q] = fmaxf(v + __ldg(&a.bias[c + q]), 0.0f);
+            }
+          }
         }
         if (!interior) continue;
         if (MODE == kToPadded) {
@@ -370,11 +425,6 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
           uint4* dst = a.out + (size_t)b * (N / 8) * OUT.rows;
 #pragma unroll
           for (int g = 0; g < N / 8; ++g) dst[g * OUT.rows + ro] = pack8(acc + 8 * g);
-        } else if (MODE == kToPlain) {
-          float* dst = a.out_plain + ((size_t)b * IN.D * IN.D * IN.D + (z * IN.D + y) * IN.D + x) * N;
-#pragma unroll
-          for (int c = 0; c < N; c += 4)
-            *reinterpret_cast<float4*>(dst + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
         } else {
           float yv = __ldg(a.b_out);
 #pragma unroll
@@ -391,7 +441,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
           }
         }
       }
-      // this warp's accumulator reads are done (tmem_ld16 waits for them)
+      // this warp's accumulator reads are done (each waited for)
       fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(kAccE + st));
@@ -405,8 +455,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(ConvArgs a) {
 }
 
 // Input window of block b in the 10^3 layout (one channel group: residual / s and
-// cell mask of the cells x - 1, x and x + 1, two zero channels; the rows at the
-// window's x ends, whose neighbours are another line's, are never a tap's centre)
+// cell mask of the cells x - 1, x and x + 1, two zero channels)
 // and the block scale s (max |residual| over the window).
 // z_zero (not null when the network's output replaces z): a block whose window
 // holds no residual is skipped by every layer, so its correction, zero, is
@@ -417,7 +466,7 @@ __global__ void __launch_bounds__(512) k_tc_gather(GridView g, const float* __re
                                                    float* __restrict__ scale, T* __restrict__ z_zero) {
   constexpr PadGeom W = geom10();
   __shared__ float red[16];
-  __shared__ float2 win[1002];  // (residual, mask) of the window, one entry of margin at each end
+  __shared__ float2 win[1000];  // (residual, mask) of the window
   const int b = blockIdx.x;
   float rv[2], mv[2], mx = 0.0f;
 #pragma unroll
@@ -452,28 +501,30 @@ __global__ void __launch_bounds__(512) k_tc_gather(GridView g, const float* __re
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const int i = threadIdx.x + 512 * k;
-    if (i < 1000) win[i + 1] = make_float2(sc > 0.0f ? rv[k] / sc : 0.0f, mv[k]);
+    if (i < 1000) win[i] = make_float2(sc > 0.0f ? rv[k] / sc : 0.0f, mv[k]);
   }
-  if (threadIdx.x < 2) win[threadIdx.x * 1001] = make_float2(0.0f, 0.0f);
   __syncthreads();
   uint4* dst = x + (size_t)b * W.rows;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const int i = threadIdx.x + 512 * k;
-    if (i < 1000) {  // window row (hz+1, hy+1, hx+1) == i in the 10^3 layout: its cell and the two beside it in x
-      const float2 lo = win[i], at = win[i + 1], hi = win[i + 2];
+    const int x0 = i % 10 - 1;
+    if (i < 1000 && x0 >= 0 && x0 < 8) {  // a row of the window's layout: its cell and the two beside it in x
+      const float2 lo = win[i - 1], at = win[i], hi = win[i + 1];
       const float v[8] = {lo.x, lo.y, at.x, at.y, hi.x, hi.y, 0.f, 0.f};
-      dst[i] = pack8(v);
+      dst[i / 10 * 8 + x0] = pack8(v);
     }
   }
   if (threadIdx.x == 0) scale[b] = sc;
 }
 
-// 2x average pooling between padded layouts (G channel groups). One thread per (block, coarse cell, group).
+// 2x average pooling from a padded layout (G channel groups) to the next padded
+// layout, or from 4^3 to the 2^3 layer's operand, [cell][group][block]. One thread
+// per (block, coarse cell, group).
 template <int DIN, int G>
-__global__ void k_tc_pool(const uint4* __restrict__ in, uint4* __restrict__ out, int nb) {
+__global__ void k_tc_pool(const uint4* __restrict__ in, uint4* __restrict__ out, int nb, long long cap) {
   constexpr PadGeom I = DIN == 8 ? geom8() : geom4();
-  constexpr PadGeom O = DIN == 8 ? geom4() : geom2();
+  constexpr PadGeom O = geom4();
   constexpr int H = DIN / 2, H3 = H * H * H;
   const long long total = (long long)nb * H3 * G;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -492,8 +543,101 @@ __global__ void k_tc_pool(const uint4* __restrict__ in, uint4* __restrict__ out,
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) s[j] *= 0.125f;
-    out[(size_t)b * G * O.rows + (size_t)gi * O.rows + pad_row(O, x, y, z)] = pack8(s);
+    const size_t at = DIN == 8 ? (size_t)b * G * O.rows + (size_t)gi * O.rows + pad_row(O, x, y, z)
+                               : (size_t)(c * G + gi) * cap + b;
+    out[at] = pack8(s);
   }
+}
+
+// The 2^3 layer (32 -> 64 channels): every output cell's taps cover the block's eight
+// cells, so one output cell of 128 blocks is a GEMM with M = 128 blocks, N = 64 and
+// K = 8 cells x 32 channels. One CTA per 128 blocks and output cell; operand columns
+// [K group][block], 32 bulk copies, 16 MMAs. Bound by the copies' latency. As a
+// convolution over padded boxes (8 of 128 rows useful, 108 KB of weights per CTA) it
+// took 33.7 us at 1.9k blocks, now 6.3. Rows past the last block hold whatever the
+// shared memory held: they reach their own, dropped outputs only.
+__global__ void __launch_bounds__(kBtThreads) k_bt_tc(const uint4* __restrict__ in, long long cap,
+                                                      const uint4* __restrict__ weights, const float* __restrict__ bias,
+                                                      float* __restrict__ out, int nb, int* error) {
+  constexpr int K_GROUPS = 32, N = 64;
+  constexpr uint32_t A_BYTES = K_GROUPS * 128u * 16u, W_BYTES = K_GROUPS * N * 16u;
+  constexpr uint32_t IDESC = instr_desc(128, N);
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + A_BYTES + W_BYTES);  // operands arrived, accumulators written
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b0 = blockIdx.x * 128, cell = blockIdx.y;
+  const uint32_t rows = (uint32_t)min(128, nb - b0);
+  const uint32_t a_addr = smem_u32(smem), w_addr = a_addr + A_BYTES;
+  const uint32_t full = smem_u32(bars), done = smem_u32(bars + 1);
+  if (tid == 0) {
+    mbar_init(full);
+    mbar_init(done);
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"((uint32_t)N));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  if (warp == 4) {
+    if (lane == 0) {
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full),
+                   "r"(W_BYTES + K_GROUPS * rows * 16u)
+                   : "memory");
+      bulk_copy_part(w_addr, weights + (size_t)cell * (W_BYTES / 16), W_BYTES, full);
+      for (int k = 0; k < K_GROUPS; ++k)
+        bulk_copy_part(a_addr + (uint32_t)k * 2048u, in + (size_t)k * cap + b0, rows * 16u, full);
+      if (mbar_wait(full, 0u)) {
+        const uint64_t ad = smem_desc(a_addr, 2048u, 128u), bd = smem_desc(w_addr, N * 16u, 128u);
+#pragma unroll
+        for (int k = 0; k < K_GROUPS / 2; ++k)
+          mma_bf16(tmem, ad + (uint64_t)(k * 256), bd + (uint64_t)(k * 2 * N), IDESC, k != 0 ? 1u : 0u);
+      } else {
+        atomicExch(error, 1);
+        mbar_wait(full, 0u);  // once more, for the copies still in flight
+      }
+      mma_commit(done);  // arrives once every MMA this thread issued has completed
+      if (!mbar_wait(done, 0u)) atomicExch(error, 1);
+    }
+  } else {
+    // (the copy's bounded waits come first, hence up to three bounds here)
+    bool ok = false;
+    for (int tries = 0; tries < 4 && !ok; ++tries) ok = mbar_wait(done, 0u);
+    fence_after_sync();
+    if (ok) {
+      const int b = b0 + 32 * warp + lane;
+      float* dst = out + ((size_t)b * 8 + cell) * N;
+#pragma unroll
+      for (int c = 0; c < N; c += 16) {
+        uint32_t v[16];
+        tmem_ld16_async(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c, v);
+        tmem_ld_wait();
+        tmem_ld_done(v);
+        if (b < nb) {
+#pragma unroll
+          for (int q = 0; q < 16; q += 4) {
+            float4 o;
+            o.x = fmaxf(__uint_as_float(v[q]) + __ldg(&bias[c + q]), 0.0f);
+            o.y = fmaxf(__uint_as_float(v[q + 1]) + __ldg(&bias[c + q + 1]), 0.0f);
+            o.z = fmaxf(__uint_as_float(v[q + 2]) + __ldg(&bias[c + q + 2]), 0.0f);
+            o.w = fmaxf(__uint_as_float(v[q + 3]) + __ldg(&bias[c + q + 3]), 0.0f);
+            *reinterpret_cast<float4*>(dst + c + q) = o;
+          }
+        }
+      }
+    } else if (lane == 0) {
+      atomicExch(error, 1);
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)N));
 }
 
 // u2 = relu(up(W_u2 bt + b_u2) + s2) at 4^3 (32 channels): one CTA per block,
@@ -590,23 +734,28 @@ __global__ void __launch_bounds__(256) k_tc_upadd1(const uint4* __restrict__ d2,
   }
 }
 
-// Packs one FP32 conv layer (w[co][ci][27]) into [27][kc][2][cout][8] BF16 with
-// input channels padded to 16 * kc (zeros); the first layer (two channels) into
-// [5][2][cout][8]: K half h of chunk p is (dz, dy) row 2p + h, channel 2 dx + ci.
+// Packs one FP32 conv layer (w[co][ci][27]) into [9 (dz, dy)][kc][2][3 dx][cout][8]
+// BF16 with 16 * kc = cin input channels; the first layer (two channels) into
+// [5][2][cout][8]: K half h of chunk p is (dz, dy) row 2p + h, channel 2 dx + ci;
+// the 2^3 layer (cout = 64) into [output cell][input cell x 4 groups][cout][8].
 __global__ void k_pack_conv(const float* __restrict__ w, int cin, int cout, int kc, __nv_bfloat16* __restrict__ out) {
-  const int total = (cin == 2 ? 5 : 27 * kc) * 2 * cout * 8;
+  const int total = cout == 64 ? 8 * 32 * 64 * 8 : (cin == 2 ? 5 : 27 * kc) * 2 * cout * 8;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int j = i & 7;
     const int n = (i >> 3) % cout;
-    const int kh = (i / (8 * cout)) & 1;
     int ci, tap;
-    if (cin == 2) {
-      const int row = 2 * (i / (16 * cout)) + kh;
+    if (cout == 64) {
+      const int kg = (i / (8 * cout)) & 31, o = i / (256 * cout), c = kg >> 2;
+      ci = (kg & 3) * 8 + j;
+      tap = (((c >> 2) - (o >> 2) + 1) * 3 + ((c >> 1) & 1) - ((o >> 1) & 1) + 1) * 3 + (c & 1) - (o & 1) + 1;
+    } else if (cin == 2) {
+      const int row = i / (8 * cout);
       ci = row < 9 && j < 6 ? j & 1 : cin;
       tap = row * 3 + (j >> 1);
     } else {
-      ci = (i / (16 * cout)) % kc * 16 + kh * 8 + j;
-      tap = i / (16 * cout * kc);
+      const int kh = (i / (24 * cout)) & 1;
+      ci = (i / (48 * cout)) % kc * 16 + kh * 8 + j;
+      tap = i / (48 * cout * kc) * 3 + (i / (8 * cout)) % 3;
     }
     out[i] = __float2bfloat16_rn(ci < cin ? w[((size_t)n * cin + ci) * 27 + tap] : 0.0f);
   }
@@ -616,14 +765,13 @@ __global__ void k_pack_conv(const float* __restrict__ w, int cin, int cout, int 
 // SM's 512 columns.
 template <int KG, int N, int MODE, int IN_KIND, int OUT_KIND>
 constexpr int conv_ctas_per_sm() {
-  constexpr PadGeom IN = IN_KIND == 10 ? geom10() : (IN_KIND == 8 ? geom8() : (IN_KIND == 4 ? geom4() : geom2()));
-  return 512 / (2 * tc_cols(IN.tiles * N));
+  return 512 / (2 * tc_cols(in_geom(IN_KIND).tiles * mma_columns(KG, N)));
 }
 
 template <int KG, int N, int MODE, int IN_KIND, int OUT_KIND>
 constexpr size_t conv_smem() {
-  constexpr PadGeom IN = IN_KIND == 10 ? geom10() : (IN_KIND == 8 ? geom8() : (IN_KIND == 4 ? geom4() : geom2()));
-  constexpr size_t bytes = (size_t)weight_chunks(KG) * 2u * N * 16u + 2u * (size_t)KG * IN.rows * 16u + 9 * 8 + 8;
+  constexpr PadGeom IN = in_geom(IN_KIND);
+  constexpr size_t bytes = (size_t)weight_chunks(KG) * 2u * mma_columns(KG, N) * 16u + 2u * (size_t)KG * IN.rows * 16u + 9 * 8 + 8;
   // Ask for enough shared memory that one more CTA than the TMEM allows does
   // not fit the SM (228 KB, 1 KB reserved per CTA), so no TMEM allocation
   // waits for another CTA's release.
@@ -644,7 +792,18 @@ cudaError_t launch_conv(const ConvArgs& a, int sms, cudaStream_t s) {
   const int per_sm = by_smem < cap ? by_smem : cap;
   const int grid = a.nb < sms * per_sm ? a.nb : sms * per_sm;
   ++g_kernel_launches;
-  kern<<<grid, kTcThreads, smem, s>>>(a);
+  kern<<<grid, conv_threads(IN_KIND), smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_bt(const uint4* in, long long cap, const uint4* weights, const float* bias, float* out, int nb,
+                      int* error, cudaStream_t s) {
+  // 96 KB of operands: two CTAs an SM, 128 of its 512 TMEM columns
+  constexpr int smem = 32 * (128 + 64) * 16 + 2 * 8 + 8;
+  static unsigned long long configured = 0;
+  if (first_on_device(configured)) cudaFuncSetAttribute(k_bt_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  ++g_kernel_launches;
+  k_bt_tc<<<dim3((nb + 127) / 128, 8), kBtThreads, smem, s>>>(in, cap, weights, bias, out, nb, error);
   return cudaGetLastError();
 }
 
@@ -665,7 +824,7 @@ UNetTcLayout unet_tc_layout() {
   L.p1 = take(2 * geom4().rows);
   L.e2a = take(4 * geom4().rows);
   L.s2 = take(4 * geom4().rows);
-  L.p2 = take(4 * geom2().rows);
+  L.p2 = take(8 * 4);
   L.u2 = take(4 * geom4().rows);
   L.d2 = take(4 * geom4().rows);
   L.rows_per_block = off;
@@ -676,7 +835,7 @@ UNetTcLayout unet_tc_layout() {
   for (int k = 0; k < 7; ++k) {
     const int kc = cin[k] >= 32 ? 2 : 1;
     L.w_off[k] = w;
-    w += (cin[k] == 2 ? 5ll : 27ll * kc) * 2 * cout[k] * 8;
+    w += cout[k] == 64 ? 8ll * 32 * 64 * 8 : (cin[k] == 2 ? 5ll : 27ll * kc) * 2 * cout[k] * 8;
   }
   L.w_total = w;
   return L;
@@ -725,7 +884,7 @@ cudaError_t unet_tc_apply(const GridView& g, const float* params, const __nv_bfl
   a.in = base(L.t8); a.weights = wp(1); a.bias = params + P.bias[1]; a.out = base(L.s1);
   if ((e = launch_conv<2, 16, kToPadded, 8, 8>(a, sms, s)) != cudaSuccess) return e;
   g_kernel_launches += 1;
-  k_tc_pool<8, 2><<<(nb * 64 * 2 + 255) / 256, 256, 0, s>>>(base(L.s1), base(L.p1), nb);
+  k_tc_pool<8, 2><<<(nb * 64 * 2 + 255) / 256, 256, 0, s>>>(base(L.s1), base(L.p1), nb, cap);
   // e2a: p1 -> e2a
   a.in = base(L.p1); a.weights = wp(2); a.bias = params + P.bias[2]; a.out = base(L.e2a);
   if ((e = launch_conv<2, 32, kToPadded, 4, 4>(a, sms, s)) != cudaSuccess) return e;
@@ -733,14 +892,13 @@ cudaError_t unet_tc_apply(const GridView& g, const float* params, const __nv_bfl
   a.in = base(L.e2a); a.weights = wp(3); a.bias = params + P.bias[3]; a.out = base(L.s2);
   if ((e = launch_conv<4, 32, kToPadded, 4, 4>(a, sms, s)) != cudaSuccess) return e;
   g_kernel_launches += 1;
-  k_tc_pool<4, 4><<<(nb * 8 * 4 + 255) / 256, 256, 0, s>>>(base(L.s2), base(L.p2), nb);
+  k_tc_pool<4, 4><<<(nb * 8 * 4 + 255) / 256, 256, 0, s>>>(base(L.s2), base(L.p2), nb, cap);
   // bt: p2 -> bt (plain FP32)
-  a.in = base(L.p2); a.weights = wp(4); a.bias = params + P.bias[4]; a.out = nullptr; a.out_plain = bt;
-  if ((e = launch_conv<4, 64, kToPlain, 2, 2>(a, sms, s)) != cudaSuccess) return e;
+  if ((e = launch_bt(base(L.p2), cap, wp(4), params + P.bias[4], bt, nb, error, s)) != cudaSuccess) return e;
   g_kernel_launches += 1;
   k_tc_upadd2<<<nb, 256, 0, s>>>(bt, base(L.s2), params + P.offset[5], params + P.bias[5], base(L.u2));
   // d2: u2 -> d2
-  a.in = base(L.u2); a.weights = wp(5); a.bias = params + P.bias[6]; a.out = base(L.d2); a.out_plain = nullptr;
+  a.in = base(L.u2); a.weights = wp(5); a.bias = params + P.bias[6]; a.out = base(L.d2);
   if ((e = launch_conv<4, 32, kToPadded, 4, 4>(a, sms, s)) != cudaSuccess) return e;
   g_kernel_launches += 1;
   k_tc_upadd1<<<nb, 256, 0, s>>>(base(L.d2), base(L.s1), params + P.offset[7], params + P.bias[7], base(L.t8));

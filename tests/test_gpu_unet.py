@@ -451,3 +451,50 @@ def test_tensor_core_convolutions_at_item_counts(batch):
         assert _rel(g[off:off + nw], g_ref[off:off + nw]) <= 3e-2, name
         assert _rel(g[off + nw:off + nw + nb], g_ref[off + nw:off + nw + nb]) <= 3e-2, name
         off += nw + nb
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (6, 5, 2), (7, 3, 3), (1, 5, 10)])
+def test_tensor_core_inference_at_block_counts(shape):
+    """The inference where the 2^3 layer's tiles of 128 blocks end (8, 126, 128 and 132 active
+    blocks: a box of full blocks at the lattice's corner and the next layer), against the FP32
+    forward, with the first third of the blocks without residual: 3e-2 of the largest value, as
+    the test above."""
+    import ctypes
+
+    import torch
+
+    n = 96
+    axes = [(np.arange(8 * k) + 0.5) / n for k in shape]
+    x = np.stack([a.ravel() for a in np.meshgrid(*axes, indexing="ij")])
+    count = x.shape[1]
+    soa = np.zeros((15, count), np.float32)
+    soa[0:3] = x
+    src, dst = _t(soa), torch.zeros((15, count), device="cuda")
+
+    def parts(t):
+        p = fb.Particles()
+        p.x[:] = [t[d].data_ptr() for d in range(3)]
+        p.v[:] = [t[3 + d].data_ptr() for d in range(3)]
+        p.c[:] = [t[6 + d].data_ptr() for d in range(9)]
+        p.mass, p.count = None, count
+        return p
+
+    ctx = fb.LiquidContext(n, capacity=count)
+    lib, rep, a, b = fb.library(), fb.Report(), parts(src), parts(dst)
+    assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(a), None, ctypes.byref(rep)) == fb.OK
+    assert lib.fl_sort_particles_by_block(ctx.handle, ctypes.byref(a), ctypes.byref(b), None, ctypes.byref(rep)) == fb.OK
+    nb = len(ctx.active_blocks())
+    assert nb == np.prod([k + 1 for k in shape])
+    rng = np.random.default_rng(nb)
+    r = rng.normal(size=(nb, 512))
+    if nb > 27:
+        r[: nb // 3] = 0.0  # blocks whose whole window holds no residual are skipped
+    r = _t(r.ravel())
+    ctx.set_learned_preconditioner(_t(U.init_params(9) + 0.01 * rng.normal(size=U.param_count())))
+    z, ref = torch.zeros(nb * 512, device="cuda"), torch.zeros(nb * 512, device="cuda")
+    ctx.apply_learned(r, z, kernels=0)
+    ctx.apply_learned(r, ref, kernels=1)
+    z, ref = z.cpu().numpy(), ref.cpu().numpy()
+    assert np.any(ref != 0.0)
+    assert _rel(z, ref) <= 3e-2
+    ctx.close()
