@@ -526,9 +526,7 @@ int pressure_solve(fl_context* c, const float* const u_pred[3], float* const u_n
   ++g_kernel_launches;
   k_set_target<<<1, 1, 0, s>>>(c->st, opt->rel_tol);
   FL_CUDA(cudaMemsetAsync(c->lv_x[0], 0, sizeof(T) * (size_t)n, s));
-  FL_CUDA(cudaMemsetAsync(c->d[0], 0, sizeof(float) * (size_t)n, s));
-  FL_CUDA(cudaMemsetAsync(c->d[1], 0, sizeof(float) * (size_t)n, s));
-  FL_CUDA(cudaMemsetAsync(c->r[1], 0, sizeof(float) * (size_t)n, s));
+  // (d and the previous r need no zeros: a solve's first iteration uses neither)
   int total = 0, refinements = 0;
   bool converged = false;
   int status = FL_OK;

@@ -286,17 +286,31 @@ __global__ void k_coarsen(GridView g, LevelDesc F, LevelPtrs<T> fp, LevelDesc C,
 }
 
 // diag = anchor + sum of the six face coefficients (after coarsening, since a
-// cell's high faces belong to its neighbours). Levels >= 1.
+// cell's high faces belong to its neighbours). Levels >= 1, all in one launch:
+// level l's cells are those of CTAs first[l] .. first[l + 1] - 1.
 template <typename T>
-__global__ void k_level_diag(GridView g, LevelDesc L, LevelPtrs<T> lp) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+struct DiagArgs {
+  GridView g;
+  int levels;
+  unsigned first[13];
+  LevelDesc desc[12];
+  LevelPtrs<T> ptr[12];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads) k_level_diag(const __grid_constant__ DiagArgs<T> A) {
+  int l = 1;
+  while (l + 1 < A.levels && blockIdx.x >= A.first[l + 1]) ++l;
+  const LevelDesc& L = A.desc[l];
+  const LevelPtrs<T>& lp = A.ptr[l];
+  const long long i = (blockIdx.x - A.first[l]) * (long long)kThreads + threadIdx.x;
   if (i >= L.count) return;
   const CellPos p = cell_pos(L, i);
   float d = lp.anchor[i];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     d += ld(&lp.k[a][i]);
-    const long long hi = level_nbr(g, L, p, a, +1);
+    const long long hi = level_nbr(A.g, L, p, a, +1);
     if (hi >= 0) d += ld(&lp.k[a][hi]);
   }
   lp.diag[i] = lp.fluid[i] ? d : 1.0f;
@@ -779,7 +793,6 @@ __global__ void __launch_bounds__(1024) k_direction_finish(int nb, const double*
       st->done = 1;
     }
     st->alpha = st->rz / tot;
-    st->rz_prev = st->rz;
   }
 }
 
@@ -1255,13 +1268,42 @@ __global__ void k_dots(int n, const T* __restrict__ z, const float* __restrict__
   }
 }
 
-// e += alpha d; r_next = r - alpha q; ||r_next||^2 -> stop test.
-__global__ void k_update(int n, const float* __restrict__ d, const float* __restrict__ q, const float* __restrict__ r,
-                         float* __restrict__ r_next, float* __restrict__ e, double* partial, SolverState* st) {
+// e += alpha d; r_next = r - alpha q; ||r_next||^2 -> stop test. With kAlpha
+// every CTA forms alpha itself from the nb per-block partials of d.q (as
+// k_direction_finish does otherwise): up to kFuseAlphaBlocks blocks that is a few
+// loads a thread, less than the launch between the two kernels (with one diagonal
+// launch for all levels, the 32^3 host step 1081 -> 1052 us, the 128^3 substep
+// 1.006 -> 1.022 times the speed before). Above, every CTA would read more
+// partials than its own vector pieces, 80 KB at the 256^3 splash's 10k blocks.
+constexpr int kFuseAlphaBlocks = 1024;
+
+template <bool kAlpha>
+__global__ void __launch_bounds__(kThreads)
+    k_update(int n, int nb, const double* __restrict__ dq, const float* __restrict__ d, const float* __restrict__ q,
+             const float* __restrict__ r, float* __restrict__ r_next, float* __restrict__ e, double* partial,
+             SolverState* st) {
   grid_dependency_wait();
   if (st->done) return;
   __shared__ double red[kThreads / 32];
-  const float alpha = (float)st->alpha;
+  float alpha;
+  if (kAlpha) {
+    __shared__ double total;
+    double acc = 0.0;
+    for (int k = threadIdx.x; k < nb; k += kThreads) acc += dq[k];
+    acc = block_sum<kThreads>(acc, red);
+    if (threadIdx.x == 0) total = acc;
+    __syncthreads();
+    if (!(total > 0.0) || !isfinite(total)) {  // the same in every CTA
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->status = kAborted;
+        st->done = 1;
+      }
+      return;
+    }
+    alpha = (float)(st->rz / total);
+  } else {
+    alpha = (float)st->alpha;
+  }
   double rr = 0.0;
   // Four cells per thread and iteration (n is a multiple of 512): 16-byte accesses.
   const float4* d4 = reinterpret_cast<const float4*>(d);
@@ -1290,6 +1332,7 @@ __global__ void k_update(int n, const float* __restrict__ d, const float* __rest
     const double t = finish_sum(partial, 1, 0, red);
     if (threadIdx.x == 0) {
       st->rr = t;
+      st->rz_prev = st->rz;
       st->inner_iter += 1;
       st->total_iter += 1;
       if (st->learned && !st->fallback) {
@@ -1760,10 +1803,18 @@ cudaError_t launch_pressure_setup(const GridView& g, const int* cell_start, unsi
     k_coarsen<T><<<blocks_for(H.desc[l].count), kThreads, 0, s>>>(g, H.desc[l - 1], H.ptr[l - 1], H.desc[l],
                                                                    H.ptr[l]);
   }
+  DiagArgs<T> A;
+  A.g = g;
+  A.levels = H.levels;
+  unsigned ctas = 0;
   for (int l = 1; l < H.levels; ++l) {
-    ++g_kernel_launches;
-    k_level_diag<T><<<blocks_for(H.desc[l].count), kThreads, 0, s>>>(g, H.desc[l], H.ptr[l]);
+    A.first[l] = ctas;
+    A.desc[l] = H.desc[l];
+    A.ptr[l] = H.ptr[l];
+    ctas += blocks_for(H.desc[l].count);
   }
+  ++g_kernel_launches;
+  k_level_diag<T><<<ctas, kThreads, 0, s>>>(A);
   return cudaGetLastError();
 }
 
@@ -1810,11 +1861,19 @@ cudaError_t launch_fcg_iteration(const GridView& g, const MgHierarchy<T>& H, con
   }
   const T* z = H.ptr[0].x;
   const unsigned grid = reduce_grid(n);
-  g_kernel_launches += 4;
+  g_kernel_launches += 3;
   launch_dep(k_dots<T>, grid, kThreads, 0, s, n, z, r_cur, r_prev, partial, st);
   launch_dep(k_direction_tiled<T, kDirectionCpt>, g.nb, 512 / kDirectionCpt, 0, s, g, H.ptr[0], z, d_old, d_new, q, partial, st);
-  launch_dep(k_direction_finish, 1, 1024, 0, s, g.nb, partial, st);
-  launch_dep(k_update, grid, kThreads, 0, s, n, d_new, q, r_cur, r_prev, e, partial, st);
+  double* update_partial = partial + g.nb;  // (the d.q partials are read until the update ends)
+  if (g.nb <= kFuseAlphaBlocks) {
+    launch_dep(k_update<true>, grid, kThreads, 0, s, n, g.nb, (const double*)partial, d_new, q, r_cur, r_prev, e,
+               update_partial, st);
+  } else {
+    ++g_kernel_launches;
+    launch_dep(k_direction_finish, 1, 1024, 0, s, g.nb, partial, st);
+    launch_dep(k_update<false>, grid, kThreads, 0, s, n, g.nb, (const double*)partial, d_new, q, r_cur, r_prev, e,
+               update_partial, st);
+  }
   return cudaGetLastError();
 }
 

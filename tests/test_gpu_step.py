@@ -291,3 +291,24 @@ def test_topology_from_unordered_particles(count):
         assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(p), None, ctypes.byref(rep)) == code
         assert rep.first_bad_index == count - 1
     ctx.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [24, 144, 152])
+def test_flexible_cg_scalars_by_block_count(precision, n):
+    """The flexible-CG scalars are summed by the kernels that use them up to 1024 active blocks (24^3:
+    27, 144^3: 1000) and by kernels of their own above (152^3: 1331). Both reach the 1e-6 FP64
+    residual, and a second solve of the same system repeats the first's bits."""
+    ctx, soa, m = dam_break_context(n)
+    tp, opt = fb.transfer_params(scenes.DT, m), fb.default_pressure_options(precision=precision)
+    code, diag = ctx.step(tp, opt)
+    assert code == fb.OK and diag.relative_residual <= 1e-6
+    assert (diag.active_blocks <= 1024) == (n < 150)
+    runs = []
+    for _ in range(2):
+        code, d = ctx.project(tp, opt)
+        assert code == fb.OK and d.relative_residual <= 1e-6 and d.iterations <= 20
+        f = ctx.fields()
+        runs.append(fb.copy_to_host(f["pressure"], d.active_blocks * 512, np.float64))
+    np.testing.assert_array_equal(runs[0], runs[1])
+    ctx.close()
