@@ -638,6 +638,65 @@ __global__ void __launch_bounds__(256 / CPT)
   }
 }
 
+// The V-cycle's last sweep (colour 0, as k_smooth0_tiled MODE 0) with the block's
+// parts of the two dot products that follow it, z.r and z.r_prev: b is the CG
+// residual r, and every value of z is in the CTA's hands. They go to
+// dots[2 blk] and dots[2 blk + 1].
+template <typename T, int CPT>
+__global__ void __launch_bounds__(256 / CPT)
+    k_smooth0_dots(GridView g, LevelPtrs<T> lp, const float* __restrict__ b, const float* __restrict__ r_prev,
+                   double* __restrict__ dots, const int* done) {
+  constexpr int NT = 256 / CPT;
+  grid_dependency_wait();
+  if (*done) return;
+  __shared__ float sh[kShell0];
+  __shared__ double red[2 * (NT / 32)];
+  const int blk = blockIdx.x, t = threadIdx.x;
+  const T* __restrict__ x = lp.x;
+  unsigned m[CPT];
+  float b0[CPT], p0[CPT], b1[CPT], p1[CPT], v[CPT], di[CPT];
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    const int i = blk * 512 + t + k * NT;
+    m[k] = lp.mask[i];
+    di[k] = lp.diag[i];
+    b0[k] = b[i];
+    v[k] = ld(&x[i + 256]);
+    p0[k] = r_prev[i];
+    b1[k] = b[i + 256];
+    p1[k] = r_prev[i + 256];
+  }
+  load_halo0<NT, 192, true>(g, blk, 1, sh, [&](int j) { return ld(&x[rb_id(j)]); });
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) sh[sidx(nat_of(256 + t + k * NT))] = v[k];
+  __syncthreads();
+  double zr = 0.0, zp = 0.0;
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    zr += (double)v[k] * (double)b1[k];
+    zp += (double)v[k] * (double)p1[k];
+    if (!(m[k] & 64u)) continue;
+    const int c = t + k * NT;
+    const float s = (b0[k] + nbr_sum0(sh, sidx(nat_of(c)), m[k])) / di[k];
+    st_T(&lp.x[blk * 512 + c], s);
+    const double z = (double)round_T<T>(s);
+    zr += z * (double)b0[k];
+    zp += z * (double)p0[k];
+  }
+  zr = warp_sum(zr);
+  zp = warp_sum(zp);
+  if ((t & 31) == 0) {
+    red[2 * (t >> 5)] = zr;
+    red[2 * (t >> 5) + 1] = zp;
+  }
+  __syncthreads();
+  if (t < 2) {
+    double sum = 0.0;
+    for (int w = 0; w < NT / 32; ++w) sum += red[2 * w + t];
+    dots[2 * blk + t] = sum;
+  }
+}
+
 // Level-0 residual restricted to level 1: all 512 cells of the block and its
 // face halos staged in shared memory.
 template <typename T, int CPT>
@@ -723,20 +782,66 @@ __global__ void __launch_bounds__(512 / CPT)
   }
 }
 
+// Up to this many blocks the flexible-CG scalars are summed by the kernels that
+// use them, every CTA alike, from per-block parts: a few loads a thread, less
+// than a reduction kernel of its own costs in launch and tail (z.r and z.r_prev by
+// the last sweep and the direction: 32^3 host step 1052 -> 1015 us, 128^3 substep
+// 1.022 -> 1.048 times the speed before; alpha by the update: 1081 -> 1052 us and
+// 1.006 -> 1.022, with one diagonal launch for all levels). Above, every CTA would
+// read more partials than its own cells, 160 KB at the 256^3 splash's 10k blocks,
+// and one last CTA summing them was slower than the separate kernel there.
+constexpr int kFuseBlocks = 1024;
+
 // d = z + beta d_old and q = A d for one block, d staged with its halo; the
 // block's d.q partial goes to partial[blk].
-template <typename T, int CPT>
+// With kDots every CTA first forms beta from the per-block parts of z.r and
+// z.r_prev (k_dots does otherwise), CTA 0 keeping z.r for the update.
+template <typename T, int CPT, bool kDots>
 __global__ void __launch_bounds__(512 / CPT)
     k_direction_tiled(GridView g, LevelPtrs<T> L0, const T* __restrict__ z, const float* __restrict__ d_old,
-                      float* __restrict__ d_new, float* __restrict__ q, double* partial, SolverState* st) {
+                      float* __restrict__ d_new, float* __restrict__ q, double* partial,
+                      const double* __restrict__ dots, SolverState* st) {
   constexpr int NT = 512 / CPT;
   grid_dependency_wait();
   if (st->done) return;
   __shared__ float sh[kShell0];
   __shared__ double red[NT / 32];
   const int blk = blockIdx.x, t = threadIdx.x;
-  const float beta = (float)st->beta;
   const bool first = st->inner_iter == 0;
+  float beta;
+  if (kDots) {
+    __shared__ double total[2];
+    const double rz_prev = st->rz_prev;
+    double zr = 0.0, zp = 0.0;
+    for (int k = t; k < g.nb; k += NT) {
+      zr += dots[2 * k];
+      zp += dots[2 * k + 1];
+    }
+    zr = block_sum<NT>(zr, red);
+    zp = block_sum<NT>(zp, red);
+    if (t == 0) {
+      total[0] = zr;
+      total[1] = zp;
+    }
+    __syncthreads();
+    zr = total[0];
+    zp = total[1];
+    if (!(zr > 0.0) || !isfinite(zr)) {  // the same in every CTA
+      if (blk == 0 && t == 0) {
+        st->status = kAborted;
+        st->done = 1;
+      }
+      return;
+    }
+    const double exact = first ? 0.0 : (zr - zp) / rz_prev;
+    beta = (float)exact;
+    if (blk == 0 && t == 0) {
+      st->beta = exact;
+      st->rz = zr;
+    }
+  } else {
+    beta = (float)st->beta;
+  }
   unsigned m[CPT];
   float dg[CPT], di[CPT];
 #pragma unroll
@@ -1270,13 +1375,7 @@ __global__ void k_dots(int n, const T* __restrict__ z, const float* __restrict__
 
 // e += alpha d; r_next = r - alpha q; ||r_next||^2 -> stop test. With kAlpha
 // every CTA forms alpha itself from the nb per-block partials of d.q (as
-// k_direction_finish does otherwise): up to kFuseAlphaBlocks blocks that is a few
-// loads a thread, less than the launch between the two kernels (with one diagonal
-// launch for all levels, the 32^3 host step 1081 -> 1052 us, the 128^3 substep
-// 1.006 -> 1.022 times the speed before). Above, every CTA would read more
-// partials than its own vector pieces, 80 KB at the 256^3 splash's 10k blocks.
-constexpr int kFuseAlphaBlocks = 1024;
-
+// k_direction_finish does otherwise).
 template <bool kAlpha>
 __global__ void __launch_bounds__(kThreads)
     k_update(int n, int nb, const double* __restrict__ dq, const float* __restrict__ d, const float* __restrict__ q,
@@ -1731,7 +1830,7 @@ static void restrict_level(const GridView& g, const MgHierarchy<T>& H, int l, co
 
 template <typename T>
 static void vcycle(const GridView& g, const MgHierarchy<T>& H, const float* r0, const MgOptions& opt,
-                   const int* done, cudaStream_t s) {
+                   const int* done, cudaStream_t s, const float* r_prev = nullptr, double* dots = nullptr) {
   const int L = H.levels;
   // The last dense level and the coarsest in one CTA when both fit.
   const bool tail = L >= 2 && !H.desc[L - 2].sparse && H.desc[L - 2].count <= kTailMaxCells &&
@@ -1768,11 +1867,14 @@ static void vcycle(const GridView& g, const MgHierarchy<T>& H, const float* r0, 
   }
   for (int l = top - 1; l >= 0; --l) {
     const float* bl = l == 0 ? r0 : H.b[l];
-    smooth<T>(g, H, l, bl, 1, 2, done, s);
-    smooth<T>(g, H, l, bl, 0, 0, done, s);
-    for (int sw = 1; sw < opt.post; ++sw) {
-      smooth<T>(g, H, l, bl, 1, 0, done, s);
-      smooth<T>(g, H, l, bl, 0, 0, done, s);
+    for (int sw = 0; sw < opt.post; ++sw) {
+      smooth<T>(g, H, l, bl, 1, sw == 0 ? 2 : 0, done, s);
+      if (l == 0 && sw == opt.post - 1 && dots != nullptr) {
+        ++g_kernel_launches;
+        launch_dep(k_smooth0_dots<T, kSmooth0Cpt>, g.nb, 256 / kSmooth0Cpt, 0, s, g, H.ptr[0], bl, r_prev, dots, done);
+      } else {
+        smooth<T>(g, H, l, bl, 0, 0, done, s);
+      }
     }
   }
 }
@@ -1847,11 +1949,17 @@ cudaError_t launch_fcg_iteration(const GridView& g, const MgHierarchy<T>& H, con
                                  float* r_prev, float* d_old, float* d_new, float* q, float* e, double* partial,
                                  SolverState* st, const int* done, cudaStream_t s, const PrecondHook* hook) {
   const int n = g.nb * kBlockCells;
+  // The dot products' and the update's parts: partial[0, nb) d.q, then up to
+  // kReduceCtas of ||r||^2, then (in the last sweep, without a learned
+  // correction after it) the pairs of z.r and z.r_prev.
+  const bool fused = hook == nullptr && g.nb <= kFuseBlocks;
+  double* update_partial = partial + g.nb;
+  double* dots = update_partial + kReduceCtas;
   if (hook != nullptr && !hook->compose) {
     const cudaError_t e = hook->apply(hook->ctx, r_cur, H.ptr[0].x, s);
     if (e != cudaSuccess) return e;
   } else {
-    vcycle<T>(g, H, r_cur, opt, done, s);
+    vcycle<T>(g, H, r_cur, opt, done, s, r_prev, fused ? dots : nullptr);
     if (hook != nullptr) {  // the learned correction from the V-cycle's residual, added to z (q as scratch)
       ++g_kernel_launches;
       k_residual0_tiled<T, kResidualCpt><<<g.nb, 512 / kResidualCpt, 0, s>>>(g, H.ptr[0], r_cur, q, done);
@@ -1861,11 +1969,17 @@ cudaError_t launch_fcg_iteration(const GridView& g, const MgHierarchy<T>& H, con
   }
   const T* z = H.ptr[0].x;
   const unsigned grid = reduce_grid(n);
-  g_kernel_launches += 3;
-  launch_dep(k_dots<T>, grid, kThreads, 0, s, n, z, r_cur, r_prev, partial, st);
-  launch_dep(k_direction_tiled<T, kDirectionCpt>, g.nb, 512 / kDirectionCpt, 0, s, g, H.ptr[0], z, d_old, d_new, q, partial, st);
-  double* update_partial = partial + g.nb;  // (the d.q partials are read until the update ends)
-  if (g.nb <= kFuseAlphaBlocks) {
+  g_kernel_launches += 2;
+  if (fused) {
+    launch_dep(k_direction_tiled<T, kDirectionCpt, true>, g.nb, 512 / kDirectionCpt, 0, s, g, H.ptr[0], z, d_old, d_new,
+               q, partial, (const double*)dots, st);
+  } else {
+    ++g_kernel_launches;
+    launch_dep(k_dots<T>, grid, kThreads, 0, s, n, z, r_cur, r_prev, partial, st);
+    launch_dep(k_direction_tiled<T, kDirectionCpt, false>, g.nb, 512 / kDirectionCpt, 0, s, g, H.ptr[0], z, d_old,
+               d_new, q, partial, (const double*)nullptr, st);
+  }
+  if (g.nb <= kFuseBlocks) {
     launch_dep(k_update<true>, grid, kThreads, 0, s, n, g.nb, (const double*)partial, d_new, q, r_cur, r_prev, e,
                update_partial, st);
   } else {
