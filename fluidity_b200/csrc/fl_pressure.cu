@@ -26,15 +26,25 @@
 // Gauss-Seidel, `pre` sweeps red->black before and `post` sweeps black->red
 // after the coarse correction (symmetric); the restriction into a level also
 // performs that level's first sweep; the coarsest level is solved by
-// `coarse_sweeps` symmetric sweeps inside one CTA's shared memory, together
-// with the last dense level when both fit (k_coarse_tail). x and k are stored
-// as T (FP32 or BF16), arithmetic is FP32.
+// `coarse_sweeps` symmetric sweeps in shared memory, and it and the levels above
+// it that fit run as one cluster kernel (k_coarse_cluster). x and k are stored
+// as T (FP32 or BF16; the cluster's iterates in FP32), arithmetic is FP32.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
+
+#include <atomic>
 
 #include "fl_internal.cuh"
 #include "fl_kernels.h"
 
 namespace fl {
+
+// Lets the grid that depends on this one start its CTAs once all of this grid's
+// have started: called by the restriction into the cluster kernel, whose loads of
+// the coarse operator then overlap it. Everywhere else the dependent kernel has
+// nothing to do before its wait and its CTAs only take the running grid's place
+// (every kernel calling it: 1.96 against 1.88 ms for the 128^3 substep).
+__device__ __forceinline__ void release_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 constexpr int kThreads = 256;
 constexpr int kReduceCtas = 4 * 148;  // fixed grid of the reduction kernels (multiple of the SM count)
@@ -377,6 +387,7 @@ __global__ void __launch_bounds__(512)
     k_restrict_sparse(GridView g, LevelPtrs<T> fp, const float* __restrict__ fb, float* cb, int cdx, int cdy,
                       LevelPtrs<T> cp, int cparity, int seed, const int* done) {
   static_assert(LS == 1 || LS == 2, "level 0 has its own kernel");
+  if (!seed) release_dependents();
   grid_dependency_wait();
   if (*done) return;
   constexpr int S = 1 << LS, S3 = S * S * S, BPC = 512 / S3;
@@ -705,6 +716,7 @@ __global__ void __launch_bounds__(512 / CPT)
                       LevelPtrs<T> cp, int seed, const int* done) {
   constexpr int NT = 512 / CPT;
   static_assert(NT >= 64, "one thread per level-1 cell of the block");
+  if (!seed) release_dependents();
   grid_dependency_wait();
   if (*done) return;
   __shared__ float sh[kShell0];
@@ -949,6 +961,7 @@ __global__ void k_smooth_dense(LevelDesc L, LevelPtrs<T> lp, const float* __rest
 template <typename T>
 __global__ void k_restrict_dense(LevelDesc F, LevelPtrs<T> fp, const float* __restrict__ fb, LevelDesc C, float* cb,
                                  LevelPtrs<T> cp, int seed, const int* done) {
+  if (!seed) release_dependents();
   grid_dependency_wait();
   if (*done) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1072,184 +1085,607 @@ __global__ void __launch_bounds__(1024) k_coarse_solve(LevelDesc L, LevelPtrs<T>
   for (int i = threadIdx.x; i < n; i += blockDim.x) st_T(&lp.x[i], lp.fluid[i] ? x[i] : 0.0f);
 }
 
-// Coarse tail of the V-cycle in one CTA: the last dense level F (at most
-// kTailMaxCells cells) pre-smoothed, its residual restricted to the coarsest
-// level C, C solved by symmetric sweeps, then F corrected and post-smoothed,
-// all in shared memory. The sweeps, restriction and coarsest solve are those
-// of k_smooth_dense, k_restrict_dense and k_coarse_solve, in the same order;
-// F's iterate stays in FP32 between them (one launch instead of ten).
-constexpr int kTailMaxCells = 4096;
-constexpr int kTailThreads = 1024;
-constexpr int kTailCpt = kTailMaxCells / kTailThreads;
+// ----------------------------------------------------------------- coarse levels in one cluster
 
-__host__ __device__ constexpr size_t tail_smem_bytes(int nf, int nc) {
-  return sizeof(float) * (7 * (size_t)nf + 6 * (size_t)nc) + (size_t)nf;
+// The V-cycle from level l0 down to the coarsest and back in ONE launch: a
+// cluster of up to 16 CTAs holds every level's operator, right-hand side and
+// iterate in its shared memory, values of neighbouring CTAs are read through
+// distributed shared memory, and the sweeps are separated by cluster barriers.
+// Bound by latency, not by bandwidth: a coarse colour sweep is a few hundred
+// nanoseconds of work, so as a launch of its own it costs its launch and two
+// dependent global round trips, and the coarsest pair in one CTA is limited by
+// one SM's issue rate. A sweep with its barrier takes ~1 us here. In place of two
+// launches per sweep above a one-CTA tail: the 32^3 host step 1015 -> 926 us (levels
+// from 1 on), the 128^3 substep 1.048 -> 1.104 times the speed before both (levels
+// from 2 on, 28 us a V-cycle), the 256^3 splash's even (levels from 3 on).
+// The operator does not change during a solve, so it is loaded before the
+// wait for the previous kernel and overlaps that kernel's tail.
+// Sparse levels (1: 4^3, 2: 2^3 cells per block) are dealt by runs of `per`
+// blocks, cells red-black within the block; dense levels by runs of 2^shift
+// linear cells; the coarsest level is held and solved by every CTA, which
+// saves the exchange of its result. The sums are those of k_smooth_sparse,
+// k_smooth_dense, the restrictions and k_coarse_solve in the same order; the
+// iterates stay in FP32 between sweeps.
+constexpr int kClThreads = 1024;
+constexpr int kClMaxLevels = 12;
+constexpr size_t kClSmemMax = 227 * 1024;
+constexpr int kClCoarsestMax = 1024;  // one cell per thread
+// Cells of a level per CTA. A sweep over more is bound by the 16 SMs' issue rate
+// and the per-level kernels on the whole chip win: with 8192 the 256^3 splash ran
+// at 0.973 times the speed of the solver before and the 104 x 184 x 136 column
+// drop at 0.926, with 2048 at 1.013 and 1.053.
+constexpr int kClCellsMax = 2048;
+
+struct ClLevel {
+  int per;    // blocks per CTA (sparse) or log2 of the cells per CTA (dense)
+  int cells;  // cells of one CTA
+  int x, b, d, r, k, nbr;  // byte offsets in shared memory (r: dense levels, nbr: sparse levels)
+};
+
+template <typename T>
+struct ClArgs {
+  GridView g;
+  int l0, levels, pre, post, sweeps, ctas;
+  int xc, bc, dc, kc;  // coarsest level's arrays
+  const float* b0;
+  const int* done;
+  LevelDesc desc[kClMaxLevels];
+  LevelPtrs<T> ptr[kClMaxLevels];
+  ClLevel lay[kClMaxLevels];
+};
+
+// Shared-memory layout for the levels l0 .. L - 1 on `ctas` CTAs; the bytes of one CTA.
+template <typename T>
+static size_t cl_layout(const MgHierarchy<T>& H, int nb, int l0, int ctas, ClArgs<T>& A) {
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    const size_t o = off;
+    off += (bytes + 15) / 16 * 16;
+    return (int)o;
+  };
+  for (int l = l0; l < H.levels - 1; ++l) {
+    const LevelDesc& D = H.desc[l];
+    ClLevel& P = A.lay[l];
+    P = ClLevel{};
+    if (D.sparse) {
+      P.per = (nb + ctas - 1) / ctas;
+      P.cells = P.per * D.S * D.S * D.S;
+      P.nbr = take(sizeof(unsigned) * 6 * P.per);
+    } else {
+      while (((long long)ctas << P.per) < D.count) ++P.per;
+      P.cells = 1 << P.per;
+      P.r = take(sizeof(float) * P.cells);
+    }
+    P.x = take(sizeof(float) * P.cells);
+    P.b = take(sizeof(float) * P.cells);
+    P.d = take(sizeof(float) * P.cells);
+    P.k = take(sizeof(T) * 6 * P.cells);
+    if (P.cells > kClCellsMax) return kClSmemMax + 1;
+    if (off > kClSmemMax) return off;
+  }
+  const size_t nc = (size_t)H.desc[H.levels - 1].count;
+  A.xc = take(sizeof(float) * nc);
+  A.bc = take(sizeof(float) * nc);
+  A.dc = take(sizeof(float) * nc);
+  A.kc = take(sizeof(float) * 3 * nc);
+  return off;
+}
+
+__device__ __forceinline__ unsigned cl_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Address of shared-memory address `a` of this CTA in CTA `rank` of the cluster.
+__device__ __forceinline__ unsigned cl_map(unsigned a, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float cl_ld(unsigned a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void cl_st(unsigned a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cl_sync() { cooperative_groups::this_cluster().sync(); }
+
+// One CTA's view of a level in shared memory.
+template <typename T>
+struct ClView {
+  float *x, *b, *d, *r;
+  T* k;           // [6][cells], axis/direction order
+  unsigned* nbr;  // [block][6]: cluster address of the neighbouring block's x
+  unsigned xa, ba, da, ra;  // shared addresses of x, b, d and r
+  int cells, per;
+};
+template <typename T>
+__device__ __forceinline__ ClView<T> cl_view(unsigned char* sm, const ClLevel& P) {
+  ClView<T> v;
+  v.x = reinterpret_cast<float*>(sm + P.x);
+  v.b = reinterpret_cast<float*>(sm + P.b);
+  v.d = reinterpret_cast<float*>(sm + P.d);
+  v.r = reinterpret_cast<float*>(sm + P.r);
+  v.k = reinterpret_cast<T*>(sm + P.k);
+  v.nbr = reinterpret_cast<unsigned*>(sm + P.nbr);
+  const unsigned base = (unsigned)__cvta_generic_to_shared(sm);
+  v.xa = base + P.x;
+  v.ba = base + P.b;
+  v.da = base + P.d;
+  v.ra = base + P.r;
+  v.cells = P.cells;
+  v.per = P.per;
+  return v;
+}
+
+// Sparse levels: cell (x, y, z) of a block sits at colour * HALF + row * (S / 2) + x / 2.
+template <int LS>
+struct ClSparse {
+  static constexpr int S = 1 << LS, S3 = S * S * S, HALF = S3 / 2;
+  static __device__ __forceinline__ int at(int x, int y, int z) {
+    return ((x + y + z) & 1) * HALF + ((z * S + y) * S + x) / 2;
+  }
+};
+
+template <typename T, int LS>
+__device__ void cl_load_sparse(const GridView& g, const LevelPtrs<T>& lp, const ClView<T>& v, int blocks, int first) {
+  using Q = ClSparse<LS>;
+  for (int e = threadIdx.x; e < blocks * 6; e += kClThreads) {
+    const int q = e % 6, a = q >> 1, dir = (q & 1) ? 1 : -1;
+    const int n = g.nbr27[(first + e / 6) * 27 + 13 + dir * (a == 0 ? 1 : (a == 1 ? 3 : 9))];
+    const int to = n >= 0 ? n : first + e / 6;  // a missing block is never weighted: any valid address
+    v.nbr[e] = cl_map(v.xa + (unsigned)(to % v.per) * Q::S3 * 4u, (unsigned)(to / v.per));
+  }
+  for (int c = threadIdx.x; c < blocks * Q::S3; c += kClThreads) {
+    const int bl = c / Q::S3, l = c % Q::S3, blk = first + bl, i = blk * Q::S3 + l;
+    const int x = l & (Q::S - 1), y = (l >> LS) & (Q::S - 1), z = l >> (2 * LS);
+    const int o = bl * Q::S3 + Q::at(x, y, z);
+    const bool fluid = lp.fluid[i] != 0;
+    const float d = lp.diag[i];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const int jn = nbr_s<LS>(g, blk, l, q >> 1, (q & 1) ? 1 : -1);
+      st_T(&v.k[q * v.cells + o], jn >= 0 ? ld(&lp.k[q >> 1][(q & 1) ? jn : i]) : 0.0f);
+    }
+    v.d[o] = fluid ? d : 0.0f;
+    v.x[o] = 0.0f;
+  }
+}
+
+// The six neighbours of one cell position in a block: where they sit in their
+// block's part of x, and which of them lie in the cell's own block. Worked out
+// once per sweep: a thread keeps its position and strides over blocks.
+template <int LS>
+struct ClNeighbours {
+  int at[6];
+  unsigned own;  // bit q: neighbour q is in the same block
+  __device__ __forceinline__ ClNeighbours(int x, int y, int z) {
+    using Q = ClSparse<LS>;
+    const int c[3] = {x, y, z};
+    own = 0;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const int a = q >> 1, dir = (q & 1) ? 1 : -1;
+      int n[3] = {c[0], c[1], c[2]};
+      n[a] += dir;
+      if (n[a] >= 0 && n[a] < Q::S) own |= 1u << q;
+      n[a] &= Q::S - 1;
+      at[q] = Q::at(n[0], n[1], n[2]);
+    }
+  }
+};
+
+// s plus (minus) the six weighted neighbours of cell o of local block bl, in axis/direction order.
+template <typename T, int LS>
+__device__ __forceinline__ float cl_sum_sparse(const ClView<T>& v, const ClNeighbours<LS>& n, int bl, int o, float s,
+                                               bool minus) {
+  using Q = ClSparse<LS>;
+  float kq[6], xq[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    kq[q] = ld(&v.k[q * v.cells + o]);
+    xq[q] = (n.own >> q) & 1u ? v.x[bl * Q::S3 + n.at[q]] : cl_ld(v.nbr[bl * 6 + q] + 4u * (unsigned)n.at[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < 6; ++q)
+    if (kq[q] != 0.0f) s = fmaf(minus ? -kq[q] : kq[q], xq[q], s);
+  return s;
+}
+
+template <typename T, int LS>
+__device__ void cl_sweep_sparse(const ClView<T>& v, int blocks, int color) {
+  using Q = ClSparse<LS>;
+  const int j = threadIdx.x % Q::HALF, row = j / (Q::S / 2), y = row & (Q::S - 1), z = row >> LS;
+  const ClNeighbours<LS> n(2 * (j % (Q::S / 2)) + ((y + z + color) & 1), y, z);
+  for (int bl = threadIdx.x / Q::HALF; bl < blocks; bl += kClThreads / Q::HALF) {
+    const int o = bl * Q::S3 + color * Q::HALF + j;
+    const float d = v.d[o];
+    if (d != 0.0f) v.x[o] = cl_sum_sparse<T, LS>(v, n, bl, o, v.b[o], false) / d;
+  }
+}
+
+// Residual summed over 2x2x2 children in (z, y, x) order: level 1 into level 2's
+// cell of the same block (b and the colour-0 first sweep), level 2 into the
+// dense cell of the block.
+template <typename T, int LS, typename F>
+__device__ void cl_restrict_sparse(const ClView<T>& v, int blocks, F store) {
+  using Q = ClSparse<LS>;
+  const int l = threadIdx.x % Q::S3, x = l & (Q::S - 1), y = (l >> LS) & (Q::S - 1), z = l >> (2 * LS);
+  const ClNeighbours<LS> n(x, y, z);
+  const int at = Q::at(x, y, z), warp_bl = (threadIdx.x & ~31) / Q::S3;
+  for (int k = 0; warp_bl + k < blocks; k += kClThreads / Q::S3) {  // uniform over the warp
+    const int bl = threadIdx.x / Q::S3 + k;
+    float res = 0.0f;
+    if (bl < blocks) {
+      const int o = bl * Q::S3 + at;
+      const float d = v.d[o];
+      if (d != 0.0f) res = v.b[o] - cl_sum_sparse<T, LS>(v, n, bl, o, d * v.x[o], true);
+    }
+    float sum = 0.0f;
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch)
+      sum += __shfl_down_sync(0xffffffffu, res, (ch & 1) + ((ch >> 1) & 1) * Q::S + (ch >> 2) * Q::S * Q::S);
+    if (bl < blocks && !((x | y | z) & 1)) store(bl, x / 2, y / 2, z / 2, sum);
+  }
+}
+
+__device__ __forceinline__ int dense_colour(const LevelDesc& L, int i) {
+  return (i % L.dim[0] + (i / L.dim[0]) % L.dim[1] + i / (L.dim[0] * L.dim[1]) + L.parity) & 1;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kTailThreads)
-    k_coarse_tail(LevelDesc F, LevelPtrs<T> fp, const float* __restrict__ fb, LevelDesc C, LevelPtrs<T> cp,
-                  float* __restrict__ cb, int pre, int post, int sweeps, const int* done) {
-  grid_dependency_wait();
-  if (*done) return;
-  extern __shared__ float sm[];
-  const int nf = (int)F.count, nc = (int)C.count;
-  float* x = sm;                 // F iterate
-  float* bf = x + nf;            // F right-hand side
-  float* df = bf + nf;           // F diagonal
-  float* kf[3] = {df + nf, df + 2 * nf, df + 3 * nf};
-  float* xc = df + 4 * nf;       // C iterate
-  float* bc = xc + nc;           // C right-hand side
-  float* dc = bc + nc;           // C diagonal of fluid cells, 0 elsewhere
-  float* kc[3] = {dc + nc, dc + 2 * nc, dc + 3 * nc};
-  float* rf = kc[2] + nc;        // F residual before the restriction
-  unsigned char* ff = reinterpret_cast<unsigned char*>(rf + nf);  // F fluid flags
-  const int t = threadIdx.x;
-  for (int i = t; i < nf; i += kTailThreads) {
-    x[i] = 0.0f;
-    bf[i] = fb[i];
-    df[i] = fp.diag[i];
-    ff[i] = fp.fluid[i];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) kf[a][i] = ld(&fp.k[a][i]);
-  }
-  for (int i = t; i < nc; i += kTailThreads) {
-    xc[i] = 0.0f;
-    dc[i] = cp.fluid[i] ? cp.diag[i] : 0.0f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) kc[a][i] = ld(&cp.k[a][i]);
-  }
-  // This thread's F cells, worked out once (in `info`): the in-range face
-  // neighbours (bits 0-5, axis/direction order), the colour (bit 6) and
-  // whether the cell exists (bit 7).
-  const int nx = F.dim[0], nxy = F.dim[0] * F.dim[1];
-  unsigned info[kTailCpt];
-#pragma unroll
-  for (int j = 0; j < kTailCpt; ++j) {
-    const int i = t + j * kTailThreads;
-    const int c0 = i % nx, c1 = (i / nx) % F.dim[1], c2 = i / nxy;
-    unsigned m = 0;
-    m |= (c0 > 0 ? 1u : 0u) | (c0 + 1 < F.dim[0] ? 2u : 0u);
-    m |= (c1 > 0 ? 4u : 0u) | (c1 + 1 < F.dim[1] ? 8u : 0u);
-    m |= (c2 > 0 ? 16u : 0u) | (c2 + 1 < F.dim[2] ? 32u : 0u);
-    info[j] = m | ((unsigned)((c0 + c1 + c2 + F.parity) & 1) << 6) | (i < nf ? 128u : 0u);
-  }
-  const int off[6] = {-1, 1, -nx, nx, -nxy, nxy};  // face neighbours in axis/direction order
-  __syncthreads();
-  // One colour sweep on F: mode 1 from zero, mode 2 with the coarse correction
-  // added to the neighbour values read (as k_smooth_dense).
-  auto sweep = [&](int color, int mode) {
-#pragma unroll
-    for (int j = 0; j < kTailCpt; ++j) {
-      const unsigned inf = info[j];
-      const int i = t + j * kTailThreads;
-      if (!(inf & 128u) || (int)((inf >> 6) & 1u) != color || !ff[i]) continue;
-      float s = bf[i];
-      if (mode != 1) {
-        const int c[3] = {i % nx, (i / nx) % F.dim[1], i / nxy};  // used by mode 2 only
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-          if (!((inf >> q) & 1u)) continue;
-          const int a = q >> 1, jn = i + off[q];
-          const float kq = (q & 1) ? kf[a][jn] : kf[a][i];
-          float xv = x[jn];
-          if (mode == 2) {
-            int n[3] = {c[0], c[1], c[2]};
-            n[a] += (q & 1) ? 1 : -1;
-            xv += xc[dense_id(C, n[0] >> 1, n[1] >> 1, n[2] >> 1)];
-          }
-          if (kq != 0.0f) s = fmaf(kq, xv, s);
-        }
-      }
-      x[i] = s / df[i];
-    }
-    __syncthreads();
-  };
-  sweep(0, 1);
-  sweep(1, 0);
-  for (int sw = 1; sw < pre; ++sw) {
-    sweep(0, 0);
-    sweep(1, 0);
-  }
-  // Residual of F (every cell, all threads), then restricted to C in the
-  // children order of k_restrict_dense, one thread per C cell.
-#pragma unroll
-  for (int j = 0; j < kTailCpt; ++j) {
-    const unsigned inf = info[j];
-    const int i = t + j * kTailThreads;
-    if (!(inf & 128u) || !ff[i]) continue;
-    float ax = df[i] * x[i];
+__device__ void cl_load_dense(const LevelDesc& L, const LevelPtrs<T>& lp, const ClView<T>& v, int first) {
+  const int nx = L.dim[0], nxy = L.dim[0] * L.dim[1];
+  for (int c = threadIdx.x; c < v.cells; c += kClThreads) {
+    const int i = first + c;
+    v.x[c] = 0.0f;
+    v.b[c] = 0.0f;  // cells of inactive blocks receive no sum
+    v.d[c] = 0.0f;
+    if (i >= (int)L.count) continue;
+    const int p[3] = {i % nx, (i / nx) % L.dim[1], i / nxy};
+    const int step[3] = {1, nx, nxy};
+    const bool fluid = lp.fluid[i] != 0;
+    const float d = lp.diag[i];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
-      if (!((inf >> q) & 1u)) continue;
-      const int a = q >> 1, jn = i + off[q];
-      const float kq = (q & 1) ? kf[a][jn] : kf[a][i];
-      if (kq != 0.0f) ax = fmaf(-kq, x[jn], ax);
+      const int a = q >> 1;
+      const bool ok = (q & 1) ? p[a] + 1 < L.dim[a] : p[a] > 0;
+      st_T(&v.k[q * v.cells + c], ok ? ld(&lp.k[a][(q & 1) ? i + step[a] : i]) : 0.0f);
     }
-    rf[i] = bf[i] - ax;
+    if (fluid) v.d[c] = dense_colour(L, i) == 0 ? d : -d;  // the sign holds the colour
   }
-  __syncthreads();
-  for (int I = t; I < nc; I += kTailThreads) {
-    const int X = I % C.dim[0], Y = (I / C.dim[0]) % C.dim[1], Z = I / (C.dim[0] * C.dim[1]);
-    float sum = 0.0f;
+}
+
+// x of dense cell j (r of it with `addr` = the residuals' address): own or another CTA's.
+template <typename T>
+__device__ __forceinline__ float cl_dense_at(const ClView<T>& v, const float* own, unsigned addr, int j, int first) {
+  const int c = j - first;
+  if (c >= 0 && c < v.cells) return own[c];
+  return cl_ld(cl_map(addr + 4u * (unsigned)(j & (v.cells - 1)), (unsigned)(j >> v.per)));
+}
+
+template <typename T>
+__device__ __forceinline__ float cl_sum_dense(const LevelDesc& L, const ClView<T>& v, int first, int c, float s,
+                                              bool minus) {
+  const int nx = L.dim[0], nxy = L.dim[0] * L.dim[1];
+  const int step[6] = {-1, 1, -nx, nx, -nxy, nxy};
+  float kq[6], xq[6];
 #pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-      const int c[3] = {2 * X + (ch & 1), 2 * Y + ((ch >> 1) & 1), 2 * Z + (ch >> 2)};
-      if (c[0] >= F.dim[0] || c[1] >= F.dim[1] || c[2] >= F.dim[2]) continue;
-      const int id = dense_id(F, c[0], c[1], c[2]);
-      if (ff[id]) sum += rf[id];
+  for (int q = 0; q < 6; ++q) {
+    kq[q] = ld(&v.k[q * v.cells + c]);
+    xq[q] = kq[q] != 0.0f ? cl_dense_at(v, v.x, v.xa, first + c + step[q], first) : 0.0f;
+  }
+#pragma unroll
+  for (int q = 0; q < 6; ++q)
+    if (kq[q] != 0.0f) s = fmaf(minus ? -kq[q] : kq[q], xq[q], s);
+  return s;
+}
+
+template <typename T>
+__device__ void cl_sweep_dense(const LevelDesc& L, const ClView<T>& v, int first, int color) {
+  for (int c = threadIdx.x; c < v.cells; c += kClThreads) {
+    const float d = color == 0 ? v.d[c] : -v.d[c];
+    if (d > 0.0f) v.x[c] = cl_sum_dense(L, v, first, c, v.b[c], false) / d;
+  }
+}
+
+// Sum over the children of coarse cell I (of level C) of the finer dense level's residuals.
+template <typename T>
+__device__ __forceinline__ float cl_children(const LevelDesc& F, const ClView<T>& fv, int ffirst, const LevelDesc& C,
+                                             int I) {
+  const int X = I % C.dim[0], Y = (I / C.dim[0]) % C.dim[1], Z = I / (C.dim[0] * C.dim[1]);
+  float r[8];
+#pragma unroll
+  for (int ch = 0; ch < 8; ++ch) {
+    const int x = 2 * X + (ch & 1), y = 2 * Y + ((ch >> 1) & 1), z = 2 * Z + (ch >> 2);
+    const bool inside = x < F.dim[0] && y < F.dim[1] && z < F.dim[2];
+    r[ch] = inside ? cl_dense_at(fv, fv.r, fv.ra, dense_id(F, x, y, z), ffirst) : 0.0f;
+  }
+  float sum = 0.0f;
+#pragma unroll
+  for (int ch = 0; ch < 8; ++ch) sum += r[ch];
+  return sum;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kClThreads, 1) k_coarse_cluster(const __grid_constant__ ClArgs<T> A) {
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  const int t = threadIdx.x;
+  const unsigned rank = cl_rank();
+  const int last = A.levels - 1;
+  const LevelDesc& C = A.desc[last];
+  const LevelPtrs<T>& cp = A.ptr[last];
+  float* xc = reinterpret_cast<float*>(cl_smem + A.xc);
+  float* bc = reinterpret_cast<float*>(cl_smem + A.bc);
+  float* dc = reinterpret_cast<float*>(cl_smem + A.dc);
+  float* kc = reinterpret_cast<float*>(cl_smem + A.kc);
+  const unsigned bca = (unsigned)__cvta_generic_to_shared(bc);
+  const int nc = (int)C.count;
+  auto first_of = [&](int l) { return A.desc[l].sparse ? (int)rank * A.lay[l].per : (int)rank << A.lay[l].per; };
+  auto blocks_of = [&](int l) { return max(0, min(A.lay[l].per, A.g.nb - (int)rank * A.lay[l].per)); };
+  // the operator (constant during the solve)
+  for (int l = A.l0; l < last; ++l) {
+    const ClView<T> v = cl_view<T>(cl_smem, A.lay[l]);
+    if (l == 1)
+      cl_load_sparse<T, 2>(A.g, A.ptr[l], v, blocks_of(l), first_of(l));
+    else if (l == 2)
+      cl_load_sparse<T, 1>(A.g, A.ptr[l], v, blocks_of(l), first_of(l));
+    else
+      cl_load_dense(A.desc[l], A.ptr[l], v, first_of(l));
+  }
+  for (int i = t; i < nc; i += kClThreads) {
+    xc[i] = 0.0f;
+    bc[i] = 0.0f;  // cells of inactive blocks receive no sum
+    dc[i] = cp.fluid[i] ? cp.diag[i] : 0.0f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) kc[a * nc + i] = ld(&cp.k[a][i]);
+  }
+  grid_dependency_wait();
+  const bool skip = *A.done != 0;  // the same for every CTA
+  if (skip) return;
+  // level l0: right-hand side and first sweep (colour 0 from zero)
+  {
+    const ClView<T> v = cl_view<T>(cl_smem, A.lay[A.l0]);
+    const int first = first_of(A.l0);
+    __syncthreads();
+    if (A.l0 < 3) {
+      const int LS = 3 - A.l0, S = 1 << LS, S3 = S * S * S, n = blocks_of(A.l0) * S3;
+      for (int c = t; c < n; c += kClThreads) {
+        const int bl = c / S3, l = c % S3, x = l & (S - 1), y = (l >> LS) & (S - 1), z = l >> (2 * LS);
+        const int o = bl * S3 + (((x + y + z) & 1) ? S3 / 2 : 0) + ((z * S + y) * S + x) / 2;
+        const float bi = A.b0[(size_t)first * S3 + c], d = v.d[o];
+        v.b[o] = bi;
+        if (d != 0.0f && !((x + y + z) & 1)) v.x[o] = bi / d;
+      }
+    } else {
+      for (int c = t; c < v.cells; c += kClThreads) {
+        const int i = first + c;
+        if (i >= (int)A.desc[A.l0].count || v.d[c] == 0.0f) continue;
+        const float bi = A.b0[i];
+        v.b[c] = bi;
+        if (v.d[c] > 0.0f) v.x[c] = bi / v.d[c];
+      }
     }
-    bc[I] = sum;
-    cb[I] = sum;
+  }
+  cl_sync();
+  auto sweep = [&](int l, int color) {
+    const ClView<T> v = cl_view<T>(cl_smem, A.lay[l]);
+    if (l == 1)
+      cl_sweep_sparse<T, 2>(v, blocks_of(l), color);
+    else if (l == 2)
+      cl_sweep_sparse<T, 1>(v, blocks_of(l), color);
+    else
+      cl_sweep_dense(A.desc[l], v, first_of(l), color);
+    cl_sync();
+  };
+  for (int l = A.l0; l < last; ++l) {
+    sweep(l, 1);
+    for (int sw = 1; sw < A.pre; ++sw) {
+      sweep(l, 0);
+      sweep(l, 1);
+    }
+    // residual, restricted to the next level with that level's first sweep
+    const ClView<T> v = cl_view<T>(cl_smem, A.lay[l]);
+    const int first = first_of(l);
+    if (l == 1) {
+      const ClView<T> w = cl_view<T>(cl_smem, A.lay[2]);
+      cl_restrict_sparse<T, 2>(v, blocks_of(l), [&](int bl, int x, int y, int z, float sum) {
+        const int o = bl * 8 + ClSparse<1>::at(x, y, z);
+        w.b[o] = sum;
+        if (w.d[o] != 0.0f && !((x + y + z) & 1)) w.x[o] = sum / w.d[o];
+      });
+    } else if (l == 2) {
+      const LevelDesc& D = A.desc[3];
+      cl_restrict_sparse<T, 1>(v, blocks_of(l), [&](int bl, int, int, int, float sum) {
+        const int* co = A.g.coord + 3 * (first + bl);
+        const int X = co[0] - A.g.blo[0], Y = co[1] - A.g.blo[1], Z = co[2] - A.g.blo[2];
+        const int id = (Z * D.dim[1] + Y) * D.dim[0] + X;
+        if (last == 3) {  // the coarsest level: every CTA's copy
+          for (int c = 0; c < A.ctas; ++c) cl_st(cl_map(bca + 4u * (unsigned)id, (unsigned)c), sum);
+          return;
+        }
+        const ClView<T> w = cl_view<T>(cl_smem, A.lay[3]);
+        const unsigned to = (unsigned)(id >> w.per), at = 4u * (unsigned)(id & (w.cells - 1));
+        cl_st(cl_map(w.ba + at, to), sum);
+        const float d = cl_ld(cl_map(w.da + at, to));
+        if (d > 0.0f) cl_st(cl_map(w.xa + at, to), sum / d);
+      });
+    } else {
+      for (int c = t; c < v.cells; c += kClThreads) {
+        const float d = fabsf(v.d[c]);
+        v.r[c] = d != 0.0f ? v.b[c] - cl_sum_dense(A.desc[l], v, first, c, d * v.x[c], true) : 0.0f;
+      }
+      cl_sync();
+      const LevelDesc& D = A.desc[l + 1];
+      if (l + 1 == last) {
+        for (int I = t; I < nc; I += kClThreads) bc[I] = cl_children(A.desc[l], v, first, D, I);
+      } else {
+        const ClView<T> w = cl_view<T>(cl_smem, A.lay[l + 1]);
+        const int wfirst = first_of(l + 1);
+        for (int c = t; c < w.cells; c += kClThreads) {
+          const int I = wfirst + c;
+          if (I >= (int)D.count) continue;
+          const float sum = cl_children(A.desc[l], v, first, D, I);
+          w.b[c] = sum;
+          if (w.d[c] > 0.0f) w.x[c] = sum / w.d[c];
+        }
+      }
+    }
+    if (l + 1 < last || l == 2) cl_sync();
   }
   __syncthreads();
-  // Coarsest level: symmetric red-black sweeps, one cell per thread (as k_coarse_solve).
-  {
-    const int i = t;
+  // coarsest level: symmetric red-black sweeps, one cell per thread (as k_coarse_solve)
+  if (t < (nc + 31) / 32 * 32) {
+    const int i = t, nx = C.dim[0], ny = C.dim[1], nz = C.dim[2];
     bool active = false;
     int color = 0;
     float kk[6] = {0, 0, 0, 0, 0, 0}, inv = 0.0f, bi = 0.0f;
     int nb[6] = {0, 0, 0, 0, 0, 0};
-    const int nx = C.dim[0], ny = C.dim[1], nz = C.dim[2];
     if (i < nc && dc[i] != 0.0f) {
       active = true;
       const int X = i % nx, Y = (i / nx) % ny, Z = i / (nx * ny);
       color = (X + Y + Z + C.parity) & 1;
       inv = 1.0f / dc[i];
       bi = bc[i];
-      if (X > 0) { kk[0] = kc[0][i]; nb[0] = i - 1; }
-      if (X + 1 < nx) { kk[1] = kc[0][i + 1]; nb[1] = i + 1; }
-      if (Y > 0) { kk[2] = kc[1][i]; nb[2] = i - nx; }
-      if (Y + 1 < ny) { kk[3] = kc[1][i + nx]; nb[3] = i + nx; }
-      if (Z > 0) { kk[4] = kc[2][i]; nb[4] = i - nx * ny; }
-      if (Z + 1 < nz) { kk[5] = kc[2][i + nx * ny]; nb[5] = i + nx * ny; }
+      if (X > 0) { kk[0] = kc[i]; nb[0] = i - 1; }
+      if (X + 1 < nx) { kk[1] = kc[i + 1]; nb[1] = i + 1; }
+      if (Y > 0) { kk[2] = kc[nc + i]; nb[2] = i - nx; }
+      if (Y + 1 < ny) { kk[3] = kc[nc + i + nx]; nb[3] = i + nx; }
+      if (Z > 0) { kk[4] = kc[2 * nc + i]; nb[4] = i - nx * ny; }
+      if (Z + 1 < nz) { kk[5] = kc[2 * nc + i + nx * ny]; nb[5] = i + nx * ny; }
     }
-    for (int pass = 0; pass < 4 * sweeps; ++pass) {
+    const int warps = (nc + 31) / 32 * 32;
+    for (int pass = 0; pass < 4 * A.sweeps; ++pass) {
       const int half = pass % 2;
-      const int c = pass < 2 * sweeps ? half : 1 - half;
+      const int c = pass < 2 * A.sweeps ? half : 1 - half;
       if (active && color == c) {
-        float sacc = bi;
+        float s = bi;
 #pragma unroll
-        for (int q = 0; q < 6; ++q) sacc = fmaf(kk[q], xc[nb[q]], sacc);
-        xc[i] = sacc * inv;
+        for (int q = 0; q < 6; ++q) s = fmaf(kk[q], xc[nb[q]], s);
+        xc[i] = s * inv;
       }
-      __syncthreads();
+      asm volatile("barrier.sync 1, %0;" ::"r"(warps) : "memory");
     }
-    if (i < nc) st_T(&cp.x[i], cp.fluid[i] ? xc[i] : 0.0f);
   }
   __syncthreads();
-  sweep(1, 2);
-  sweep(0, 0);
-  for (int sw = 1; sw < post; ++sw) {
-    sweep(1, 0);
-    sweep(0, 0);
+  // back up: correct colour 0 (all the first sweep reads), then sweep 1, 0, ...
+  for (int l = last - 1; l >= A.l0; --l) {
+    const ClView<T> v = cl_view<T>(cl_smem, A.lay[l]);
+    const int first = first_of(l);
+    if (l < 3) {
+      const int LS = 3 - l, S = 1 << LS, HALF = S * S * S / 2, n = blocks_of(l) * HALF;
+      for (int e = t; e < n; e += kClThreads) {
+        const int bl = e / HALF, j = e % HALF, o = bl * 2 * HALF + j;
+        if (v.d[o] == 0.0f) continue;
+        if (l == 1) {
+          const int row = j / 2, y = row & 3, z = row >> 2, x = 2 * (j & 1) + ((y + z) & 1);
+          const ClView<T> w = cl_view<T>(cl_smem, A.lay[2]);
+          v.x[o] += w.x[bl * 8 + ClSparse<1>::at(x >> 1, y >> 1, z >> 1)];
+        } else {
+          const int* co = A.g.coord + 3 * (first + bl);
+          const LevelDesc& D = A.desc[3];
+          const int id = ((co[2] - A.g.blo[2]) * D.dim[1] + (co[1] - A.g.blo[1])) * D.dim[0] + (co[0] - A.g.blo[0]);
+          if (last == 3) {
+            v.x[o] += xc[id];
+          } else {
+            const ClView<T> w = cl_view<T>(cl_smem, A.lay[3]);
+            v.x[o] += cl_dense_at(w, w.x, w.xa, id, first_of(3));
+          }
+        }
+      }
+    } else {
+      const LevelDesc& F = A.desc[l];
+      const LevelDesc& D = A.desc[l + 1];
+      for (int c = t; c < v.cells; c += kClThreads) {
+        const int i = first + c;
+        if (!(v.d[c] > 0.0f)) continue;
+        const int id = dense_id(D, (i % F.dim[0]) >> 1, ((i / F.dim[0]) % F.dim[1]) >> 1,
+                                (i / (F.dim[0] * F.dim[1])) >> 1);
+        if (l + 1 == last) {
+          v.x[c] += xc[id];
+        } else {
+          const ClView<T> w = cl_view<T>(cl_smem, A.lay[l + 1]);
+          v.x[c] += cl_dense_at(w, w.x, w.xa, id, first_of(l + 1));
+        }
+      }
+    }
+    cl_sync();
+    for (int sw = 0; sw < A.post; ++sw) {
+      sweep(l, 1);
+      sweep(l, 0);
+    }
   }
-  for (int i = t; i < nf; i += kTailThreads)
-    if (ff[i]) st_T(&fp.x[i], x[i]);
+  // the finest of these levels' iterate, for the prolongation above it (after the
+  // last sweep's barrier no CTA reads another's shared memory)
+  const ClView<T> v = cl_view<T>(cl_smem, A.lay[A.l0]);
+  T* xout = A.ptr[A.l0].x;
+  const int first = first_of(A.l0);
+  if (A.l0 < 3) {
+    const int LS = 3 - A.l0, S = 1 << LS, S3 = S * S * S, n = blocks_of(A.l0) * S3;
+    for (int c = t; c < n; c += kClThreads) {
+      const int bl = c / S3, l = c % S3, x = l & (S - 1), y = (l >> LS) & (S - 1), z = l >> (2 * LS);
+      const int o = bl * S3 + (((x + y + z) & 1) ? S3 / 2 : 0) + ((z * S + y) * S + x) / 2;
+      if (v.d[o] != 0.0f) st_T(&xout[(size_t)first * S3 + c], v.x[o]);
+    }
+  } else {
+    for (int c = t; c < v.cells; c += kClThreads)
+      if (v.d[c] != 0.0f) st_T(&xout[first + c], v.x[c]);
+  }
+}
+
+// CTAs of the largest cluster the device runs with a full shared-memory request: 16, 8 or 0 (none).
+template <typename T>
+static int cl_ctas() {
+  static std::atomic<int> known[64];  // 0: not asked yet, else 1 + the answer
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (known[dev] == 0) {
+    int answer = 0;
+    auto* kernel = k_coarse_cluster<T>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmemMax) == cudaSuccess &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+      for (int ctas = 16; ctas >= 8 && answer == 0; ctas /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(kClThreads);
+        cfg.dynamicSmemBytes = kClSmemMax;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = ctas;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters >= 1) answer = ctas;
+      }
+    }
+    cudaGetLastError();
+    known[dev] = 1 + answer;
+  }
+  return known[dev] - 1;
+}
+
+// The finest level the cluster kernel can take (smallest l0 >= 1 whose levels
+// fit its shared memory), or 0 where it takes none: the device runs no such
+// cluster, the coarsest level has more cells than a CTA has threads, or only
+// the coarsest level would be left. The limits are kClCellsMax's and the shared
+// memory's.
+template <typename T>
+static int cl_first_level(const MgHierarchy<T>& H, int nb, ClArgs<T>& A) {
+  if (H.levels > kClMaxLevels || H.desc[H.levels - 1].count > kClCoarsestMax) return 0;
+  A.ctas = cl_ctas<T>();
+  if (A.ctas == 0) return 0;
+  for (int l0 = 1; l0 < H.levels - 1; ++l0)
+    if (cl_layout(H, nb, l0, A.ctas, A) <= kClSmemMax) return l0;
+  return 0;
 }
 
 // ----------------------------------------------------------------- CG kernels (level 0, grid-stride)
-
 
 // r64 = b' - A p64 (FP64) for one 8^3 block; r = (float)r64; e = 0; the
 // block's ||r64||^2 goes to partial[blk]. One CTA per block with CPT cells per
@@ -1756,6 +2192,26 @@ static void launch_dep(void (*kernel)(P...), unsigned grid, unsigned block, size
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // a failure is left for cudaGetLastError()
 }
 
+// The same for one cluster that is the whole grid.
+template <typename P, typename A>
+static void launch_dep_cluster(void (*kernel)(P), unsigned ctas, unsigned block, size_t smem, cudaStream_t s,
+                               const A& arg) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = ctas;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  cudaLaunchKernelEx(&cfg, kernel, arg);  // a failure is left for cudaGetLastError()
+}
+
 template <typename T, int LS>
 static void smooth_sparse(const GridView& g, const MgHierarchy<T>& H, int l, const float* bl, int color, int mode,
                           const int* done, cudaStream_t s) {
@@ -1832,10 +2288,9 @@ template <typename T>
 static void vcycle(const GridView& g, const MgHierarchy<T>& H, const float* r0, const MgOptions& opt,
                    const int* done, cudaStream_t s, const float* r_prev = nullptr, double* dots = nullptr) {
   const int L = H.levels;
-  // The last dense level and the coarsest in one CTA when both fit.
-  const bool tail = L >= 2 && !H.desc[L - 2].sparse && H.desc[L - 2].count <= kTailMaxCells &&
-                    H.desc[L - 1].count <= kTailThreads;
-  const int top = tail ? L - 2 : L - 1;  // levels smoothed by the per-level kernels: [0, top)
+  ClArgs<T> A;
+  const int l0 = cl_first_level(H, g.nb, A);
+  const int top = l0 > 0 ? l0 : L - 1;  // levels smoothed by the per-level kernels: [0, top)
   for (int l = 0; l < top; ++l) {
     const float* bl = l == 0 ? r0 : H.b[l];
     // colour 0's first sweep (from zero) is folded into colour 1's kernel on
@@ -1847,17 +2302,22 @@ static void vcycle(const GridView& g, const MgHierarchy<T>& H, const float* r0, 
     }
     restrict_level<T>(g, H, l, bl, l + 1 < top, done, s);
   }
-  if (tail) {
-    const LevelDesc& F = H.desc[L - 2];
-    const LevelDesc& C = H.desc[L - 1];
-    const size_t smem = tail_smem_bytes((int)F.count, (int)C.count);
-    static unsigned long long configured = 0;
-    if (first_on_device(configured))
-      cudaFuncSetAttribute(k_coarse_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)tail_smem_bytes(kTailMaxCells, kTailThreads));
+  if (l0 > 0) {
+    const size_t smem = cl_layout(H, g.nb, l0, A.ctas, A);
+    A.g = g;
+    A.l0 = l0;
+    A.levels = L;
+    A.pre = opt.pre;
+    A.post = opt.post;
+    A.sweeps = opt.coarse_sweeps;
+    A.b0 = H.b[l0];
+    A.done = done;
+    for (int l = 0; l < L; ++l) {
+      A.desc[l] = H.desc[l];
+      A.ptr[l] = H.ptr[l];
+    }
     ++g_kernel_launches;
-    launch_dep(k_coarse_tail<T>, 1, kTailThreads, smem, s, F, H.ptr[L - 2], (const float*)H.b[L - 2], C,
-               H.ptr[L - 1], H.b[L - 1], opt.pre, opt.post, opt.coarse_sweeps, done);
+    launch_dep_cluster(k_coarse_cluster<T>, (unsigned)A.ctas, kClThreads, smem, s, A);
   } else {
     const LevelDesc& C = H.desc[L - 1];
     const size_t smem = (size_t)C.count * 6 * sizeof(float);
@@ -2039,6 +2499,8 @@ cudaError_t launch_to_natural(const GridView& g, const MgHierarchy<T>& H, float*
 }
 
 void configure_pressure_kernels() {
+  cl_ctas<float>();  // asked here, outside any stream capture
+  cl_ctas<__nv_bfloat16>();
   static bool done = false;
   if (done) return;
   cudaFuncSetAttribute(k_coarse_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 6 * (int)sizeof(float));

@@ -312,3 +312,32 @@ def test_flexible_cg_scalars_by_block_count(precision, n):
         runs.append(fb.copy_to_host(f["pressure"], d.active_blocks * 512, np.float64))
     np.testing.assert_array_equal(runs[0], runs[1])
     ctx.close()
+
+
+@pytest.mark.parametrize("precision,tol", [(0, 1e-5), (1, 3e-2)])
+@pytest.mark.parametrize("n,levels", [(24, 4), (40, 5), (72, 6), (176, 0)])
+def test_vcycle_coarse_levels_in_a_cluster(precision, tol, n, levels):
+    """One V-cycle against the FP64 restatement where the levels below level 0 or 1 run in one
+    cluster: odd block lattices (3, 5, 9 and 22 blocks), fewer blocks than CTAs, the coarsest level
+    right below the in-block ones (4 levels) and, at 176^3 in FP32, more blocks than level 1 may have."""
+    import torch
+
+    ctx, soa, m = dam_break_context(n)
+    ctx.step(fb.transfer_params(scenes.DT, m), fb.default_pressure_options())
+    blocks, f = ctx.active_blocks(), read_fields(ctx, n)
+    ct = np.where(f["cell_type"] == 255, 2, f["cell_type"]).astype(np.uint8)
+    r_dense = np.random.default_rng(n).normal(size=ct.shape) * (ct == 1)
+    loc = np.arange(512)
+    gx, gy, gz = ((blocks[:, d:d + 1] * 8 + (loc >> 3 * d & 7)).ravel() for d in range(3))
+    r_dev = torch.from_numpy(r_dense[gz, gy, gx].astype(np.float32)).cuda()
+    z_dev = torch.zeros_like(r_dev)
+    opt = fb.default_pressure_options(precision=precision, levels=levels)
+    assert fb.library().fl_apply_vcycle(ctx.handle, r_dev.data_ptr(), z_dev.data_ptr(), ctypes.byref(opt), None) == fb.OK
+    torch.cuda.synchronize()
+    if levels == 0:  # the library's rule: the first dense level of at most 512 cells is the coarsest
+        levels = next(l for l in range(4, 12) if (-(-(n // 8) // 2 ** (l - 4))) ** 3 <= 512)
+    z = fb.sparse_cells_to_dense(blocks, z_dev.cpu().numpy(), (n, n, n))
+    zo = oracle.vcycle(box_for(n), ct, r_dense, levels=levels, pre=opt.pre_sweeps, post=opt.post_sweeps,
+                       coarse_sweeps=opt.coarse_sweeps)
+    assert rel_err(z, zo, ct == 1) <= tol
+    ctx.close()
