@@ -138,6 +138,21 @@ __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16* p) {
 // launched without that attribute, it returns at once.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The wait for a kernel that loads through const __restrict__ pointers before any
+// branch: the compiler takes what they point to as read-only and may move such a
+// load above the wait, so the pointers come out of it as new values.
+template <typename P>
+__device__ __forceinline__ void behind_wait(P& p) {
+  size_t a = __cvta_generic_to_global(p);
+  asm volatile("" : "+l"(a));
+  p = static_cast<P>(__cvta_global_to_generic(a));
+}
+template <typename... P>
+__device__ __forceinline__ void grid_dependency_wait(P&... p) {
+  grid_dependency_wait();
+  (behind_wait(p), ...);
+}
+
 // Four consecutive values from a 4-element-aligned position (16 B for FP32, 8 B for BF16).
 template <typename T>
 __device__ __forceinline__ void ld4(const T* p, float v[4]) {

@@ -10,6 +10,30 @@
 
 namespace fl {
 
+// Launch with programmatic stream serialization: the kernel may be scheduled
+// while its predecessor on the stream drains, hiding the launch gap between
+// many short kernels: a V-cycle's, a training step's (64 items on the tensor cores
+// 429 -> 335 us, 45 in FP32 549 -> 448) and the learned layers' (one application at
+// 1.9k blocks 259 -> 234).
+// Every kernel launched this way calls grid_dependency_wait() before it reads
+// or writes what an earlier kernel may still touch, so the ordering is the
+// stream's (and, the wait being unconditional, transitive: each grid completes
+// only after its own predecessor).
+template <typename... P, typename... A>
+void launch_dep(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // a failure is left for cudaGetLastError()
+}
+
 struct P2GMergeParams {
   int mode;             // 0: raw mass + momentum; 1: normalize + gravity (+ walls)
   int walls;            // apply the stationary-wall condition on solid-adjacent faces

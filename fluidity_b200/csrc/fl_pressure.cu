@@ -2170,29 +2170,7 @@ __global__ void k_from_rb(int n, const float* in_rb, float* out_nat) {
 
 // ----------------------------------------------------------------- host orchestration
 
-// Launch with programmatic stream serialization: the kernel may be scheduled
-// while its predecessor on the stream drains, hiding the launch gap between
-// the many short kernels of a V-cycle. Every kernel launched this way calls
-// grid_dependency_wait() before anything else, so it reads no input before the
-// predecessor grid has completed (and, the wait being unconditional, each
-// grid completes only after its own predecessor: the ordering is transitive).
-template <typename... P, typename... A>
-static void launch_dep(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                       A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // a failure is left for cudaGetLastError()
-}
-
-// The same for one cluster that is the whole grid.
+// launch_dep for one cluster that is the whole grid.
 template <typename P, typename A>
 static void launch_dep_cluster(void (*kernel)(P), unsigned ctas, unsigned block, size_t smem, cudaStream_t s,
                                const A& arg) {

@@ -76,6 +76,7 @@ template <int S, bool VALID, bool DATA>
 __global__ void __launch_bounds__(kConvThreads) k_conv3(const float* __restrict__ in, int cin, const float* __restrict__ w,
                                                const float* __restrict__ bias, int cout, float* __restrict__ out,
                                                int relu, const float* __restrict__ act) {
+  grid_dependency_wait(in, w, bias, act);
   using T = ConvTile<S>;
   constexpr int E = S + 2, S3 = S * S * S, EIN = VALID ? E : S, EIN3 = EIN * EIN * EIN, OFF = VALID ? 0 : 1;
   constexpr int kSlabs = S / T::kZ, kCells = (T::kZ + 2) * E * E;
@@ -196,6 +197,7 @@ template <bool DATA>
 __global__ void __launch_bounds__(256) k_conv3_2(const float* __restrict__ in, int cin, const float* __restrict__ w,
                                                  const float* __restrict__ bias, int cout, int batch,
                                                  float* __restrict__ out, int relu, const float* __restrict__ act) {
+  grid_dependency_wait(in, w, bias, act);
   extern __shared__ __align__(16) float conv_smem[];
   float* wt = conv_smem;
   float* tile = wt + cin * 27 * kConv2W;
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(256) k_conv3_2(const float* __restrict__ in, i
 __global__ void k_conv1_fwd(const float* __restrict__ in, int cin, const float* __restrict__ w,
                             const float* __restrict__ bias, int cout, int s3, long long total,
                             float* __restrict__ out) {
+  grid_dependency_wait(in, w, bias);
   for (long long i = blockIdx.x * (long long)kT + threadIdx.x; i < total; i += (long long)gridDim.x * kT) {
     const int cell = (int)(i % s3);
     const int co = (int)((i / s3) % cout);
@@ -277,6 +280,7 @@ __global__ void k_conv1_fwd(const float* __restrict__ in, int cin, const float* 
 
 // 2x average pooling: out [B][C][(S/2)^3] from in [B][C][S^3].
 __global__ void k_pool(const float* __restrict__ in, int S, long long total, float* __restrict__ out) {
+  grid_dependency_wait(in);
   const int H = S / 2, H3 = H * H * H, S3 = S * S * S;
   for (long long i = blockIdx.x * (long long)kT + threadIdx.x; i < total; i += (long long)gridDim.x * kT) {
     const int c = (int)(i % H3);
@@ -293,6 +297,7 @@ __global__ void k_pool(const float* __restrict__ in, int S, long long total, flo
 // out = relu(coarse[parent] + skip) at resolution S.
 __global__ void k_up_add_relu(const float* __restrict__ coarse, const float* __restrict__ skip, int S, long long total,
                               float* __restrict__ out) {
+  grid_dependency_wait(coarse, skip);
   const int H = S / 2, S3 = S * S * S, H3 = H * H * H;
   for (long long i = blockIdx.x * (long long)kT + threadIdx.x; i < total; i += (long long)gridDim.x * kT) {
     const int c = (int)(i % S3);
@@ -333,6 +338,7 @@ template <int S, bool VALID, int CIN>
 __global__ void __launch_bounds__(WgradTile<S, VALID, CIN>::kThreads)
     k_conv3_wgrad(const float* __restrict__ in, const float* __restrict__ g, int cout, int batch, int units,
                   float* __restrict__ part) {
+  grid_dependency_wait(in, g);
   using T = WgradTile<S, VALID, CIN>;
   constexpr int E = S + 2, S3 = S * S * S, EIN = VALID ? E : S, EIN3 = EIN * EIN * EIN, OFF = VALID ? 0 : 1;
   constexpr int kInCells = (T::kZ + 2) * E * E, kOutCells = T::kZ * S * S;
@@ -407,6 +413,7 @@ __global__ void __launch_bounds__(WgradTile<S, VALID, CIN>::kThreads)
 // every eighth row, then the eight sums in order.
 __global__ void __launch_bounds__(kT) k_wgrad_sum(const float* __restrict__ part, int rows, int nw, int cout,
                                                   float* __restrict__ dw, float* __restrict__ db) {
+  grid_dependency_wait(part);
   __shared__ float red[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int e = blockIdx.x * 32 + lane, n = nw + cout;
@@ -434,6 +441,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT) k_conv1_bwd_weight(const float* __restrict__ in, int cin,
                                                          const float* __restrict__ g, int cout, int s3, int batch,
                                                          float* __restrict__ dw, float* __restrict__ db) {
+  grid_dependency_wait(in, g);
   __shared__ float red[2 * (NT / 32)];
   const int ci = blockIdx.x, co = blockIdx.y;
   float a = 0.0f, bs = 0.0f;
@@ -467,6 +475,7 @@ __global__ void __launch_bounds__(NT) k_conv1_bwd_weight(const float* __restrict
 // din[b][ci][o] = (sum_co w[co][ci] g[b][co][o]) * (act > 0).
 __global__ void k_conv1_bwd_data(const float* __restrict__ g, int cout, const float* __restrict__ w, int cin, int s3,
                                  long long total, const float* __restrict__ act, float* __restrict__ din) {
+  grid_dependency_wait(g, w, act);
   for (long long i = blockIdx.x * (long long)kT + threadIdx.x; i < total; i += (long long)gridDim.x * kT) {
     const int o = (int)(i % s3);
     const int ci = (int)((i / s3) % cin);
@@ -482,6 +491,7 @@ __global__ void k_conv1_bwd_data(const float* __restrict__ g, int cout, const fl
 
 // out[b][c][coarse] = sum of the 8 children of g at resolution S.
 __global__ void k_up_back(const float* __restrict__ g, int S, long long total, float* __restrict__ out) {
+  grid_dependency_wait(g);
   const int H = S / 2, H3 = H * H * H, S3 = S * S * S;
   for (long long i = blockIdx.x * (long long)kT + threadIdx.x; i < total; i += (long long)gridDim.x * kT) {
     const int c = (int)(i % H3);
@@ -498,6 +508,7 @@ __global__ void k_up_back(const float* __restrict__ g, int S, long long total, f
 // out = (ga + gp[parent] / 8) * (act > 0) at resolution S.
 __global__ void k_pool_back_add_mask(const float* __restrict__ ga, const float* __restrict__ gp,
                                      const float* __restrict__ act, int S, long long total, float* __restrict__ out) {
+  grid_dependency_wait(ga, gp, act);
   const int H = S / 2, S3 = S * S * S, H3 = H * H * H;
   for (long long i = blockIdx.x * (long long)kT + threadIdx.x; i < total; i += (long long)gridDim.x * kT) {
     const int c = (int)(i % S3);
@@ -750,11 +761,11 @@ void conv3_fwd(const float* in, int cin, const float* w, const float* bias, int 
                cudaStream_t s) {
   ++g_kernel_launches;
   if constexpr (S == 2)
-    k_conv3_2<false><<<dim3((batch + 31) / 32, cout / 8), 256, conv2_smem(cin), s>>>(in, cin, w, bias, cout, batch, out,
-                                                                                     relu, nullptr);
+    launch_dep(k_conv3_2<false>, dim3((batch + 31) / 32, cout / 8), 256, conv2_smem(cin), s, in, cin, w, bias, cout,
+               batch, out, relu, nullptr);
   else
-    k_conv3<S, VALID, false><<<dim3(batch * (S / ConvTile<S>::kZ), cout / 16), kConvThreads, ConvTile<S>::smem(cin), s>>>(
-        in, cin, w, bias, cout, out, relu, nullptr);
+    launch_dep(k_conv3<S, VALID, false>, dim3(batch * (S / ConvTile<S>::kZ), cout / 16), kConvThreads,
+               ConvTile<S>::smem(cin), s, in, cin, w, bias, cout, out, relu, nullptr);
 }
 
 // g has the layer's cout channels, din its cin: the roles of k_conv3's cin and cout.
@@ -763,11 +774,11 @@ void conv3_bwd_data(const float* g, int cout, const float* w, int cin, const flo
                     cudaStream_t s) {
   ++g_kernel_launches;
   if constexpr (S == 2)
-    k_conv3_2<true><<<dim3((batch + 31) / 32, cin / 8), 256, conv2_smem(cout), s>>>(g, cout, w, nullptr, cin, batch,
-                                                                                    din, 0, act);
+    launch_dep(k_conv3_2<true>, dim3((batch + 31) / 32, cin / 8), 256, conv2_smem(cout), s, g, cout, w, nullptr, cin,
+               batch, din, 0, act);
   else
-    k_conv3<S, false, true><<<dim3(batch * (S / ConvTile<S>::kZ), cin / 16), kConvThreads, ConvTile<S>::smem(cout), s>>>(
-        g, cout, w, nullptr, cin, din, 0, act);
+    launch_dep(k_conv3<S, false, true>, dim3(batch * (S / ConvTile<S>::kZ), cin / 16), kConvThreads,
+               ConvTile<S>::smem(cout), s, g, cout, w, nullptr, cin, din, 0, act);
 }
 
 template <int S, bool VALID, int CIN>
@@ -778,7 +789,8 @@ void wgrad(const float* in, const float* g, int cout, int batch, float* part, fl
   // two CTAs per SM where the units and the partial rows' space allow it
   const int ctas = (int)std::min<long long>({(long long)units, 2 * 148, kWgradPart / ((long long)T::kSplit * (nw + cout))});
   ++g_kernel_launches;
-  k_conv3_wgrad<S, VALID, CIN><<<dim3(ctas, cout / 16), T::kThreads, T::kSmem, s>>>(in, g, cout, batch, units, part);
+  launch_dep(k_conv3_wgrad<S, VALID, CIN>, dim3(ctas, cout / 16), T::kThreads, T::kSmem, s, in, g, cout, batch, units,
+             part);
   wgrad_sum(part, ctas * T::kSplit, nw, cout, dw, db, s);
 }
 
@@ -821,7 +833,7 @@ void bwd3_weight(UNetTcTrain* tc, cudaError_t& e, int layer, const float* in, in
 
 void wgrad_sum(const float* part, int rows, int nw, int cout, float* dw, float* db, cudaStream_t s) {
   ++g_kernel_launches;
-  k_wgrad_sum<<<(nw + cout + 31) / 32, kT, 0, s>>>(part, rows, nw, cout, dw, db);
+  launch_dep(k_wgrad_sum, (nw + cout + 31) / 32, kT, 0, s, part, rows, nw, cout, dw, db);
 }
 
 UNetLayout unet_layout() {
@@ -918,20 +930,20 @@ cudaError_t unet_forward(const float* P, const float* x, int batch, float* cache
   fwd3<8, true>(tc, tce, 0, A + C.x, 2, W(0), Bi(0), 16, A + C.e1a, batch, 1, s);
   fwd3<8, false>(tc, tce, 1, A + C.e1a, 16, W(1), Bi(1), 16, A + C.s1, batch, 1, s);
   g_kernel_launches += 1;
-  k_pool<<<grid_for(B * 16 * 64), kT, 0, s>>>(A + C.s1, 8, B * 16 * 64, A + C.p1);
+  launch_dep(k_pool, grid_for(B * 16 * 64), kT, 0, s, A + C.s1, 8, B * 16 * 64, A + C.p1);
   fwd3<4, false>(tc, tce, 2, A + C.p1, 16, W(2), Bi(2), 32, A + C.e2a, batch, 1, s);
   fwd3<4, false>(tc, tce, 3, A + C.e2a, 32, W(3), Bi(3), 32, A + C.s2, batch, 1, s);
   g_kernel_launches += 1;
-  k_pool<<<grid_for(B * 32 * 8), kT, 0, s>>>(A + C.s2, 4, B * 32 * 8, A + C.p2);
+  launch_dep(k_pool, grid_for(B * 32 * 8), kT, 0, s, A + C.s2, 4, B * 32 * 8, A + C.p2);
   fwd3<2, false>(tc, tce, 4, A + C.p2, 32, W(4), Bi(4), 64, A + C.bt, batch, 1, s);
   g_kernel_launches += 6;
-  k_conv1_fwd<<<grid_for(B * 32 * 8), kT, 0, s>>>(A + C.bt, 64, W(5), Bi(5), 32, 8, B * 32 * 8, A + C.c2);
-  k_up_add_relu<<<grid_for(B * 32 * 64), kT, 0, s>>>(A + C.c2, A + C.s2, 4, B * 32 * 64, A + C.u2);
+  launch_dep(k_conv1_fwd, grid_for(B * 32 * 8), kT, 0, s, A + C.bt, 64, W(5), Bi(5), 32, 8, B * 32 * 8, A + C.c2);
+  launch_dep(k_up_add_relu, grid_for(B * 32 * 64), kT, 0, s, A + C.c2, A + C.s2, 4, B * 32 * 64, A + C.u2);
   fwd3<4, false>(tc, tce, 6, A + C.u2, 32, W(6), Bi(6), 32, A + C.d2, batch, 1, s);
-  k_conv1_fwd<<<grid_for(B * 16 * 64), kT, 0, s>>>(A + C.d2, 32, W(7), Bi(7), 16, 64, B * 16 * 64, A + C.c1);
-  k_up_add_relu<<<grid_for(B * 16 * 512), kT, 0, s>>>(A + C.c1, A + C.s1, 8, B * 16 * 512, A + C.u1);
+  launch_dep(k_conv1_fwd, grid_for(B * 16 * 64), kT, 0, s, A + C.d2, 32, W(7), Bi(7), 16, 64, B * 16 * 64, A + C.c1);
+  launch_dep(k_up_add_relu, grid_for(B * 16 * 512), kT, 0, s, A + C.c1, A + C.s1, 8, B * 16 * 512, A + C.u1);
   fwd3<8, false>(tc, tce, 8, A + C.u1, 16, W(8), Bi(8), 16, A + C.d1, batch, 1, s);
-  k_conv1_fwd<<<grid_for(B * 512), kT, 0, s>>>(A + C.d1, 16, W(9), Bi(9), 1, 512, B * 512, A + C.y);
+  launch_dep(k_conv1_fwd, grid_for(B * 512), kT, 0, s, A + C.d1, 16, W(9), Bi(9), 1, 512, B * 512, A + C.y);
   if (y != nullptr && y != A + C.y)
     cudaMemcpyAsync(y, A + C.y, sizeof(float) * 512 * B, cudaMemcpyDeviceToDevice, s);
   if (tce != cudaSuccess) return tce;
@@ -952,32 +964,34 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   auto GB = [&](int l) { return G + L.bias[l]; };
   // out layer (16 -> 1)
   g_kernel_launches += 2;
-  k_conv1_bwd_weight<1024><<<dim3(16, 1), 1024, 0, s>>>(A + C.d1, 16, gy, 1, 512, batch, GW(9), GB(9));
-  k_conv1_bwd_data<<<grid_for(B * 16 * 512), kT, 0, s>>>(gy, 1, W(9), 16, 512, B * 16 * 512, A + C.d1, A + C.g8a);
+  launch_dep(k_conv1_bwd_weight<1024>, dim3(16, 1), 1024, 0, s, A + C.d1, 16, gy, 1, 512, batch, GW(9), GB(9));
+  launch_dep(k_conv1_bwd_data, grid_for(B * 16 * 512), kT, 0, s, gy, 1, W(9), 16, 512, B * 16 * 512, A + C.d1,
+             A + C.g8a);
   // d1 (conv3 16->16 on u1); gu1 pre-activation -> g8b
   bwd3_weight<8, false>(tc, tce, 8, A + C.u1, 16, A + C.g8a, 16, batch, A + C.part, GW(8), GB(8), s);
   bwd3_data<8>(tc, tce, 8, A + C.g8a, 16, W(8), 16, A + C.u1, A + C.g8b, batch, s);
   // u1 = relu(up(c1) + s1): c1 = conv1(d2, 32->16)
   g_kernel_launches += 3;
-  k_up_back<<<grid_for(B * 16 * 64), kT, 0, s>>>(A + C.g8b, 8, B * 16 * 64, A + C.g4c);
-  k_conv1_bwd_weight<kT><<<dim3(32, 16), kT, 0, s>>>(A + C.d2, 32, A + C.g4c, 16, 64, batch, GW(7), GB(7));
-  k_conv1_bwd_data<<<grid_for(B * 32 * 64), kT, 0, s>>>(A + C.g4c, 16, W(7), 32, 64, B * 32 * 64, A + C.d2,
-                                                        A + C.g4a);
+  launch_dep(k_up_back, grid_for(B * 16 * 64), kT, 0, s, A + C.g8b, 8, B * 16 * 64, A + C.g4c);
+  launch_dep(k_conv1_bwd_weight<kT>, dim3(32, 16), kT, 0, s, A + C.d2, 32, A + C.g4c, 16, 64, batch, GW(7), GB(7));
+  launch_dep(k_conv1_bwd_data, grid_for(B * 32 * 64), kT, 0, s, A + C.g4c, 16, W(7), 32, 64, B * 32 * 64, A + C.d2,
+             A + C.g4a);
   // d2 (conv3 32->32 on u2); gu2 pre-activation -> g4b
   bwd3_weight<4, false>(tc, tce, 6, A + C.u2, 32, A + C.g4a, 32, batch, A + C.part, GW(6), GB(6), s);
   bwd3_data<4>(tc, tce, 6, A + C.g4a, 32, W(6), 32, A + C.u2, A + C.g4b, batch, s);
   // u2 = relu(up(c2) + s2): c2 = conv1(bt, 64->32)
   g_kernel_launches += 3;
-  k_up_back<<<grid_for(B * 32 * 8), kT, 0, s>>>(A + C.g4b, 4, B * 32 * 8, A + C.g2b);
-  k_conv1_bwd_weight<kT><<<dim3(64, 32), kT, 0, s>>>(A + C.bt, 64, A + C.g2b, 32, 8, batch, GW(5), GB(5));
-  k_conv1_bwd_data<<<grid_for(B * 64 * 8), kT, 0, s>>>(A + C.g2b, 32, W(5), 64, 8, B * 64 * 8, A + C.bt, A + C.g2a);
+  launch_dep(k_up_back, grid_for(B * 32 * 8), kT, 0, s, A + C.g4b, 4, B * 32 * 8, A + C.g2b);
+  launch_dep(k_conv1_bwd_weight<kT>, dim3(64, 32), kT, 0, s, A + C.bt, 64, A + C.g2b, 32, 8, batch, GW(5), GB(5));
+  launch_dep(k_conv1_bwd_data, grid_for(B * 64 * 8), kT, 0, s, A + C.g2b, 32, W(5), 64, 8, B * 64 * 8, A + C.bt,
+             A + C.g2a);
   // bt (conv3 32->64 on p2) -> gp2 (g2b, 32 channels)
   bwd3_weight<2, false>(tc, tce, 4, A + C.p2, 32, A + C.g2a, 64, batch, A + C.part, GW(4), GB(4), s);
   bwd3_data<2>(tc, tce, 4, A + C.g2a, 64, W(4), 32, nullptr, A + C.g2b, batch, s);
   // s2 gradient: (gu2 + pool_back(gp2)) * (s2 > 0) -> g4a
   g_kernel_launches += 1;
-  k_pool_back_add_mask<<<grid_for(B * 32 * 64), kT, 0, s>>>(A + C.g4b, A + C.g2b, A + C.s2, 4, B * 32 * 64,
-                                                            A + C.g4a);
+  launch_dep(k_pool_back_add_mask, grid_for(B * 32 * 64), kT, 0, s, A + C.g4b, A + C.g2b, A + C.s2, 4, B * 32 * 64,
+             A + C.g4a);
   // e2b (conv3 32->32 on e2a) -> ge2a (g4c)
   bwd3_weight<4, false>(tc, tce, 3, A + C.e2a, 32, A + C.g4a, 32, batch, A + C.part, GW(3), GB(3), s);
   bwd3_data<4>(tc, tce, 3, A + C.g4a, 32, W(3), 32, A + C.e2a, A + C.g4c, batch, s);
@@ -986,8 +1000,8 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   bwd3_data<4>(tc, tce, 2, A + C.g4c, 32, W(2), 16, nullptr, A + C.g4b, batch, s);
   // s1 gradient: (gu1 + pool_back(gp1)) * (s1 > 0) -> g8a
   g_kernel_launches += 1;
-  k_pool_back_add_mask<<<grid_for(B * 16 * 512), kT, 0, s>>>(A + C.g8b, A + C.g4b, A + C.s1, 8, B * 16 * 512,
-                                                             A + C.g8a);
+  launch_dep(k_pool_back_add_mask, grid_for(B * 16 * 512), kT, 0, s, A + C.g8b, A + C.g4b, A + C.s1, 8, B * 16 * 512,
+             A + C.g8a);
   // e1b (conv3 16->16 on e1a) -> ge1a (g8c)
   bwd3_weight<8, false>(tc, tce, 1, A + C.e1a, 16, A + C.g8a, 16, batch, A + C.part, GW(1), GB(1), s);
   bwd3_data<8>(tc, tce, 1, A + C.g8a, 16, W(1), 16, A + C.e1a, A + C.g8c, batch, s);

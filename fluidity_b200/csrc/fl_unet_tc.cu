@@ -282,6 +282,9 @@ __global__ void __launch_bounds__(conv_threads(IN_KIND)) k_conv_tc(ConvArgs a) {
                  "r"((uint32_t)(2 * NCOLS)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  // Until here nothing that the kernel before this one writes (the weights were
+  // packed before the window's gather): its end and this prologue overlap.
+  grid_dependency_wait();
   fence_async_smem();  // the weights, stored by every thread, before the MMAs read them
   fence_before_sync();
   __syncthreads();
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(conv_threads(IN_KIND)) k_conv_tc(ConvArgs a) {
       const int b = (int)blockIdx.x + j * (int)gridDim.x;
       if (b >= a.nb) return -1;
       ++j;
-      if (a.scale == nullptr || __ldg(&a.scale[b]) != 0.0f) return b;
+      if (a.scale == nullptr || a.scale[b] != 0.0f) return b;
     }
   };
 
@@ -523,6 +526,7 @@ __global__ void __launch_bounds__(512) k_tc_gather(GridView g, const float* __re
 // per (block, coarse cell, group).
 template <int DIN, int G>
 __global__ void k_tc_pool(const uint4* __restrict__ in, uint4* __restrict__ out, int nb, long long cap) {
+  grid_dependency_wait(in);
   constexpr PadGeom I = DIN == 8 ? geom8() : geom4();
   constexpr PadGeom O = geom4();
   constexpr int H = DIN / 2, H3 = H * H * H;
@@ -579,6 +583,7 @@ __global__ void __launch_bounds__(kBtThreads) k_bt_tc(const uint4* __restrict__ 
                  "r"((uint32_t)N));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  grid_dependency_wait();
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -647,6 +652,7 @@ __global__ void __launch_bounds__(kBtThreads) k_bt_tc(const uint4* __restrict__ 
 __global__ void __launch_bounds__(256) k_tc_upadd2(const float* __restrict__ bt, const uint4* __restrict__ s2,
                                                    const float* __restrict__ w, const float* __restrict__ bias,
                                                    uint4* __restrict__ u2) {
+  grid_dependency_wait(bt, s2);
   constexpr PadGeom L = geom4();
   __shared__ float c2[8][32];
   __shared__ float wt[64][33];  // the 1x1 weights transposed: a warp's 32 output channels read one row (padded:
@@ -681,6 +687,7 @@ __global__ void __launch_bounds__(256) k_tc_upadd2(const float* __restrict__ bt,
 __global__ void __launch_bounds__(256) k_tc_upadd1(const uint4* __restrict__ d2, const uint4* __restrict__ s1,
                                                    const float* __restrict__ w, const float* __restrict__ bias,
                                                    uint4* __restrict__ u1) {
+  grid_dependency_wait(d2, s1);
   constexpr PadGeom L4 = geom4();
   constexpr PadGeom L8 = geom8();
   __shared__ float din[64][33];
@@ -792,7 +799,7 @@ cudaError_t launch_conv(const ConvArgs& a, int sms, cudaStream_t s) {
   const int per_sm = by_smem < cap ? by_smem : cap;
   const int grid = a.nb < sms * per_sm ? a.nb : sms * per_sm;
   ++g_kernel_launches;
-  kern<<<grid, conv_threads(IN_KIND), smem, s>>>(a);
+  launch_dep(kern, grid, conv_threads(IN_KIND), smem, s, a);
   return cudaGetLastError();
 }
 
@@ -803,7 +810,7 @@ cudaError_t launch_bt(const uint4* in, long long cap, const uint4* weights, cons
   static unsigned long long configured = 0;
   if (first_on_device(configured)) cudaFuncSetAttribute(k_bt_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   ++g_kernel_launches;
-  k_bt_tc<<<dim3((nb + 127) / 128, 8), kBtThreads, smem, s>>>(in, cap, weights, bias, out, nb, error);
+  launch_dep(k_bt_tc, dim3((nb + 127) / 128, 8), kBtThreads, smem, s, in, cap, weights, bias, out, nb, error);
   return cudaGetLastError();
 }
 
@@ -884,7 +891,7 @@ cudaError_t unet_tc_apply(const GridView& g, const float* params, const __nv_bfl
   a.in = base(L.t8); a.weights = wp(1); a.bias = params + P.bias[1]; a.out = base(L.s1);
   if ((e = launch_conv<2, 16, kToPadded, 8, 8>(a, sms, s)) != cudaSuccess) return e;
   g_kernel_launches += 1;
-  k_tc_pool<8, 2><<<(nb * 64 * 2 + 255) / 256, 256, 0, s>>>(base(L.s1), base(L.p1), nb, cap);
+  launch_dep(k_tc_pool<8, 2>, (nb * 64 * 2 + 255) / 256, 256, 0, s, base(L.s1), base(L.p1), nb, cap);
   // e2a: p1 -> e2a
   a.in = base(L.p1); a.weights = wp(2); a.bias = params + P.bias[2]; a.out = base(L.e2a);
   if ((e = launch_conv<2, 32, kToPadded, 4, 4>(a, sms, s)) != cudaSuccess) return e;
@@ -892,16 +899,16 @@ cudaError_t unet_tc_apply(const GridView& g, const float* params, const __nv_bfl
   a.in = base(L.e2a); a.weights = wp(3); a.bias = params + P.bias[3]; a.out = base(L.s2);
   if ((e = launch_conv<4, 32, kToPadded, 4, 4>(a, sms, s)) != cudaSuccess) return e;
   g_kernel_launches += 1;
-  k_tc_pool<4, 4><<<(nb * 8 * 4 + 255) / 256, 256, 0, s>>>(base(L.s2), base(L.p2), nb, cap);
+  launch_dep(k_tc_pool<4, 4>, (nb * 8 * 4 + 255) / 256, 256, 0, s, base(L.s2), base(L.p2), nb, cap);
   // bt: p2 -> bt (plain FP32)
   if ((e = launch_bt(base(L.p2), cap, wp(4), params + P.bias[4], bt, nb, error, s)) != cudaSuccess) return e;
   g_kernel_launches += 1;
-  k_tc_upadd2<<<nb, 256, 0, s>>>(bt, base(L.s2), params + P.offset[5], params + P.bias[5], base(L.u2));
+  launch_dep(k_tc_upadd2, nb, 256, 0, s, bt, base(L.s2), params + P.offset[5], params + P.bias[5], base(L.u2));
   // d2: u2 -> d2
   a.in = base(L.u2); a.weights = wp(5); a.bias = params + P.bias[6]; a.out = base(L.d2);
   if ((e = launch_conv<4, 32, kToPadded, 4, 4>(a, sms, s)) != cudaSuccess) return e;
   g_kernel_launches += 1;
-  k_tc_upadd1<<<nb, 256, 0, s>>>(base(L.d2), base(L.s1), params + P.offset[7], params + P.bias[7], base(L.t8));
+  launch_dep(k_tc_upadd1, nb, 256, 0, s, base(L.d2), base(L.s1), params + P.offset[7], params + P.bias[7], base(L.t8));
   // d1 + output layer: u1 (in t8) -> z
   a.in = base(L.t8); a.weights = wp(6); a.bias = params + P.bias[8]; a.out = nullptr;
   a.w_out = params + P.offset[9]; a.b_out = params + P.bias[9]; a.type = type; a.z = z;

@@ -15,10 +15,10 @@
 // operands and by launch latency, so warp-level MMAs (m16n8k16), which read
 // their operands from where they were staged and need no tensor-memory
 // allocation or epilogue copy, are enough to take the matrix work off the
-// critical path. A training step of 64 items takes 429 us; with im2col operands
+// critical path. A training step of 64 items takes 335 us; with im2col operands
 // written to memory and library GEMMs between them (92 + 20 launches) it took 664,
 // with up to 32 channels per CTA and several items per weight-gradient unit (so 8
-// to 64 CTAs a layer) 494.
+// to 64 CTAs a layer) 494, without programmatic launches 429.
 // Bias, ReLU and the ReLU mask are applied in the epilogue. Sums and every
 // result are FP32, as are the parameters and Adam's state; every reduction has a
 // fixed order. The FP32 kernels of fl_unet.cu remain the exact path.
@@ -99,6 +99,7 @@ __host__ __device__ constexpr int pack_index(int layer) {
 
 // Element e of the forward (data = 0) or data-gradient half of the table.
 __global__ void k_pack(const float* __restrict__ params, UNetLayout L, int data, __nv_bfloat16* __restrict__ out) {
+  grid_dependency_wait(params);
   constexpr PackTable T = pack_table();
   const int first = data ? T.l[1].data : 0, end = data ? T.total : T.l[1].data;
   const int e = first + blockIdx.x * blockDim.x + threadIdx.x;
@@ -178,6 +179,7 @@ template <int S, bool VALID, int CIN, int COUT, bool DATA>
 __global__ void __launch_bounds__(kConvThreads)
     k_conv_mma(const float* __restrict__ in, const __nv_bfloat16* __restrict__ w, const float* __restrict__ bias,
                float* __restrict__ out, int batch, int relu, const float* __restrict__ act) {
+  grid_dependency_wait(in, w, bias, act);
   using C = ConvShape<S>;
   using T = Tile<S, CIN, C::kItems, C::kZ>;
   constexpr int kSlabs = S / C::kZ, S3 = S * S * S, kNw = C::kCo / 8 / C::kWn;
@@ -308,6 +310,7 @@ template <int S, bool VALID, int CIN, int COUT>
 __global__ void __launch_bounds__(kWgradThreads)
     k_wgrad_mma(const float* __restrict__ in, const float* __restrict__ g, int batch, int units,
                 float* __restrict__ part) {
+  grid_dependency_wait(in, g);
   using W = WgradShape<S, CIN, COUT>;
   using T = typename W::T;
   constexpr int kSlabs = S / W::kZ, S3 = S * S * S, kM = W::kCo / 16, kN = CIN == 2 ? 1 : CIN / 8;
@@ -416,13 +419,13 @@ cudaError_t conv(const UNetTcTrain& t, int layer, bool data, const float* in, co
   ++g_kernel_launches;
   static unsigned long long configured[2] = {0, 0};
   if constexpr (VALID) {
-    k_conv_mma<S, VALID, CIN, COUT, false><<<grid, kConvThreads, smem, s>>>(in, t.w + p.fwd, bias, out, batch, relu,
-                                                                            nullptr);
+    launch_dep(k_conv_mma<S, VALID, CIN, COUT, false>, grid, kConvThreads, smem, s, in, t.w + p.fwd, bias, out, batch,
+               relu, nullptr);
   } else {
     auto* kernel = data ? k_conv_mma<S, VALID, CIN, COUT, true> : k_conv_mma<S, VALID, CIN, COUT, false>;
     if (first_on_device(configured[data]))
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kernel<<<grid, kConvThreads, smem, s>>>(in, t.w + (data ? p.data : p.fwd), bias, out, batch, relu, act);
+    launch_dep(kernel, grid, kConvThreads, smem, s, in, t.w + (data ? p.data : p.fwd), bias, out, batch, relu, act);
   }
   return cudaGetLastError();
 }
@@ -437,7 +440,8 @@ cudaError_t wgrad(const float* in, const float* g, int batch, float* part, float
   if (first_on_device(configured))
     cudaFuncSetAttribute(k_wgrad_mma<S, VALID, CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W::kSmem);
   ++g_kernel_launches;
-  k_wgrad_mma<S, VALID, CIN, COUT><<<dim3(ctas, COUT / W::kCo), kWgradThreads, W::kSmem, s>>>(in, g, batch, units, part);
+  launch_dep(k_wgrad_mma<S, VALID, CIN, COUT>, dim3(ctas, COUT / W::kCo), kWgradThreads, W::kSmem, s, in, g,
+             batch, units, part);
   wgrad_sum(part, ctas, nw, COUT, dw, db, s);
   return cudaGetLastError();
 }
@@ -462,7 +466,7 @@ cudaError_t unet_tc_train_pack(const UNetTcTrain& t, const float* params, bool d
   constexpr PackTable T = pack_table();
   const int n = data ? T.total - T.l[1].data : T.l[1].data;
   ++g_kernel_launches;
-  k_pack<<<(n + 255) / 256, 256, 0, s>>>(params, unet_layout(), data ? 1 : 0, t.w);
+  launch_dep(k_pack, (n + 255) / 256, 256, 0, s, params, unet_layout(), data ? 1 : 0, t.w);
   return cudaGetLastError();
 }
 

@@ -498,3 +498,30 @@ def test_tensor_core_inference_at_block_counts(shape):
     assert np.any(ref != 0.0)
     assert _rel(z, ref) <= 3e-2
     ctx.close()
+
+
+@pytest.mark.parametrize("tensor_cores", [False, True])
+def test_training_passes_in_a_row_are_ordered(tensor_cores):
+    """Kernels of a pass may be scheduled before their predecessors end, and each waits before it reads:
+    Adam, forward and backward issued in a row give the bits that the same calls give with the device
+    idle before each."""
+    import torch
+
+    rng = np.random.default_rng(15)
+    x, gy = _t(rng.normal(size=(45, 2, 10, 10, 10))), _t(rng.normal(size=(45, 512)))
+    th = _t(U.init_params(2) + 0.01 * rng.normal(size=U.param_count()))
+    unet = fb.UNet(45, tensor_cores=tensor_cores)
+    results = []
+    for idle in (True, False, False):
+        p, m, v = th.clone(), torch.zeros_like(th), torch.zeros_like(th)
+        y, g = torch.zeros((45, 512), device="cuda"), torch.zeros_like(th)
+        for step in range(1, 13):
+            for call in (lambda: unet.forward(p, x, y), lambda: unet.backward(p, gy, g),
+                         lambda: fb.UNet.adam_step(p, g, m, v, step)):
+                call()
+                if idle:
+                    torch.cuda.synchronize()
+        results.append(torch.cat([p, g, y.ravel()]).cpu().numpy())
+    for r in results[1:]:
+        np.testing.assert_array_equal(r, results[0])
+    unet.close()
