@@ -950,9 +950,34 @@ cudaError_t unet_forward(const float* P, const float* x, int batch, float* cache
   return cudaGetLastError();
 }
 
+cudaError_t unet_side_create(UNetSide* side) {
+  cudaError_t e = cudaStreamCreateWithFlags(&side->s, cudaStreamNonBlocking);
+  cudaEvent_t* events[] = {&side->fork[0], &side->fork[1], &side->fork[2], &side->fork[3],
+                           &side->fork[4], &side->fork[5], &side->read,    &side->join};
+  for (cudaEvent_t* v : events)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+  if (e != cudaSuccess) unet_side_destroy(side);
+  return e;
+}
+
+void unet_side_destroy(UNetSide* side) {
+  for (cudaEvent_t v : side->fork)
+    if (v != nullptr) cudaEventDestroy(v);
+  if (side->read != nullptr) cudaEventDestroy(side->read);
+  if (side->join != nullptr) cudaEventDestroy(side->join);
+  if (side->s != nullptr) cudaStreamDestroy(side->s);
+  *side = UNetSide{};
+}
+
 // Gradient of sum(gy * y) with respect to the parameters, from the cache of the last forward.
+// A layer's kernels fill a part of the chip at training batches, and the weight gradients
+// (over half of the time) feed nothing: they run on the side stream, each forked off once
+// its output gradient is there, beside the chain of data gradients on `s`; `s` joins them
+// at the end. The chain reuses the first half's gradient buffers only after the side
+// stream has read them (`read`). A training step of 64 items on the tensor cores 335 ->
+// 301 us, of 45 in FP32 448 -> 407.
 cudaError_t unet_backward(const float* P, float* cache, const float* gy, int batch, float* G, cudaStream_t s,
-                          UNetTcTrain* tc) {
+                          const UNetSide& side, UNetTcTrain* tc) {
   configure_unet_kernels();
   cudaError_t tce = tc != nullptr ? unet_tc_train_pack(*tc, P, true, s) : cudaSuccess;
   const UNetLayout L = unet_layout();
@@ -962,51 +987,66 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   auto W = [&](int l) { return P + L.offset[l]; };
   auto GW = [&](int l) { return G + L.offset[l]; };
   auto GB = [&](int l) { return G + L.bias[l]; };
+  const cudaStream_t w = side.s;
+  auto fork = [&](int k) {  // the side stream goes on from here
+    cudaEventRecord(side.fork[k], s);
+    cudaStreamWaitEvent(w, side.fork[k], 0);
+  };
   // out layer (16 -> 1)
   g_kernel_launches += 2;
-  launch_dep(k_conv1_bwd_weight<1024>, dim3(16, 1), 1024, 0, s, A + C.d1, 16, gy, 1, 512, batch, GW(9), GB(9));
   launch_dep(k_conv1_bwd_data, grid_for(B * 16 * 512), kT, 0, s, gy, 1, W(9), 16, 512, B * 16 * 512, A + C.d1,
              A + C.g8a);
+  fork(0);
+  launch_dep(k_conv1_bwd_weight<1024>, dim3(16, 1), 1024, 0, w, A + C.d1, 16, gy, 1, 512, batch, GW(9), GB(9));
   // d1 (conv3 16->16 on u1); gu1 pre-activation -> g8b
-  bwd3_weight<8, false>(tc, tce, 8, A + C.u1, 16, A + C.g8a, 16, batch, A + C.part, GW(8), GB(8), s);
+  bwd3_weight<8, false>(tc, tce, 8, A + C.u1, 16, A + C.g8a, 16, batch, A + C.part, GW(8), GB(8), w);
   bwd3_data<8>(tc, tce, 8, A + C.g8a, 16, W(8), 16, A + C.u1, A + C.g8b, batch, s);
   // u1 = relu(up(c1) + s1): c1 = conv1(d2, 32->16)
   g_kernel_launches += 3;
   launch_dep(k_up_back, grid_for(B * 16 * 64), kT, 0, s, A + C.g8b, 8, B * 16 * 64, A + C.g4c);
-  launch_dep(k_conv1_bwd_weight<kT>, dim3(32, 16), kT, 0, s, A + C.d2, 32, A + C.g4c, 16, 64, batch, GW(7), GB(7));
   launch_dep(k_conv1_bwd_data, grid_for(B * 32 * 64), kT, 0, s, A + C.g4c, 16, W(7), 32, 64, B * 32 * 64, A + C.d2,
              A + C.g4a);
+  fork(1);
+  launch_dep(k_conv1_bwd_weight<kT>, dim3(32, 16), kT, 0, w, A + C.d2, 32, A + C.g4c, 16, 64, batch, GW(7), GB(7));
   // d2 (conv3 32->32 on u2); gu2 pre-activation -> g4b
-  bwd3_weight<4, false>(tc, tce, 6, A + C.u2, 32, A + C.g4a, 32, batch, A + C.part, GW(6), GB(6), s);
+  bwd3_weight<4, false>(tc, tce, 6, A + C.u2, 32, A + C.g4a, 32, batch, A + C.part, GW(6), GB(6), w);
   bwd3_data<4>(tc, tce, 6, A + C.g4a, 32, W(6), 32, A + C.u2, A + C.g4b, batch, s);
   // u2 = relu(up(c2) + s2): c2 = conv1(bt, 64->32)
   g_kernel_launches += 3;
   launch_dep(k_up_back, grid_for(B * 32 * 8), kT, 0, s, A + C.g4b, 4, B * 32 * 8, A + C.g2b);
-  launch_dep(k_conv1_bwd_weight<kT>, dim3(64, 32), kT, 0, s, A + C.bt, 64, A + C.g2b, 32, 8, batch, GW(5), GB(5));
   launch_dep(k_conv1_bwd_data, grid_for(B * 64 * 8), kT, 0, s, A + C.g2b, 32, W(5), 64, 8, B * 64 * 8, A + C.bt,
              A + C.g2a);
+  fork(2);
+  launch_dep(k_conv1_bwd_weight<kT>, dim3(64, 32), kT, 0, w, A + C.bt, 64, A + C.g2b, 32, 8, batch, GW(5), GB(5));
+  cudaEventRecord(side.read, w);
   // bt (conv3 32->64 on p2) -> gp2 (g2b, 32 channels)
-  bwd3_weight<2, false>(tc, tce, 4, A + C.p2, 32, A + C.g2a, 64, batch, A + C.part, GW(4), GB(4), s);
+  bwd3_weight<2, false>(tc, tce, 4, A + C.p2, 32, A + C.g2a, 64, batch, A + C.part, GW(4), GB(4), w);
+  cudaStreamWaitEvent(s, side.read, 0);  // g2b, g4c, g4a and g8a are written again from here
   bwd3_data<2>(tc, tce, 4, A + C.g2a, 64, W(4), 32, nullptr, A + C.g2b, batch, s);
   // s2 gradient: (gu2 + pool_back(gp2)) * (s2 > 0) -> g4a
   g_kernel_launches += 1;
   launch_dep(k_pool_back_add_mask, grid_for(B * 32 * 64), kT, 0, s, A + C.g4b, A + C.g2b, A + C.s2, 4, B * 32 * 64,
              A + C.g4a);
   // e2b (conv3 32->32 on e2a) -> ge2a (g4c)
-  bwd3_weight<4, false>(tc, tce, 3, A + C.e2a, 32, A + C.g4a, 32, batch, A + C.part, GW(3), GB(3), s);
   bwd3_data<4>(tc, tce, 3, A + C.g4a, 32, W(3), 32, A + C.e2a, A + C.g4c, batch, s);
+  fork(3);
+  bwd3_weight<4, false>(tc, tce, 3, A + C.e2a, 32, A + C.g4a, 32, batch, A + C.part, GW(3), GB(3), w);
   // e2a (conv3 16->32 on p1) -> gp1 (g4b, 16 channels)
-  bwd3_weight<4, false>(tc, tce, 2, A + C.p1, 16, A + C.g4c, 32, batch, A + C.part, GW(2), GB(2), s);
+  bwd3_weight<4, false>(tc, tce, 2, A + C.p1, 16, A + C.g4c, 32, batch, A + C.part, GW(2), GB(2), w);
   bwd3_data<4>(tc, tce, 2, A + C.g4c, 32, W(2), 16, nullptr, A + C.g4b, batch, s);
   // s1 gradient: (gu1 + pool_back(gp1)) * (s1 > 0) -> g8a
   g_kernel_launches += 1;
   launch_dep(k_pool_back_add_mask, grid_for(B * 16 * 512), kT, 0, s, A + C.g8b, A + C.g4b, A + C.s1, 8, B * 16 * 512,
              A + C.g8a);
   // e1b (conv3 16->16 on e1a) -> ge1a (g8c)
-  bwd3_weight<8, false>(tc, tce, 1, A + C.e1a, 16, A + C.g8a, 16, batch, A + C.part, GW(1), GB(1), s);
+  fork(4);
+  bwd3_weight<8, false>(tc, tce, 1, A + C.e1a, 16, A + C.g8a, 16, batch, A + C.part, GW(1), GB(1), w);
   bwd3_data<8>(tc, tce, 1, A + C.g8a, 16, W(1), 16, A + C.e1a, A + C.g8c, batch, s);
   // e1a (valid conv3 2->16 on x)
-  bwd3_weight<8, true>(tc, tce, 0, A + C.x, 2, A + C.g8c, 16, batch, A + C.part, GW(0), GB(0), s);
+  fork(5);
+  bwd3_weight<8, true>(tc, tce, 0, A + C.x, 2, A + C.g8c, 16, batch, A + C.part, GW(0), GB(0), w);
+  cudaEventRecord(side.join, w);
+  cudaStreamWaitEvent(s, side.join, 0);
   if (tce != cudaSuccess) return tce;
   return cudaGetLastError();
 }
@@ -1182,6 +1222,7 @@ struct fl_unet {
   int device = 0;
   int max_batch = 0;
   float* cache = nullptr;
+  fl::UNetSide side;
   fl::UNetTcTrain* tc = nullptr;  // set: the 3x3x3 training convolutions run on the tensor cores
 };
 
@@ -1220,6 +1261,12 @@ int fl_unet_create(int max_batch, fl_unet** out) {
     delete u;
     return FL_RESOURCE_EXHAUSTED;
   }
+  if (fl::unet_side_create(&u->side) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(u->cache);
+    delete u;
+    return FL_RESOURCE_EXHAUSTED;
+  }
   cudaMemset(u->cache, 0, bytes);
   *out = u;
   return FL_OK;
@@ -1232,6 +1279,7 @@ int fl_unet_destroy(fl_unet* u) {
     delete u->tc;
   }
   cudaFree(u->cache);
+  fl::unet_side_destroy(&u->side);
   delete u;
   return FL_OK;
 }
@@ -1281,7 +1329,7 @@ int fl_unet_backward(fl_unet* u, const float* params, const float* grad_output, 
     return FL_INVALID_ARGUMENT;
   if (batch > u->max_batch) return FL_RESOURCE_EXHAUSTED;
   return unet_code(fl::unet_backward(params, u->cache, grad_output, batch, grad_params,
-                                     static_cast<cudaStream_t>(stream), u->tc));
+                                     static_cast<cudaStream_t>(stream), u->side, u->tc));
 }
 
 int fl_unet_masked_mse(const float* output, const float* target, const float* mask, int batch, int relative,

@@ -58,8 +58,16 @@ cudaError_t conv3_bwd_weight_tc(int layer, const float* in, const float* g, int 
 // the tensor cores, BF16 operands with FP32 accumulation.
 cudaError_t unet_forward(const float* params, const float* x, int batch, float* cache, float* y, cudaStream_t s,
                          UNetTcTrain* tc = nullptr);
+// The backward's second stream, for the weight gradients: the chain of data
+// gradients does not wait for them (see unet_backward).
+struct UNetSide {
+  cudaStream_t s = nullptr;
+  cudaEvent_t fork[6] = {}, read = nullptr, join = nullptr;
+};
+cudaError_t unet_side_create(UNetSide* side);
+void unet_side_destroy(UNetSide* side);
 cudaError_t unet_backward(const float* params, float* cache, const float* grad_y, int batch, float* grad_params,
-                          cudaStream_t s, UNetTcTrain* tc = nullptr);
+                          cudaStream_t s, const UNetSide& side, UNetTcTrain* tc = nullptr);
 cudaError_t unet_masked_mse(const float* y, const float* target, const float* mask, int batch, int relative,
                             float* loss, float* grad, cudaStream_t s);
 cudaError_t unet_block_residual_loss(const float* y, const float* x, int batch, float* loss, float* grad,

@@ -525,3 +525,36 @@ def test_training_passes_in_a_row_are_ordered(tensor_cores):
     for r in results[1:]:
         np.testing.assert_array_equal(r, results[0])
     unet.close()
+
+
+@pytest.mark.parametrize("tensor_cores", [False, True])
+def test_weight_gradients_end_before_the_stream_goes_on(tensor_cores):
+    """The weight gradients run beside the data gradients on a stream of the handle's own: what the
+    caller's stream does right after the backward (overwriting its inputs, another forward into the same
+    activations) does not reach them. The same bits as with the device idle in between."""
+    import torch
+
+    rng = np.random.default_rng(17)
+    x, gy = _t(rng.normal(size=(40, 2, 10, 10, 10))), _t(rng.normal(size=(40, 512)))
+    th = _t(U.init_params(4) + 0.01 * rng.normal(size=U.param_count()))
+    unet = fb.UNet(40, tensor_cores=tensor_cores)
+    stream = torch.cuda.Stream()
+    grads = []
+    torch.cuda.synchronize()
+    for idle in (True, False, False):
+        with torch.cuda.stream(stream):
+            p, up, y, g = th.clone(), gy.clone(), torch.zeros((40, 512), device="cuda"), torch.zeros_like(th)
+            unet.forward(p, x, y, stream=stream.cuda_stream)
+            unet.backward(p, up, g, stream=stream.cuda_stream)
+            if idle:
+                torch.cuda.synchronize()
+            out = g.clone()
+            p.zero_()
+            up.fill_(float("nan"))
+            unet.forward(p, x, y, stream=stream.cuda_stream)
+        torch.cuda.synchronize()
+        grads.append(out.cpu().numpy())
+    assert np.all(np.isfinite(grads[0])) and np.any(grads[0] != 0.0)
+    for g in grads[1:]:
+        np.testing.assert_array_equal(g, grads[0])
+    unet.close()
