@@ -47,9 +47,10 @@ constexpr int kT = 256;
 // amortised: a thread owns four x-adjacent cells and kCo output channels, so
 // one input row (a 16- and an 8-byte shared load) serves 3 taps x 4 cells x
 // kCo channels in packed FMAs (channel pairs). A training step of 45
-// items takes 549 us; with one output per thread and an input and a weight load
+// items takes 407 us; with one output per thread and an input and a weight load
 // per FMA it took 1821, with one group of 128 threads per CTA here and at most one
-// CTA per SM in the weight gradients 629. Staging is most of what is left.
+// CTA per SM in the weight gradients 629, with one stream and plain launches 549.
+// Staging is most of what is left.
 // One CTA per item, slab of kZ output planes and 16 output channels, two groups
 // of 128 threads each taking half of the input channels; the slab's zero-padded input (rows padded to a multiple of four
 // words, planes so that the eight lanes of a 16-byte access touch all banks)
