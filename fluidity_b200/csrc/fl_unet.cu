@@ -47,7 +47,7 @@ constexpr int kT = 256;
 // amortised: a thread owns four x-adjacent cells and kCo output channels, so
 // one input row (a 16- and an 8-byte shared load) serves 3 taps x 4 cells x
 // kCo channels in packed FMAs (channel pairs). A training step of 45
-// items takes 407 us; with one output per thread and an input and a weight load
+// items takes 404 us; with one output per thread and an input and a weight load
 // per FMA it took 1821, with one group of 128 threads per CTA here and at most one
 // CTA per SM in the weight gradients 629, with one stream and plain launches 549.
 // Staging is most of what is left.
@@ -295,16 +295,33 @@ __global__ void k_pool(const float* __restrict__ in, int S, long long total, flo
   }
 }
 
-// out = relu(coarse[parent] + skip) at resolution S.
-__global__ void k_up_add_relu(const float* __restrict__ coarse, const float* __restrict__ skip, int S, long long total,
-                              float* __restrict__ out) {
-  grid_dependency_wait(coarse, skip);
-  const int H = S / 2, S3 = S * S * S, H3 = H * H * H;
+// out = relu(up(conv1(in)) + skip): a thread forms one output channel of one of the
+// H^3 coarse cells and adds it to the cell's eight children at resolution 2H, which
+// are loaded first. Bound by its launch and one round trip; as two kernels with the
+// coarse sums between them a training step took 302 us instead of 299 (64 items,
+// tensor cores) and 408 instead of 404 (45, FP32).
+__global__ void k_up_conv1_relu(const float* __restrict__ in, int cin, const float* __restrict__ w,
+                                const float* __restrict__ bias, const float* __restrict__ skip, int cout, int H,
+                                long long total, float* __restrict__ out) {
+  grid_dependency_wait(in, w, bias, skip);
+  const int S = 2 * H, H3 = H * H * H;
   for (long long i = blockIdx.x * (long long)kT + threadIdx.x; i < total; i += (long long)gridDim.x * kT) {
-    const int c = (int)(i % S3);
-    const long long bc = i / S3;
-    const int z = c / (S * S), y = (c / S) % S, x = c % S;
-    out[i] = fmaxf(coarse[bc * H3 + ((z >> 1) * H + (y >> 1)) * H + (x >> 1)] + skip[i], 0.0f);
+    const int cell = (int)(i % H3), co = (int)((i / H3) % cout);
+    const long long b = i / ((long long)H3 * cout);
+    const int x = cell % H, y = (cell / H) % H, z = cell / (H * H);
+    const long long fine = (b * cout + co) * 8 * H3 + ((long long)(2 * z) * S + 2 * y) * S + 2 * x;
+    float2 child[4];  // pairs along x
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      child[k] = *reinterpret_cast<const float2*>(skip + fine + (k >> 1) * S * S + (k & 1) * S);
+    float acc = bias[co];
+    const float* src = in + (size_t)b * cin * H3 + cell;
+#pragma unroll 8
+    for (int ci = 0; ci < cin; ++ci) acc = fmaf(__ldg(&w[co * cin + ci]), src[(size_t)ci * H3], acc);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      *reinterpret_cast<float2*>(out + fine + (k >> 1) * S * S + (k & 1) * S) =
+          make_float2(fmaxf(acc + child[k].x, 0.0f), fmaxf(acc + child[k].y, 0.0f));
   }
 }
 
@@ -871,10 +888,8 @@ UNetCache unet_cache_layout(int batch) {
   C.s2 = take(32 * 64);
   C.p2 = take(32 * 8);
   C.bt = take(64 * 8);
-  C.c2 = take(32 * 8);
   C.u2 = take(32 * 64);
   C.d2 = take(32 * 64);
-  C.c1 = take(16 * 64);
   C.u1 = take(16 * 512);
   C.d1 = take(16 * 512);
   C.y = take(512);
@@ -937,12 +952,12 @@ cudaError_t unet_forward(const float* P, const float* x, int batch, float* cache
   g_kernel_launches += 1;
   launch_dep(k_pool, grid_for(B * 32 * 8), kT, 0, s, A + C.s2, 4, B * 32 * 8, A + C.p2);
   fwd3<2, false>(tc, tce, 4, A + C.p2, 32, W(4), Bi(4), 64, A + C.bt, batch, 1, s);
-  g_kernel_launches += 6;
-  launch_dep(k_conv1_fwd, grid_for(B * 32 * 8), kT, 0, s, A + C.bt, 64, W(5), Bi(5), 32, 8, B * 32 * 8, A + C.c2);
-  launch_dep(k_up_add_relu, grid_for(B * 32 * 64), kT, 0, s, A + C.c2, A + C.s2, 4, B * 32 * 64, A + C.u2);
+  g_kernel_launches += 3;
+  launch_dep(k_up_conv1_relu, grid_for(B * 32 * 8), kT, 0, s, A + C.bt, 64, W(5), Bi(5), A + C.s2, 32, 2, B * 32 * 8,
+             A + C.u2);
   fwd3<4, false>(tc, tce, 6, A + C.u2, 32, W(6), Bi(6), 32, A + C.d2, batch, 1, s);
-  launch_dep(k_conv1_fwd, grid_for(B * 16 * 64), kT, 0, s, A + C.d2, 32, W(7), Bi(7), 16, 64, B * 16 * 64, A + C.c1);
-  launch_dep(k_up_add_relu, grid_for(B * 16 * 512), kT, 0, s, A + C.c1, A + C.s1, 8, B * 16 * 512, A + C.u1);
+  launch_dep(k_up_conv1_relu, grid_for(B * 16 * 64), kT, 0, s, A + C.d2, 32, W(7), Bi(7), A + C.s1, 16, 4, B * 16 * 64,
+             A + C.u1);
   fwd3<8, false>(tc, tce, 8, A + C.u1, 16, W(8), Bi(8), 16, A + C.d1, batch, 1, s);
   launch_dep(k_conv1_fwd, grid_for(B * 512), kT, 0, s, A + C.d1, 16, W(9), Bi(9), 1, 512, B * 512, A + C.y);
   if (y != nullptr && y != A + C.y)
@@ -1002,7 +1017,7 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   // d1 (conv3 16->16 on u1); gu1 pre-activation -> g8b
   bwd3_weight<8, false>(tc, tce, 8, A + C.u1, 16, A + C.g8a, 16, batch, A + C.part, GW(8), GB(8), w);
   bwd3_data<8>(tc, tce, 8, A + C.g8a, 16, W(8), 16, A + C.u1, A + C.g8b, batch, s);
-  // u1 = relu(up(c1) + s1): c1 = conv1(d2, 32->16)
+  // u1 = relu(up(conv1(d2, 32->16)) + s1)
   g_kernel_launches += 3;
   launch_dep(k_up_back, grid_for(B * 16 * 64), kT, 0, s, A + C.g8b, 8, B * 16 * 64, A + C.g4c);
   launch_dep(k_conv1_bwd_data, grid_for(B * 32 * 64), kT, 0, s, A + C.g4c, 16, W(7), 32, 64, B * 32 * 64, A + C.d2,
@@ -1012,7 +1027,7 @@ cudaError_t unet_backward(const float* P, float* cache, const float* gy, int bat
   // d2 (conv3 32->32 on u2); gu2 pre-activation -> g4b
   bwd3_weight<4, false>(tc, tce, 6, A + C.u2, 32, A + C.g4a, 32, batch, A + C.part, GW(6), GB(6), w);
   bwd3_data<4>(tc, tce, 6, A + C.g4a, 32, W(6), 32, A + C.u2, A + C.g4b, batch, s);
-  // u2 = relu(up(c2) + s2): c2 = conv1(bt, 64->32)
+  // u2 = relu(up(conv1(bt, 64->32)) + s2)
   g_kernel_launches += 3;
   launch_dep(k_up_back, grid_for(B * 32 * 8), kT, 0, s, A + C.g4b, 4, B * 32 * 8, A + C.g2b);
   launch_dep(k_conv1_bwd_data, grid_for(B * 64 * 8), kT, 0, s, A + C.g2b, 32, W(5), 64, 8, B * 64 * 8, A + C.bt,

@@ -21,7 +21,7 @@ struct UNetLayout {
 
 // Offsets (floats) of each activation / scratch tensor in a training cache of `batch` items.
 struct UNetCache {
-  long long x, e1a, s1, p1, e2a, s2, p2, bt, c2, u2, d2, c1, u1, d1, y;
+  long long x, e1a, s1, p1, e2a, s2, p2, bt, u2, d2, u1, d1, y;
   long long activations;
   long long g8a, g8b, g8c, g4a, g4b, g4c, g2a, g2b, part;
   long long total;

@@ -15,7 +15,7 @@
 // operands and by launch latency, so warp-level MMAs (m16n8k16), which read
 // their operands from where they were staged and need no tensor-memory
 // allocation or epilogue copy, are enough to take the matrix work off the
-// critical path. A training step of 64 items takes 301 us; with im2col operands
+// critical path. A training step of 64 items takes 299 us; with im2col operands
 // written to memory and library GEMMs between them (92 + 20 launches) it took 664,
 // with up to 32 channels per CTA and several items per weight-gradient unit (so 8
 // to 64 CTAs a layer) 494, without programmatic launches 429, with the weight
