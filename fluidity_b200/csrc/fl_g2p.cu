@@ -360,9 +360,10 @@ cudaError_t launch_g2p(const GridView& g, const ParticlesView& p, const int* cel
   if (g.nb == 0 || p.count == 0) return cudaSuccess;
   ++g_kernel_launches;
   if (full_out != nullptr) {
-    static unsigned long long configured = 0;
-    if (first_on_device(configured))
+    static OncePerDevice configured;
+    once_on_device(configured, [] {
       cudaFuncSetAttribute(k_g2p_full, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFullSmem);
+    });
     k_g2p_full<<<g.nb, kG2PThreads, kFullSmem, s>>>(g, p, cell_start, u[0], u[1], u[2], u_old ? u_old[0] : nullptr,
                                                     u_old ? u_old[1] : nullptr, u_old ? u_old[2] : nullptr, full_out,
                                                     rep);

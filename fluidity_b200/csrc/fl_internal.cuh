@@ -20,22 +20,19 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fl_once.h"
+
 namespace fl {
 
-// Host-side once-per-device flag: true the first time it is asked for the
-// current device (bit d of `mask` records device d). Set-up such as a
-// function's shared-memory attribute applies to the current device only, so
-// a process that drives several GPUs repeats it on each.
-inline bool first_on_device(unsigned long long& mask) {
+// Runs `set` once for the current device, before any caller returns.
+template <typename F>
+inline void once_on_device(OncePerDevice& done, F&& set) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+  if (cudaGetDevice(&dev) != cudaSuccess) {
     cudaGetLastError();
-    return true;
+    dev = -1;
   }
-  const unsigned long long bit = 1ull << dev;
-  if (mask & bit) return false;
-  mask |= bit;
-  return true;
+  done.run(dev, set);
 }
 
 constexpr int kBlockAxis = 8;

@@ -367,13 +367,13 @@ cudaError_t launch_p2g(const GridView& g, const ParticlesView& p, const int* cel
                        cudaStream_t s, const unsigned int* order) {
   if (g.nb == 0) return cudaSuccess;
   const size_t smem = sizeof(float2) * kP2GWarps * kWarpTileMax;
-  static unsigned long long configured = 0;
-  if (first_on_device(configured)) {
+  static OncePerDevice configured;
+  once_on_device(configured, [&] {
     cudaFuncSetAttribute(k_p2g_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     // two CTAs per SM: 2 x 30 KB of warp tiles in the 64 KB shared-memory
     // carveout (28% of 228 KB); the rest of the SM's 256 KB stays L1
     cudaFuncSetAttribute(k_p2g_tile, cudaFuncAttributePreferredSharedMemoryCarveout, 28);
-  }
+  });
   ++g_kernel_launches;
   k_p2g_tile<<<g.nb, kP2GThreads, smem, s>>>(g, p, order, cell_start, tiles, rep);
   ++g_kernel_launches;

@@ -2534,12 +2534,12 @@ cudaError_t launch_to_natural(const GridView& g, const MgHierarchy<T>& H, float*
 void configure_pressure_kernels() {
   cl_ctas<float>();  // asked here, outside any stream capture
   cl_ctas<__nv_bfloat16>();
-  static bool done = false;
-  if (done) return;
-  cudaFuncSetAttribute(k_coarse_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 6 * (int)sizeof(float));
-  cudaFuncSetAttribute(k_coarse_solve<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       8192 * 6 * (int)sizeof(float));
-  done = true;
+  static OncePerDevice configured;
+  once_on_device(configured, [] {
+    constexpr int smem = 8192 * 6 * (int)sizeof(float);
+    cudaFuncSetAttribute(k_coarse_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(k_coarse_solve<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
 }
 
 #define FL_INSTANTIATE(T)                                                                                         \

@@ -911,24 +911,24 @@ UNetCache unet_cache_layout(int batch) {
 }
 
 void configure_unet_kernels() {
-  static bool done = false;
-  if (done) return;
-  auto allow = [](auto* kernel, size_t bytes) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  };
-  allow(k_conv3<8, true, false>, ConvTile<8>::smem(2));
-  allow(k_conv3<8, false, false>, ConvTile<8>::smem(16));
-  allow(k_conv3<8, false, true>, ConvTile<8>::smem(16));
-  allow(k_conv3<4, false, false>, ConvTile<4>::smem(32));
-  allow(k_conv3<4, false, true>, ConvTile<4>::smem(32));
-  allow(k_conv3_2<false>, conv2_smem(32));
-  allow(k_conv3_2<true>, conv2_smem(64));
-  allow(k_conv3_wgrad<8, true, 2>, WgradTile<8, true, 2>::kSmem);
-  allow(k_conv3_wgrad<8, false, 16>, WgradTile<8, false, 16>::kSmem);
-  allow(k_conv3_wgrad<4, false, 16>, WgradTile<4, false, 16>::kSmem);
-  allow(k_conv3_wgrad<4, false, 32>, WgradTile<4, false, 32>::kSmem);
-  allow(k_conv3_wgrad<2, false, 32>, WgradTile<2, false, 32>::kSmem);
-  done = true;
+  static OncePerDevice configured;
+  once_on_device(configured, [] {
+    auto allow = [](auto* kernel, size_t bytes) {
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    allow(k_conv3<8, true, false>, ConvTile<8>::smem(2));
+    allow(k_conv3<8, false, false>, ConvTile<8>::smem(16));
+    allow(k_conv3<8, false, true>, ConvTile<8>::smem(16));
+    allow(k_conv3<4, false, false>, ConvTile<4>::smem(32));
+    allow(k_conv3<4, false, true>, ConvTile<4>::smem(32));
+    allow(k_conv3_2<false>, conv2_smem(32));
+    allow(k_conv3_2<true>, conv2_smem(64));
+    allow(k_conv3_wgrad<8, true, 2>, WgradTile<8, true, 2>::kSmem);
+    allow(k_conv3_wgrad<8, false, 16>, WgradTile<8, false, 16>::kSmem);
+    allow(k_conv3_wgrad<4, false, 16>, WgradTile<4, false, 16>::kSmem);
+    allow(k_conv3_wgrad<4, false, 32>, WgradTile<4, false, 32>::kSmem);
+    allow(k_conv3_wgrad<2, false, 32>, WgradTile<2, false, 32>::kSmem);
+  });
 }
 
 // Forward pass of `batch` items; every activation is kept in `cache` (layout unet_cache_layout).
@@ -1078,9 +1078,10 @@ cudaError_t unet_block_residual_loss(const float* y, const float* x, int batch, 
                                      cudaStream_t s) {
   ++g_kernel_launches;
   constexpr size_t smem = kLossWarps * kLossWarpBytes;
-  static unsigned long long configured = 0;
-  if (first_on_device(configured))
+  static OncePerDevice configured;
+  once_on_device(configured, [] {
     cudaFuncSetAttribute(k_block_residual_loss, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
   k_block_residual_loss<<<kLossCtas, kLossWarps * 32, smem, s>>>(y, x, batch, loss, grad);
   return cudaGetLastError();
 }

@@ -791,9 +791,9 @@ template <int KG, int N, int MODE, int IN_KIND, int OUT_KIND>
 cudaError_t launch_conv(const ConvArgs& a, int sms, cudaStream_t s) {
   constexpr size_t smem = conv_smem<KG, N, MODE, IN_KIND, OUT_KIND>();
   auto kern = k_conv_tc<KG, N, MODE, IN_KIND, OUT_KIND>;
-  static unsigned long long configured = 0;
-  if (first_on_device(configured))
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static OncePerDevice configured;
+  once_on_device(configured,
+                 [&] { cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
   const int by_smem = (int)(233472 / (smem + 1024));
   const int cap = conv_ctas_per_sm<KG, N, MODE, IN_KIND, OUT_KIND>();
   const int per_sm = by_smem < cap ? by_smem : cap;
@@ -807,8 +807,8 @@ cudaError_t launch_bt(const uint4* in, long long cap, const uint4* weights, cons
                       int* error, cudaStream_t s) {
   // 96 KB of operands: two CTAs an SM, 128 of its 512 TMEM columns
   constexpr int smem = 32 * (128 + 64) * 16 + 2 * 8 + 8;
-  static unsigned long long configured = 0;
-  if (first_on_device(configured)) cudaFuncSetAttribute(k_bt_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static OncePerDevice configured;
+  once_on_device(configured, [] { cudaFuncSetAttribute(k_bt_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   ++g_kernel_launches;
   launch_dep(k_bt_tc, dim3((nb + 127) / 128, 8), kBtThreads, smem, s, in, cap, weights, bias, out, nb, error);
   return cudaGetLastError();

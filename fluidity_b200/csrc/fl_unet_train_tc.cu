@@ -418,14 +418,14 @@ cudaError_t conv(const UNetTcTrain& t, int layer, bool data, const float* in, co
   const PackLayer p = pack_table().l[pack_index(layer)];
   const dim3 grid((unsigned)((batch + C::kItems - 1) / C::kItems * (S / C::kZ)), COUT / C::kCo);
   ++g_kernel_launches;
-  static unsigned long long configured[2] = {0, 0};
+  static OncePerDevice configured[2];
   if constexpr (VALID) {
     launch_dep(k_conv_mma<S, VALID, CIN, COUT, false>, grid, kConvThreads, smem, s, in, t.w + p.fwd, bias, out, batch,
                relu, nullptr);
   } else {
     auto* kernel = data ? k_conv_mma<S, VALID, CIN, COUT, true> : k_conv_mma<S, VALID, CIN, COUT, false>;
-    if (first_on_device(configured[data]))
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    once_on_device(configured[data],
+                   [&] { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
     launch_dep(kernel, grid, kConvThreads, smem, s, in, t.w + (data ? p.data : p.fwd), bias, out, batch, relu, act);
   }
   return cudaGetLastError();
@@ -437,9 +437,10 @@ cudaError_t wgrad(const float* in, const float* g, int batch, float* part, float
   constexpr int nw = COUT * CIN * 27;
   const int units = (batch + W::kItems - 1) / W::kItems * (S / W::kZ);
   const int ctas = (int)std::min<long long>({(long long)units, 148, kWgradPart / (nw + COUT)});
-  static unsigned long long configured = 0;
-  if (first_on_device(configured))
+  static OncePerDevice configured;
+  once_on_device(configured, [] {
     cudaFuncSetAttribute(k_wgrad_mma<S, VALID, CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)W::kSmem);
+  });
   ++g_kernel_launches;
   launch_dep(k_wgrad_mma<S, VALID, CIN, COUT>, dim3(ctas, COUT / W::kCo), kWgradThreads, W::kSmem, s, in, g,
              batch, units, part);

@@ -558,3 +558,72 @@ def test_weight_gradients_end_before_the_stream_goes_on(tensor_cores):
     for g in grads[1:]:
         np.testing.assert_array_equal(g, grads[0])
     unet.close()
+
+
+FIRST_CALLS = """
+import threading
+import torch
+import fluidity_b200 as fb
+
+threads, tensor_cores = 6, {tensor_cores}
+torch.manual_seed(1)
+x = torch.randn((8, 2, 10, 10, 10), device="cuda")
+x[:, 1] = 1.0
+p = 0.1 * torch.randn(fb.UNet.param_count(), device="cuda")
+torch.cuda.synchronize()
+start, results = threading.Barrier(threads), [None] * threads
+
+
+def work(k):
+    net = fb.UNet(8, tensor_cores=tensor_cores)
+    y, g, gy, loss = torch.zeros((8, 512), device="cuda"), torch.zeros_like(p), torch.zeros((8, 512), device="cuda"), torch.zeros(1, device="cuda")
+    torch.cuda.synchronize()
+    start.wait()
+    net.forward(p, x, y)
+    fb.UNet.block_residual_loss(y, x, loss, gy)
+    net.backward(p, gy, g)
+    torch.cuda.synchronize()
+    results[k] = torch.cat([y.ravel(), g, loss])
+    net.close()
+
+
+ts = [threading.Thread(target=work, args=(k,)) for k in range(threads)]
+[t.start() for t in ts]
+[t.join() for t in ts]
+assert all(r is not None and bool(torch.isfinite(r).all()) for r in results), [r is None for r in results]
+assert all(torch.equal(r, results[0]) for r in results)
+"""
+
+
+@pytest.mark.parametrize("tensor_cores", [False, True])
+def test_first_calls_of_several_threads(tensor_cores):
+    """Threads with a handle each whose first passes start together, in a process of their own so that
+    no kernel's shared-memory attribute is set yet: no launch precedes it, and all get the same bits."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    root = Path(__file__).resolve().parent.parent
+    r = subprocess.run([sys.executable, "-c", FIRST_CALLS.format(tensor_cores=tensor_cores)], cwd=root, timeout=300,
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_network_on_a_second_device():
+    """Kernel attributes belong to a device: after a pass on one GPU the same pass runs on another."""
+    import torch
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    rng, results = np.random.default_rng(3), []
+    x, gy, th = rng.normal(size=(4, 2, 10, 10, 10)), rng.normal(size=(4, 512)), U.init_params(2)
+    for device in (0, 1):
+        with torch.cuda.device(device):
+            net, P, X, DY = fb.UNet(4), _t(th), _t(x), _t(gy)
+            Y, G = torch.zeros((4, 512), device="cuda"), torch.zeros_like(P)
+            net.forward(P, X, Y)
+            net.backward(P, DY, G)
+            torch.cuda.synchronize()
+            results.append(torch.cat([Y.ravel(), G]).cpu().numpy())
+            net.close()
+    np.testing.assert_array_equal(results[0], results[1])
