@@ -867,10 +867,8 @@ __global__ void __launch_bounds__(512 / CPT)
       zp += sums[w].y;
     }
     if (!(zr > 0.0) || !isfinite(zr)) {  // the same in every CTA
-      if (blk == 0 && t == 0) {
-        st->status = kAborted;
-        st->done = 1;
-      }
+      // (the update raises `done`: CTAs of this grid may not have read it yet)
+      if (blk == 0 && t == 0) st->status = kAborted;
       return;
     }
     const double exact = first ? 0.0 : (zr - zp) / rz_prev;
@@ -1846,7 +1844,9 @@ __global__ void k_dots(int n, const T* __restrict__ z, const float* __restrict__
 
 // e += alpha d; r_next = r - alpha q; ||r_next||^2 -> stop test. With kAlpha
 // every CTA forms alpha itself from the nb per-block partials of d.q (as
-// k_direction_finish does otherwise).
+// k_direction_finish does otherwise); where that or the direction broke down,
+// all CTAs leave e and r as they are and the last one ends the solve. `done` and
+// `status` change in the last CTA alone, when every other has read them.
 template <bool kAlpha>
 __global__ void __launch_bounds__(kThreads)
     k_update(int n, int nb, const double* __restrict__ dq, const float* __restrict__ d, const float* __restrict__ q,
@@ -1872,6 +1872,7 @@ __global__ void __launch_bounds__(kThreads)
     ev = e4[i];
   };
   if (kAlpha) {
+    const bool broken = st->status != 0;  // by the direction
     if (i < count) load();  // in flight while alpha is formed
     __shared__ double sums[kThreads / 32];
     double acc = 0.0;
@@ -1883,10 +1884,11 @@ __global__ void __launch_bounds__(kThreads)
     double total = sums[0];
 #pragma unroll
     for (int w = 1; w < kThreads / 32; ++w) total += sums[w];
-    if (!(total > 0.0) || !isfinite(total)) {  // the same in every CTA
-      if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (broken || !(total > 0.0) || !isfinite(total)) {  // the same in every CTA
+      if (last_block(st) && threadIdx.x == 0) {
         st->status = kAborted;
         st->done = 1;
+        st->ticket = 0;
       }
       return;
     }

@@ -341,3 +341,38 @@ def test_vcycle_coarse_levels_in_a_cluster(precision, tol, n, levels):
                        coarse_sweeps=opt.coarse_sweeps)
     assert rel_err(z, zo, ct == 1) <= tol
     ctx.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n", [24, 144, 152])
+def test_solve_that_breaks_down_ends_and_leaves_no_trace(precision, n):
+    """A predicted velocity that is not a number makes z.r not positive: the solve ends with ABORTED
+    where the kernels that use the CG scalars sum them (27 and 1000 blocks) and where kernels of their
+    own do (1331), after no iteration, and the next solve gives the bits of the one before."""
+    import torch
+
+    ctx, _, m = dam_break_context(n)
+    tp, opt = fb.transfer_params(scenes.DT, m), fb.default_pressure_options(precision=precision)
+    code, diag = ctx.step(tp, opt)
+    assert code == fb.OK
+    f, cells = ctx.fields(), diag.active_blocks * 512
+    u = [torch.from_numpy(fb.copy_to_host(f["u_pred"][a], cells, np.float32)).cuda() for a in range(3)]
+    out = [torch.zeros(cells, device="cuda") for _ in range(3)]
+    arr = lambda ts: (ctypes.c_void_p * 3)(*[t.data_ptr() for t in ts])  # noqa: E731
+    broken = [t.clone() for t in u]
+    fluid = int(np.flatnonzero(fb.copy_to_host(f["cell_type"], cells, np.uint8) == 1)[-1])
+    broken[1][fluid] = float("nan")
+    p = torch.zeros(cells, dtype=torch.float64, device="cuda")
+    pressures = []
+    for velocities, want in ((u, fb.OK), (broken, fb.ABORTED), (u, fb.OK), (broken, fb.ABORTED), (u, fb.OK)):
+        d = fb.PressureDiagnostics()
+        code = fb.library().fl_pressure_project(ctx.handle, arr(velocities), arr(out), ctypes.byref(tp), ctypes.byref(opt),
+                                                ctypes.byref(d), p.data_ptr(), None)
+        assert code == want
+        if code == fb.OK:
+            pressures.append(p.cpu().numpy())
+        else:
+            assert d.status == fb.ABORTED and d.iterations == 0
+    for other in pressures[1:]:
+        np.testing.assert_array_equal(other, pressures[0])
+    ctx.close()
