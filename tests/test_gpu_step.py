@@ -376,3 +376,19 @@ def test_solve_that_breaks_down_ends_and_leaves_no_trace(precision, n):
     for other in pressures[1:]:
         np.testing.assert_array_equal(other, pressures[0])
     ctx.close()
+
+
+def test_short_states_in_a_context_of_large_capacity():
+    """Upload and download of a few particles where the arrays lie 2^31 bytes apart, more than
+    the pitch that the device states for strided copies (76 GB of device memory, none of it touched beyond the particles)."""
+    import torch
+
+    if torch.cuda.mem_get_info()[0] < 90e9:
+        pytest.skip("needs 90 GB of free device memory")
+    rng = np.random.default_rng(8)
+    soa = [rng.uniform(0.2, 0.8, size=(15, k)).astype(np.float32) for k in (1000, 7)]
+    ctx = fb.LiquidContext(16, capacity=2 ** 29)
+    for s in soa:
+        ctx.upload(s)
+        np.testing.assert_array_equal(ctx.download(), s)
+    ctx.close()
