@@ -35,10 +35,16 @@ __device__ __forceinline__ bool lattice_cell_of(const GridView& g, const float x
 }
 
 // Particles per thread in k_mark_blocks, k_cell_keys and k_scatter_index: a CTA
-// of 256 threads covers 1024 consecutive particles, particle k * 256 + t of the
-// CTA's range on thread t, with every independent load of the four issued together.
+// of 256 threads covers 1024 consecutive particles, with every independent load
+// of a thread's four issued together.
 constexpr int kSortIlp = 4;
 constexpr int kSortThreads = 256;
+
+// This thread's first particle in k_cell_keys: a warp covers 32 kSortIlp
+// consecutive ones, particle 32 k + lane of them on its lane.
+__device__ __forceinline__ unsigned long long sort_first() {
+  return ((unsigned long long)blockIdx.x * kSortThreads + (threadIdx.x & ~31u)) * kSortIlp + (threadIdx.x & 31u);
+}
 
 // HBM-bound: 12 B of positions per particle. Particles arrive nearly in cell
 // order, so a warp holds one or two runs of equal blocks: only the first lane of
@@ -138,11 +144,11 @@ __global__ void k_build_nbr27(GridView g, int* nbr27) {
 __global__ void __launch_bounds__(kSortThreads)
     k_cell_keys(GridView g, ParticlesView p, unsigned int* keys, unsigned int* index, int* counts,
                 DeviceReport* rep) {
-  const unsigned long long i0 = (unsigned long long)blockIdx.x * (kSortIlp * kSortThreads) + threadIdx.x;
+  const unsigned long long i0 = sort_first();
   float X[kSortIlp][3];
 #pragma unroll
   for (int k = 0; k < kSortIlp; ++k) {
-    const unsigned long long i = i0 + (unsigned long long)k * kSortThreads;
+    const unsigned long long i = i0 + (unsigned long long)k * 32;
 #pragma unroll
     for (int d = 0; d < 3; ++d) X[k][d] = i < p.count ? lattice_coord(g, p.x[d][i], d) : 0.0f;
   }
@@ -150,7 +156,7 @@ __global__ void __launch_bounds__(kSortThreads)
   bool fin_k[kSortIlp];
 #pragma unroll
   for (int k = 0; k < kSortIlp; ++k) {
-    const unsigned long long i = i0 + (unsigned long long)k * kSortThreads;
+    const unsigned long long i = i0 + (unsigned long long)k * 32;
     bool fin = true, inside = true;
     int bidx = 0, l = 0;
     if (i < p.count) {
@@ -169,27 +175,43 @@ __global__ void __launch_bounds__(kSortThreads)
     o[k] = (i < p.count && fin && inside) ? g.table[bidx] : -1;
     lcell[k] = l;
   }
-  // One counter update per particle, all four in flight: particles arrive nearly
-  // in cell order, but after a step a warp's 32 lie in some 20 cells, so joining
-  // equal keys first saves few updates and serializes the four. The ranks within
-  // a cell are unique; k_sort_cells_block fixes their final order. A warp
-  // match before the updates took 262 us at the 256^3 splash, this 168.
+  // One counter update per run of equal keys in the warp, all four in flight: the
+  // run's first lane adds its length and the others take the ranks that follow.
+  // The ranks within a cell are unique; k_sort_cells_block fixes their final
+  // order, the sooner the closer to it they are. Particles in cell order are runs
+  // of a whole cell, which as single updates queue for one address: 2.1M
+  // particles in order at 8, 16 and 64 per cell took 12, 20 and 52 us, now 13
+  // each, and k_sort_cells_block at 64 went from 460 to 67. After a step a warp's 32
+  // lie in some 20 cells and runs save little: 157 us at the 256^3 splash, 169 with
+  // single updates, 203 with the four in turn, 260 with a warp match (which in
+  // random order at 64 per cell leaves ranks that the block sort orders in 144 us
+  // instead of 240; at up to 24 per cell the runs win there too, 37 against 45).
   unsigned int key[kSortIlp], rank[kSortIlp];
+  int head[kSortIlp];  // lane of the run's first particle
+  const int lane = (int)(threadIdx.x & 31);
 #pragma unroll
   for (int k = 0; k < kSortIlp; ++k) {
-    const unsigned long long i = i0 + (unsigned long long)k * kSortThreads;
-    key[k] = 0xffffffffu;
+    const unsigned long long i = i0 + (unsigned long long)k * 32;
+    key[k] = o[k] >= 0 ? (unsigned int)o[k] * 512u + (unsigned int)lcell[k] : 0xffffffffu;
+    const unsigned int before = __shfl_up_sync(0xffffffffu, key[k], 1);
+    const unsigned int heads = __ballot_sync(0xffffffffu, lane == 0 || before != key[k]);
+    head[k] = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
     rank[k] = 0;
-    if (o[k] >= 0) {
-      key[k] = (unsigned int)o[k] * 512u + (unsigned int)lcell[k];
-      rank[k] = (unsigned int)atomicAdd(&counts[key[k]], 1);
-    } else if (i < p.count) {  // not finite: out of range; else outside the lattice or in an inactive block
-      report_error(rep, fin_k[k] ? kFailedPrecondition : kOutOfRange, i);
+    if (o[k] < 0) {
+      if (i < p.count)  // not finite: out of range; else outside the lattice or in an inactive block
+        report_error(rep, fin_k[k] ? kFailedPrecondition : kOutOfRange, i);
+    } else if (head[k] == lane) {
+      const unsigned int after = lane < 31 ? heads >> (lane + 1) : 0u;
+      const int length = after != 0u ? __ffs(after) : 32 - lane;
+      rank[k] = (unsigned int)atomicAdd(&counts[key[k]], length);
     }
   }
 #pragma unroll
+  for (int k = 0; k < kSortIlp; ++k)
+    rank[k] = __shfl_sync(0xffffffffu, rank[k], head[k]) + (unsigned int)(lane - head[k]);
+#pragma unroll
   for (int k = 0; k < kSortIlp; ++k) {
-    const unsigned long long i = i0 + (unsigned long long)k * kSortThreads;
+    const unsigned long long i = i0 + (unsigned long long)k * 32;
     if (i < p.count) {
       keys[i] = key[k];
       index[i] = rank[k];  // arrival rank within the cell (order not yet deterministic)

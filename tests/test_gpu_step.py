@@ -392,3 +392,46 @@ def test_short_states_in_a_context_of_large_capacity():
         ctx.upload(s)
         np.testing.assert_array_equal(ctx.download(), s)
     ctx.close()
+
+
+@pytest.mark.parametrize("per", [1, 31, 32, 33, 129])
+@pytest.mark.parametrize("order", ["cells", "pairs", "reversed"])
+def test_sort_of_runs_of_equal_cells(per, order):
+    """Particles whose cells come in runs around a warp's 32 lanes and the 128 particles of its four
+    turns (a cell after the other, two cells in turn, the cells backwards), with a last warp that is not
+    full: the stable cell sort, and a particle without a cell in the middle of a run is reported."""
+    import torch
+
+    n, cells = 32, 37
+    rng = np.random.default_rng(per)
+    cell = np.repeat(np.arange(cells), per)
+    if order == "pairs":
+        cell = np.concatenate([cell[0::2], cell[1::2]]) if per == 1 else cell.reshape(cells, per)[:36].reshape(18, 2, per).transpose(
+            0, 2, 1).ravel()
+    elif order == "reversed":
+        cell = cell[::-1]
+    x = np.stack([8 + cell % 8, 8 + cell // 8, np.full_like(cell, 9)]) + rng.uniform(0.05, 0.95, size=(3, len(cell)))
+    soa = np.zeros((15, len(cell)), np.float32)
+    soa[0:3] = x / n
+    soa[3] = np.arange(len(cell))
+    src, dst = torch.from_numpy(soa).cuda(), torch.zeros(soa.shape, device="cuda")
+
+    def parts(t):
+        p = fb.Particles()
+        p.x[:] = [t[d].data_ptr() for d in range(3)]
+        p.v[:] = [t[3 + d].data_ptr() for d in range(3)]
+        p.c[:] = [t[6 + d].data_ptr() for d in range(9)]
+        p.mass, p.count = None, soa.shape[1]
+        return p
+
+    ctx, lib, rep = fb.LiquidContext(n, capacity=len(cell)), fb.library(), fb.Report()
+    a, b = parts(src), parts(dst)
+    assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(a), None, ctypes.byref(rep)) == fb.OK
+    assert lib.fl_sort_particles_by_block(ctx.handle, ctypes.byref(a), ctypes.byref(b), None, ctypes.byref(rep)) == fb.OK
+    np.testing.assert_array_equal(dst.cpu().numpy(), soa[:, sort_permutation(soa, n)])
+    bad = len(cell) // 2
+    src[0, bad] = float("nan")
+    assert lib.fl_sort_particles_by_block(ctx.handle, ctypes.byref(a), ctypes.byref(b), None,
+                                          ctypes.byref(rep)) == fb.OUT_OF_RANGE
+    assert rep.first_bad_index == bad
+    ctx.close()
