@@ -435,3 +435,44 @@ def test_sort_of_runs_of_equal_cells(per, order):
                                           ctypes.byref(rep)) == fb.OUT_OF_RANGE
     assert rep.first_bad_index == bad
     ctx.close()
+
+
+def test_sort_gathers_only_particles_that_have_a_cell():
+    """Particles without a cell leave the sort's index shorter than the particles: in a context whose
+    index still holds a longer sort's entries, and in a fresh one, the rest arrives in order and nothing
+    from past the input (here: the longer sort's particles, in the same tensor) reaches the output."""
+    import torch
+
+    n = 32
+    rng = np.random.default_rng(21)
+    for before in (0, 5000):
+        ctx, lib, rep = fb.LiquidContext(n, capacity=5000), fb.library(), fb.Report()
+        soa = np.zeros((15, 5000), np.float32)
+        soa[0:3] = rng.uniform(0.2, 0.8, size=(3, 5000))
+        soa[3], soa[3, 700:] = np.arange(5000), -1.0
+        src = torch.from_numpy(soa).cuda()
+        for count, bad in ((before, 0), (700, 5)):
+            if count == 0:
+                continue
+            dst = torch.full((15, 5000), 7.0, device="cuda")
+            views = []
+            for t in (src, dst):
+                p = fb.Particles()
+                p.x[:] = [t[d].data_ptr() for d in range(3)]
+                p.v[:] = [t[3 + d].data_ptr() for d in range(3)]
+                p.c[:] = [t[6 + d].data_ptr() for d in range(9)]
+                p.mass, p.count = None, count
+                views.append(p)
+            a, b = views
+            assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(a), None, ctypes.byref(rep)) == fb.OK
+            good = np.ones(count, bool)
+            good[rng.choice(count, bad, replace=False)] = False
+            src[1, torch.from_numpy(np.flatnonzero(~good)).cuda()] = float("nan")
+            code = lib.fl_sort_particles_by_block(ctx.handle, ctypes.byref(a), ctypes.byref(b), None, ctypes.byref(rep))
+            assert code == (fb.OUT_OF_RANGE if bad else fb.OK)
+            kept = soa[:, :count][:, good]
+            got = dst.cpu().numpy()
+            np.testing.assert_array_equal(got[:, :count - bad], kept[:, sort_permutation(kept, n)])
+            if bad:
+                assert np.all(got[3, count - bad:count] >= 0.0) and np.all(got[:, count:] == 7.0)
+        ctx.close()
