@@ -40,33 +40,40 @@ __device__ __forceinline__ bool lattice_cell_of(const GridView& g, const float x
 constexpr int kSortIlp = 4;
 constexpr int kSortThreads = 256;
 
-// This thread's first particle in k_cell_keys: a warp covers 32 kSortIlp
-// consecutive ones, particle 32 k + lane of them on its lane.
+// This thread's first particle in k_mark_blocks and k_cell_keys: a warp covers
+// 32 kSortIlp consecutive ones in kSortIlp turns, particle 32 k + lane of them on its lane.
 __device__ __forceinline__ unsigned long long sort_first() {
   return ((unsigned long long)blockIdx.x * kSortThreads + (threadIdx.x & ~31u)) * kSortIlp + (threadIdx.x & 31u);
 }
 
-// HBM-bound: 12 B of positions per particle. Particles arrive nearly in cell
-// order, so a warp holds one or two runs of equal blocks: only the first lane of
-// a run looks the block up, and it stores only where the byte is still 0
-// (contended same-address stores serialize in L2). With one particle per thread
-// and a warp match instead of the runs, a 256^3 splash substep took 8143 us (now
-// 8107) and the 120 x 104 x 88 transfers 621 us (now 616).
+// 12 B of positions per particle, but bound by the marks: those of the blocks that
+// the resident CTAs are in share a few sectors, so every lookup that L1 does not
+// hold and every store goes to one L2 slice. Particles arrive nearly in cell order:
+// a warp's 128 consecutive ones are a few runs of equal blocks, only a run's first
+// particle looks its block up, one turn after the other, and stores where the mark is
+// still 0. Where a turn has more than kMarkRuns runs the particles are in no order,
+// and a warp match finds the blocks. 2.1M particles in order take 30 us, with runs
+// joined only within a turn and the four lookups together 77, with one particle per
+// thread and a match always 42; in random order 40, 75 and 42, without the match 60;
+// the 256^3 splash's moved ones 262, 470 and 470, the 128^3 dam break's 36, 35 and 35.
+constexpr int kMarkRuns = 8;
+
 __global__ void __launch_bounds__(kSortThreads)
     k_mark_blocks(GridView g, ParticlesView p, unsigned char* occ, DeviceReport* rep) {
-  const unsigned long long i0 = (unsigned long long)blockIdx.x * (kSortIlp * kSortThreads) + threadIdx.x;
+  const unsigned long long i0 = sort_first();
   float x[kSortIlp][3];
 #pragma unroll
   for (int k = 0; k < kSortIlp; ++k) {
-    const unsigned long long i = i0 + (unsigned long long)k * kSortThreads;
+    const unsigned long long i = i0 + (unsigned long long)k * 32;
 #pragma unroll
     for (int d = 0; d < 3; ++d) x[k][d] = i < p.count ? p.x[d][i] : 0.0f;
   }
+  const int lane = (int)(threadIdx.x & 31);
   int idx[kSortIlp];
   bool look[kSortIlp];
 #pragma unroll
   for (int k = 0; k < kSortIlp; ++k) {
-    const unsigned long long i = i0 + (unsigned long long)k * kSortThreads;
+    const unsigned long long i = i0 + (unsigned long long)k * 32;
     idx[k] = -1;
     if (i < p.count) {
       int cell[3];
@@ -83,15 +90,19 @@ __global__ void __launch_bounds__(kSortThreads)
       else
         idx[k] = (b[2] * g.bdim[1] + b[1]) * g.bdim[0] + b[0];  // at most 2^21 blocks
     }
-    const int before = __shfl_up_sync(0xffffffffu, idx[k], 1);
-    look[k] = idx[k] >= 0 && ((threadIdx.x & 31) == 0 || before != idx[k]);
+    // the particle before: the lane below's, or for lane 0 the last lane's of the turn before
+    const int below = __shfl_up_sync(0xffffffffu, idx[k], 1);
+    const int last = k > 0 ? __shfl_sync(0xffffffffu, idx[k > 0 ? k - 1 : 0], 31) : -1;
+    look[k] = idx[k] >= 0 && (lane == 0 ? last : below) != idx[k];
   }
-  bool store[kSortIlp];
 #pragma unroll
-  for (int k = 0; k < kSortIlp; ++k) store[k] = look[k] && occ[idx[k]] == 0;
-#pragma unroll
-  for (int k = 0; k < kSortIlp; ++k)
-    if (store[k]) occ[idx[k]] = 1;
+  for (int k = 0; k < kSortIlp; ++k) {
+    if (__popc(__ballot_sync(0xffffffffu, look[k])) > kMarkRuns) {  // no order: a block's first lane looks
+      const unsigned same = __match_any_sync(0xffffffffu, idx[k]);
+      look[k] = idx[k] >= 0 && lane == __ffs(same) - 1;
+    }
+    if (look[k] && occ[idx[k]] == 0) occ[idx[k]] = 1;
+  }
 }
 
 __global__ void k_flag_active(GridView g, const unsigned char* occ, int* flag, int total) {

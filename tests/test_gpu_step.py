@@ -258,17 +258,31 @@ def test_empty_and_invalid_particles():
     assert e.value.code == fb.RESOURCE_EXHAUSTED
 
 
-@pytest.mark.parametrize("count", [1, 31, 33, 1023, 1024, 1025, 5000])
-def test_topology_from_unordered_particles(count):
-    """Blocks marked by particles in no order, at counts around a warp and around the 1024
-    particles of a CTA, against the blocks (and their ring) found on the host; a particle that
-    has no block is reported with its index."""
+def _in_runs(count, rng, n, run):
+    """Positions whose blocks come in runs of `run` particles (0: in no order, some blocks with many)."""
+    if run == 0:
+        x = rng.uniform(1.0 / n, 1.0 - 1.0 / n, size=(3, count))
+        x[0, ::2] *= 0.25
+        return x
+    blocks = rng.permutation((n // 8) ** 3)[: -(-count // run)]
+    b = np.repeat(np.stack([blocks % 8, blocks // 8 % 8, blocks // 64]), run, axis=1)[:, :count]
+    return (8 * b + rng.uniform(0.01, 7.99, size=(3, count))) / n
+
+
+@pytest.mark.parametrize("run", [0, 3, 4, 5, 31, 33, 128, 200])
+@pytest.mark.parametrize("count", [1, 31, 33, 127, 129, 1023, 1024, 1025, 5000])
+def test_topology_from_unordered_particles(count, run):
+    """Blocks marked by particles in no order and in runs of a block (around the 8 runs a turn of 32
+    and around a warp's 128 particles), at counts around a turn, a warp and the 1024 particles of a CTA,
+    against the blocks (and their ring) found on the host; a particle that has no block is reported with
+    its index."""
     import torch
 
+    if run and count > run * 512:
+        pytest.skip("more runs than blocks")
     n, rng = 64, np.random.default_rng(count)
     soa = np.zeros((15, count), np.float32)
-    soa[0:3] = rng.uniform(1.0 / n, 1.0 - 1.0 / n, size=(3, count))
-    soa[0, ::2] *= 0.25  # uneven: some blocks with many particles
+    soa[0:3] = _in_runs(count, rng, n, run)
     ctx = fb.LiquidContext(n, capacity=count)
     dev = torch.from_numpy(soa).cuda()
     p = fb.Particles()
