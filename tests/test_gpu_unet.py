@@ -390,11 +390,14 @@ def _open_network(seed):
     return th
 
 
-@pytest.mark.parametrize("batch", [1, 5, 33, 40])
+@pytest.mark.parametrize("batch", [1, 5, 33, 40, 160])
 def test_fp32_convolutions_at_item_counts(batch):
-    """The FP32 forward and backward at item counts around the items a CTA takes (4, 32) and the
-    work units of one CTA per SM (40 items are 160 slabs), against the FP64 oracle: sums of at most
-    864 FP32 terms in the forward, 20k in a gradient, 1e-4 per layer; twice gives the same bits."""
+    """The FP32 forward and backward at item counts around the items a CTA takes at 2^3 (32 in the
+    convolutions, 4 in the weight gradients; one elsewhere) and, at 160, with more work units in every
+    layer's weight gradient than it has CTAs (640 slabs against 296 at 8^3, 160 items against 151 and 75
+    at 4^3, 40 groups against 37 at 2^3), so that CTAs take a second one; against the FP64 oracle:
+    sums of at most 864 FP32 terms in the forward, 82k in a gradient, 1e-4 per layer; twice gives the
+    same bits."""
     import torch
 
     rng = np.random.default_rng(batch)
@@ -421,11 +424,13 @@ def test_fp32_convolutions_at_item_counts(batch):
         off += nw + nb
 
 
-@pytest.mark.parametrize("batch", [1, 3, 17, 40])
+@pytest.mark.parametrize("batch", [1, 3, 17, 40, 160])
 def test_tensor_core_convolutions_at_item_counts(batch):
-    """The tensor-core forward, and the backward from the FP32 forward's cache, at item counts
-    around the items a CTA takes (2, 4, 16) and the work units of one CTA per SM, against the FP64
-    oracle at BF16 tolerances (as test_tensor_core_training_matches_oracle_at_bf16_tolerance)."""
+    """The tensor-core forward, and the backward from the FP32 forward's cache, at item counts around
+    the four items a CTA takes at 2^3 (one elsewhere) and, at 160, with more work units in every layer's
+    weight gradient than it has CTAs (320 slabs against 148 at 8^3, 160 items against 148 and 75 at
+    4^3, 40 groups against 37 at 2^3), against the FP64 oracle at BF16 tolerances (as
+    test_tensor_core_training_matches_oracle_at_bf16_tolerance)."""
     import torch
 
     rng = np.random.default_rng(batch)
@@ -453,12 +458,8 @@ def test_tensor_core_convolutions_at_item_counts(batch):
         off += nw + nb
 
 
-@pytest.mark.parametrize("shape", [(1, 1, 1), (6, 5, 2), (7, 3, 3), (1, 5, 10)])
-def test_tensor_core_inference_at_block_counts(shape):
-    """The inference where the 2^3 layer's tiles of 128 blocks end (8, 126, 128 and 132 active
-    blocks: a box of full blocks at the lattice's corner and the next layer), against the FP32
-    forward, with the first third of the blocks without residual: 3e-2 of the largest value, as
-    the test above."""
+def _box_of_blocks(shape):
+    """A context whose active blocks are a box of full blocks at the lattice's corner and the next layer."""
     import ctypes
 
     import torch
@@ -483,8 +484,20 @@ def test_tensor_core_inference_at_block_counts(shape):
     lib, rep, a, b = fb.library(), fb.Report(), parts(src), parts(dst)
     assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(a), None, ctypes.byref(rep)) == fb.OK
     assert lib.fl_sort_particles_by_block(ctx.handle, ctypes.byref(a), ctypes.byref(b), None, ctypes.byref(rep)) == fb.OK
+    assert len(ctx.active_blocks()) == np.prod([k + 1 for k in shape])
+    return ctx
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (6, 5, 2), (7, 3, 3), (1, 5, 10)])
+def test_tensor_core_inference_at_block_counts(shape):
+    """The inference where the 2^3 layer's tiles of 128 blocks end (8, 126, 128 and 132 active
+    blocks: a box of full blocks at the lattice's corner and the next layer), against the FP32
+    forward, with the first third of the blocks without residual: 3e-2 of the largest value, as
+    the test above."""
+    import torch
+
+    ctx = _box_of_blocks(shape)
     nb = len(ctx.active_blocks())
-    assert nb == np.prod([k + 1 for k in shape])
     rng = np.random.default_rng(nb)
     r = rng.normal(size=(nb, 512))
     if nb > 27:
@@ -497,6 +510,38 @@ def test_tensor_core_inference_at_block_counts(shape):
     z, ref = z.cpu().numpy(), ref.cpu().numpy()
     assert np.any(ref != 0.0)
     assert _rel(z, ref) <= 3e-2
+    ctx.close()
+
+
+@pytest.mark.parametrize("shape", [(4, 4, 5), (8, 10, 2), (11, 9, 10)])
+def test_tensor_core_inference_with_several_blocks_per_cta(shape):
+    """The inference where a CTA of the convolutions takes block after block through its two operand and
+    two accumulator stages: 150 and 297 blocks, one or two more than one CTA per SM and two, and 1320,
+    four and more for each of two CTAs per SM. The residual is zero in parts of the box, so that
+    blocks to skip lie between others in a CTA's sequence. Against the FP32 forward, each
+    block for itself: 3e-2 of its largest value, as the tests above for all of them."""
+    import torch
+
+    ctx = _box_of_blocks(shape)
+    blocks = ctx.active_blocks()
+    nb = len(blocks)
+    rng = np.random.default_rng(nb)
+    r = rng.normal(size=(nb, 512))
+    if nb > 1000:  # cubes of 4^3 blocks all over the box
+        r[(blocks // 4).sum(1) % 2 == 1] = 0.0
+    else:
+        r[blocks[:, 0] < len(np.unique(blocks[:, 0])) // 2] = 0.0
+    near = {tuple(b + d) for b in blocks[np.any(r != 0.0, 1)] for d in np.indices((3, 3, 3)).reshape(3, -1).T - 1}
+    idle = np.array([tuple(b) not in near for b in blocks])
+    assert 0 < idle.sum() < nb // 2
+    r = _t(r.ravel())
+    ctx.set_learned_preconditioner(_t(U.init_params(9) + 0.01 * rng.normal(size=U.param_count())))
+    z, ref = torch.full((nb * 512,), 5.0, device="cuda"), torch.full((nb * 512,), 5.0, device="cuda")
+    ctx.apply_learned(r, z, kernels=0)
+    ctx.apply_learned(r, ref, kernels=1)
+    z, ref = z.cpu().numpy().reshape(nb, 512), ref.cpu().numpy().reshape(nb, 512)
+    assert np.all(z[idle] == 0.0) and np.all(ref[idle] == 0.0)
+    assert np.all(np.abs(z - ref).max(1) <= 3e-2 * np.abs(ref).max(1))
     ctx.close()
 
 
