@@ -601,78 +601,94 @@ __global__ void __launch_bounds__(1024) k_masked_mse(const float* __restrict__ y
 // over the V items whose block holds residual. The zero correction scores at
 // most 1; a network that inverts A_b on its block scores 0.
 //
-// Bound by latency: an item is 12 KB. One cluster of 8 CTAs x 16 warps, a warp
-// per item (16 cells per lane, no CTA barrier in the item loop), so 128 items
-// are in flight at once; V and the loss are summed over the cluster through
-// distributed shared memory in item order, so no scratch memory and no second
-// launch is needed and the call stays bitwise reproducible. With one CTA taking
-// the items in turn a BF16 training step of 64 items took 801 us, now 676 us.
-constexpr int kLossCtas = 8, kLossWarps = 16, kLossMaxItems = 1024;
+// Bound by latency: an item is 12 KB. One cluster of 8 CTAs x 16 warps, four warps
+// per item (four cells per thread, a barrier of their own), so 32 items are in
+// flight at once; V and the loss are summed over the cluster through distributed
+// shared memory in item order, so no scratch memory and no second launch is
+// needed and the call stays bitwise reproducible. One item takes 15 us, 64 16 and
+// 1024 114; with a warp per item 23, 25 and 131, with a CTA per item 15, 26 and
+// 260, and with one CTA taking all items in turn 12, 210 and 3230.
+constexpr int kLossCtas = 8, kLossWarps = 16, kLossItemWarps = 4, kLossMaxItems = 1024;
 constexpr int kLossFlags = 1024;  // bytes: 1000 window flags, padded
-constexpr size_t kLossWarpBytes = kLossFlags + sizeof(float) * 512;
+constexpr size_t kLossItemBytes = kLossFlags + sizeof(float) * 512;
 
 __global__ void __cluster_dims__(kLossCtas, 1, 1) __launch_bounds__(kLossWarps * 32)
     k_block_residual_loss(const float* __restrict__ y, const float* __restrict__ x, int batch,
                           float* __restrict__ loss, float* __restrict__ grad) {
   constexpr int kMine = kLossMaxItems / kLossCtas;
+  constexpr int kGroups = kLossWarps / kLossItemWarps, kThreads = 32 * kLossItemWarps, kCells = 512 / kThreads;
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ double den[kMine], num[kMine];
+  __shared__ double parts[kLossWarps];
   __shared__ int valid_cta;
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned char* flag = dyn + warp * kLossWarpBytes;  // bit 0 fluid, bit 1 not solid
+  const int group = warp / kLossItemWarps, t = threadIdx.x % kThreads;  // the item's warps, the thread among theirs
+  unsigned char* flag = dyn + group * kLossItemBytes;  // bit 0 fluid, bit 1 not solid
   float* vec = reinterpret_cast<float*>(flag + kLossFlags);
   if (threadIdx.x == 0) valid_cta = 0;
   for (int k = threadIdx.x; k < kMine; k += kLossWarps * 32) num[k] = 0.0;
   __syncthreads();
+  auto sync = [&] { asm volatile("barrier.sync %0, %1;" ::"r"(1 + group), "n"(kThreads) : "memory"); };
+  // over the item's threads, the warps' sums in order (parts may be written again after the next sync)
+  auto item_sum = [&](double v) {
+    v = warp_sum(v);
+    if (lane == 0) parts[warp] = v;
+    sync();
+    v = parts[group * kLossItemWarps];
+#pragma unroll
+    for (int w = 1; w < kLossItemWarps; ++w) v += parts[group * kLossItemWarps + w];
+    return v;
+  };
   auto window = [](int l) { return ((l >> 6) + 1) * 100 + (((l >> 3) & 7) + 1) * 10 + (l & 7) + 1; };
   // pass 1: |r_b|^2 per item and the number of items with residual (item b: CTA b % 8, slot b / 8)
-  for (int slot = warp; slot * kLossCtas + rank < batch; slot += kLossWarps) {
+  for (int slot = group; slot * kLossCtas + rank < batch; slot += kGroups) {
     const float* xb = x + (size_t)(slot * kLossCtas + rank) * 2000;
     double v = 0.0;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int w = window(lane + 32 * k);
+    for (int k = 0; k < kCells; ++k) {
+      const int w = window(t + kThreads * k);
       const float m = xb[1000 + w], r = xb[w];
       if (m == 1.0f) v += (double)r * (double)r;
     }
-    v = warp_sum(v);
-    if (lane == 0) {
+    v = item_sum(v);
+    if (t == 0) {
       den[slot] = v;
       if (v > 0.0) atomicAdd(&valid_cta, 1);
     }
+    sync();  // the next item's sum overwrites the parts
   }
   cluster.sync();
   int valid = 0;
 #pragma unroll
   for (int c = 0; c < kLossCtas; ++c) valid += *cluster.map_shared_rank(&valid_cta, c);
   // pass 2: residual after the correction, the loss and its gradient
-  for (int slot = warp; slot * kLossCtas + rank < batch; slot += kLossWarps) {
+  for (int slot = group; slot * kLossCtas + rank < batch; slot += kGroups) {
     const size_t b = (size_t)slot * kLossCtas + rank;
     const float* xb = x + b * 2000;
-    float yv[16], rv[16];
+    float yv[kCells], rv[kCells];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      yv[k] = y[b * 512 + lane + 32 * k];
-      rv[k] = xb[window(lane + 32 * k)];
+    for (int k = 0; k < kCells; ++k) {
+      yv[k] = y[b * 512 + t + kThreads * k];
+      rv[k] = xb[window(t + kThreads * k)];
     }
 #pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-      const int i = lane + 32 * k;
+    for (int k = 0; k < 2 * kCells; ++k) {
+      const int i = t + kThreads * k;
       if (i < 1000) {
         const float m = xb[1000 + i];
         flag[i] = (unsigned char)((m == 1.0f ? 1 : 0) | (m >= 0.0f ? 2 : 0));
       }
     }
-    __syncwarp();
+    sync();
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int l = lane + 32 * k;
+    for (int k = 0; k < kCells; ++k) {
+      const int l = t + kThreads * k;
       if (!(flag[window(l)] & 1)) yv[k] = 0.0f;
       vec[l] = yv[k];
     }
-    __syncwarp();
+    sync();
     const int dw[6] = {-1, 1, -10, 10, -100, 100}, dl[6] = {-1, 1, -8, 8, -64, 64};
     // the sum of the block's fluid neighbours of cell l and (diag) its open faces
     auto neighbours = [&](int l, float* diag) {
@@ -688,23 +704,23 @@ __global__ void __cluster_dims__(kLossCtas, 1, 1) __launch_bounds__(kLossWarps *
       *diag = d;
       return off;
     };
-    float rho[16], dg[16];
+    float rho[kCells], dg[kCells];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int l = lane + 32 * k;
+    for (int k = 0; k < kCells; ++k) {
+      const int l = t + kThreads * k;
       const float off = neighbours(l, &dg[k]);
       rho[k] = (flag[window(l)] & 1) ? rv[k] - (dg[k] * yv[k] - off) : 0.0f;
     }
-    __syncwarp();
+    sync();
 #pragma unroll
-    for (int k = 0; k < 16; ++k) vec[lane + 32 * k] = rho[k];
-    __syncwarp();
+    for (int k = 0; k < kCells; ++k) vec[t + kThreads * k] = rho[k];
+    sync();
     const double d = den[slot];
     const double scale = d > 0.0 ? 1.0 / (valid * fmax(d, 1.0)) : 0.0;
     double acc = 0.0;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int l = lane + 32 * k;
+    for (int k = 0; k < kCells; ++k) {
+      const int l = t + kThreads * k;
       acc += scale * (double)rho[k] * (double)rho[k];
       if (grad != nullptr) {
         float arho = 0.0f;
@@ -716,9 +732,9 @@ __global__ void __cluster_dims__(kLossCtas, 1, 1) __launch_bounds__(kLossWarps *
         grad[b * 512 + l] = (float)(-2.0 * scale * (double)arho);
       }
     }
-    acc = warp_sum(acc);
-    if (lane == 0) num[slot] = acc;
-    __syncwarp();  // the next item overwrites flag and vec
+    acc = item_sum(acc);
+    if (t == 0) num[slot] = acc;
+    sync();  // the next item overwrites flag and vec
   }
   cluster.sync();
   if (rank == 0 && warp == 0 && loss != nullptr) {
@@ -1077,11 +1093,7 @@ cudaError_t unet_masked_mse(const float* y, const float* t, const float* m, int 
 cudaError_t unet_block_residual_loss(const float* y, const float* x, int batch, float* loss, float* grad,
                                      cudaStream_t s) {
   ++g_kernel_launches;
-  constexpr size_t smem = kLossWarps * kLossWarpBytes;
-  static OncePerDevice configured;
-  once_on_device(configured, [] {
-    cudaFuncSetAttribute(k_block_residual_loss, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  });
+  constexpr size_t smem = kLossWarps / kLossItemWarps * kLossItemBytes;  // 12 KB
   k_block_residual_loss<<<kLossCtas, kLossWarps * 32, smem, s>>>(y, x, batch, loss, grad);
   return cudaGetLastError();
 }
