@@ -48,18 +48,23 @@ __device__ __forceinline__ unsigned long long sort_first() {
 
 // 12 B of positions per particle, but bound by the marks: those of the blocks that
 // the resident CTAs are in share a few sectors, so every lookup that L1 does not
-// hold and every store goes to one L2 slice. Particles arrive nearly in cell order:
-// a warp's 128 consecutive ones are a few runs of equal blocks, only a run's first
-// particle looks its block up, one turn after the other, and stores where the mark is
-// still 0. Where a turn has more than kMarkRuns runs the particles are in no order,
-// and a warp match finds the blocks. 2.1M particles in order take 30 us, with runs
-// joined only within a turn and the four lookups together 77, with one particle per
-// thread and a match always 42; in random order 40, 75 and 42, without the match 60;
-// the 256^3 splash's moved ones 262, 470 and 470, the 128^3 dam break's 36, 35 and 35.
+// hold and every store goes to one L2 slice. Particles arrive nearly in cell order, so
+// a warp's 128 consecutive ones are a few runs of equal blocks: a run's first particle
+// brings its block to the warp's list (one a lane), the warps' lists meet in a table of
+// the CTA, and only then is each block looked up, and stored where its mark is still 0.
+// Where a turn has more than kMarkRuns runs the particles are in no order, and a warp
+// match finds the blocks to look up. In us, this | a lookup per run of a warp | per run of
+// a turn, the four turns' together | one particle per thread and a match:
+//   2.1M in order 17 | 20 | 77 | 43, in random order 38 | 39 | 67 | 43,
+//   moved by a step: 0.3M 9 | 12 | 8 | 22, 1.9M 16 | 27 | 28 | 35, 2.0M 21 | 33 | 36 | 35,
+//   29.6M 226 | 268 | 465 | 470. (Storing without the lookup: 11 in order, 460 at 29.6M.)
 constexpr int kMarkRuns = 8;
+constexpr int kMarkTable = 64;
 
 __global__ void __launch_bounds__(kSortThreads)
     k_mark_blocks(GridView g, ParticlesView p, unsigned char* occ, DeviceReport* rep) {
+  __shared__ int table[kMarkTable];
+  if (threadIdx.x < kMarkTable) table[threadIdx.x] = -1;
   const unsigned long long i0 = sort_first();
   float x[kSortIlp][3];
 #pragma unroll
@@ -95,13 +100,35 @@ __global__ void __launch_bounds__(kSortThreads)
     const int last = k > 0 ? __shfl_sync(0xffffffffu, idx[k > 0 ? k - 1 : 0], 31) : -1;
     look[k] = idx[k] >= 0 && (lane == 0 ? last : below) != idx[k];
   }
+  // the warp's list: at most kMarkRuns blocks a turn, hence at most 32
+  static_assert(kMarkRuns * kSortIlp <= 32, "one block a lane");
+  int mine = -1, found = 0;
 #pragma unroll
   for (int k = 0; k < kSortIlp; ++k) {
-    if (__popc(__ballot_sync(0xffffffffu, look[k])) > kMarkRuns) {  // no order: a block's first lane looks
+    unsigned heads = __ballot_sync(0xffffffffu, look[k]);
+    if (__popc(heads) > kMarkRuns) {  // no order: a block's first lane looks
       const unsigned same = __match_any_sync(0xffffffffu, idx[k]);
-      look[k] = idx[k] >= 0 && lane == __ffs(same) - 1;
+      if (idx[k] >= 0 && lane == __ffs(same) - 1 && occ[idx[k]] == 0) occ[idx[k]] = 1;
+      heads = 0u;
     }
-    if (look[k] && occ[idx[k]] == 0) occ[idx[k]] = 1;
+    while (heads != 0u) {
+      const int block = __shfl_sync(0xffffffffu, idx[k], __ffs(heads) - 1);
+      if (!__any_sync(0xffffffffu, mine == block)) {
+        if (lane == found) mine = block;
+        ++found;
+      }
+      heads &= ~__ballot_sync(0xffffffffu, idx[k] == block);
+    }
+  }
+  __syncthreads();  // (the table's first values)
+  if (mine >= 0) {
+    const int other = atomicCAS(&table[mine % kMarkTable], -1, mine);
+    if (other >= 0 && other != mine && occ[mine] == 0) occ[mine] = 1;  // the entry is another block's
+  }
+  __syncthreads();
+  if (threadIdx.x < kMarkTable) {
+    const int block = table[threadIdx.x];
+    if (block >= 0 && occ[block] == 0) occ[block] = 1;
   }
 }
 
