@@ -18,6 +18,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <new>
 #include <tuple>
 #include <utility>
 #include <vector>
@@ -866,14 +867,23 @@ int create_context(const fl_grid_desc* grid, uint64_t particle_capacity, bool so
   if (particle_capacity >= (1ULL << 31)) return FL_RESOURCE_EXHAUSTED;
   int st = device_ready();
   if (st != FL_OK) return st;
-  fl_context* c = new fl_context();
+  // Host memory first: running out of it is an error code, not an exception for the C caller.
+  fl_context* c = nullptr;
+  std::vector<std::pair<void**, size_t>> pieces;
+  try {
+    pieces.reserve(192);  // more than the pieces below, so that none of them allocates
+    c = new fl_context();
+    if (!solver) c->host = new HostBlock();
+  } catch (const std::bad_alloc&) {
+    delete c;
+    return FL_RESOURCE_EXHAUSTED;
+  }
   cudaGetDevice(&c->device);
   c->desc = *grid;
   c->pcap = std::max<uint64_t>(particle_capacity, 1);
   c->lattice = (int)lattice;
   const size_t cells = (size_t)lattice * kBlockCells;
   // The slab's pieces: listed first, then placed (512-byte aligned) in one allocation.
-  std::vector<std::pair<void**, size_t>> pieces;
   size_t total = 0;
   auto piece = [&](auto** p, size_t bytes) {
     pieces.emplace_back(reinterpret_cast<void**>(p), total);
@@ -959,8 +969,6 @@ int create_context(const fl_grid_desc* grid, uint64_t particle_capacity, bool so
       c->host = nullptr;
       chk(FL_RESOURCE_EXHAUSTED);
     }
-  } else {
-    c->host = new HostBlock();
   }
   if (c->host != nullptr) {
     c->nb_host = &c->host->nb;
