@@ -798,10 +798,13 @@ __global__ void __launch_bounds__(512 / CPT)
 // use them, every CTA alike, from per-block parts: a few loads a thread, less
 // than a reduction kernel of its own costs in launch and tail (z.r and z.r_prev by
 // the last sweep and the direction: 32^3 host step 1052 -> 1015 us, 128^3 substep
-// 1.022 -> 1.048 times the speed before; alpha by the update: 1081 -> 1052 us and
-// 1.006 -> 1.022, with one diagonal launch for all levels). Above, every CTA would
-// read more partials than its own cells, 160 KB at the 256^3 splash's 10k blocks,
-// and one last CTA summing them was slower than the separate kernel there.
+// 2.5% less; alpha by the update, with one diagonal launch for all levels: 1081 ->
+// 1052 us and 1.6% less). Above, every CTA would read more partials than its own
+// cells, 160 KB at the 256^3 splash's 10k blocks, and one last CTA summing them
+// was slower than the separate kernel there. Measured at 27, 368 and 729 blocks on
+// this side and at 10.7k on the other: where between them the two meet is not
+// known, and need not be one place for alpha (read by at most kReduceCtas CTAs) and
+// beta (read by one a block).
 constexpr int kFuseBlocks = 1024;
 
 // d = z + beta d_old and q = A d for one block, d staged with its halo; the
@@ -1129,8 +1132,10 @@ __global__ void __launch_bounds__(1024) k_coarse_solve(LevelDesc L, LevelPtrs<T>
 // dependent global round trips, and the coarsest pair in one CTA is limited by
 // one SM's issue rate. A sweep with its barrier takes ~1 us here. In place of two
 // launches per sweep above a one-CTA tail: the 32^3 host step 1015 -> 926 us (levels
-// from 1 on), the 128^3 substep 1.048 -> 1.104 times the speed before both (levels
-// from 2 on, 28 us a V-cycle), the 256^3 splash's even (levels from 3 on).
+// from 1 on), the 128^3 substep 5% less (levels from 2 on, 28 us a V-cycle), the
+// 256^3 splash's even (levels from 3 on). Under the profiler (128^3 dam break, 40 us)
+// its SMs issue in 22% of cycles; the barriers are the top stall, missing
+// instructions the next.
 // The operator does not change during a solve, so it is loaded before the
 // wait for the previous kernel and overlaps that kernel's tail.
 // Sparse levels (1: 4^3, 2: 2^3 cells per block) are dealt by runs of `per`
@@ -1144,9 +1149,10 @@ constexpr int kClMaxLevels = 12;
 constexpr size_t kClSmemMax = 227 * 1024;
 constexpr int kClCoarsestMax = 1024;  // one cell per thread
 // Cells of a level per CTA. A sweep over more is bound by the 16 SMs' issue rate
-// and the per-level kernels on the whole chip win: with 8192 the 256^3 splash ran
-// at 0.973 times the speed of the solver before and the 104 x 184 x 136 column
-// drop at 0.926, with 2048 at 1.013 and 1.053.
+// and the per-level kernels on the whole chip win: against per-level kernels with a
+// one-CTA tail, the 256^3 splash substep took 2.8% more time with 8192 and the 104 x 184 x
+// 136 column drop 8.0% more, with 2048 1.3% and 5.0% less. (Nothing between was
+// measured.)
 constexpr int kClCellsMax = 2048;
 
 struct ClLevel {

@@ -43,19 +43,20 @@ constexpr int kT = 256;
 // The FP32 3x3x3 convolutions, forward and data gradient. Both are
 //   out[b][o][cell] = f(sum_i sum_tap W[o][i][tap] in[b][i][cell + tap - 1]),
 // the data gradient with i over the layer's output channels and
-// W[o][i][tap] = w[i][o][26 - tap]. Bound by the FP32 pipe once the loads are
-// amortised: a thread owns four x-adjacent cells and kCo output channels, so
-// one input row (a 16- and an 8-byte shared load) serves 3 taps x 4 cells x
-// kCo channels in packed FMAs (channel pairs). A training step of 45
-// items takes 404 us; with one output per thread and an input and a weight load
-// per FMA it took 1821, with one group of 128 threads per CTA here and at most one
-// CTA per SM in the weight gradients 629, with one stream and plain launches 549.
-// Staging is most of what is left.
+// W[o][i][tap] = w[i][o][26 - tap]. Bound by latency: at 45 items an SM holds 8 to 16
+// warps, which issue in 30-36% of cycles and wait for what they stage first. A
+// thread owns four x-adjacent cells and kCo output channels, so one input row (a
+// 16- and an 8-byte shared load) serves 3 taps x 4 cells x kCo channels in packed
+// FMAs (channel pairs). A training step of 45 items takes 392 us; with one output per
+// thread and an input and a weight load per FMA it took 1821, with one group of 128
+// threads per CTA here and at most one CTA per SM in the weight gradients 629, with
+// one stream and plain launches 549.
 // One CTA per item, slab of kZ output planes and 16 output channels, two groups
-// of 128 threads each taking half of the input channels; the slab's zero-padded input (rows padded to a multiple of four
-// words, planes so that the eight lanes of a 16-byte access touch all banks)
-// and the 16 channels' weights ([input channel][tap][channel]) are staged in
-// shared memory. Sums run over input channels, then taps in ascending order.
+// of 128 threads each taking half of the input channels; the slab's zero-padded
+// input (rows padded to a multiple of four words, planes so that the eight lanes of
+// a 16-byte access touch all banks) and the 16 channels' weights ([input
+// channel][tap][channel]) are staged in shared memory. Sums run over input
+// channels, then taps in ascending order.
 template <int S>
 struct ConvTile {
   static constexpr int kZ = S == 8 ? 2 : 4;   // output planes per CTA
@@ -1324,7 +1325,7 @@ int fl_unet_set_tensor_cores(fl_unet* u, int enable) {
     return FL_OK;
   }
   if (u->tc != nullptr) return FL_OK;
-  if (u->max_batch > fl::kUNetTcMaxBatch) return FL_OUT_OF_RANGE;  // 32-bit operand indexing
+  if (u->max_batch > fl::kUNetTcMaxBatch) return FL_OUT_OF_RANGE;
   int st = fl::check_device();
   if (st != FL_OK) return st;
   auto* t = new fl::UNetTcTrain();

@@ -43,7 +43,9 @@ void wgrad_sum(const float* part, int rows, int nw, int cout, float* dw, float* 
 struct UNetTcTrain {
   __nv_bfloat16* w = nullptr;
 };
-constexpr int kUNetTcMaxBatch = 8192;  // largest batch of the tensor-core path
+// Largest batch of the tensor-core path: the limit that its entry point states. (No index
+// of its kernels needs one, and no larger batch has been run.)
+constexpr int kUNetTcMaxBatch = 8192;
 cudaError_t unet_tc_train_create(UNetTcTrain* t);
 void unet_tc_train_destroy(UNetTcTrain* t);
 cudaError_t unet_tc_train_pack(const UNetTcTrain& t, const float* params, bool data, cudaStream_t s);
