@@ -53,13 +53,17 @@ __device__ __forceinline__ unsigned long long sort_first() {
 // brings its block to the warp's list (one a lane), the warps' lists meet in a table of
 // the CTA, and only then is each block looked up, and stored where its mark is still 0.
 // Where a turn has more than kMarkRuns runs the particles are in no order, and a warp
-// match finds the blocks to look up. In us, this | a lookup per run of a warp | per run of
-// a turn, the four turns' together | one particle per thread and a match:
-//   2.1M in order 17 | 20 | 77 | 43, in random order 38 | 39 | 67 | 43,
-//   moved by a step: 0.3M 9 | 12 | 8 | 22, 1.9M 16 | 27 | 28 | 35, 2.0M 21 | 33 | 36 | 35,
-//   29.6M 226 | 268 | 465 | 470. (Storing without the lookup: 11 in order, 460 at 29.6M.)
+// match finds the blocks to look up. Up to kMarkFew CTAs (three an SM) there is little to
+// queue for and the runs' first particles look their blocks up together, one round trip.
+// In us, this | joined at every size | lookups per run of a turn, together | one particle
+// per thread and a match:
+//   moved by a step: 27k 2.4 | 3.0 | 2.3 | 2.0, 0.1M 2.5 | 5.6 | 2.4 | 2.4, 0.4M 6.7 | 10 | 8 | 21,
+//   1.9M 23 | 23 | 28 | 35, 2.0M 22 | 22 | 34 | 35, 29.6M 230 | 230 | 480 | 470;
+//   in order: 0.26M 3 | 6 | 7 | 30, 0.5M 9 | 9 | 47 | 43 (together 18), 2.1M 18 | 18 | 77 | 43;
+//   in random order: 0.26M 3 | 5 | 7 | 4, 0.5M 13 | 13 | 23 | 8, 2.1M 42 | 42 | 65 | 43.
 constexpr int kMarkRuns = 8;
 constexpr int kMarkTable = 64;
+constexpr unsigned kMarkFew = 3 * 148;
 
 __global__ void __launch_bounds__(kSortThreads)
     k_mark_blocks(GridView g, ParticlesView p, unsigned char* occ, DeviceReport* rep) {
@@ -99,6 +103,15 @@ __global__ void __launch_bounds__(kSortThreads)
     const int below = __shfl_up_sync(0xffffffffu, idx[k], 1);
     const int last = k > 0 ? __shfl_sync(0xffffffffu, idx[k > 0 ? k - 1 : 0], 31) : -1;
     look[k] = idx[k] >= 0 && (lane == 0 ? last : below) != idx[k];
+  }
+  if (gridDim.x <= kMarkFew) {
+    bool store[kSortIlp];
+#pragma unroll
+    for (int k = 0; k < kSortIlp; ++k) store[k] = look[k] && occ[idx[k]] == 0;
+#pragma unroll
+    for (int k = 0; k < kSortIlp; ++k)
+      if (store[k]) occ[idx[k]] = 1;
+    return;
   }
   // the warp's list: at most kMarkRuns blocks a turn, hence at most 32
   static_assert(kMarkRuns * kSortIlp <= 32, "one block a lane");

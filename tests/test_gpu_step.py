@@ -259,28 +259,31 @@ def test_empty_and_invalid_particles():
 
 
 def _in_runs(count, rng, n, run):
-    """Positions whose blocks come in runs of `run` particles (0: in no order, some blocks with many)."""
+    """Positions whose blocks come in runs of `run` particles (0: in no order, some blocks with many).
+    Runs beyond 12 are of the same 12 blocks, so that most blocks of the lattice stay empty, and six
+    particles anywhere among them are alone in their blocks: each of those marks is made once."""
     if run == 0:
         x = rng.uniform(1.0 / n, 1.0 - 1.0 / n, size=(3, count))
-        x[0, ::2] *= 0.25
+        x[:, ::2] *= 0.25
         return x
-    blocks = rng.permutation((n // 8) ** 3)[: -(-count // run)]
-    b = np.repeat(np.stack([blocks % 8, blocks // 8 % 8, blocks // 64]), run, axis=1)[:, :count]
-    return (8 * b + rng.uniform(0.01, 7.99, size=(3, count))) / n
+    blocks = rng.permutation((n // 8) ** 3)
+    of = np.repeat(np.resize(blocks[:12], -(-count // run)), run)[:count]
+    if count > 1000:
+        of[rng.choice(count, 6, replace=False)] = blocks[12:18]
+    return (8 * np.stack([of % (n // 8), of // (n // 8) % (n // 8), of // (n // 8) ** 2]) +
+            rng.uniform(0.01, 7.99, size=(3, count))) / n
 
 
 @pytest.mark.parametrize("run", [0, 3, 4, 5, 31, 33, 128, 200])
-@pytest.mark.parametrize("count", [1, 31, 33, 127, 129, 1023, 1024, 1025, 5000])
+@pytest.mark.parametrize("count", [1, 31, 33, 127, 129, 1023, 1024, 1025, 5000, 454656, 454657, 500003])
 def test_topology_from_unordered_particles(count, run):
     """Blocks marked by particles in no order and in runs of a block (around the 8 runs a turn of 32
-    and around a warp's 128 particles), at counts around a turn, a warp and the 1024 particles of a CTA,
-    against the blocks (and their ring) found on the host; a particle that has no block is reported with
-    its index."""
+    and around a warp's 128 particles), at counts around a turn, a warp, the 1024 particles of a CTA and
+    the 444 CTAs above which a CTA's blocks are joined before they are looked up, against the blocks
+    (and their ring) found on the host; a particle that has no block is reported with its index."""
     import torch
 
-    if run and count > run * 512:
-        pytest.skip("more runs than blocks")
-    n, rng = 64, np.random.default_rng(count)
+    n, rng = 128, np.random.default_rng(count)
     soa = np.zeros((15, count), np.float32)
     soa[0:3] = _in_runs(count, rng, n, run)
     ctx = fb.LiquidContext(n, capacity=count)
@@ -293,12 +296,12 @@ def test_topology_from_unordered_particles(count, run):
     lib, rep = fb.library(), fb.Report()
     assert lib.fl_topology_from_particles(ctx.handle, ctypes.byref(p), None, ctypes.byref(rep)) == fb.OK
     blk = np.floor(soa[0:3] * np.float32(n)).astype(int) // 8
-    occ = np.zeros((10, 10, 10), bool)
+    occ = np.zeros((18, 18, 18), bool)
     for dz in range(3):
         for dy in range(3):
             for dx in range(3):
                 occ[blk[2] + dz, blk[1] + dy, blk[0] + dx] = True
-    z, y, x = np.nonzero(occ[1:9, 1:9, 1:9])
+    z, y, x = np.nonzero(occ[1:17, 1:17, 1:17])
     np.testing.assert_array_equal(ctx.active_blocks(), np.stack([x, y, z], 1))
     for bad, code in ((np.nan, fb.OUT_OF_RANGE), (1.5, fb.FAILED_PRECONDITION)):
         dev[1, count - 1] = bad
