@@ -232,8 +232,13 @@ __global__ void __launch_bounds__(kG2PThreads, kG2PMinBlocks)
 // memory (rows of 25 words: no conflicts) and stored as 24 contiguous 128-byte
 // lines; a lane storing its own record touches 32 lines per instruction. The
 // 120 x 104 x 88 transfers, whose gather this is, went from 616 to 534 us with the
-// staged records and to 500 with the pairs.
+// staged records, to 500 with the pairs and to 484 with the tile's lookups in batches.
 constexpr int kFullRow = 25;
+// Tile entries of a thread in flight at once, lookups before values: the 13 entries are two
+// dependent round trips each, and with three CTAs an SM one entry after another left blocks
+// of few particles behind the kernel that shared the step's four (17 a block, no old field: 56 ->
+// 60 us at 1.9k blocks; now 53, and 240 instead of 248 at 512 a block with one).
+constexpr int kFullBatch = 7;
 constexpr size_t kFullSmem = sizeof(float) * (6 * kTileFaces + kG2PThreads * kFullRow);
 
 __global__ void __launch_bounds__(kG2PThreads, 3)
@@ -246,12 +251,26 @@ __global__ void __launch_bounds__(kG2PThreads, 3)
   if (b == 0 && t == 0 && rep != nullptr) rep->compiled_architecture = compiled_arch();
   const int pbeg = cell_start[b * kBlockCells], pend = cell_start[(b + 1) * kBlockCells];
   if (pbeg == pend) return;
-  const float* un[3] = {u0, u1, u2};
-  const float* uo[3] = {o0, o1, o2};
-  for (int n = t; n < 3 * kTileFaces; n += kG2PThreads) {
-    int a;
-    const long long src = tile_source(g, b, n, &a);
-    tile[n] = make_float2(src >= 0 ? un[a][src] : 0.0f, src >= 0 && o0 != nullptr ? uo[a][src] : 0.0f);
+#pragma unroll 1
+  for (int n0 = t; n0 < 3 * kTileFaces; n0 += kFullBatch * kG2PThreads) {
+    int src[kFullBatch];  // at most 2^21 blocks of 512 faces
+#pragma unroll
+    for (int k = 0; k < kFullBatch; ++k) {
+      const int n = n0 + k * kG2PThreads;
+      int a;
+      src[k] = n < 3 * kTileFaces ? (int)tile_source(g, b, n, &a) : -1;
+    }
+    float2 v[kFullBatch];
+#pragma unroll
+    for (int k = 0; k < kFullBatch; ++k) {
+      const int a = (n0 + k * kG2PThreads) / kTileFaces;
+      const float* fresh = a == 0 ? u0 : (a == 1 ? u1 : u2);
+      const float* old = a == 0 ? o0 : (a == 1 ? o1 : o2);
+      v[k] = make_float2(src[k] >= 0 ? fresh[src[k]] : 0.0f, src[k] >= 0 && o0 != nullptr ? old[src[k]] : 0.0f);
+    }
+#pragma unroll
+    for (int k = 0; k < kFullBatch; ++k)
+      if (n0 + k * kG2PThreads < 3 * kTileFaces) tile[n0 + k * kG2PThreads] = v[k];
   }
   __syncthreads();
   const int bc[3] = {g.coord[3 * b] * 8, g.coord[3 * b + 1] * 8, g.coord[3 * b + 2] * 8};
