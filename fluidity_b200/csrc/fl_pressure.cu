@@ -1152,7 +1152,8 @@ constexpr int kClCoarsestMax = 1024;  // one cell per thread
 // and the per-level kernels on the whole chip win: against per-level kernels with a
 // one-CTA tail, the 256^3 splash substep took 2.8% more time with 8192 and the 104 x 184 x
 // 136 column drop 8.0% more, with 2048 1.3% and 5.0% less. (Nothing between was
-// measured.)
+// measured. With a single post-sweep, not the default, the 192^3 splash's solve in
+// FP32 takes 2% more: fewer sweeps share the cluster's fixed cost.)
 constexpr int kClCellsMax = 2048;
 
 struct ClLevel {
